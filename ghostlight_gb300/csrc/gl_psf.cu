@@ -6,7 +6,8 @@
 // staged in shared memory once per CTA; one thread per (source, pupil sample)
 // walks the wavelengths with the reference-formulation primary trace; the
 // splat is bilinear, or a normalised Gaussian of the configured physical
-// width, clipped to the source's tile.
+// width, clipped to the source's tile.  A wide Gaussian takes the dense kernel
+// below: the tile as a sum of outer products in registers.
 #include "gl_internal.h"
 #include "gl_render.h"
 
@@ -14,6 +15,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -37,6 +39,11 @@ struct PsfArgs {
     float* out_g;
     float* out_b;
     int tile_smem;       // 1: the CTA's source tile is accumulated in shared memory
+    // dense path: landings [source][wavelength][sample] (weight < 0: none near
+    // the tile), of n_land wavelengths from l_base on; samples per CTA in steps
+    // of the CTA's threads
+    float4* land;
+    int l_base, n_land, s_base, rounds;
 };
 
 // Adds a ray-wavelength's weighted colour to one composite pixel: into the
@@ -72,9 +79,12 @@ __device__ __forceinline__ void deposit(const PsfArgs& A, float* tile, int tx, i
     }
 }
 
+template <bool LAND>
 __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* lens, const float* at, float* tile,
                                               int si, int gi);
 
+// LAND: the landings go to A.land instead of the tiles (the dense path).
+template <bool LAND>
 __global__ void __launch_bounds__(kPsfThreads) psf_kernel(PsfArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -98,10 +108,10 @@ __global__ void __launch_bounds__(kPsfThreads) psf_kernel(PsfArgs A)
         for (int i = threadIdx.x; i < planes * tile_px; i += blockDim.x) tile[i] = 0.0f;
     }
     __syncthreads();
-    const int si = blockIdx.x;
+    const int si = LAND ? A.s_base + blockIdx.x : blockIdx.x;
     const int gi = blockIdx.y * kPsfThreads + threadIdx.x;
-    if (si < A.n_src && gi < A.n_grid) psf_trace_one(A, lens, at, tile, si, gi);
-    if (!A.tile_smem || si >= A.n_src) return;
+    if (si < A.n_src && gi < A.n_grid) psf_trace_one<LAND>(A, lens, at, tile, si, gi);
+    if (LAND || !A.tile_smem || si >= A.n_src) return;
     __syncthreads();
     const gl_psf_source S = A.src[si];
     float* outs[3] = {A.out_r, A.out_g, A.out_b};
@@ -117,7 +127,9 @@ __global__ void __launch_bounds__(kPsfThreads) psf_kernel(PsfArgs A)
 }
 
 // One pupil sample of one source through every wavelength, splatted into the
-// source's tile (tile != nullptr: the CTA's shared-memory copy of it).
+// source's tile (tile != nullptr: the CTA's shared-memory copy of it).  LAND:
+// landings (px, py, weight) of the wavelengths in hand instead of the splat.
+template <bool LAND>
 __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* lens, const float* at, float* tile,
                                               int si, int gi)
 {
@@ -127,8 +139,15 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
     const V3 dir = normalized(v3(bx, by, 1.0f));
     const V3 org = v3(uv.x * A.front_R - kSpawnOffset * bx, uv.y * A.front_R - kSpawnOffset * by, A.start_z);
     const int tx_min = S.tile_x0, ty_min = S.tile_y0, tx_max = S.tile_x0 + A.tile_w, ty_max = S.tile_y0 + A.tile_h;
-    for (int l = 0; l < A.n_spec; ++l)
+    const int l0 = LAND ? A.l_base : 0, l1 = LAND ? A.l_base + A.n_land : A.n_spec;
+    for (int l = l0; l < l1; ++l)
     {
+        float4* land = nullptr;
+        if (LAND)
+        {
+            land = A.land + ((size_t)(si - A.s_base) * A.n_land + (l - l0)) * A.n_grid + gi;
+            land->z = -1.0f;
+        }
         const float4 sp = A.spec[l];
         const TraceOut r = trace_primary(lens, A.n_surf, at + l * A.n_surf, org, dir, sp.x);
         if (r.status != GL_TRACE_OK || !isfinite(r.x) || !isfinite(r.y)) continue;
@@ -138,6 +157,11 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
         if (tx < -margin || tx > (float)A.tile_w + margin || ty < -margin || ty > (float)A.tile_h + margin) continue;
         const float px = tx + (float)S.tile_x0, py = ty + (float)S.tile_y0;
         const float w = r.w * A.ray_weight;
+        if (LAND)
+        {
+            *land = make_float4(px, py, w, 0.0f);
+            continue;
+        }
         const float lum = (S.r + S.g + S.b) * (1.0f / 3.0f) * sp.z * w;
         const float cr = S.r * sp.y * w, cg = S.g * sp.z * w, cb = S.b * sp.w * w;
         if (A.sigma_px <= 0.0f)
@@ -191,15 +215,194 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
     }
 }
 
+// ---- dense Gaussian tiles ---------------------------------------------------
+// The Gaussian of a landing is an outer product gx(x) gy(y), so a source's
+// tile at one wavelength is the matrix product Gy^T diag(w) Gx over the rays
+// that land near it: no exponentials per tap (2 (2R + 1) per ray instead of
+// 2 (2R + 1)^2) and no shared-memory atomics (3 per tap).  One CTA holds the
+// tile of one (source, wavelength, range of pupil samples) in registers, 8 x 8
+// pixels per thread; it
+//   1. packs the landings near the tile, as psf_kernel<true> left them, into a
+//      list;
+//   2. for 32 landings at a time writes the rows gx and gy (zero outside the
+//      window, gy times weight / sum of the window) to shared memory, one warp
+//      per landing, and adds their outer products, each group of threads that
+//      covers the tile taking every G-th landing;
+//   3. sums the groups through shared memory and adds the tile, times the
+//      wavelength's colour weights, to the composite.
+// Bound by the FP32 pipes in step 2 (64 FMA per 4 shared 16-byte loads); the
+// trace before it is most of the time left.  8 x 8 tiles of 64^2, 16
+// wavelengths, radius 13 (the default settings): 3.96 -> 0.44 ms for both
+// kernels.  The trace stays a kernel of its own (landings through a scratch
+// that fits L2): inlined here it rounded some landings differently.
+constexpr int kDenseChunk = 32;       // landings per outer-product step
+constexpr size_t kDenseLandings = (size_t)4 << 20;   // 64 MB: stays in L2 between the two kernels
+constexpr int kDenseRoundsMax = 16;   // pupil samples per thread and CTA, at most
+
+struct DenseGeom {
+    int tx, ty, groups;               // 8 x 8 blocks across and down the tile, thread groups that cover it
+};
+
+__host__ __device__ inline DenseGeom dense_geom(int tile_w, int tile_h)
+{
+    DenseGeom g;
+    g.tx = (tile_w + 7) / 8;
+    g.ty = (tile_h + 7) / 8;
+    g.groups = g.tx * g.ty <= kPsfThreads ? kPsfThreads / (g.tx * g.ty) : 0;
+    return g;
+}
+
+// floats: the landing list, then the gx / gy rows, which the group sum reuses
+// as one plane
+inline size_t dense_smem_floats(const DenseGeom& g, int rounds)
+{
+    const size_t rows = (size_t)kDenseChunk * 8 * (g.tx + g.ty), plane = (size_t)64 * g.tx * g.ty;
+    return 4 * (size_t)rounds * kPsfThreads + std::max(rows, plane);
+}
+
+__global__ void __launch_bounds__(kPsfThreads, 2) psf_dense_kernel(PsfArgs A)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int n_list;
+    const DenseGeom G = dense_geom(A.tile_w, A.tile_h);
+    const int W8 = 8 * G.tx, H8 = 8 * G.ty;
+    float4* list = reinterpret_cast<float4*>(smem_raw);              // local px, py, weight
+    float* gx = reinterpret_cast<float*>(list + A.rounds * kPsfThreads);         // [landing][W8]
+    float* gy = gx + kDenseChunk * W8;                               // [landing][H8]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int si = A.s_base + blockIdx.x, l = A.l_base + blockIdx.y;
+    if (tid == 0) n_list = 0;
+    __syncthreads();
+    const gl_psf_source S = A.src[si];
+    const float4 sp = A.spec[l];
+    const int R = A.radius_px;
+    const float4* land = A.land + ((size_t)blockIdx.x * A.n_land + blockIdx.y) * A.n_grid;
+    for (int q = 0; q < A.rounds; ++q)
+    {
+        const int gi = (blockIdx.z * A.rounds + q) * kPsfThreads + tid;
+        float4 e = make_float4(0.0f, 0.0f, -1.0f, 0.0f);
+        if (gi < A.n_grid) e = land[gi];
+        const bool in = e.z >= 0.0f;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        int base = 0;
+        if (lane == 0 && m) base = atomicAdd(&n_list, __popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (in) list[base + __popc(m & ((1u << lane) - 1u))] = e;
+    }
+    __syncthreads();
+    const int n = n_list;
+    if (n == 0) return;
+    const float inv2 = 1.0f / (2.0f * A.sigma_px * A.sigma_px);
+    const int per = G.tx * G.ty, grp = tid / per, cell = tid - grp * per;
+    const int mx = (cell % G.tx) * 8, my = (cell / G.tx) * 8;
+    float acc[8][8] = {};
+    for (int c0 = 0; c0 < n; c0 += kDenseChunk)
+    {
+        const int cnt = min(kDenseChunk, n - c0);
+        for (int r = warp; r < cnt; r += kPsfThreads / 32)
+        {
+            const float4 e = list[c0 + r];
+            const int cx = (int)floorf(e.x), cy = (int)floorf(e.y);
+            const float ox = e.x - ((float)cx + 0.5f), oy = e.y - ((float)cy + 0.5f);
+            // window offset of this lane: R <= 16, at most 33 entries per axis
+            float wx = 0.0f, wy = 0.0f;
+            for (int d = lane - R; d <= R; d += 32)
+            {
+                const float dx = (float)d - ox, dy = (float)d - oy;
+                wx += expf(-(dx * dx) * inv2);
+                wy += expf(-(dy * dy) * inv2);
+            }
+            #pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                wx += __shfl_xor_sync(0xffffffffu, wx, o);
+                wy += __shfl_xor_sync(0xffffffffu, wy, o);
+            }
+            const float ws = wx * wy;
+            const float amp = ws > 1e-20f ? e.z / ws : 0.0f;
+            const int lx = cx - S.tile_x0, ly = cy - S.tile_y0;
+            for (int i = lane; i < W8; i += 32)
+            {
+                const float dx = (float)(i - lx) - ox;
+                gx[r * W8 + i] = (i < A.tile_w && abs(i - lx) <= R) ? expf(-(dx * dx) * inv2) : 0.0f;
+            }
+            for (int i = lane; i < H8; i += 32)
+            {
+                const float dy = (float)(i - ly) - oy;
+                gy[r * H8 + i] = (i < A.tile_h && abs(i - ly) <= R) ? expf(-(dy * dy) * inv2) * amp : 0.0f;
+            }
+        }
+        __syncthreads();
+        if (grp < G.groups)
+        {
+            for (int r = grp; r < cnt; r += G.groups)
+            {
+                const float4* px = reinterpret_cast<const float4*>(gx + r * W8 + mx);
+                const float4* py = reinterpret_cast<const float4*>(gy + r * H8 + my);
+                const float4 x0 = px[0], x1 = px[1], y0 = py[0], y1 = py[1];
+                const float vx[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+                const float vy[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+                #pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    #pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[j][i] = fmaf(vy[j], vx[i], acc[j][i]);
+            }
+        }
+        __syncthreads();
+    }
+    // sum of the groups, in order, in the rows' place (the loop ended on a barrier)
+    float* sum = gx;
+    for (int g = 0; g < G.groups; ++g)
+    {
+        if (grp == g)
+        {
+            #pragma unroll
+            for (int j = 0; j < 8; ++j)
+                #pragma unroll
+                for (int i = 0; i < 8; ++i)
+                {
+                    float* q = sum + (my + j) * W8 + mx + i;
+                    *q = g == 0 ? acc[j][i] : *q + acc[j][i];
+                }
+        }
+        __syncthreads();
+    }
+    const float lum = (S.r + S.g + S.b) * (1.0f / 3.0f) * sp.z;
+    const float c[3] = {A.mono ? lum : S.r * sp.y, S.g * sp.z, S.b * sp.w};
+    float* outs[3] = {A.out_r, A.out_g, A.out_b};
+    const int planes = A.mono ? 1 : 3;
+    for (int t = tid; t < A.tile_w * A.tile_h; t += kPsfThreads)
+    {
+        const int y = t / A.tile_w, x = t - y * A.tile_w;
+        const int xi = S.tile_x0 + x, yi = S.tile_y0 + y;
+        if (xi < 0 || xi >= A.comp_w || yi < 0 || yi >= A.comp_h) continue;
+        const float v = sum[y * W8 + x];
+        if (v == 0.0f) continue;
+        for (int pl = 0; pl < planes; ++pl)
+            if (c[pl] != 0.0f) atomicAdd(outs[pl] + (size_t)yi * A.comp_w + xi, c[pl] * v);
+    }
+}
+
+// The dense kernel pays for the whole tile per landing, the sparse one for the
+// (2R + 1)^2 taps.  Atlas of 64 sources, 16 wavelengths, 64^2 grid, sparse
+// against dense: 64^2 tiles, R = 2 0.40 / 0.43 ms, R = 3 0.52 / 0.43, R = 13
+// 3.96 / 0.44; 32^2 tiles, R = 2 0.41 / 0.42, R = 3 0.55 / 0.42; 128^2 tiles,
+// R = 3 0.43 / 0.48, R = 4 0.54 / 0.48 (the trace is 0.35 of each).
+inline bool dense_tile(int tile_w, int tile_h, float sigma_px, int radius_px)
+{
+    const DenseGeom g = dense_geom(tile_w, tile_h);
+    return sigma_px > 0.0f && g.groups >= 1 && radius_px >= (64 * g.tx * g.ty <= 8192 ? 3 : 4);
+}
+
 }  // namespace
 }  // namespace gl
 
 using namespace gl;
 
-// The render of both entries: `ordered` takes the scratch (lens records,
-// index table, spectrum, sources, pupil grid: one block) from the device's
-// stream-ordered pool and frees it in stream order without waiting; otherwise
-// plain allocations and a wait on the stream before they are freed.
+// The render of both entries: the scratch (lens records, index table,
+// spectrum, sources, pupil grid: one block, one copy) comes from the device's
+// stream-ordered pool and is freed in stream order; the plain entry then waits
+// for the stream, `ordered` does not.
 static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_psf_source* sources, int n_sources,
                            const gl_pupil_sample* grid, int n_grid, const gl_spectral_sample* spec, int n_spec,
                            int tile_w, int tile_h, int composite_w, int composite_h, float mm_per_pixel,
@@ -229,21 +432,21 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
     }
     build_ior_tables(surfaces, n_surfaces, lams.data(), n_spec, at.data(), bf.data());
     cudaStream_t st = (cudaStream_t)stream;
-    // one scratch block, each part 256-byte aligned
+    // one scratch block, each part 256-byte aligned, filled by one copy
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t o_recs = 0, o_at = o_recs + up(recs.size() * sizeof(SurfRec)), o_spec = o_at + up(at.size() * sizeof(float)),
                  o_src = o_spec + up(sp.size() * sizeof(float4)), o_grid = o_src + up((size_t)n_sources * sizeof(gl_psf_source)),
                  total = o_grid + up((size_t)n_grid * sizeof(float2));
+    std::vector<char> host(total, 0);
+    std::memcpy(host.data() + o_recs, recs.data(), recs.size() * sizeof(SurfRec));
+    std::memcpy(host.data() + o_at, at.data(), at.size() * sizeof(float));
+    std::memcpy(host.data() + o_spec, sp.data(), sp.size() * sizeof(float4));
+    std::memcpy(host.data() + o_src, sources, (size_t)n_sources * sizeof(gl_psf_source));
+    std::memcpy(host.data() + o_grid, grid, (size_t)n_grid * sizeof(float2));
     char* block = nullptr;
-    cudaError_t e;
-    if (ordered)
-    {
-        cudaMemPool_t pool;
-        e = shared_device_pool(dev, &pool);
-        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&block), total, pool, st);
-    }
-    else
-        e = cudaMalloc(&block, total);
+    cudaMemPool_t pool;
+    cudaError_t e = shared_device_pool(dev, &pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&block), total, pool, st);
     if (e != cudaSuccess)
         return fail(e == cudaErrorMemoryAllocation ? GL_ERR_OOM : GL_ERR_CUDA, std::string("psf_render: ") + cudaGetErrorString(e));
     SurfRec* d_recs = reinterpret_cast<SurfRec*>(block + o_recs);
@@ -251,18 +454,32 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
     float4* d_spec = reinterpret_cast<float4*>(block + o_spec);
     gl_psf_source* d_src = reinterpret_cast<gl_psf_source*>(block + o_src);
     float2* d_grid = reinterpret_cast<float2*>(block + o_grid);
-    e = cudaMemcpyAsync(d_recs, recs.data(), recs.size() * sizeof(SurfRec), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_at, at.data(), at.size() * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_spec, sp.data(), sp.size() * sizeof(float4), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_src, sources, (size_t)n_sources * sizeof(gl_psf_source), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_grid, grid, (size_t)n_grid * sizeof(float2), cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(block, host.data(), total, cudaMemcpyHostToDevice, st);
     // the CTA's source tile in shared memory when it fits (96 KB of tile)
     const size_t tile_bytes = (size_t)(monochromatic ? 1 : 3) * tile_w * tile_h * sizeof(float);
     const bool tile_smem = tile_bytes <= 96 * 1024;
-    const size_t smem = recs.size() * sizeof(SurfRec) + at.size() * sizeof(float) + (tile_smem ? tile_bytes + 16 : 0);
+    const DenseGeom dg = dense_geom(tile_w, tile_h);
+    // samples per CTA: as many as keep about four CTAs per resident slot (two
+    // per SM), so that few CTAs add the same tile to the composite
+    int rounds = kDenseRoundsMax, n_sm = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    auto dense_z = [&](int r) { return ((long long)n_grid + r * kPsfThreads - 1) / (r * kPsfThreads); };
+    while (rounds > 1 && dense_z(rounds) * n_sources * n_spec < 8LL * n_sm) rounds /= 2;
+    const size_t dense_smem = dense_smem_floats(dg, rounds) * sizeof(float);
+    const bool dense = dense_tile(tile_w, tile_h, splat_sigma_px, splat_radius_px) && dense_smem <= 220 * 1024 &&
+                       (size_t)n_grid <= kDenseLandings;
+    // landings of as many sources and wavelengths at a time as fit the scratch
+    const int land_l = dense ? (int)std::min<size_t>(std::min(n_spec, 65535), kDenseLandings / n_grid) : 0;
+    const int land_s = dense ? (int)std::min<size_t>(n_sources, std::max<size_t>(1, kDenseLandings / ((size_t)n_grid * land_l))) : 0;
+    float4* d_land = nullptr;
+    if (e == cudaSuccess && dense)
+        e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&d_land), sizeof(float4) * (size_t)land_s * land_l * n_grid, pool, st);
+    const size_t smem = recs.size() * sizeof(SurfRec) + at.size() * sizeof(float) + (tile_smem && !dense ? tile_bytes + 16 : 0);
     if (e == cudaSuccess && smem > 48 * 1024)
-        e = (cudaError_t)raise_smem_limit((const void*)psf_kernel, smem);
+        e = (cudaError_t)raise_smem_limit(dense ? (const void*)psf_kernel<true> : (const void*)psf_kernel<false>, smem);
+    if (e == cudaSuccess && dense && dense_smem > 47 * 1024)   // the kernel has a static word besides
+        e = (cudaError_t)raise_smem_limit((const void*)psf_dense_kernel, dense_smem);
+    int launches = dense ? 0 : 1;
     if (e == cudaSuccess)
     {
         PsfArgs A;
@@ -274,24 +491,39 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
         A.mono = monochromatic ? 1 : 0;
         A.sigma_px = splat_sigma_px; A.radius_px = splat_radius_px;
         A.out_r = d_out_r; A.out_g = d_out_g; A.out_b = d_out_b;
-        A.tile_smem = tile_smem ? 1 : 0;
-        const dim3 g((unsigned)n_sources, (unsigned)((n_grid + kPsfThreads - 1) / kPsfThreads));
-        psf_kernel<<<g, kPsfThreads, smem, st>>>(A);
+        A.tile_smem = tile_smem && !dense ? 1 : 0;
+        A.land = d_land;
+        A.l_base = 0; A.n_land = 0; A.s_base = 0;
+        A.rounds = rounds;
+        const unsigned blocks = (unsigned)((n_grid + kPsfThreads - 1) / kPsfThreads);
+        if (!dense) psf_kernel<false><<<dim3((unsigned)n_sources, blocks), kPsfThreads, smem, st>>>(A);
+        for (int s0 = 0; dense && s0 < n_sources; s0 += land_s)
+            for (int l0 = 0; l0 < n_spec; l0 += land_l)
+            {
+                const unsigned ns = (unsigned)std::min(land_s, n_sources - s0);
+                A.s_base = s0; A.l_base = l0;
+                A.n_land = std::min(land_l, n_spec - l0);
+                psf_kernel<true><<<dim3(ns, blocks), kPsfThreads, smem, st>>>(A);
+                psf_dense_kernel<<<dim3(ns, (unsigned)A.n_land, (unsigned)dense_z(rounds)), kPsfThreads, dense_smem, st>>>(A);
+                launches += 2;
+            }
         e = cudaGetLastError();
     }
-    if (ordered)
+    if (d_land)
     {
-        const cudaError_t f = cudaFreeAsync(block, st);
+        const cudaError_t f = cudaFreeAsync(d_land, st);
         if (e == cudaSuccess) e = f;
     }
-    else
+    const cudaError_t f = cudaFreeAsync(block, st);
+    if (e == cudaSuccess) e = f;
+    if (!ordered)
     {
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        cudaFree(block);
+        const cudaError_t w = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = w;
     }
     if (e != cudaSuccess)
         return fail(e == cudaErrorMemoryAllocation ? GL_ERR_OOM : GL_ERR_CUDA, std::string("psf_render: ") + cudaGetErrorString(e));
-    g_last_launches = 1;
+    g_last_launches = launches;
     return GL_OK;
 }
 
