@@ -196,33 +196,53 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 //
 //   W_x[k][j] = exp(-2 pi i s_x(l) (j - c_j)(k - c_x)),  same for y.
 //
-// Step 1: T'[k][i] = sum_j W_x[k][j] A[i][j]          (K_out x n, complex)
-// Step 2: E[l][k]  = sum_i W_y[l][i] T'[k][i]         (K_out x K_out, complex)
+// The operand A is real and the phase is odd in d = j - c_j, so the sums run
+// over |d| only, on A's even and odd parts about the centre:
+//   A_ee, A_oe, A_eo, A_oo   (first letter: row parity, second: column parity;
+//                             even = A[+d] + A[-d], odd = A[+d] - A[-d])
+// with C = cos, S = sin of the phase at d >= 0 (nh of them, half of n):
+//   step 1   Te_r = C A_ee, To_r = C A_oe, Te_i = -S A_eo, To_i = -S A_oo
+//   step 2   Re E = C_y Te_r + S_y To_i,   Im E = C_y Te_i - S_y To_r
+// (Te / To the even and odd parts of T over the pupil rows).  Both steps take
+// half the products of the unfolded form, the matrices half the memory, and
+// Re E and Im E accumulate directly.  The pixel-integrated (box) form needs
+// Re E only: Te_r and To_i, a quarter of the products.
 //
 // FORM 0 (split BF16): every operand X is stored as X_hi = bf16(X) and
-// X_lo = bf16(X - X_hi); the three-term product A_hi B_hi + A_hi B_lo +
-// A_lo B_hi is one GEMM over a tripled reduction axis, A' = [hi | hi | lo],
-// B' = [hi | lo | hi].  FORM 1 (TF32): FP32 operands, kind::tf32 MMAs.
-// Accumulation is FP32 in TMEM throughout.
+// X_lo = bf16(X - X_hi), rows [hi | lo]; each 128-byte step of the reduction
+// loads the four tiles once and accumulates A_hi B_hi + A_hi B_lo + A_lo B_hi.
+// FORM 1 (TF32): FP32 operands, kind::tf32 MMAs, not folded: sums of two
+// operand entries round differently in 11 bits, and this form's results are
+// its roundings.  Step 1 makes [Tr | Ti] = [Wr | Wi] A, step 2 accumulates
+// D1 = Wr [Tr | Ti], D2 = Wi [Tr | Ti] and combines them (Re E = D1[Tr] -
+// D2[Ti], Im E = D1[Ti] + D2[Tr]); the box form makes D1[Tr] and D2[Ti] only.
+// FORM 2 (FP32 on the CUDA cores) is folded.  Accumulation is FP32 in TMEM (or
+// registers) throughout.
 //
-// Complex products: T' holds, per 128 output columns, the two row blocks
-// [Tr | Ti]; step 2 stages them next to each other in shared memory and
-// accumulates two products with the same B operand, D1 = Wr [Tr | Ti] and
-// D2 = Wi [Tr | Ti] (N = 2 x tile width each), which its epilogue combines:
-// Re E = Wr Tr - Wi Ti = D1[Tr] - D2[Ti], Im E = Wr Ti + Wi Tr = D1[Ti] +
-// D2[Tr].
+// 512^2 pupil to 2048^2, 31 wavelengths, split BF16: step 1 233 -> 109 us, step
+// 2 1093 -> 550 us.  Step 2 issues 1536 cycles of MMA per 96 KB stage, two
+// stages deep, and runs its tensor pipe at about 60%: bound by the operand
+// stream from L2 (62 bytes per cycle and SM at full rate).
+//
+// Storage (Kp = 2 nh bf16, or nh floats; rows of Kp; unfolded: nh = n):
+//   W'  [lam][C | S][k]                                  TF32: [Wr | Wi]
+//   A'  [ee | oe | eo | oo][row d]   box: [ee | oo]      (nhr rows each; TF32: A)
+//   T'  [lam][k / 128][Te_r | Te_i | To_i | -To_r][k % 128]   box: [Te_r | To_i]
+//                                                        TF32: [Tr | Ti]
 // ===========================================================================
 namespace gl {
 namespace {
 
 constexpr int kMdftThreads = 192;     // warps 0-3 epilogue, warp 4 TMA, warp 5 MMA
+constexpr int kTf32 = 1;              // the form that is not folded
 constexpr int kOpTile = 128 * 128;    // bytes of one 128-row x 128-byte operand tile
 
 struct MdftArgs {
-    int KA;       // rows of the A operand per (wavelength, re/im part): Kx in step 1, Ky in step 2
-    int Kx;       // output width = T' k range; row stride of the output planes
+    int KA;       // rows of the A operand per (wavelength, C / S part): Kx in step 1, Ky in step 2
     int NBm;      // 128-row blocks of the A operand (step 1: Kx / 128, step 2: Ky / 128)
-    int n, n_lambda, Kp, nkb, NB, NI, n_units;   // NB = Kx / 128 (T' blocks per wavelength)
+    int nh, nhr;                      // folded reduction length (multiple of 16), rows per parity block of A'
+    int nkb;                          // 128-byte steps of one folded reduction
+    int NB, NI, n_units;              // T' blocks per wavelength (Kx / 128), step-1 tiles across nh
     void* tprime;                     // step 1 output / step 2 B operand
     float* out_r;
     float* out_g;
@@ -232,7 +252,6 @@ struct MdftArgs {
     // step-2 output placement: plan pixel (l, k) -> frame (y0 + l, x0 + k) of
     // planes out_w wide, kept when l < win_h and k < win_w
     int out_w, x0, y0, win_w, win_h;
-    int box;                          // 1: accumulate Re E (pixel-integrated form); 0: |E|^2
     float4 tint;                      // per-launch colour factor on the weights
     int lam_base;                     // first wavelength of this launch's range
     int NBt;                          // step 2: output tiles per row of the frame (Kx / tile width)
@@ -251,9 +270,9 @@ __host__ __device__ constexpr uint32_t idesc_any(int M, int N)
     return FORM == 0 ? tc::idesc_bf16(M, N, false) : tc::idesc_tf32(M, N, false);
 }
 
-__device__ __forceinline__ void store_split16(__nv_bfloat16* row, int n, int i0, const float (&v)[16], float sign)
+__device__ __forceinline__ void store_split16(__nv_bfloat16* row, int nh, int i0, const float (&v)[16], float sign)
 {
-    // [hi | lo | hi] at columns i0, n + i0, 2n + i0
+    // [hi | lo] at columns i0, nh + i0
     __align__(16) __nv_bfloat16 hi[16], lo[16];
     #pragma unroll
     for (int j = 0; j < 16; ++j)
@@ -265,30 +284,46 @@ __device__ __forceinline__ void store_split16(__nv_bfloat16* row, int n, int i0,
     const uint4* h4 = reinterpret_cast<const uint4*>(hi);
     const uint4* l4 = reinterpret_cast<const uint4*>(lo);
     uint4* d0 = reinterpret_cast<uint4*>(row + i0);
-    uint4* d1 = reinterpret_cast<uint4*>(row + n + i0);
-    uint4* d2 = reinterpret_cast<uint4*>(row + 2 * n + i0);
+    uint4* d1 = reinterpret_cast<uint4*>(row + nh + i0);
     d0[0] = h4[0]; d0[1] = h4[1];
     d1[0] = l4[0]; d1[1] = l4[1];
-    d2[0] = h4[0]; d2[1] = h4[1];
 }
 
+// Shared-memory stages of one CTA and its accumulators.  A stage holds two A
+// tiles of 128 rows (folded: hi and lo; TF32: Wr and Wi) and the row blocks of
+// B (folded: hi and lo of each), as many stages as fit, four at most.
+template <int FORM, int STEP, int TN, bool BOX>
+struct MdftShape {
+    static constexpr bool kFold = FORM != kTf32;
+    static constexpr int kBSets = kFold ? 2 : 1;
+    static constexpr int kBlocks = kFold ? (BOX ? 1 : 2) : STEP;    // row blocks of B per unit and set
+    static constexpr int kRows = STEP == 2 ? TN : 128;              // rows of one block
+    static constexpr int kN = (!kFold && STEP == 2 && BOX) ? TN : kBlocks * kRows;   // MMA N
+    static constexpr int kBBytes = kBlocks * kRows * 128;
+    static constexpr int kStageBytes = 2 * kOpTile + kBSets * kBBytes;
+    static constexpr int kStages = 212992 / kStageBytes < 4 ? 212992 / kStageBytes : 4;
+    static constexpr int kAccCols = kFold ? kN : 2 * kN;            // TMEM columns of a unit (TF32: D1 and D2)
+    static constexpr int kAccBufs = kAccCols <= 256 ? 2 : 1;
+    static constexpr int kParts = (kFold && STEP == 1) ? 2 : 1;     // units per tile: C and S apart
+    // reductions per unit: C and S, step by step in turn (the two cancel far
+    // from the centre: one after the other the sum would grow in between)
+    static constexpr int kPhases = (kFold && STEP == 2) ? 2 : 1;
+    // step 2's epilogue turns 32 x 32 blocks of the tile per warp
+    static constexpr int kTurn = STEP == 2 ? 4 * 32 * 33 * 4 : 0;
+    static constexpr int kSmem = kStages * kStageBytes + kTurn + 1024;
+};
+
 // TN (step 2): complex output columns per unit, 128 or 64 (the autotuner's
-// tile-shape knob).  A 64-column unit stages three 64-row blocks of T' (8 KB
-// each, box rows 64 in tB) and issues N = 128 MMAs; its smaller stages allow
-// a three-deep pipeline, and twice the units spread a small frame over more
-// SMs.
-template <int FORM, int STEP, int TN = 128>
+// tile-shape knob); twice the units spread a small frame over more SMs.
+template <int FORM, int STEP, int TN, bool BOX>
 __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_constant__ CUtensorMap tA,
                                                               const __grid_constant__ CUtensorMap tB, MdftArgs args)
 {
     static_assert(TN == 128 || TN == 64, "tile width");
-    constexpr int kBBytes = (STEP == 2) ? 2 * TN * 128 : kOpTile;   // B operand bytes per stage
-    constexpr int kStagesM = (STEP == 2) ? (TN == 128 ? 3 : 4) : 4;
-    constexpr int kStageBytes = 2 * kOpTile + kBBytes;
-    // accumulator buffers in TMEM's 512 columns: a unit of step 2 takes
-    // 4 TN columns (D1 and D2), so the 128-column tile is single-buffered
-    constexpr int kAccBufs = (STEP == 2 && TN == 128) ? 1 : 2;
+    using Sh = MdftShape<FORM, STEP, TN, BOX>;
+    constexpr int kStagesM = Sh::kStages;
     constexpr int kbe = (FORM == 0) ? 64 : 32;                   // reduction elements per 128-byte row
+    constexpr int kStep = (FORM == 0) ? 16 : 8;                  // and per MMA
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align1024(smem_raw);
     __shared__ uint64_t full[kStagesM], empty[kStagesM], acc_full[2], acc_empty[2], mma_done;
@@ -317,7 +352,8 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
     const int G = gridDim.x;
     const int u0 = blockIdx.x, u1 = args.n_units;
 
-    auto decode = [&](int u, int& lam, int& mb, int& xb) {
+    auto decode = [&](int u, int& lam, int& mb, int& xb, int& part) {
+        part = 0;
         if (STEP == 2)
         {
             // wavelength-major: all output tiles of one wavelength, then the next
@@ -330,10 +366,12 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
         }
         else
         {
-            lam = args.lam_base + u / (args.NBm * args.NI);
-            const int r = u % (args.NBm * args.NI);
-            mb = r / args.NI;
-            xb = r % args.NI;
+            const int per = args.NBm * args.NI * Sh::kParts;
+            lam = args.lam_base + u / per;
+            const int r = u % per;
+            part = r % Sh::kParts;                  // C, then S
+            mb = (r / Sh::kParts) / args.NI;
+            xb = (r / Sh::kParts) % args.NI;
         }
     };
 
@@ -345,34 +383,43 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
             bool stop = false;
             for (int u = u0; u < u1 && !stop; u += G)
             {
-                int lam, mb, xb;
-                decode(u, lam, mb, xb);
-                const int rowA = (lam * 2) * args.KA + mb * 128;
-                for (int kb = 0; kb < args.nkb; ++kb, ++it)
+                int lam, mb, xb, part;
+                decode(u, lam, mb, xb, part);
                 {
-                    const int s = it % kStagesM, r = it / kStagesM;
-                    if (it >= kStagesM && !tc::mbar_wait(&empty[s], (r - 1) & 1, err, tc::TC_TIMEOUT_EMPTY)) { stop = true; break; }
-                    uint8_t* st = smem + s * kStageBytes;
-                    tc::mbar_expect_tx(&full[s], kStageBytes);
-                    const int x = kb * kbe;
-                    tc::tma_load_2d(st, &tA, x, rowA, &full[s]);
-                    tc::tma_load_2d(st + kOpTile, &tA, x, rowA + args.KA, &full[s]);
-                    if (STEP == 2)
+                    for (int kk0 = 0; kk0 < Sh::kPhases * args.nkb; ++kk0, ++it)
                     {
-                        // rows [Tr | Ti] of this tile's columns: T' holds them in
-                        // 128-row blocks, a 64-column tile takes one half of each
-                        const int xb128 = (TN == 128) ? xb : (xb >> 1);
-                        const int half = (TN == 128) ? 0 : (xb & 1) * 64;
-                        const int rowB = ((lam * args.NB + xb128) * 2) * 128 + half;
+                        const int kb = kk0 / Sh::kPhases, cs = STEP == 2 ? kk0 % Sh::kPhases : part;
+                        const int rowA = (lam * 2 + cs) * args.KA + mb * 128;
+                        const int s = it % kStagesM, r = it / kStagesM;
+                        if (it >= kStagesM && !tc::mbar_wait(&empty[s], (r - 1) & 1, err, tc::TC_TIMEOUT_EMPTY)) { stop = true; break; }
+                        uint8_t* st = smem + s * Sh::kStageBytes;
+                        tc::mbar_expect_tx(&full[s], Sh::kStageBytes);
+                        const int x = kb * kbe;
+                        tc::tma_load_2d(st, &tA, x, rowA, &full[s]);
+                        if (Sh::kFold) tc::tma_load_2d(st + kOpTile, &tA, args.nh + x, rowA, &full[s]);
+                        else tc::tma_load_2d(st + kOpTile, &tA, x, rowA + args.KA, &full[s]);
                         #pragma unroll
-                        for (int j = 0; j < 2; ++j)
-                            tc::tma_load_2d(st + 2 * kOpTile + j * TN * 128, &tB, x, rowB + j * 128, &full[s]);
+                        for (int t = 0; t < Sh::kBSets; ++t)
+                            #pragma unroll
+                            for (int j = 0; j < Sh::kBlocks; ++j)
+                            {
+                                const int q = cs * Sh::kBlocks + j;
+                                int rowB;
+                                if (STEP == 2)
+                                {
+                                    // T' holds each part in blocks of 128 columns; a
+                                    // 64-column tile takes one half of each
+                                    const int xb128 = (TN == 128) ? xb : (xb >> 1);
+                                    const int half = (TN == 128) ? 0 : (xb & 1) * 64;
+                                    rowB = ((lam * args.NB + xb128) * (Sh::kPhases * Sh::kBlocks) + q) * 128 + half;
+                                }
+                                else
+                                    rowB = q * args.nhr + xb * 128;
+                                tc::tma_load_2d(st + 2 * kOpTile + t * Sh::kBBytes + j * Sh::kRows * 128, &tB,
+                                                t * args.nh + x, rowB, &full[s]);
+                            }
+                        ++issued;
                     }
-                    else
-                    {
-                        tc::tma_load_2d(st + 2 * kOpTile, &tB, x, xb * 128, &full[s]);
-                    }
-                    ++issued;
                 }
             }
             for (int q = (issued > kStagesM ? issued - kStagesM : 0); q < issued; ++q)
@@ -384,44 +431,42 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
     {
         if (lane == 0)
         {
-            const uint32_t id2 = idesc_any<FORM>(128, 2 * TN);
-            const uint32_t id128 = idesc_any<FORM>(128, 128);
+            const uint32_t id = idesc_any<FORM>(128, Sh::kN);
             int it = 0, ui = 0;
             bool stop = false;
             for (int u = u0; u < u1 && !stop; u += G, ++ui)
             {
-                const int b = ui % kAccBufs, ur = ui / kAccBufs;
-                if (ui >= kAccBufs && !tc::mbar_wait(&acc_empty[b], (ur - 1) & 1, err, tc::TC_TIMEOUT_ACC_FREE)) break;
+                const int b = ui % Sh::kAccBufs, ur = ui / Sh::kAccBufs;
+                if (ui >= Sh::kAccBufs && !tc::mbar_wait(&acc_empty[b], (ur - 1) & 1, err, tc::TC_TIMEOUT_ACC_FREE)) break;
                 tc::tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)(b * 256);
-                for (int kb = 0; kb < args.nkb; ++kb, ++it)
+                for (int kk0 = 0; kk0 < Sh::kPhases * args.nkb; ++kk0, ++it)
                 {
+                    const int kb = kk0 / Sh::kPhases;
                     const int s = it % kStagesM, r = it / kStagesM;
                     if (!tc::mbar_wait(&full[s], r & 1, err, tc::TC_TIMEOUT_FULL)) { stop = true; break; }
                     tc::tc_fence_after();
-                    uint8_t* st = smem + s * kStageBytes;
-                    const uint64_t aR = tc::sw128_desc(tc::smem_u32(st));
-                    const uint64_t aI = tc::sw128_desc(tc::smem_u32(st + kOpTile));
-                    if (STEP == 2)
+                    uint8_t* st = smem + s * Sh::kStageBytes;
+                    const uint64_t a0 = tc::sw128_desc(tc::smem_u32(st));
+                    const uint64_t a1 = tc::sw128_desc(tc::smem_u32(st + kOpTile));
+                    const uint64_t b0 = tc::sw128_desc(tc::smem_u32(st + 2 * kOpTile));
+                    // folded: the lo set; TF32 box: the Ti block
+                    const uint64_t b1 = tc::sw128_desc(tc::smem_u32(st + 2 * kOpTile + (Sh::kFold ? Sh::kBBytes : Sh::kRows * 128)));
+                    // the last step of a reduction may be partly past nh (whatever lies there is not multiplied)
+                    const int left = (args.nh - kb * kbe) / kStep;
+                    #pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
                     {
-                        // D1 = Wr [Tr | Ti] at d, D2 = Wi [Tr | Ti] at d + 2 TN
-                        const uint64_t bRI = tc::sw128_desc(tc::smem_u32(st + 2 * kOpTile));   // [Tr | Ti]
-                        #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
+                        if (kk >= left) break;
+                        const uint32_t acc = (kk0 | kk) != 0;
+                        mma_any<FORM>(d, a0 + 2 * kk, b0 + 2 * kk, id, acc);
+                        if (Sh::kFold)
                         {
-                            mma_any<FORM>(d, aR + 2 * kk, bRI + 2 * kk, id2, (kb | kk) != 0);
-                            mma_any<FORM>(d + 2 * TN, aI + 2 * kk, bRI + 2 * kk, id2, (kb | kk) != 0);
+                            mma_any<FORM>(d, a0 + 2 * kk, b1 + 2 * kk, id, 1);
+                            mma_any<FORM>(d, a1 + 2 * kk, b0 + 2 * kk, id, 1);
                         }
-                    }
-                    else
-                    {
-                        const uint64_t bM = tc::sw128_desc(tc::smem_u32(st + 2 * kOpTile));
-                        #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                        {
-                            mma_any<FORM>(d, aR + 2 * kk, bM + 2 * kk, id128, (kb | kk) != 0);
-                            mma_any<FORM>(d + 128, aI + 2 * kk, bM + 2 * kk, id128, (kb | kk) != 0);
-                        }
+                        else
+                            mma_any<FORM>(d + Sh::kN, a1 + 2 * kk, (STEP == 2 && BOX ? b1 : b0) + 2 * kk, id, acc);
                     }
                     tc::mma_commit(&empty[s]);
                 }
@@ -440,9 +485,9 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
         const int row = warp * 32 + lane;
         for (int u = u0; u < u1; u += G, ++ui)
         {
-            int lam, mb, xb;
-            decode(u, lam, mb, xb);
-            const int b = ui % kAccBufs, ur = ui / kAccBufs;
+            int lam, mb, xb, part;
+            decode(u, lam, mb, xb, part);
+            const int b = ui % Sh::kAccBufs, ur = ui / Sh::kAccBufs;
             const bool ok = tc::mbar_wait(&acc_full[b], ur & 1, err, tc::TC_TIMEOUT_ACC);
             tc::tc_fence_after();
             const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * 256);
@@ -450,84 +495,118 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
             {
                 const float4 w0 = args.weights[lam];
                 const float4 w = make_float4(w0.x * args.tint.x, w0.y * args.tint.y, w0.z * args.tint.z, 0.0f);
-                const int l = mb * 128 + row;
-                const bool row_in = l < args.win_h;
-                const size_t orow = (size_t)(args.y0 + l) * (size_t)args.out_w + (size_t)args.x0;
+                // A TMEM lane is a row of the tile, so a thread holds 32 columns
+                // of one row; turned through shared memory, a warp adds whole
+                // 128-byte row pieces to the planes: 16-byte vector atomics
+                // where every row starts on a 16-byte boundary, else scalar
+                // ones.  Adding each thread's own row left the warp's 32 rows
+                // in 32 sectors per instruction and bound the kernel: 512^2 ->
+                // 2048^2 x 31 650 -> 550 us, a 389 x 301 window 118 -> 42 us.
+                float* turn = reinterpret_cast<float*>(smem + kStagesM * Sh::kStageBytes) + warp * (32 * 33);
+                const int lrow = mb * 128 + warp * 32;
+                const size_t o0 = (size_t)(args.y0 + lrow) * (size_t)args.out_w + (size_t)args.x0 + (size_t)xb * TN;
+                const bool vec = ((args.out_w | args.x0) & 3) == 0;
+                const int rows = min(32, args.win_h - lrow);
                 #pragma unroll 1
-                for (int c = 0; c < TN / 16; ++c)
+                for (int c = 0; c < TN / 32; ++c)
                 {
-                    // Re E = D1[Tr] - D2[Ti], Im E = D1[Ti] + D2[Tr]
-                    float re[16], im[16], u2[16], v2[16];
-                    tc::tmem_ld16(ta + (uint32_t)(c * 16), re);
-                    tc::tmem_ld16(ta + (uint32_t)TN + (uint32_t)(c * 16), im);
-                    tc::tmem_ld16(ta + (uint32_t)(2 * TN) + (uint32_t)(c * 16), u2);
-                    tc::tmem_ld16(ta + (uint32_t)(3 * TN) + (uint32_t)(c * 16), v2);
                     #pragma unroll
-                    for (int j = 0; j < 16; ++j)
+                    for (int h = 0; h < 2; ++h)
                     {
-                        re[j] -= v2[j];
-                        im[j] += u2[j];
-                    }
-                    if (!ok || !row_in) continue;
-                    const int kc = xb * TN + c * 16;
-                    #pragma unroll
-                    for (int j = 0; j < 16; j += 4)
-                    {
-                        float I[4];
-                        #pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            I[q] = args.box ? re[j + q] : re[j + q] * re[j + q] + im[j + q] * im[j + q];
-                        const int k = kc + j;
-                        const size_t o = orow + (size_t)k;
-                        if (k + 3 < args.win_w && (o & 3) == 0)
+                        float re[16], im[16];
+                        const uint32_t tc0 = ta + (uint32_t)(c * 32 + h * 16);
+                        tc::tmem_ld16(tc0, re);
+                        if (!BOX) tc::tmem_ld16(tc0 + TN, im);
+                        if (!Sh::kFold)
                         {
-                            atomicAdd(reinterpret_cast<float4*>(args.out_r + o), make_float4(w.x * I[0], w.x * I[1], w.x * I[2], w.x * I[3]));
-                            atomicAdd(reinterpret_cast<float4*>(args.out_g + o), make_float4(w.y * I[0], w.y * I[1], w.y * I[2], w.y * I[3]));
-                            atomicAdd(reinterpret_cast<float4*>(args.out_b + o), make_float4(w.z * I[0], w.z * I[1], w.z * I[2], w.z * I[3]));
-                        }
-                        else
-                        {
+                            // Re E = D1[Tr] - D2[Ti], Im E = D1[Ti] + D2[Tr]
+                            float u[16];
+                            tc::tmem_ld16(tc0 + (BOX ? TN : 3 * TN), u);
                             #pragma unroll
-                            for (int q = 0; q < 4; ++q)
+                            for (int j = 0; j < 16; ++j) re[j] -= u[j];
+                            if (!BOX)
                             {
-                                if (k + q >= args.win_w) break;
-                                atomicAdd(args.out_r + o + q, w.x * I[q]);
-                                atomicAdd(args.out_g + o + q, w.y * I[q]);
-                                atomicAdd(args.out_b + o + q, w.z * I[q]);
+                                tc::tmem_ld16(tc0 + 2 * TN, u);
+                                #pragma unroll
+                                for (int j = 0; j < 16; ++j) im[j] += u[j];
+                            }
+                        }
+                        #pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            turn[lane * 33 + h * 16 + j] = BOX ? re[j] : re[j] * re[j] + im[j] * im[j];
+                    }
+                    __syncwarp();
+                    const int kc = xb * TN + c * 32;
+                    if (ok && vec)
+                    {
+                        const int col = (lane & 7) * 4;
+                        for (int r = lane >> 3; r < rows; r += 4)
+                        {
+                            const float* t = turn + r * 33 + col;
+                            const size_t o = o0 + (size_t)r * args.out_w + c * 32 + col;
+                            if (kc + col + 3 < args.win_w)
+                            {
+                                atomicAdd(reinterpret_cast<float4*>(args.out_r + o), make_float4(w.x * t[0], w.x * t[1], w.x * t[2], w.x * t[3]));
+                                atomicAdd(reinterpret_cast<float4*>(args.out_g + o), make_float4(w.y * t[0], w.y * t[1], w.y * t[2], w.y * t[3]));
+                                atomicAdd(reinterpret_cast<float4*>(args.out_b + o), make_float4(w.z * t[0], w.z * t[1], w.z * t[2], w.z * t[3]));
+                            }
+                            else
+                            {
+                                #pragma unroll
+                                for (int q = 0; q < 4; ++q)
+                                {
+                                    if (kc + col + q >= args.win_w) break;
+                                    atomicAdd(args.out_r + o + q, w.x * t[q]);
+                                    atomicAdd(args.out_g + o + q, w.y * t[q]);
+                                    atomicAdd(args.out_b + o + q, w.z * t[q]);
+                                }
                             }
                         }
                     }
+                    else if (ok && kc + lane < args.win_w)
+                    {
+                        for (int r = 0; r < rows; ++r)
+                        {
+                            const float v = turn[r * 33 + lane];
+                            const size_t o = o0 + (size_t)r * args.out_w + c * 32 + lane;
+                            atomicAdd(args.out_r + o, w.x * v);
+                            atomicAdd(args.out_g + o, w.y * v);
+                            atomicAdd(args.out_b + o, w.z * v);
+                        }
+                    }
+                    __syncwarp();
                 }
             }
             else
             {
-                // T' rows of this k: [Tr | Ti] blocks of 128 rows.
-                const int k = row;
-                const size_t blk = ((size_t)(lam * args.NB + mb) * 2) * 128;
-                #pragma unroll 1
-                for (int c = 0; c < 8; ++c)
+                // T' rows of this k.  The C part gives (Te_r, To_r), the S part
+                // (-Te_i, -To_i); step 2 wants [Te_r | Te_i | To_i | -To_r].  TF32:
+                // (Tr, Ti) as they are.
+                constexpr int kOut = Sh::kFold ? Sh::kBlocks : 2;
+                const size_t blk = (size_t)(lam * args.NB + mb) * (Sh::kParts * kOut) * 128;
+                #pragma unroll
+                for (int j = 0; j < kOut; ++j)
                 {
-                    float re[16], im[16];
-                    tc::tmem_ld16(ta + (uint32_t)(c * 16), re);
-                    tc::tmem_ld16(ta + 128u + (uint32_t)(c * 16), im);
-                    if (!ok) continue;
-                    const int i0 = xb * 128 + c * 16;
-                    if (FORM == 0)
+                    const int dst = !Sh::kFold ? j : (BOX ? part : (part == 0 ? (j == 0 ? 0 : 3) : (j == 0 ? 1 : 2)));
+                    const float sign = (!Sh::kFold || (part == 0 && j == 0)) ? 1.0f : -1.0f;
+                    #pragma unroll 1
+                    for (int c = 0; c < 8; ++c)
                     {
-                        __nv_bfloat16* T = static_cast<__nv_bfloat16*>(args.tprime);
-                        store_split16(T + (blk + 0 * 128 + k) * (size_t)args.Kp, args.n, i0, re, 1.0f);
-                        store_split16(T + (blk + 1 * 128 + k) * (size_t)args.Kp, args.n, i0, im, 1.0f);
-                    }
-                    else
-                    {
-                        float* T = static_cast<float*>(args.tprime);
-                        float* r0 = T + (blk + 0 * 128 + k) * (size_t)args.Kp + i0;
-                        float* r1 = T + (blk + 1 * 128 + k) * (size_t)args.Kp + i0;
-                        #pragma unroll
-                        for (int j = 0; j < 16; j += 4)
+                        float v[16];
+                        tc::tmem_ld16(ta + (uint32_t)(j * 128 + c * 16), v);
+                        const int i0 = xb * 128 + c * 16;
+                        if (!ok || i0 >= args.nh) continue;
+                        if (FORM == 0)
                         {
-                            *reinterpret_cast<float4*>(r0 + j) = make_float4(re[j], re[j + 1], re[j + 2], re[j + 3]);
-                            *reinterpret_cast<float4*>(r1 + j) = make_float4(im[j], im[j + 1], im[j + 2], im[j + 3]);
+                            __nv_bfloat16* T = static_cast<__nv_bfloat16*>(args.tprime);
+                            store_split16(T + (blk + dst * 128 + row) * (size_t)(2 * args.nh), args.nh, i0, v, sign);
+                        }
+                        else
+                        {
+                            float* r0 = static_cast<float*>(args.tprime) + (blk + dst * 128 + row) * (size_t)args.nh + i0;
+                            #pragma unroll
+                            for (int q = 0; q < 16; q += 4)
+                                *reinterpret_cast<float4*>(r0 + q) = make_float4(sign * v[q], sign * v[q + 1], sign * v[q + 2], sign * v[q + 3]);
                         }
                     }
                 }
@@ -541,69 +620,104 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
     if (warp == 5) tc::tmem_dealloc(tmem, 512);
 }
 
-// DFT matrices W'[lam][part][k][Kp]: part 0 = Re, 1 = Im of
-// exp(-2 pi i s(lam) (j - cj)(k - ck)).  The phase is formed in FP32
-// double-float arithmetic (Dekker / Ogita-Rump-Oishi error-free products
-// with FMA): s = s_hi + s_lo and ck = ck_hi + ck_lo are split on the host,
-// a = j - cj is exact (cj a half-integer), b = k - ck is carried as a
-// two-float sum, and the product's integer cycles are removed from
-// the leading term exactly; the reduced phase is accurate to ~1e-9 cycles,
-// then evaluated with sincospif.  (The FP64 units of this part are slow.)
-// With box set each entry also carries the pixel-box factor sinc(s (j - cj))
-// of the reference's pixel-integrated form (mdft_render.cu:109-135).
-// FORM 0 stores [hi | hi | lo] along the reduction axis, FORM 1 the FP32 value.
-template <int FORM>
-__global__ void mdft_dft_kernel(void* out, int n_lambda, int K_rows, int n, int Kp, const float2* __restrict__ scale,
-                                float ck_hi, float ck_lo, float cj, int box)
+// DFT matrices W'[lam][C | S][k][Kp]: cos and sin of 2 pi s(lam) d (k - ck) at
+// the folded distances d = m (centre cj whole) or m + 1/2, zero from nf on
+// (TF32: cos and -sin at every d = m - cj).
+// The phase is formed in FP32 double-float arithmetic (Dekker /
+// Ogita-Rump-Oishi error-free products with FMA): s = s_hi + s_lo and
+// ck = ck_hi + ck_lo are split on the host, d is exact, b = k - ck is carried
+// as a two-float sum, and the product's integer cycles are removed from the
+// leading term exactly; the reduced phase is accurate to ~1e-9 cycles, then
+// evaluated with sincospif.  (The FP64 units of this part are slow.)
+// With box set each entry also carries the pixel-box factor sinc(s d) of the
+// reference's pixel-integrated form (mdft_render.cu:109-135).
+// The factor depends on (wavelength, d) alone: a plan's table, made once.  A
+// thread makes two neighbouring entries of a row, so the stores are whole words
+// and no index is divided in the inner loop.  Bound by the instructions of the
+// phase and sincospif.  W_x' and W_y' of a 640^2 operand, 512 x 384 outputs, 31
+// wavelengths: 141 us in the unfolded layout (with the factor made per entry),
+// 33 us now.
+struct DftRows {
+    void* out;
+    const float2* scale;
+    const float* amp;                  // [lam][nh]
+    float ck_hi, ck_lo;
+    int K;
+};
+
+// amp[lam][m]: 1 (box: sinc(s d)) up to nf, 0 past it
+__global__ void mdft_amp_kernel(float* __restrict__ amp, const float2* __restrict__ scale, int nh, int nf, float d0,
+                                int box)
 {
-    const size_t total = (size_t)n_lambda * K_rows * n;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
+    const int lam = blockIdx.x;
+    const float2 sc = scale[lam];
+    for (int m = threadIdx.x; m < nh; m += blockDim.x)
     {
-        const int j = (int)(e % n);
-        const int k = (int)((e / n) % K_rows);
-        const int lam = (int)(e / ((size_t)n * K_rows));
-        const float2 sc = scale[lam];                  // (s_hi, s_lo)
-        const float a = (float)j - cj;                 // exact
-        // b = k - ck as bh + bl: Knuth's two-sum of k and -ck_hi, then -ck_lo
-        const float kf = (float)k;
-        const float bh = kf - ck_hi;
-        const float bb = bh - kf;
-        const float bl = ((kf - (bh - bb)) + (-ck_hi - bb)) - ck_lo;
-        const float p1 = a * bh;
-        const float e1 = fmaf(a, bh, -p1);             // a*bh = p1 + e1 exactly
-        const float m_lo = e1 + a * bl;
-        const float q = sc.x * p1;
-        const float eq = fmaf(sc.x, p1, -q);           // s_hi*p1 = q + eq exactly
-        const float rest = eq + sc.x * m_lo + sc.y * p1;
-        float fr = (q - rintf(q)) + rest;              // q - rint(q) is exact
-        fr -= rintf(fr);
-        float sv, cv;
-        sincospif(2.0f * fr, &sv, &cv);
-        float amp = 1.0f;
-        if (box)
+        float v = m < nf ? 1.0f : 0.0f;
+        if (box && m < nf)
         {
-            // pixel-box factor of the pixel-integrated form: sinc(m s), m = j - cj
-            // the lag, s = pixel pitch / pattern period at this wavelength
-            const float x = a * (sc.x + sc.y);
-            amp = fabsf(x) < 1e-7f ? 1.0f : sinpif(x) / (3.14159265358979323846f * x);
+            // pixel-box factor of the pixel-integrated form: d the lag, s =
+            // pixel pitch / pattern period at this wavelength
+            const float x = ((float)m + d0) * (sc.x + sc.y);
+            v = fabsf(x) < 1e-7f ? 1.0f : sinpif(x) / (3.14159265358979323846f * x);
         }
-        const float re = amp * cv, im = -amp * sv;
-        const size_t rr = ((size_t)(lam * 2 + 0) * K_rows + k) * Kp;
-        const size_t ri = ((size_t)(lam * 2 + 1) * K_rows + k) * Kp;
+        amp[(size_t)lam * nh + m] = v;
+    }
+}
+
+template <int FORM>
+__global__ void __launch_bounds__(256) mdft_dft_kernel(DftRows R, int n_lambda, int nh, float d0)
+{
+    const int row = blockIdx.x * blockDim.y + threadIdx.y;
+    if (row >= n_lambda * R.K) return;
+    const int lam = row / R.K, k = row - lam * R.K;
+    const float* amps = R.amp + (size_t)lam * nh;
+    const float2 sc = R.scale[lam];                // (s_hi, s_lo)
+    // b = k - ck as bh + bl: Knuth's two-sum of k and -ck_hi, then -ck_lo
+    const float kf = (float)k;
+    const float bh = kf - R.ck_hi;
+    const float bb = bh - kf;
+    const float bl = ((kf - (bh - bb)) + (-R.ck_hi - bb)) - R.ck_lo;
+    const int Kp = FORM == 0 ? 2 * nh : nh;
+    const size_t rc = ((size_t)(lam * 2 + 0) * R.K + k) * Kp, rs = ((size_t)(lam * 2 + 1) * R.K + k) * Kp;
+    for (int m = 2 * threadIdx.x; m < nh; m += 2 * blockDim.x)
+    {
+        float cv[2], sv[2];
+        #pragma unroll
+        for (int q = 0; q < 2; ++q)
+        {
+            const float a = (float)(m + q) + d0;   // exact
+            const float p1 = a * bh;
+            const float e1 = fmaf(a, bh, -p1);             // a*bh = p1 + e1 exactly
+            const float m_lo = e1 + a * bl;
+            const float qq = sc.x * p1;
+            const float eq = fmaf(sc.x, p1, -qq);          // s_hi*p1 = qq + eq exactly
+            const float rest = eq + sc.x * m_lo + sc.y * p1;
+            float fr = (qq - rintf(qq)) + rest;            // qq - rint(qq) is exact
+            fr -= rintf(fr);
+            sincospif(2.0f * fr, &sv[q], &cv[q]);
+            const float amp = amps[m + q];
+            cv[q] *= amp;
+            sv[q] = FORM == kTf32 ? -amp * sv[q] : amp * sv[q];
+        }
         if (FORM == 0)
         {
-            __nv_bfloat16* W = static_cast<__nv_bfloat16*>(out);
-            const __nv_bfloat16 rh = __float2bfloat16_rn(re), ih = __float2bfloat16_rn(im);
-            const __nv_bfloat16 rl = __float2bfloat16_rn(re - __bfloat162float(rh));
-            const __nv_bfloat16 il = __float2bfloat16_rn(im - __bfloat162float(ih));
-            W[rr + j] = rh; W[rr + n + j] = rh; W[rr + 2 * n + j] = rl;
-            W[ri + j] = ih; W[ri + n + j] = ih; W[ri + 2 * n + j] = il;
+            __nv_bfloat16* W = static_cast<__nv_bfloat16*>(R.out);
+            __nv_bfloat162 ch, cl, sh, sl;
+            ch.x = __float2bfloat16_rn(cv[0]); ch.y = __float2bfloat16_rn(cv[1]);
+            sh.x = __float2bfloat16_rn(sv[0]); sh.y = __float2bfloat16_rn(sv[1]);
+            cl.x = __float2bfloat16_rn(cv[0] - __bfloat162float(ch.x)); cl.y = __float2bfloat16_rn(cv[1] - __bfloat162float(ch.y));
+            sl.x = __float2bfloat16_rn(sv[0] - __bfloat162float(sh.x)); sl.y = __float2bfloat16_rn(sv[1] - __bfloat162float(sh.y));
+            *reinterpret_cast<__nv_bfloat162*>(W + rc + m) = ch;
+            *reinterpret_cast<__nv_bfloat162*>(W + rc + nh + m) = cl;
+            *reinterpret_cast<__nv_bfloat162*>(W + rs + m) = sh;
+            *reinterpret_cast<__nv_bfloat162*>(W + rs + nh + m) = sl;
         }
         else
         {
-            float* W = static_cast<float*>(out);
-            W[rr + j] = re;
-            W[ri + j] = im;
+            float* W = static_cast<float*>(R.out);
+            *reinterpret_cast<float2*>(W + rc + m) = make_float2(cv[0], cv[1]);
+            *reinterpret_cast<float2*>(W + rs + m) = make_float2(sv[0], sv[1]);
         }
     }
 }
@@ -676,151 +790,234 @@ __global__ void pupil_build_kernel(float* __restrict__ out, int N, float fill, P
     out[idx] = (env ? acc : (float)cnt) * (1.0f / 16.0f);
 }
 
-// Pupil amplitude A[i][j] (float, n x n) -> B operand [hi | lo | hi] or FP32.
+// Operand A[i][j] (float, n x n) -> its even and odd parts about the centre,
+// A'[part][row d][col d'], split BF16 [hi | lo] or FP32.  i1 / i2 are the
+// indices at +d and -d (outside the operand: zero); d = 0 of a whole centre
+// counts once in the even part.
 template <int FORM>
-__global__ void mdft_mask_kernel(const float* __restrict__ a, void* out, int n, int Kp)
+__device__ __forceinline__ void mdft_fold_one(const float* __restrict__ a, void* out, int n, int nh, int nhr, int nf,
+                                              int h2, int box, int x, int y)
 {
-    const size_t total = (size_t)n * n;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
+    const int Kp = FORM == 0 ? 2 * nh : nh;
+    if (FORM == kTf32)                               // not folded: nh = n
     {
-        const int j = (int)(e % n), i = (int)(e / n);
-        const float v = a[e];
+        static_cast<float*>(out)[(size_t)y * Kp + x] = a[(size_t)y * n + x];
+        return;
+    }
+    const int base = (h2 + 1) >> 1;                  // index at the smallest distance
+    auto at = [&](int r, int c) {
+        return (r >= 0 && r < n && c >= 0 && c < n) ? a[(size_t)r * n + c] : 0.0f;
+    };
+    const int r1 = base + y, r2 = h2 - r1, c1 = base + x, c2 = h2 - c1;
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};           // ee, oe, eo, oo
+    if (x < nf && y < nf)
+    {
+        const float p = at(r1, c1), q = c1 == c2 ? 0.0f : at(r1, c2);
+        const float s = r1 == r2 ? 0.0f : at(r2, c1), t = (r1 == r2 || c1 == c2) ? 0.0f : at(r2, c2);
+        const bool ro = r1 != r2, co = c1 != c2;     // no odd part at distance 0
+        v[0] = (p + q) + (s + t);
+        v[1] = ro ? (p + q) - (s + t) : 0.0f;
+        v[2] = co ? (p - q) + (s - t) : 0.0f;
+        v[3] = ro && co ? (p - q) - (s - t) : 0.0f;
+    }
+    const int parts = box ? 2 : 4;
+    #pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+        if (k >= parts) break;
+        const float w = box ? (k == 0 ? v[0] : v[3]) : v[k];
+        const size_t o = ((size_t)k * nhr + y) * Kp + x;
         if (FORM == 0)
         {
             __nv_bfloat16* M = static_cast<__nv_bfloat16*>(out);
-            const __nv_bfloat16 h = __float2bfloat16_rn(v);
-            const __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(h));
-            M[(size_t)i * Kp + j] = h; M[(size_t)i * Kp + n + j] = l; M[(size_t)i * Kp + 2 * n + j] = h;
+            const __nv_bfloat16 h = __float2bfloat16_rn(w);
+            M[o] = h;
+            M[o + nh] = __float2bfloat16_rn(w - __bfloat162float(h));
         }
         else
         {
-            static_cast<float*>(out)[(size_t)i * Kp + j] = v;
+            static_cast<float*>(out)[o] = w;
         }
     }
+}
+
+// The blocks past the nh rows zero the output planes and the error word, in
+// place of four memset nodes.
+template <int FORM>
+__global__ void __launch_bounds__(128) mdft_fold_kernel(const float* __restrict__ a, void* out, int n, int nh, int nhr,
+                                                        int nf, int h2, int box, float* z0, float* z1, float* z2,
+                                                        size_t npx, int* err)
+{
+    const int y = blockIdx.x;
+    if (y >= nh)
+    {
+        const size_t at = (size_t)(y - nh) * blockDim.x + threadIdx.x, all = (size_t)(gridDim.x - nh) * blockDim.x;
+        if (at == 0) *err = 0;
+        float* planes[3] = {z0, z1, z2};
+        #pragma unroll
+        for (int c = 0; c < 3; ++c)
+        {
+            const bool vec = (reinterpret_cast<uintptr_t>(planes[c]) & 15) == 0;
+            const size_t quads = vec ? npx / 4 : 0;
+            for (size_t i = at; i < quads; i += all)
+                reinterpret_cast<float4*>(planes[c])[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (size_t i = 4 * quads + at; i < npx; i += all) planes[c][i] = 0.0f;
+        }
+        return;
+    }
+    for (int x = threadIdx.x; x < nh; x += blockDim.x) mdft_fold_one<FORM>(a, out, n, nh, nhr, nf, h2, box, x, y);
 }
 
 
 // ---- FP32 CUDA-core form -------------------------------------------------------
-// Register-tiled FP32 products on the SIMT pipes over the TF32 form's storage
-// (W' [lam][2][K_out][n], T' [lam][NB][3][128][n]); 256 threads, 128x128
-// tiles, 8x8 outputs per thread, K chunks of 16 staged in shared memory.
-constexpr int kSB = 128, kSK = 16;
+// The same folded products in FP32 FMAs over the TF32 form's storage.  A CTA
+// makes a 64 x 64 tile of every row block of a unit (step 1: one parity of T;
+// step 2: Re E and Im E over both), 256 threads of 4 x 4 per block, reduction
+// chunks of 16 staged in shared memory one chunk ahead.  Step 2 adds its
+// wavelengths' colours up in registers; a frame of few tiles is also split over
+// wavelength ranges (n_ranges), whose CTAs add into the planes with atomics.
+// Bound by the FP32 pipes: 32 FMA per three 16-byte shared loads (box: 16 per
+// two).  256^2 pupil to 512^2, 8 wavelengths: both steps 1.75 -> 0.09 ms (the
+// unfolded form looped over the wavelengths in 16 CTAs of 128 x 128 tiles).
+constexpr int kSB = 64, kSK = 16;
 
-__global__ void __launch_bounds__(256) mdft_simt_step1(const float* __restrict__ W, const float* __restrict__ A,
-                                                       float* __restrict__ T, int K_out, int n, int NB, int lam_base)
+template <int STEP, bool BOX>
+__global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restrict__ W, const float* __restrict__ B,
+                                                           MdftArgs args, int lam1, int n_ranges)
 {
-    // K_out = rows of W_x per (wavelength, part) = Kx
-    __shared__ float sWr[kSK][kSB + 4], sWi[kSK][kSB + 4], sA[kSK][kSB + 4];
-    const int lam = lam_base + (int)blockIdx.z, mb = blockIdx.y, ib = blockIdx.x;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const float* Wr = W + ((size_t)(lam * 2 + 0) * K_out + mb * kSB) * n;
-    const float* Wi = W + ((size_t)(lam * 2 + 1) * K_out + mb * kSB) * n;
-    const float* Ab = A + (size_t)(ib * kSB) * n;
-    float cr[8][8] = {}, ci[8][8] = {};
-    for (int k0 = 0; k0 < n; k0 += kSK)
+    constexpr int NBLK = BOX ? 1 : 2;
+    __shared__ __align__(16) float sA[kSK][kSB + 4];
+    __shared__ __align__(16) float sB[NBLK][kSK][kSB + 4];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int lr = tid >> 2, lc = (tid & 3) * 4;               // row and first column of this thread's staging loads
+    const int nh = args.nh, xb = blockIdx.x, mb = blockIdx.y;  // 64-wide tiles
+    int l0, l1, part = 0;
+    if (STEP == 1)
     {
-        for (int e = threadIdx.x; e < kSB * kSK; e += 256)
-        {
-            const int r = e / kSK, c = e % kSK;
-            sWr[c][r] = Wr[(size_t)r * n + k0 + c];
-            sWi[c][r] = Wi[(size_t)r * n + k0 + c];
-            sA[c][r] = Ab[(size_t)r * n + k0 + c];
-        }
-        __syncthreads();
-        #pragma unroll
-        for (int kk = 0; kk < kSK; ++kk)
-        {
-            float wr[8], wi[8], a[8];
-            #pragma unroll
-            for (int q = 0; q < 8; ++q) { wr[q] = sWr[kk][ty * 8 + q]; wi[q] = sWi[kk][ty * 8 + q]; a[q] = sA[kk][tx * 8 + q]; }
-            #pragma unroll
-            for (int p = 0; p < 8; ++p)
-                #pragma unroll
-                for (int q = 0; q < 8; ++q) { cr[p][q] += wr[p] * a[q]; ci[p][q] += wi[p] * a[q]; }
-        }
-        __syncthreads();
+        l0 = args.lam_base + (int)(blockIdx.z >> 1);
+        l1 = l0 + 1;
+        part = blockIdx.z & 1;
     }
-    const size_t blk = ((size_t)(lam * NB + mb) * 3) * 128;
-    #pragma unroll
-    for (int p = 0; p < 8; ++p)
+    else
     {
-        const int k = ty * 8 + p;
-        #pragma unroll
-        for (int q = 0; q < 8; ++q)
-        {
-            const int i = ib * kSB + tx * 8 + q;
-            T[(blk + 0 * 128 + k) * n + i] = -ci[p][q];
-            T[(blk + 1 * 128 + k) * n + i] = cr[p][q];
-            T[(blk + 2 * 128 + k) * n + i] = ci[p][q];
-        }
+        const int total = lam1 - args.lam_base, per = (total + n_ranges - 1) / n_ranges;
+        l0 = args.lam_base + (int)blockIdx.z * per;
+        l1 = min(lam1, l0 + per);
     }
-}
-
-__global__ void __launch_bounds__(256) mdft_simt_step2(const float* __restrict__ W, const float* __restrict__ T,
-                                                       const float4* __restrict__ weights, float* out_r, float* out_g,
-                                                       float* out_b, int K_rows, int K_out, int n, int NB, int lam0, int lam1,
-                                                       int box, int out_w, int x0, int y0, int win_w, int win_h,
-                                                       float4 tint)
-{
-    // K_rows = rows of W_y per (wavelength, part) = Ky; K_out = output width Kx
-    __shared__ float sWr[kSK][kSB + 4], sWi[kSK][kSB + 4], sTr[kSK][kSB + 4], sTi[kSK][kSB + 4];
-    const int mb = blockIdx.y, nb = blockIdx.x;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    for (int lam = lam0; lam < lam1; ++lam)
+    float rgb[STEP == 2 ? 3 : 1][4][4] = {};
+    for (int lam = l0; lam < l1; ++lam)
     {
-        const float* Wr = W + ((size_t)(lam * 2 + 0) * K_rows + mb * kSB) * n;
-        const float* Wi = W + ((size_t)(lam * 2 + 1) * K_rows + mb * kSB) * n;
-        const size_t blk = ((size_t)(lam * NB + nb) * 3) * 128;
-        const float* Tr = T + (blk + 128) * n;
-        const float* Ti = T + (blk + 256) * n;
-        float er[8][8] = {}, ei[8][8] = {};
-        for (int k0 = 0; k0 < n; k0 += kSK)
+        float acc[NBLK][4][4] = {};
         {
-            for (int e = threadIdx.x; e < kSB * kSK; e += 256)
+            // chunks of C and S in turn (step 2), like the tensor-core forms
+            constexpr int kPh = STEP == 2 ? 2 : 1;
+            const float* Ar = W + ((size_t)(lam * 2 + part) * args.KA + mb * kSB + lr) * nh + lc;
+            const size_t step_a = (size_t)args.KA * nh, step_b = (size_t)NBLK * (STEP == 2 ? 128 : args.nhr) * nh;
+            const float* Br[NBLK];
+            #pragma unroll
+            for (int j = 0; j < NBLK; ++j)
             {
-                const int r = e / kSK, c = e % kSK;
-                sWr[c][r] = Wr[(size_t)r * n + k0 + c];
-                sWi[c][r] = Wi[(size_t)r * n + k0 + c];
-                sTr[c][r] = Tr[(size_t)r * n + k0 + c];
-                sTi[c][r] = Ti[(size_t)r * n + k0 + c];
+                // the last tile across nh may end past nh, not past A's padded rows (nhr is a multiple of 128)
+                const size_t row = STEP == 2
+                    ? ((size_t)(lam * args.NB + (xb >> 1)) * (2 * NBLK) + j) * 128 + (xb & 1) * kSB + lr
+                    : (size_t)(part * NBLK + j) * args.nhr + xb * kSB + lr;
+                Br[j] = B + row * nh + lc;
             }
-            __syncthreads();
-            #pragma unroll 4
-            for (int kk = 0; kk < kSK; ++kk)
+            float4 pa = *reinterpret_cast<const float4*>(Ar), pb[NBLK];
+            #pragma unroll
+            for (int j = 0; j < NBLK; ++j) pb[j] = *reinterpret_cast<const float4*>(Br[j]);
+            const int chunks = kPh * (nh / kSK);
+            for (int ch = 0; ch < chunks; ++ch)
             {
-                float wr[8], wi[8], tr[8], ti[8];
+                __syncthreads();
+                sA[lc][lr] = pa.x; sA[lc + 1][lr] = pa.y; sA[lc + 2][lr] = pa.z; sA[lc + 3][lr] = pa.w;
                 #pragma unroll
-                for (int q = 0; q < 8; ++q)
+                for (int j = 0; j < NBLK; ++j)
                 {
-                    wr[q] = sWr[kk][ty * 8 + q]; wi[q] = sWi[kk][ty * 8 + q];
-                    tr[q] = sTr[kk][tx * 8 + q]; ti[q] = sTi[kk][tx * 8 + q];
+                    sB[j][lc][lr] = pb[j].x; sB[j][lc + 1][lr] = pb[j].y;
+                    sB[j][lc + 2][lr] = pb[j].z; sB[j][lc + 3][lr] = pb[j].w;
+                }
+                __syncthreads();
+                if (ch + 1 < chunks)
+                {
+                    const int k0 = ((ch + 1) / kPh) * kSK, cs = (ch + 1) % kPh;
+                    pa = *reinterpret_cast<const float4*>(Ar + cs * step_a + k0);
+                    #pragma unroll
+                    for (int j = 0; j < NBLK; ++j) pb[j] = *reinterpret_cast<const float4*>(Br[j] + cs * step_b + k0);
                 }
                 #pragma unroll
-                for (int p = 0; p < 8; ++p)
+                for (int kk = 0; kk < kSK; ++kk)
+                {
+                    const float4 a4 = *reinterpret_cast<const float4*>(&sA[kk][ty * 4]);
+                    const float av[4] = {a4.x, a4.y, a4.z, a4.w};
                     #pragma unroll
-                    for (int q = 0; q < 8; ++q)
+                    for (int j = 0; j < NBLK; ++j)
                     {
-                        er[p][q] += wr[p] * tr[q] - wi[p] * ti[q];
-                        ei[p][q] += wr[p] * ti[q] + wi[p] * tr[q];
+                        const float4 b4 = *reinterpret_cast<const float4*>(&sB[j][kk][tx * 4]);
+                        const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+                        #pragma unroll
+                        for (int p = 0; p < 4; ++p)
+                            #pragma unroll
+                            for (int q = 0; q < 4; ++q) acc[j][p][q] = fmaf(av[p], bv[q], acc[j][p][q]);
                     }
+                }
             }
-            __syncthreads();
         }
-        // this block owns the tile across wavelengths: plain read-modify-write
-        const float4 w0 = weights[lam];
-        const float4 w = make_float4(w0.x * tint.x, w0.y * tint.y, w0.z * tint.z, 0.0f);
-        #pragma unroll
-        for (int p = 0; p < 8; ++p)
+        if (STEP == 1)
         {
-            const int l = mb * kSB + ty * 8 + p;
-            if (l >= win_h) continue;
-            const size_t row = (size_t)(y0 + l) * out_w + x0 + nb * kSB + tx * 8;
+            // A rows are k, B rows the folded pupil rows: T'[block][k % 128][i]
+            float* T = static_cast<float*>(args.tprime);
+            const size_t blk = (size_t)(lam * args.NB + (mb >> 1)) * (2 * NBLK) * 128;
+            const int i0 = xb * kSB + tx * 4;
+            if (i0 >= nh) continue;
             #pragma unroll
-            for (int q = 0; q < 8; ++q)
+            for (int j = 0; j < NBLK; ++j)
             {
-                if (nb * kSB + tx * 8 + q >= win_w) continue;
-                const float I = box ? er[p][q] : er[p][q] * er[p][q] + ei[p][q] * ei[p][q];
-                out_r[row + q] += w.x * I; out_g[row + q] += w.y * I; out_b[row + q] += w.z * I;
+                const int dst = BOX ? part : (part == 0 ? (j == 0 ? 0 : 3) : (j == 0 ? 1 : 2));
+                const float sign = (part == 0 && j == 0) ? 1.0f : -1.0f;
+                #pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    *reinterpret_cast<float4*>(T + (blk + dst * 128 + (mb & 1) * kSB + ty * 4 + p) * nh + i0) =
+                        make_float4(sign * acc[j][p][0], sign * acc[j][p][1], sign * acc[j][p][2], sign * acc[j][p][3]);
+            }
+        }
+        else
+        {
+            const float4 w = args.weights[lam];
+            const float wr = w.x * args.tint.x, wg = w.y * args.tint.y, wb = w.z * args.tint.z;
+            #pragma unroll
+            for (int p = 0; p < 4; ++p)
+                #pragma unroll
+                for (int q = 0; q < 4; ++q)
+                {
+                    const float re = acc[0][p][q], im = BOX ? 0.0f : acc[NBLK - 1][p][q];
+                    const float I = BOX ? re : re * re + im * im;
+                    rgb[0][p][q] += wr * I;
+                    rgb[1 % (STEP == 2 ? 3 : 1)][p][q] += wg * I;
+                    rgb[2 % (STEP == 2 ? 3 : 1)][p][q] += wb * I;
+                }
+        }
+    }
+    if (STEP == 2)
+    {
+        float* outs[3] = {args.out_r, args.out_g, args.out_b};
+        #pragma unroll
+        for (int p = 0; p < 4; ++p)
+        {
+            const int l = mb * kSB + ty * 4 + p;
+            if (l >= args.win_h) continue;
+            const size_t row = (size_t)(args.y0 + l) * args.out_w + args.x0 + xb * kSB + tx * 4;
+            #pragma unroll
+            for (int q = 0; q < 4; ++q)
+            {
+                if (xb * kSB + tx * 4 + q >= args.win_w) continue;
+                #pragma unroll
+                for (int c = 0; c < 3; ++c)
+                {
+                    const float v = rgb[c % (STEP == 2 ? 3 : 1)][p][q];
+                    if (n_ranges > 1) atomicAdd(outs[c] + row + q, v);
+                    else outs[c][row + q] += v;                // this block owns the tile
+                }
             }
         }
     }
@@ -833,12 +1030,18 @@ constexpr double kMaxCentre = 12288.0;   // pattern centre range (pixels)
 
 struct MdftPlan {
     int n = 0, Kx = 0, Ky = 0, n_lambda = 0, form = 0, Kp = 0, elem = 2;
-    void* wx = nullptr;     // W_x' [lam][2][Kx][Kp]
-    void* wy = nullptr;     // W_y' [lam][2][Ky][Kp]
-    void* mask = nullptr;   // A'   [n][Kp]
-    void* tprime = nullptr; // T'   [lam][Kx/128][3][128][Kp]
+    // folded reduction: nf distances |j - cj|, padded to nh (16); nhr rows per
+    // part of A' (128); h2 = 2 cj
+    // (TF32, not folded: nf = nh = n); d0 = smallest distance (TF32: -cj)
+    int nf = 0, nh = 0, nhr = 0, h2 = 0;
+    float d0 = 0.0f;
+    void* wx = nullptr;     // W_x' [lam][C | S][Kx][Kp]
+    void* wy = nullptr;     // W_y' [lam][C | S][Ky][Kp]
+    void* mask = nullptr;   // A'   [4 parts, box 2][nhr][Kp]
+    void* tprime = nullptr; // T'   [lam][Kx/128][4 parts, box 2][128][Kp]
     float4* weights = nullptr;
     float2* scales = nullptr;   // [2][n_lambda] (s_hi, s_lo) device copy
+    float* amp = nullptr;       // [x, y][n_lambda][nh] factors of the matrix entries
     double cx = 0.0, cy = 0.0;
     float cj = 0.0f;            // reduction-axis centre: (n - 1) / 2, or the zero lag mc of the box form
     int box = 0;                // pixel-integrated form (the reference's MDFT engine)
@@ -854,7 +1057,7 @@ static void mdft_free(MdftPlan* p)
 {
     if (!p) return;
     cudaFree(p->wx); cudaFree(p->wy); cudaFree(p->mask); cudaFree(p->tprime);
-    cudaFree(p->weights); cudaFree(p->scales); cudaFree(p->err);
+    cudaFree(p->weights); cudaFree(p->scales); cudaFree(p->amp); cudaFree(p->err);
     delete p;
 }
 
@@ -867,24 +1070,60 @@ namespace gl {
 // Enqueue the DFT matrices of the plan's current centre.
 static cudaError_t mdft_build_matrices(MdftPlan* p, cudaStream_t st)
 {
-    const int blocks = 4 * p->sms;
-    const float cj = p->cj;
-    const int box = p->box;
     const float cxh = (float)p->cx, cxl = (float)(p->cx - (double)cxh);
     const float cyh = (float)p->cy, cyl = (float)(p->cy - (double)cyh);
-    if (p->form == 0)
+    const DftRows R[2] = {{p->wx, p->scales, p->amp, cxh, cxl, p->Kx},
+                          {p->wy, p->scales + p->n_lambda, p->amp + (size_t)p->n_lambda * p->nh, cyh, cyl, p->Ky}};
+    const int tx = p->nh >= 128 ? 64 : 32;             // two entries per thread and pass
+    const dim3 block(tx, 256 / tx);
+    for (const DftRows& r : R)
     {
-        mdft_dft_kernel<0><<<blocks, 256, 0, st>>>(p->wx, p->n_lambda, p->Kx, p->n, p->Kp, p->scales, cxh, cxl, cj, box);
-        mdft_dft_kernel<0><<<blocks, 256, 0, st>>>(p->wy, p->n_lambda, p->Ky, p->n, p->Kp, p->scales + p->n_lambda, cyh,
-                                                   cyl, cj, box);
-    }
-    else
-    {
-        mdft_dft_kernel<1><<<blocks, 256, 0, st>>>(p->wx, p->n_lambda, p->Kx, p->n, p->Kp, p->scales, cxh, cxl, cj, box);
-        mdft_dft_kernel<1><<<blocks, 256, 0, st>>>(p->wy, p->n_lambda, p->Ky, p->n, p->Kp, p->scales + p->n_lambda, cyh,
-                                                   cyl, cj, box);
+        const int grid = (p->n_lambda * r.K + (int)block.y - 1) / (int)block.y;
+        if (p->form == 0) mdft_dft_kernel<0><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
+        else if (p->form == kTf32) mdft_dft_kernel<kTf32><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
+        else mdft_dft_kernel<2><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
     }
     return cudaGetLastError();
+}
+
+// Opt one GEMM instance in to its shared memory.
+template <int FORM, int STEP, int TN, bool BOX>
+static cudaError_t mdft_prepare()
+{
+    return cudaFuncSetAttribute(mdft_kernel<FORM, STEP, TN, BOX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                MdftShape<FORM, STEP, TN, BOX>::kSmem);
+}
+
+template <int FORM, bool BOX>
+static cudaError_t mdft_prepare_all()
+{
+    cudaError_t e = mdft_prepare<FORM, 1, 128, BOX>();
+    if (e == cudaSuccess) e = mdft_prepare<FORM, 2, 128, BOX>();
+    if (e == cudaSuccess) e = mdft_prepare<FORM, 2, 64, BOX>();
+    return e;
+}
+
+template <int FORM, bool BOX>
+static void mdft_gemms(const MdftPlan* p, const MdftArgs& a1, int g1, const MdftArgs& a2, int g2, cudaStream_t st)
+{
+    mdft_kernel<FORM, 1, 128, BOX><<<g1, kMdftThreads, MdftShape<FORM, 1, 128, BOX>::kSmem, st>>>(p->t_wx, p->t_mask, a1);
+    if (p->tile_n == 64)
+        mdft_kernel<FORM, 2, 64, BOX><<<g2, kMdftThreads, MdftShape<FORM, 2, 64, BOX>::kSmem, st>>>(p->t_wy, p->t_tp64, a2);
+    else
+        mdft_kernel<FORM, 2, 128, BOX><<<g2, kMdftThreads, MdftShape<FORM, 2, 128, BOX>::kSmem, st>>>(p->t_wy, p->t_tp, a2);
+}
+
+template <bool BOX>
+static void mdft_simt(const MdftPlan* p, const MdftArgs& a1, const MdftArgs& a2, int l1, cudaStream_t st)
+{
+    const int nl = l1 - a1.lam_base;
+    const dim3 t1((p->nh + kSB - 1) / kSB, p->Kx / kSB, 2 * nl);
+    mdft_simt_kernel<1, BOX><<<t1, 256, 0, st>>>(static_cast<const float*>(p->wx), static_cast<const float*>(p->mask), a1, l1, 1);
+    // wavelength ranges until about three CTAs per SM are in flight
+    const int tiles = (p->Kx / kSB) * (p->Ky / kSB);
+    const int ranges = std::min(nl, std::max(1, (3 * p->sms + tiles - 1) / tiles));
+    const dim3 t2(p->Kx / kSB, p->Ky / kSB, ranges);
+    mdft_simt_kernel<2, BOX><<<t2, 256, 0, st>>>(static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime), a2, l1, ranges);
 }
 
 }  // namespace gl
@@ -913,13 +1152,19 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     p->n = n; p->Kx = Kx; p->Ky = Ky; p->n_lambda = n_lambda; p->form = form;
     p->cx = center_x; p->cy = center_y;
     p->box = box; p->cj = red_center;
-    p->Kp = form == 0 ? 3 * n : n;
+    p->h2 = (int)(2.0f * red_center);
+    p->nf = form == kTf32 ? n : (int)std::floor(std::max((double)red_center, (double)(n - 1) - (double)red_center)) + 1;
+    p->d0 = form == kTf32 ? -red_center : ((p->h2 & 1) ? 0.5f : 0.0f);
+    p->nh = (p->nf + 15) / 16 * 16;
+    p->nhr = (p->nh + 127) / 128 * 128;
+    p->Kp = form == 0 ? 2 * p->nh : p->nh;
     p->elem = form == 0 ? 2 : 4;
-    const int NBx = Kx / 128;
+    const int NBx = Kx / 128, parts = (box || form == kTf32) ? 2 : 4;      // of T'
+    const int mparts = form == kTf32 ? 1 : parts;                          // of A'
     const size_t wxbytes = (size_t)n_lambda * 2 * Kx * p->Kp * p->elem;
     const size_t wybytes = (size_t)n_lambda * 2 * Ky * p->Kp * p->elem;
-    const size_t mbytes = (size_t)n * p->Kp * p->elem;
-    const size_t tbytes = (size_t)n_lambda * NBx * 3 * 128 * p->Kp * p->elem;
+    const size_t mbytes = (size_t)mparts * p->nhr * p->Kp * p->elem;
+    const size_t tbytes = (size_t)n_lambda * NBx * parts * 128 * p->Kp * p->elem;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
     chk(cudaMalloc(&p->wx, wxbytes));
@@ -928,8 +1173,10 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     chk(cudaMalloc(&p->tprime, tbytes));
     chk(cudaMalloc(&p->weights, sizeof(float4) * n_lambda));
     chk(cudaMalloc(&p->scales, sizeof(float2) * 2 * n_lambda));
+    chk(cudaMalloc(&p->amp, sizeof(float) * 2 * n_lambda * p->nh));
     chk(cudaMalloc(&p->err, sizeof(int)));
     chk(cudaMemset(p->err, 0, sizeof(int)));          // a plan never executed reports no error
+    chk(cudaMemset(p->mask, 0, mbytes));              // the rows between nh and nhr stay zero
     int dev = 0;
     chk(cudaGetDevice(&dev));
     chk(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
@@ -949,25 +1196,15 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     }
     chk(cudaMemcpy(p->weights, w.data(), sizeof(float4) * n_lambda, cudaMemcpyHostToDevice));
     chk(cudaMemcpy(p->scales, sc.data(), sizeof(float2) * 2 * n_lambda, cudaMemcpyHostToDevice));
-    if (e == cudaSuccess) chk(mdft_build_matrices(p, st));
+    if (e == cudaSuccess)
+    {
+        mdft_amp_kernel<<<2 * n_lambda, 256, 0, st>>>(p->amp, p->scales, p->nh, p->nf, p->d0, box);
+        chk(mdft_build_matrices(p, st));
+    }
     chk(cudaStreamSynchronize(st));
     // shared-memory opt-in once here, so execute enqueues kernels only (graph capture)
-    {
-        const int smem1 = 4 * 3 * kOpTile + 1024, smem2 = 3 * 4 * kOpTile + 1024;
-        const int smem2h = 4 * (2 * kOpTile + 2 * 64 * 128) + 1024;
-        if (form == 0)
-        {
-            chk(cudaFuncSetAttribute(mdft_kernel<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1));
-            chk(cudaFuncSetAttribute(mdft_kernel<0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
-            chk(cudaFuncSetAttribute(mdft_kernel<0, 2, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2h));
-        }
-        else if (form == 1)
-        {
-            chk(cudaFuncSetAttribute(mdft_kernel<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1));
-            chk(cudaFuncSetAttribute(mdft_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
-            chk(cudaFuncSetAttribute(mdft_kernel<1, 2, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2h));
-        }
-    }
+    if (form == 0) chk(box ? mdft_prepare_all<0, true>() : mdft_prepare_all<0, false>());
+    else if (form == 1) chk(box ? mdft_prepare_all<1, true>() : mdft_prepare_all<1, false>());
     const CUtensorMapDataType dt = form == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const uint32_t bc = form == 0 ? 64 : 32;
     int rc = GL_OK;
@@ -975,9 +1212,9 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     {
         rc = make_tmap_2d(&p->t_wx, p->wx, dt, p->elem, (uint64_t)n_lambda * 2 * Kx, (uint64_t)p->Kp, 128, bc);
         if (!rc) rc = make_tmap_2d(&p->t_wy, p->wy, dt, p->elem, (uint64_t)n_lambda * 2 * Ky, (uint64_t)p->Kp, 128, bc);
-        if (!rc) rc = make_tmap_2d(&p->t_mask, p->mask, dt, p->elem, (uint64_t)n, (uint64_t)p->Kp, 128, bc);
-        if (!rc) rc = make_tmap_2d(&p->t_tp, p->tprime, dt, p->elem, (uint64_t)n_lambda * NBx * 3 * 128, (uint64_t)p->Kp, 128, bc);
-        if (!rc) rc = make_tmap_2d(&p->t_tp64, p->tprime, dt, p->elem, (uint64_t)n_lambda * NBx * 3 * 128, (uint64_t)p->Kp, 64, bc);
+        if (!rc) rc = make_tmap_2d(&p->t_mask, p->mask, dt, p->elem, (uint64_t)mparts * p->nhr, (uint64_t)p->Kp, 128, bc);
+        if (!rc) rc = make_tmap_2d(&p->t_tp, p->tprime, dt, p->elem, (uint64_t)n_lambda * NBx * parts * 128, (uint64_t)p->Kp, 128, bc);
+        if (!rc) rc = make_tmap_2d(&p->t_tp64, p->tprime, dt, p->elem, (uint64_t)n_lambda * NBx * parts * 128, (uint64_t)p->Kp, 64, bc);
     }
     if (e != cudaSuccess || rc)
     {
@@ -1029,62 +1266,54 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
         x0 + win_w > out_w || y0 + win_h > out_h)
         return fail(GL_ERR_INVALID, "mdft_plan_execute: the output window must lie inside the planes and the plan");
     cudaStream_t st = (cudaStream_t)stream;
-    const int NBx = p->Kx / 128, NBy = p->Ky / 128, NI = p->n / 128;
+    const int NBx = p->Kx / 128, NBy = p->Ky / 128;
     const size_t npx = (size_t)out_w * out_h;
     int launches = 0;
-    GL_CUDA_TRY(cudaMemsetAsync(p->err, 0, sizeof(int), st));
-    if (p->form == 0) mdft_mask_kernel<0><<<2 * p->sms, 256, 0, st>>>(d_pupil, p->mask, p->n, p->Kp);
-    else mdft_mask_kernel<1><<<2 * p->sms, 256, 0, st>>>(d_pupil, p->mask, p->n, p->Kp);
+    // zeroing blocks: two waves of the chip at most, one at least (the error word)
+    const size_t zero = accumulate ? 0 : npx;
+    const int fold = p->nh + (int)std::max<size_t>(1, std::min<size_t>((3 * zero / 4 + 1023) / 1024, 16 * (size_t)p->sms));
+    auto run_fold = [&](auto kernel) {
+        kernel<<<fold, 128, 0, st>>>(d_pupil, p->mask, p->n, p->nh, p->nhr, p->nf, p->h2, p->box, d_out_r, d_out_g,
+                                     d_out_b, zero, p->err);
+    };
+    if (p->form == 0) run_fold(mdft_fold_kernel<0>);
+    else if (p->form == kTf32) run_fold(mdft_fold_kernel<kTf32>);
+    else run_fold(mdft_fold_kernel<2>);
     ++launches;
-    if (!accumulate)
-    {
-        GL_CUDA_TRY(cudaMemsetAsync(d_out_r, 0, npx * sizeof(float), st));
-        GL_CUDA_TRY(cudaMemsetAsync(d_out_g, 0, npx * sizeof(float), st));
-        GL_CUDA_TRY(cudaMemsetAsync(d_out_b, 0, npx * sizeof(float), st));
-    }
     MdftArgs a;
-    a.NBt = NBx;
-    a.KA = p->Kx; a.Kx = p->Kx; a.NBm = NBx;
-    a.n = p->n; a.n_lambda = p->n_lambda; a.Kp = p->Kp;
-    a.nkb = p->Kp / (p->form == 0 ? 64 : 32);
-    a.NB = NBx; a.NI = NI;
+    a.KA = p->Kx; a.NBm = NBx; a.NBt = NBx;
+    a.nh = p->nh; a.nhr = p->nhr;
+    const int kbe = p->form == 0 ? 64 : 32;
+    a.nkb = (p->nh + kbe - 1) / kbe;
+    a.NB = NBx; a.NI = p->nhr / 128;
     a.tprime = p->tprime; a.out_r = d_out_r; a.out_g = d_out_g; a.out_b = d_out_b;
     a.weights = p->weights; a.err = p->err;
-    a.out_w = out_w; a.x0 = x0; a.y0 = y0; a.win_w = win_w; a.win_h = win_h; a.box = p->box;
+    a.out_w = out_w; a.x0 = x0; a.y0 = y0; a.win_w = win_w; a.win_h = win_h;
     a.tint = tint_rgb ? make_float4(tint_rgb[0], tint_rgb[1], tint_rgb[2], 0.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    const size_t smem1 = 4 * 3 * (size_t)kOpTile + 1024, smem2 = 3 * 4 * (size_t)kOpTile + 1024;
     const int l0 = p->lam0, l1 = p->lam1 < 0 ? p->n_lambda : p->lam1, nl = l1 - l0;
     a.lam_base = l0;
-    a.n_units = nl * NBx * NI;                          // step 1: (lambda, k block, pupil-row block)
+    a.n_units = nl * NBx * a.NI * (p->form == kTf32 ? 1 : 2);   // step 1: (lambda, k block, pupil-row block, C / S)
     const int gmax = p->ctas > 0 ? p->ctas : p->sms;
     const int g1 = std::min(a.n_units, gmax);
     MdftArgs a2 = a;
     a2.KA = p->Ky; a2.NBm = NBy;
-    const bool half = p->tile_n == 64;
     a2.NBt = p->Kx / p->tile_n;
     a2.n_units = NBy * a2.NBt * nl;                     // step 2: (lambda, output tile)
     const int g2 = std::min(a2.n_units, gmax);
-    const size_t smem2h = 4 * (2 * (size_t)kOpTile + 2 * 64 * 128) + 1024;
     if (p->form == 2)
     {
-        mdft_simt_step1<<<dim3(NI, NBx, nl), 256, 0, st>>>(static_cast<const float*>(p->wx),
-                                                           static_cast<const float*>(p->mask),
-                                                           static_cast<float*>(p->tprime), p->Kx, p->n, NBx, l0);
-        mdft_simt_step2<<<dim3(NBx, NBy), 256, 0, st>>>(static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime),
-                                                       p->weights, d_out_r, d_out_g, d_out_b, p->Ky, p->Kx, p->n, NBx,
-                                                       l0, l1, p->box, out_w, x0, y0, win_w, win_h, a.tint);
+        if (p->box) mdft_simt<true>(p, a, a2, l1, st);
+        else mdft_simt<false>(p, a, a2, l1, st);
     }
     else if (p->form == 0)
     {
-        mdft_kernel<0, 1><<<g1, kMdftThreads, smem1, st>>>(p->t_wx, p->t_mask, a);
-        if (half) mdft_kernel<0, 2, 64><<<g2, kMdftThreads, smem2h, st>>>(p->t_wy, p->t_tp64, a2);
-        else mdft_kernel<0, 2><<<g2, kMdftThreads, smem2, st>>>(p->t_wy, p->t_tp, a2);
+        if (p->box) mdft_gemms<0, true>(p, a, g1, a2, g2, st);
+        else mdft_gemms<0, false>(p, a, g1, a2, g2, st);
     }
     else
     {
-        mdft_kernel<1, 1><<<g1, kMdftThreads, smem1, st>>>(p->t_wx, p->t_mask, a);
-        if (half) mdft_kernel<1, 2, 64><<<g2, kMdftThreads, smem2h, st>>>(p->t_wy, p->t_tp64, a2);
-        else mdft_kernel<1, 2><<<g2, kMdftThreads, smem2, st>>>(p->t_wy, p->t_tp, a2);
+        if (p->box) mdft_gemms<1, true>(p, a, g1, a2, g2, st);
+        else mdft_gemms<1, false>(p, a, g1, a2, g2, st);
     }
     GL_CUDA_TRY(cudaGetLastError());
     launches += 2;
@@ -1118,7 +1347,7 @@ extern "C" int gl_mdft_plan_set_launch(gl_mdft_plan* plan, int ctas)
 {
     using namespace gl;
     if (!plan || ctas < 0) return fail(GL_ERR_INVALID, "mdft_plan_set_launch: bad arguments");
-    // one 192-thread CTA with ~161 KB of shared memory fits per SM
+    // one 192-thread CTA with up to ~193 KB of shared memory fits per SM
     plan->p->ctas = ctas == 0 ? 0 : std::min(ctas, plan->p->sms);
     return GL_OK;
 }

@@ -59,6 +59,7 @@ class MdftPlan:
         h = C.c_void_p()
         self.box = bool(box)
         rc = 0.5 * (self.n - 1) if red_center is None else float(red_center)
+        self._red_center = rc
         _native.check(self._lib.gl_mdft_plan_create3(
             self.n, self.Kx, self.Ky, self.n_lambda, D(*sx), D(*sy), cx, cy,
             (C.c_float * w.size)(*w.reshape(-1)), FORMS[form], int(self.box), rc, st, C.byref(h)), "mdft")
@@ -133,14 +134,16 @@ class MdftPlan:
         return int(v.value)
 
     def device_bytes(self) -> int:
-        """HBM the plan holds: the two DFT matrices, the operand mask and the
-        intermediate T' in the form's element type (split-BF16: three bf16
-        terms per element along K)."""
-        kp = 3 * self.n if self.form == "split_bf16" else self.n
-        elem = 2 if self.form == "split_bf16" else 4
-        nl = self.n_lambda
-        return (nl * 2 * (self.Kx + self.Ky) * kp * elem + self.n * kp * elem +
-                nl * (self.Kx // 128) * 3 * 128 * kp * elem + 32 * nl + 4)
+        """HBM the plan holds: the two folded DFT matrices (cosine and sine
+        over the distances from the reduction centre), the operand's parity
+        parts and the intermediate T' in the form's element type (split-BF16:
+        two bf16 terms per element)."""
+        tf32 = self.form == "tf32"          # not folded
+        nh = self.n if tf32 else (int(max(self._red_center, self.n - 1 - self._red_center)) + 16) // 16 * 16
+        row = nh * 4                        # two bf16 terms or one float
+        parts, nl = (2 if self.box or tf32 else 4), self.n_lambda
+        return (nl * 2 * (self.Kx + self.Ky) * row + (1 if tf32 else parts) * ((nh + 127) // 128 * 128) * row +
+                nl * parts * self.Kx * row + 32 * nl + 4)
 
     def close(self):
         if getattr(self, "_h", None):
