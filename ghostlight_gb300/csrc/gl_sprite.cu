@@ -16,9 +16,8 @@
 //     centred disc of `fill` of the grid, so most rows are zero); column FFTs
 //     over groups of NB adjacent columns whose epilogue writes |X|^2 straight
 //     to its fftshifted place and adds the block's energy to one FP64 sum;
-//   * the wavelength bake and the ds x ds box sum fused in one kernel: each
-//     coarse texel accumulates its fine texels in the reference's order, so
-//     the N x N x 3 fine sprite (805 MB at N = 8192) never exists in HBM; the
+//   * the wavelength bake and the ds x ds box sum fused in one kernel, so the
+//     N x N x 3 fine sprite (805 MB at N = 8192) never exists in HBM; the
 //     1 / energy normalisation is read on the device (no host round trip);
 //   * the splat: one thread per (source, output pixel in the footprint),
 //     float atomics into the caller's planes (sources overlap), as the
@@ -110,18 +109,6 @@ __global__ void __launch_bounds__(kSpriteThreads) sprite_cols(const float2* __re
     }
 }
 
-__device__ __forceinline__ float psf_bilinear(const float* __restrict__ psf, float fx, float fy, int N, float scale)
-{
-    if (fx < 0.0f || fy < 0.0f || fx >= (float)(N - 1) || fy >= (float)(N - 1)) return 0.0f;
-    const int x0 = (int)floorf(fx), y0 = (int)floorf(fy);
-    const float tx = fx - x0, ty = fy - y0;
-    const float* r0 = psf + (size_t)y0 * N;
-    const float* r1 = r0 + N;
-    const float a = (r0[x0] * scale) * (1.0f - tx) + (r0[x0 + 1] * scale) * tx;
-    const float b = (r1[x0] * scale) * (1.0f - tx) + (r1[x0 + 1] * scale) * tx;
-    return a * (1.0f - ty) + b * ty;
-}
-
 // Column pass of the second transform of the matrix-DFT engine's compact
 // autocorrelation (mdft_render.cu:88-99, 247-262): after the row pass of the
 // fftshifted PSF, transform the columns whose x lag lies within +-mc of zero
@@ -170,42 +157,152 @@ __global__ void __launch_bounds__(kSpriteThreads) autocorr_cols(const float2* __
     }
 }
 
-// bake over wavelength + ds x ds box sum: coarse texel (a, b) of M x M
+// Bake over wavelength + box sum of d x d fine texels (d a power of two up to
+// 32): coarse texel (a, b) of M x M.
+//
+// A lane owns one fine column and T fine rows of it; a CTA's eight warps stack
+// to 32 columns x 8 T rows.  The rows' source positions are tabled per
+// wavelength in shared memory, the column's is formed once per wavelength.
+// Neighbouring fine rows sample source rows 0.8 to 1.4 apart, so the
+// horizontal blend of the lower source row of one is mostly the upper one of
+// the next: about 2.5 loads per texel and wavelength where separate samples
+// take 4, and all loads of a thread's rows are in flight at once (carrying the
+// blend from row to row behind a branch left each row waiting for its own
+// load: 228 us).
+// The box sum goes over the thread's rows, then lanes, then (d > T) warps, in
+// a fixed order.  Every fine texel is a thread's, so a strongly minified sprite
+// (few coarse texels) still fills the chip.  Bound by load latency and issue in
+// equal parts (issue slots 56% busy, L1 49%); 16 rows per thread or more CTAs
+// per SM at fewer registers are slower.
+// N = 2048, 31 wavelengths, d = 2: 221 -> 183 us; N = 1024, 16 wavelengths,
+// d = 16 (one thread per coarse texel: 16 CTAs): 1404 -> 37 us.
+constexpr int kBakeSpec = 32;      // wavelengths staged at a time
+
+// A fine row's source row at one wavelength: y N (negative: outside), blend.
+struct __align__(8) RowAt { int off; float t; };
+
+template <int T>
 __global__ void __launch_bounds__(kSpriteThreads) sprite_bake(const float* __restrict__ psf, int N,
                                                               const float4* __restrict__ spec, int n_spec,
-                                                              float lambda_ref, int ds, int M,
+                                                              float lambda_ref, int d, int M,
                                                               const double* __restrict__ energy,
                                                               float* __restrict__ sprite)
 {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= M * M) return;
+    constexpr int kRows = kSpriteThreads / 32 * T;       // fine rows of the CTA
+    __shared__ float4 lam[kBakeSpec];                    // lambda_ref / lambda, colour weights
+    __shared__ RowAt row_at[kBakeSpec][kRows];
+    __shared__ float part[kSpriteThreads / 32][32][3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane, j0 = blockIdx.y * kRows + warp * T;
     const double e = *energy;
     const float scale = (e > 0.0) ? (float)(1.0 / e) : 0.0f;
-    const int a = idx % M, b = idx / M;
-    const float half = (float)(N / 2);
-    float sr = 0.0f, sg = 0.0f, sb = 0.0f;
-    for (int jj = 0; jj < ds; ++jj)
-        for (int ii = 0; ii < ds; ++ii)
+    const float half = (float)(N / 2), top = (float)(N - 1);
+    const float dx = (float)(i - N / 2);
+    float acc[T][3] = {};
+    for (int l0 = 0; l0 < n_spec; l0 += kBakeSpec)
+    {
+        const int nl = min(kBakeSpec, n_spec - l0);
+        __syncthreads();
+        for (int q = threadIdx.x; q < nl * kRows; q += kSpriteThreads)
         {
-            const int i = a * ds + ii, j = b * ds + jj;
-            const float dx = (float)(i - N / 2), dy = (float)(j - N / 2);
-            float cr = 0.0f, cg = 0.0f, cb = 0.0f;
-            for (int l = 0; l < n_spec; ++l)
-            {
-                const float4 s = spec[l];
-                const float k = lambda_ref / s.x;
-                const float v = psf_bilinear(psf, half + dx * k, half + dy * k, N, scale) * k * k;
-                cr += s.y * v;
-                cg += s.z * v;
-                cb += s.w * v;
-            }
-            sr += cr;
-            sg += cg;
-            sb += cb;
+            const int l = q / kRows, r = q - l * kRows;
+            const float4 s = spec[l0 + l];
+            const float k = lambda_ref / s.x;
+            const float dy = (float)((int)blockIdx.y * kRows + r - N / 2);
+            const float fy = half + dy * k;
+            const bool in = fy >= 0.0f && fy < top;
+            const int y0 = in ? (int)floorf(fy) : 0;
+            RowAt at;
+            at.off = in ? y0 * N : -1;
+            at.t = fy - (float)y0;
+            row_at[l][r] = at;
+            if (r == 0) lam[l] = make_float4(k, s.y * (k * k * scale), s.z * (k * k * scale), s.w * (k * k * scale));
         }
-    sprite[3 * (size_t)idx + 0] = sr;
-    sprite[3 * (size_t)idx + 1] = sg;
-    sprite[3 * (size_t)idx + 2] = sb;
+        __syncthreads();
+        for (int l = 0; l < nl; ++l)
+        {
+            const float4 s = lam[l];
+            const float fx = half + dx * s.x;
+            const bool in = fx >= 0.0f && fx < top;
+            if (!__any_sync(0xffffffffu, in)) continue;
+            const int x0 = in ? (int)floorf(fx) : 0;
+            const float tx = fx - (float)x0;
+            // a column outside blends to zero
+            const float b0 = in ? 1.0f - tx : 0.0f, b1 = in ? tx : 0.0f;
+            const float* col = psf + x0;
+            RowAt at[T];
+            #pragma unroll
+            for (int r = 0; r < T; ++r) at[r] = row_at[l][warp * T + r];
+            // lower source row of each fine row; the upper one where it is not
+            // the row before's (the same for the whole warp)
+            float lo[T], up[T];
+            #pragma unroll
+            for (int r = 0; r < T; ++r)
+            {
+                const int y = max(at[r].off, 0);
+                lo[r] = __ldg(col + (y + N)) * b0 + __ldg(col + (y + N + 1)) * b1;
+            }
+            #pragma unroll
+            for (int r = 0; r < T; ++r)
+            {
+                const int y = max(at[r].off, 0);
+                const bool carried = r > 0 && at[r].off == at[max(r - 1, 0)].off + N && at[max(r - 1, 0)].off >= 0;
+                up[r] = 0.0f;
+                if (!carried) up[r] = __ldg(col + y) * b0 + __ldg(col + (y + 1)) * b1;
+                else up[r] = lo[max(r - 1, 0)];
+            }
+            #pragma unroll
+            for (int r = 0; r < T; ++r)
+            {
+                const float v = at[r].off < 0 ? 0.0f : up[r] * (1.0f - at[r].t) + lo[r] * at[r].t;
+                acc[r][0] += s.y * v;
+                acc[r][1] += s.z * v;
+                acc[r][2] += s.w * v;
+            }
+        }
+    }
+    // rows of the thread, then lanes
+    const int g = min(d, T);                             // rows per sum
+    #pragma unroll
+    for (int r = 0; r < T; ++r)
+        #pragma unroll
+        for (int c = 0; c < 3; ++c)
+        {
+            float v = acc[r][c];
+            #pragma unroll
+            for (int q = 1; q < T; ++q)
+                if (r + q < T && q < g && r % g == 0) v += acc[r + q][c];
+            for (int o = 1; o < d; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (r % g == 0 && (lane & (d - 1)) == 0)
+            {
+                if (d <= T) sprite[3 * ((size_t)((j0 + r) / d) * M + i / d) + c] = v;
+                else part[warp][lane][c] = v;
+            }
+        }
+    if (d <= T) return;                                  // uniform over the grid
+    // d > T: each coarse texel is d / T warps of this CTA
+    __syncthreads();
+    const int wpt = d / T, cols = 32 / d, rows = (kSpriteThreads / 32) / wpt;
+    for (int t = threadIdx.x; t < rows * cols * 3; t += kSpriteThreads)
+    {
+        const int c = t % 3, a = (t / 3) % cols, b = t / (3 * cols);
+        float v = 0.0f;
+        for (int w = 0; w < wpt; ++w) v += part[b * wpt + w][a * d][c];
+        sprite[3 * ((size_t)(blockIdx.y * rows + b) * M + blockIdx.x * cols + a) + c] = v;
+    }
+}
+
+// The rest of a box sum above 32: f x f sums of the 32-texel sums.
+__global__ void __launch_bounds__(kSpriteThreads) sprite_box(const float* __restrict__ fine, int f, int M,
+                                                             float* __restrict__ sprite)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 3 * M * M) return;
+    const int c = t % 3, a = (t / 3) % M, b = t / (3 * M);
+    float v = 0.0f;
+    for (int y = 0; y < f; ++y)
+        for (int x = 0; x < f; ++x) v += fine[3 * ((size_t)(b * f + y) * M * f + a * f + x) + c];
+    sprite[t] = v;
 }
 
 // One output pixel of one source's footprint (offset t in its
@@ -300,7 +397,7 @@ struct SpritePlan {
     float2* work = nullptr;
     float* psf = nullptr;
     float* sprite = nullptr;
-    size_t sprite_cap = 0;       // floats; grown by the bake to 3 M^2
+    size_t sprite_cap = 0;       // floats; grown by the bake to 3 M^2 (and the scratch of a large box sum)
     float4* spec = nullptr;
     double* energy = nullptr;
     StarSource* src = nullptr;
@@ -385,7 +482,8 @@ extern "C" int gl_sprite_plan_bake(gl_sprite_plan* plan, const float* d_pupil, i
     if (ds < 1 || (ds & (ds - 1)) != 0 || ds > N / 8)
         return fail(GL_ERR_INVALID, "sprite_bake: ds must be a power of two in [1, N/8]");
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t need = 3 * (size_t)(N / ds) * (N / ds);
+    // a box sum above 32 goes through the 32-texel sums, kept behind the sprite
+    const size_t need = 3 * (size_t)(N / ds) * (N / ds) + (ds > 32 ? 3 * (size_t)(N / 32) * (N / 32) : 0);
     if (need > p->sprite_cap)
     {
         // an earlier splat on this stream may still read the old sprite
@@ -406,11 +504,22 @@ extern "C" int gl_sprite_plan_bake(gl_sprite_plan* plan, const float* d_pupil, i
         sprite_cols<2><<<N / 2, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
     else
         sprite_cols<1><<<N, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
-    const int MM = p->M * p->M;
-    sprite_bake<<<(MM + kSpriteThreads - 1) / kSpriteThreads, kSpriteThreads, 0, st>>>(
-        p->psf, N, p->spec, p->n_spec, p->lambda_ref, ds, p->M, p->energy, p->sprite);
+    // rows per thread: eight share the most loads; small grids take fewer, for
+    // enough warps (256 CTAs at least)
+    const int d = std::min(ds, 32), m1 = N / d;
+    float* fine = ds > 32 ? p->sprite + 3 * (size_t)p->M * p->M : p->sprite;
+    auto bake = [&](auto kernel, int T) {
+        kernel<<<dim3(N / 32, N / (8 * T)), kSpriteThreads, 0, st>>>(p->psf, N, p->spec, p->n_spec, p->lambda_ref, d, m1,
+                                                                     p->energy, fine);
+    };
+    if (N >= 1024) bake(sprite_bake<8>, 8);
+    else if (N >= 512 || d > 8) bake(sprite_bake<4>, 4);      // a CTA's 8 T rows hold whole box sums
+    else bake(sprite_bake<1>, 1);
+    if (ds > 32)
+        sprite_box<<<(3 * p->M * p->M + kSpriteThreads - 1) / kSpriteThreads, kSpriteThreads, 0, st>>>(fine, ds / 32, p->M,
+                                                                                                       p->sprite);
     GL_CUDA_TRY(cudaGetLastError());
-    g_last_launches = 3;
+    g_last_launches = ds > 32 ? 4 : 3;
     return GL_OK;
 }
 
