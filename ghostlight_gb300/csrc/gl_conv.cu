@@ -5,23 +5,29 @@
 // analytic glare-spread sprite splatted per source, veil_render.cu:94-243);
 // the flare path adds one: out_c = in_c (*) k, 'same' size, k centred.
 //
-// GB300 route: the transform is memory-bound, so it is laid out for HBM.
+// GB300 route:
 //   * linear convolution by zero-padded circular convolution of size P x Q,
 //     P, Q = the smallest 2^a 3^b >= image + kernel - 1 (2048 + 257 - 1 = 2304
 //     = 16 * 16 * 9: no power-of-two padding waste);
-//   * two real channels per complex transform (the kernel is real, so the
-//     real and imaginary parts of the result are the two channels);
-//   * Stockham FFTs in shared memory with large radices held in registers
-//     (16, 8, 4, 2 and 9, 3: three passes over shared memory for 2304
-//     points), twiddles from a per-plan table computed in FP64; the shared
-//     arrays carry one pad word per 16 so the strided radix writes do not
-//     collide in banks;
-//   * three HBM passes: (1) forward row FFTs, two rows per CTA; (2) per group
-//     of four columns: forward column FFT, multiply by the kernel spectrum,
-//     inverse column FFT, all in one shared-memory residency; (3) inverse row
-//     FFTs writing the cropped W x H planes.
+//   * image and kernel are real: two rows of a plane make one complex row
+//     transform, whose Hermitian parts are the two rows' spectra, so only
+//     Q / 2 + 1 columns exist;
+//   * Stockham FFTs with large radices held in registers (16, 8, 4, 2 and 9,
+//     3), 16 elements per thread and one shared-memory buffer per transform
+//     (gl_fft.cuh);
+//   * three passes: (1) forward row FFTs of two row pairs per CTA, split into
+//     the rows' half spectra; (2) per two columns: forward FFT, times the
+//     kernel spectrum, inverse FFT.  The inverse takes the radices in the
+//     opposite order, so the product stays in the registers that the last
+//     forward butterfly left it in; (3) the row pairs' spectra rebuilt, inverse
+//     row FFTs, the cropped W x H planes written from registers.
 // The kernel spectrum (normalisation 1/(PQ) folded in) is built once per plan
 // and stays resident.
+// 2048^2 x 3 (*) 257^2: 0.325 -> 0.160 ms (two planes packed in one complex
+// transform, the third alone, ping-pong buffers, 18 warps per SM before); the
+// passes take 47, 73 and 45 us cold, issue slots half busy: bound by instruction
+// issue and fetch (each CTA runs a long straight line of code once), not by HBM
+// (15%) or shared memory (40%).
 #include "gl_internal.h"
 #include "gl_fft.cuh"
 
@@ -35,207 +41,293 @@
 namespace gl {
 namespace {
 
-// HBM layout of the intermediate ("column-group tiles"): complex element
-// (row r, column q) of channel pair p at ((p * G + q / 4) * rows + r) * 4 + q % 4,
-// G = ceil(Q / 4).  A column group (4 columns x all rows) is one contiguous
-// block, so the column pass streams it with coalesced 16-byte accesses; the
-// row passes touch 32-byte pieces (4 complex) per group, whole DRAM sectors.
-__device__ __forceinline__ size_t tile_index(int pair, int G, int rows, int r, int q)
+// HBM layout of the intermediate: column pairs.  Half spectrum (row r, column
+// q <= Q / 2) of plane p at ((p G + q / 2) rows + r) 2 + q % 2, G = pairs of
+// columns, rows even.  A column pair is one contiguous block for the column
+// pass; a row pair's piece of it is one 32-byte sector for the row passes, and
+// the pieces of a CTA's row pairs are neighbours.
+__device__ __forceinline__ size_t pair_index(int plane, int G, int rows, int g, int r)
 {
-    return (((size_t)pair * G + (q >> 2)) * rows + r) * 4 + (q & 3);
+    return (((size_t)plane * G + g) * rows + r) * 2;
 }
 
-constexpr int kRowsPerCta = 2;
-constexpr int kRowLoads = 8;   // per-thread loads in flight per row pass
+constexpr int kPairs = 2;          // row pairs per CTA in the row passes
+constexpr int kColsPerCta = 2;     // one column pair per CTA in the column pass
+constexpr int kConvThreads = 384;  // 3072 points, two transforms of them, 16 elements per thread
+// Ping-pong stages (gl_fft.cuh) up to this length, in place above.  Three
+// planes, ping-pong against in place: 162 x 486 points 20.7 / 39.1 us (the
+// first is the call's own time), 512 x 729 30.9 / 37.0, 972 x 972 55.4 / 51.3,
+// 2304 x 2304 175 / 161.
+constexpr int kShort = 800;
 
-// Pass 1: forward row FFTs, two rows per CTA (rows 2b, 2b+1; blockIdx.y =
-// packed pair: 0 = in0 + i in1, 1 = in2).  An optional second layer is summed
-// in on load (flare composite = ghosts + starburst).  Rows of width W,
-// zero-padded to Q, written as column-group tiles of `rows` rows.
-__global__ void __launch_bounds__(1024) conv_rows_fwd(const float* __restrict__ in0, const float* __restrict__ in1,
-                              const float* __restrict__ in2, const float* __restrict__ add0,
-                              const float* __restrict__ add1, const float* __restrict__ add2, int W, int rows,
-                              float2* __restrict__ buf, FftDims dq, const float2* __restrict__ tw)
+struct ConvPlanes {
+    const float* in[3];
+    const float* add[3];           // a second layer summed in on load, or null
+    float* out[3];
+};
+
+// Input of pass 1: rows row0 + 2 s and the next as one complex row.
+struct RowLoad {
+    const float* in;
+    const float* add;
+    int W, H, row0;
+    __device__ __forceinline__ float2 operator()(int s, int i) const
+    {
+        const int r = row0 + 2 * s;
+        float2 z = make_float2(0.0f, 0.0f);
+        if (i < W)
+        {
+            const size_t o = (size_t)r * W + i;
+            if (r < H) z.x = in[o];
+            if (r + 1 < H) z.y = in[o + W];
+            if (add)
+            {
+                if (r < H) z.x += add[o];
+                if (r + 1 < H) z.y += add[o + W];
+            }
+        }
+        return z;
+    }
+};
+
+// Output of pass 3: real part -> row row0 + 2 s, imaginary part -> the next.
+struct RowStore {
+    float* out;
+    int W, H, row0;
+    __device__ __forceinline__ void operator()(int s, int i, float2 v) const
+    {
+        if (i >= W) return;
+        const int r = row0 + 2 * s;
+        const size_t o = (size_t)r * W + i;
+        if (r < H) out[o] = v.x;
+        if (r + 1 < H) out[o + W] = v.y;
+    }
+};
+
+// A column pair: rows at and past `rows` are zero, and not written.
+struct ColLoad {
+    const float2* base;
+    int rows;
+    __device__ __forceinline__ float2 operator()(int s, int r) const
+    {
+        return r < rows ? base[2 * (size_t)r + s] : make_float2(0.0f, 0.0f);
+    }
+};
+struct ColStore {
+    float2* base;
+    int rows;
+    __device__ __forceinline__ void operator()(int s, int r, float2 v) const
+    {
+        if (r < rows) base[2 * (size_t)r + s] = v;
+    }
+};
+struct ColMul {
+    const float2* k;
+    __device__ __forceinline__ float2 operator()(int s, int r, float2 v) const { return cmul(v, __ldg(k + 2 * (size_t)r + s)); }
+};
+
+// Pass 1: plane blockIdx.y, row pairs blockIdx.x kPairs + s.  Rows of width W,
+// zero-padded to Q.
+template <bool PP>
+__global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_rows_fwd(const __grid_constant__ ConvPlanes A, int W, int H, int rows, int G,
+                                                                float2* __restrict__ buf, const __grid_constant__ FftDims d,
+                                                                const float2* __restrict__ tw)
 {
     extern __shared__ float2 sm[];
-    const int Q = dq.n, G = (Q + 3) >> 2;
     float2* x = sm;
-    float2* y = sm + padded((size_t)Q * kRowsPerCta);
-    const int pair = blockIdx.y;
-    const int row0 = blockIdx.x * kRowsPerCta;
-    const float* re = pair == 0 ? in0 : in2;
-    const float* im = pair == 0 ? in1 : nullptr;
-    const float* are = pair == 0 ? add0 : add2;
-    const float* aim = pair == 0 ? add1 : nullptr;
-    const int total = Q * kRowsPerCta;
-    for (int e0 = 0; e0 < total; e0 += blockDim.x * kRowLoads)
+    float2* y = PP ? sm + kPairs * padded((size_t)d.n) : sm;
+    const int Q = d.n, row0 = blockIdx.x * 2 * kPairs;
+    const RowLoad load{A.in[blockIdx.y], A.add[blockIdx.y], W, H, row0};
+    if (d.nrad == 0)
     {
-        float a[kRowLoads], b[kRowLoads];
-        #pragma unroll
-        for (int u = 0; u < kRowLoads; ++u)
-        {
-            const int e = e0 + u * blockDim.x + threadIdx.x;
-            const int rr = e / Q, i = e - rr * Q;
-            const int row = row0 + rr;
-            a[u] = 0.0f; b[u] = 0.0f;
-            if (e < total && i < W && row < rows)
-            {
-                const size_t o = (size_t)row * W + i;
-                a[u] = re[o];
-                if (are) a[u] += are[o];
-                if (im) b[u] = im[o];
-                if (aim) b[u] += aim[o];
-            }
-        }
-        #pragma unroll
-        for (int u = 0; u < kRowLoads; ++u)
-        {
-            const int e = e0 + u * blockDim.x + threadIdx.x;
-            if (e < total)
-            {
-                const int rr = e / Q, i = e - rr * Q;
-                x[pad(i * kRowsPerCta + rr)] = make_float2(a[u], b[u]);
-            }
-        }
+        if (threadIdx.x < kPairs) x[fft_slot<kPairs, false>(0, threadIdx.x, Q)] = load(threadIdx.x, 0);
+        __syncthreads();
     }
-    __syncthreads();
-    const float2* r = stockham<kRowsPerCta>(x, y, dq, tw, false);
-    // two complex of one row per thread -> one 16-byte store into the tile
-    const int half = (Q + 1) / 2;
-    for (int h = threadIdx.x; h < half * kRowsPerCta; h += blockDim.x)
+    else
+        fft_any<kPairs, false, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
+    for (int st = 1; st < d.nrad; ++st) fft_any<kPairs, false, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    // Z = FFT(a + i b): FFT(a)[q] = (Z[q] + conj Z[Q - q]) / 2, FFT(b)[q] = (Z[q] - conj Z[Q - q]) / 2i;
+    // the pairs of one column pair are neighbouring sectors, so they go to neighbouring threads
+    for (int t = threadIdx.x; t < G * kPairs; t += blockDim.x)
     {
-        const int rr = h / half, q = 2 * (h - rr * half);
-        const int row = row0 + rr;
-        if (row >= rows) continue;
-        const float2 v0 = r[pad(q * kRowsPerCta + rr)];
-        const float2 v1 = (q + 1 < Q) ? r[pad((q + 1) * kRowsPerCta + rr)] : make_float2(0.0f, 0.0f);
-        *reinterpret_cast<float4*>(buf + tile_index(pair, G, rows, row, q)) = make_float4(v0.x, v0.y, v1.x, v1.y);
+        const int g = t / kPairs, s = t % kPairs, r = row0 + 2 * s;
+        if (r >= rows) continue;
+        float2 a[2], b[2];
+        #pragma unroll
+        for (int c = 0; c < 2; ++c)
+        {
+            const int q = 2 * g + c;
+            a[c] = b[c] = make_float2(0.0f, 0.0f);
+            if (q <= Q / 2)
+            {
+                const float2 z = x[fft_slot<kPairs, false>(q, s, Q)], w = x[fft_slot<kPairs, false>(q == 0 ? 0 : Q - q, s, Q)];
+                a[c] = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
+                b[c] = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
+            }
+        }
+        float4* o = reinterpret_cast<float4*>(buf + pair_index(blockIdx.y, G, rows, g, r));
+        o[0] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
+        o[1] = make_float4(b[0].x, b[0].y, b[1].x, b[1].y);
     }
 }
 
-constexpr int kColGroup = 4;      // columns per tile group in the HBM layout
-constexpr int kColsPerCta = 2;    // columns per CTA: half a group, so two CTAs fit an SM
-
-// Pass 2: two columns (half a tile group) per CTA: forward column FFT over P
-// rows (rows >= rows_in are zero), times the kernel spectrum, inverse column
-// FFT; rows [0, rows_out) back in place.  mode 1 (kernel-spectrum setup):
-// forward only, result for all P rows.  The two halves of a group are
-// neighbouring CTAs, so each 32-byte sector they share is read from DRAM once.
-__global__ void __launch_bounds__(1024) conv_cols(float2* __restrict__ buf, const float2* __restrict__ khat,
-                                                  int rows_in, int rows_out, FftDims dp, int Q, int mode,
-                                                  const float2* __restrict__ tw)
+// The middle of a column: last forward stage, times the kernel spectrum, first
+// inverse stage, all on the same registers (that stage's outputs j + p m are
+// the inputs of the inverse's first stage of the same radix).
+template <int R, class MUL>
+__device__ __forceinline__ void conv_turn(float2 (&v)[R], int it, const FftStage& d, const MUL& mul)
 {
-    extern __shared__ float2 sm[];
-    const int P = dp.n, G = (Q + 3) >> 2;
-    float2* x = sm;
-    float2* y = sm + padded((size_t)P * kColsPerCta);
-    const int g = blockIdx.x >> 1, hcol = (blockIdx.x & 1) * kColsPerCta;
-    float2* base = buf + ((size_t)blockIdx.y * G + g) * rows_in * kColGroup;
-    const int valid = max(0, min(kColsPerCta, Q - g * kColGroup - hcol));
-    if (valid == 0) return;
+    const int m = d.n / R, s = it % kColsPerCta, j = it / kColsPerCta;
+    #pragma unroll
+    for (int p = 0; p < R; ++p) v[p] = mul(s, j + p * m, v[p]);
+    dft<R>(v, 1.0f);
+}
+
+template <int R, bool PP, bool FIRST, bool LAST, class LD, class MUL, class ST>
+__device__ __forceinline__ void conv_middle(const float2* x, float2* y, const FftStage& d, const LD& ld, const MUL& mul,
+                                            const ST& st)
+{
+    constexpr int NB = kColsPerCta;
+    const int items = d.n / R * NB;
+    FftStage back = d;
+    back.Ls = 1;                       // the first stage of the way back
+    if (PP)
     {
-        constexpr int U = 8;
-        for (int r0 = 0; r0 < P; r0 += blockDim.x * U)
+        for (int it = threadIdx.x; it < items; it += blockDim.x)
         {
-            float4 v[U];
-            #pragma unroll
-            for (int u = 0; u < U; ++u)
-            {
-                const int r = r0 + u * blockDim.x + threadIdx.x;
-                v[u] = r < rows_in ? *reinterpret_cast<const float4*>(base + (size_t)r * kColGroup + hcol)
-                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-            #pragma unroll
-            for (int u = 0; u < U; ++u)
-            {
-                const int r = r0 + u * blockDim.x + threadIdx.x;
-                if (r < P)
-                {
-                    x[pad(2 * r)] = make_float2(v[u].x, v[u].y);
-                    x[pad(2 * r + 1)] = valid > 1 ? make_float2(v[u].z, v[u].w) : make_float2(0.0f, 0.0f);
-                }
-            }
+            float2 v[R];
+            fft_take<R, NB, true, false, FIRST>(v, x, it, d, ld);
+            conv_turn<R>(v, it, d, mul);
+            fft_put<R, NB, true, LAST>(v, y, it, back, st);
         }
     }
-    __syncthreads();
-    float2* f = stockham<kColsPerCta>(x, y, dp, tw, false);
-    float2* other = (f == x) ? y : x;
-    if (mode == 1)
+    else
     {
-        for (int r = threadIdx.x; r < P; r += blockDim.x)
+        constexpr int I = (16 + R - 1) / R;
+        float2 v[I][R] = {};
+        #pragma unroll
+        for (int u = 0; u < I; ++u)
         {
-            const float2 a = f[pad(2 * r)], b = f[pad(2 * r + 1)];
-            *reinterpret_cast<float4*>(base + (size_t)r * kColGroup + hcol) = make_float4(a.x, a.y, b.x, b.y);
+            const int it = threadIdx.x + u * blockDim.x;
+            if (it >= items) continue;
+            fft_take<R, NB, true, false, FIRST>(v[u], x, it, d, ld);
+            conv_turn<R>(v[u], it, d, mul);
         }
+        if (!FIRST) __syncthreads();
+        #pragma unroll
+        for (int u = 0; u < I; ++u)
+        {
+            const int it = threadIdx.x + u * blockDim.x;
+            if (it < items) fft_put<R, NB, true, LAST>(v[u], y, it, back, st);
+        }
+    }
+    if (!LAST) __syncthreads();
+}
+
+template <bool PP, bool FIRST, bool LAST, class LD, class MUL, class ST>
+__device__ __forceinline__ void conv_middle_any(float2*& x, float2*& y, const FftDims& d, const float2* __restrict__ tws,
+                                                const LD& ld, const MUL& mul, const ST& st)
+{
+    const FftStage f = fft_stage_of(d, d.nrad - 1, tws);
+    switch (d.rad[d.nrad - 1])
+    {
+    case 16: conv_middle<16, PP, FIRST, LAST>(x, y, f, ld, mul, st); break;
+    case 9: conv_middle<9, PP, FIRST, LAST>(x, y, f, ld, mul, st); break;
+    case 8: conv_middle<8, PP, FIRST, LAST>(x, y, f, ld, mul, st); break;
+    case 4: conv_middle<4, PP, FIRST, LAST>(x, y, f, ld, mul, st); break;
+    case 3: conv_middle<3, PP, FIRST, LAST>(x, y, f, ld, mul, st); break;
+    default: conv_middle<2, PP, FIRST, LAST>(x, y, f, ld, mul, st); break;
+    }
+    float2* t = x;
+    x = y;
+    y = t;
+}
+
+// Pass 2: column pair blockIdx.x of plane blockIdx.y: forward FFT over P rows
+// (rows >= rows_in are zero), times the kernel spectrum, inverse FFT; rows
+// [0, rows_in) back in place.  SETUP (kernel spectrum): forward only, all P rows.
+template <bool SETUP, bool PP>
+__global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_cols(float2* __restrict__ buf, const float2* __restrict__ khat,
+                                                            int rows_in, int rows, int k_rows, int G, const __grid_constant__ FftDims d,
+                                                            const __grid_constant__ FftDims di,
+                                                            const float2* __restrict__ tw, const float2* __restrict__ twi)
+{
+    extern __shared__ float2 sm[];
+    float2* x = sm;
+    float2* y = PP ? sm + padded((size_t)d.n * kColsPerCta) : sm;
+    const int g = blockIdx.x;
+    float2* base = buf + pair_index(blockIdx.y, G, rows, g, 0);
+    const ColLoad load{base, rows_in};
+    const ColStore store{base, rows_in};
+    if (SETUP)
+    {
+        if (d.nrad < 2)
+        {
+            if (d.nrad == 1) fft_any<2, true, false, PP, true, true>(x, y, d, 0, tw, load, store);
+            return;                                    // one point: its own transform
+        }
+        fft_any<2, true, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
+        for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+        fft_any<2, true, false, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
         return;
     }
-    const float2* kb = khat + (size_t)g * P * kColGroup + hcol;
-    for (int r = threadIdx.x; r < P; r += blockDim.x)
+    const ColMul mul{khat + pair_index(0, G, k_rows, g, 0)};
+    if (d.nrad < 2)
     {
-        const float4 k = __ldg(reinterpret_cast<const float4*>(kb + (size_t)r * kColGroup));
-        f[pad(2 * r)] = cmul(f[pad(2 * r)], make_float2(k.x, k.y));
-        f[pad(2 * r + 1)] = cmul(f[pad(2 * r + 1)], make_float2(k.z, k.w));
+        if (d.nrad == 1) conv_middle_any<PP, true, true>(x, y, d, tw, load, mul, store);
+        else if (threadIdx.x < 2) store(threadIdx.x, 0, mul(threadIdx.x, 0, load(threadIdx.x, 0)));
+        return;
     }
-    __syncthreads();
-    const float2* res = stockham<kColsPerCta>(f, other, dp, tw, true);
-    for (int r = threadIdx.x; r < rows_out; r += blockDim.x)
-    {
-        const float2 a = res[pad(2 * r)], b = res[pad(2 * r + 1)];
-        *reinterpret_cast<float4*>(base + (size_t)r * kColGroup + hcol) = make_float4(a.x, a.y, b.x, b.y);
-    }
+    fft_any<2, true, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
+    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    conv_middle_any<PP, false, false>(x, y, d, tw, FftNone{}, mul, FftNone{});
+    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, true, PP, false, false>(x, y, di, st, twi, FftNone{}, FftNone{});
+    fft_any<2, true, true, PP, false, true>(x, y, di, d.nrad - 1, twi, FftNone{}, store);
 }
 
-// Pass 3: inverse row FFTs from the tiles, two rows per CTA; real part ->
-// out0 (pair 0) / out2 (pair 1), imaginary part -> out1 (pair 0).  Crop to W.
-__global__ void __launch_bounds__(1024) conv_rows_inv(const float2* __restrict__ buf, int W, int H, float* __restrict__ out0,
-                              float* __restrict__ out1, float* __restrict__ out2, FftDims dq,
-                              const float2* __restrict__ tw)
+// Pass 3: the row pairs' transforms Z = FFT(a) + i FFT(b) from the half
+// spectra, inverse FFT, real part -> row r, imaginary part -> row r + 1.
+template <bool PP>
+__global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_rows_inv(const float2* __restrict__ buf, const __grid_constant__ ConvPlanes A, int W,
+                                                                int H, int rows, int G, const __grid_constant__ FftDims d,
+                                                                const float2* __restrict__ tw)
 {
     extern __shared__ float2 sm[];
-    const int Q = dq.n, G = (Q + 3) >> 2;
     float2* x = sm;
-    float2* y = sm + padded((size_t)Q * kRowsPerCta);
-    const int pair = blockIdx.y;
-    const int row0 = blockIdx.x * kRowsPerCta;
-    const int half = (Q + 1) / 2;
-    const int total = half * kRowsPerCta;
-    constexpr int U = 6;
-    for (int h0 = 0; h0 < total; h0 += blockDim.x * U)
+    float2* y = PP ? sm + kPairs * padded((size_t)d.n) : sm;
+    const int Q = d.n, row0 = blockIdx.x * 2 * kPairs;
+    float* out = A.out[blockIdx.y];
+    for (int t = threadIdx.x; t < G * kPairs; t += blockDim.x)
     {
-        float4 v[U];
-        #pragma unroll
-        for (int u = 0; u < U; ++u)
+        const int g = t / kPairs, s = t % kPairs, r = row0 + 2 * s;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+        if (r < rows)
         {
-            const int h = h0 + u * blockDim.x + threadIdx.x;
-            const int rr = h / half, q = 2 * (h - rr * half);
-            const int row = row0 + rr;
-            v[u] = (h < total && row < H) ? __ldg(reinterpret_cast<const float4*>(buf + tile_index(pair, G, H, row, q)))
-                                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4* p = reinterpret_cast<const float4*>(buf + pair_index(blockIdx.y, G, rows, g, r));
+            a = __ldg(p);
+            b = __ldg(p + 1);
         }
         #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int c = 0; c < 2; ++c)
         {
-            const int h = h0 + u * blockDim.x + threadIdx.x;
-            if (h < total)
-            {
-                const int rr = h / half, q = 2 * (h - rr * half);
-                x[pad(q * kRowsPerCta + rr)] = make_float2(v[u].x, v[u].y);
-                if (q + 1 < Q) x[pad((q + 1) * kRowsPerCta + rr)] = make_float2(v[u].z, v[u].w);
-            }
+            const int q = 2 * g + c;
+            if (q > Q / 2) continue;
+            const float2 u = c ? make_float2(a.z, a.w) : make_float2(a.x, a.y);
+            const float2 w = c ? make_float2(b.z, b.w) : make_float2(b.x, b.y);
+            x[fft_slot<kPairs, false>(q, s, Q)] = make_float2(u.x - w.y, u.y + w.x);
+            // conj U + i conj W at Q - q; the middle of an even Q is its own mirror
+            if (q > 0 && 2 * q != Q) x[fft_slot<kPairs, false>(Q - q, s, Q)] = make_float2(u.x + w.y, w.x - u.y);
         }
     }
     __syncthreads();
-    const float2* r = stockham<kRowsPerCta>(x, y, dq, tw, true);
-    for (int e = threadIdx.x; e < W * kRowsPerCta; e += blockDim.x)
+    const RowStore store{out, W, H, row0};
+    if (d.nrad == 0)
     {
-        const int rr = e / W, i = e - rr * W;
-        const int row = row0 + rr;
-        if (row >= H) continue;
-        const float2 v = r[pad(i * kRowsPerCta + rr)];
-        const size_t o = (size_t)row * W + i;
-        if (pair == 0) { out0[o] = v.x; out1[o] = v.y; }
-        else out2[o] = v.x;
+        if (threadIdx.x < kPairs) store(threadIdx.x, 0, x[fft_slot<kPairs, false>(0, threadIdx.x, Q)]);
+        return;
     }
+    for (int st = 0; st + 1 < d.nrad; ++st) fft_any<kPairs, false, true, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    fft_any<kPairs, false, true, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
 }
 
 int good_size(int need)
@@ -253,13 +345,17 @@ int good_size(int need)
 }  // namespace
 
 struct ConvPlan {
-    int W = 0, H = 0, KW = 0, KH = 0, P = 0, Q = 0, G = 0;
-    float2* khat = nullptr;   // column-group tiles, P rows
-    float2* buf = nullptr;    // column-group tiles, 2 pairs x H rows
-    float2* tw_p = nullptr;   // twiddles for P (== tw_q when P == Q)
-    float2* tw_q = nullptr;
+    int W = 0, H = 0, KW = 0, KH = 0, P = 0, Q = 0;
+    int G = 0, rows = 0, k_rows = 0;  // column pairs, rows of the intermediate and of the kernel spectrum (even)
+    float2* khat = nullptr;   // column pairs, k_rows rows
+    float2* buf = nullptr;    // column pairs, 3 planes x rows
+    float2* tw_q = nullptr;   // stage twiddles: rows, columns, columns in the opposite order
+    float2* tw_p = nullptr;
+    float2* tw_pi = nullptr;
+    FftDims dq{}, dp{}, dpi{};
     size_t smem_row = 0, smem_col = 0;
     int thr_row = 0, thr_col = 0;
+    bool pp_row = false, pp_col = false;      // ping-pong stages
 };
 
 }  // namespace gl
@@ -272,9 +368,28 @@ static void conv_free(ConvPlan* p)
 {
     cudaFree(p->khat);
     cudaFree(p->buf);
-    if (p->tw_p != p->tw_q) cudaFree(p->tw_p);
     cudaFree(p->tw_q);
+    cudaFree(p->tw_p);
+    cudaFree(p->tw_pi);
     delete p;
+}
+
+// Passes 1 and 2 over `planes` planes of `rows` intermediate rows.
+static void conv_fwd(const ConvPlan* p, const ConvPlanes& A, int planes, int W, int H, int rows, float2* buf, cudaStream_t st)
+{
+    const dim3 rb((unsigned)((rows + 2 * kPairs - 1) / (2 * kPairs)), planes);
+    if (p->pp_row) conv_rows_fwd<true><<<rb, p->thr_row, p->smem_row, st>>>(A, W, H, rows, p->G, buf, p->dq, p->tw_q);
+    else conv_rows_fwd<false><<<rb, p->thr_row, p->smem_row, st>>>(A, W, H, rows, p->G, buf, p->dq, p->tw_q);
+}
+
+template <bool SETUP>
+static void conv_mid(const ConvPlan* p, int planes, float2* buf, const float2* khat, int rows_in, int rows, cudaStream_t st)
+{
+    const dim3 cb(p->G, planes);
+    if (p->pp_col)
+        conv_cols<SETUP, true><<<cb, p->thr_col, p->smem_col, st>>>(buf, khat, rows_in, rows, p->k_rows, p->G, p->dp, p->dpi, p->tw_p, p->tw_pi);
+    else
+        conv_cols<SETUP, false><<<cb, p->thr_col, p->smem_col, st>>>(buf, khat, rows_in, rows, p->k_rows, p->G, p->dp, p->dpi, p->tw_p, p->tw_pi);
 }
 
 extern "C" int gl_conv2d_plan_create(int width, int height, const float* h_kernel, int kw, int kh, void* stream,
@@ -287,31 +402,23 @@ extern "C" int gl_conv2d_plan_create(int width, int height, const float* h_kerne
     p->W = width; p->H = height; p->KW = kw; p->KH = kh;
     p->Q = good_size(width + kw - 1);
     p->P = good_size(height + kh - 1);
-    p->G = (p->Q + 3) / 4;
     if (p->P > 3072 || p->Q > 3072)
     {
         delete p;
         return fail(GL_ERR_INVALID, "conv2d_plan_create: padded transform above 3072 points per axis");
     }
-    p->smem_row = 2 * padded((size_t)p->Q * kRowsPerCta) * sizeof(float2);
-    p->smem_col = 2 * padded((size_t)p->P * kColsPerCta) * sizeof(float2);
-    {
-        // one thread per butterfly of the largest-radix stage
-        const FftDims dq = make_dims(p->Q), dp = make_dims(p->P);
-        auto threads = [](const FftDims& d, int nb) {
-            int rmax = 2;
-            for (int i = 0; i < d.nrad; ++i) rmax = std::max(rmax, d.rad[i]);
-            const int t = (d.n * nb / rmax + 31) / 32 * 32;
-            return std::min(1024, std::max(64, t));
-        };
-        p->thr_row = threads(dq, kRowsPerCta);
-        p->thr_col = threads(dp, kColsPerCta);
-    }
-    if (p->smem_col > 227 * 1024 || p->smem_row > 227 * 1024)
-    {
-        delete p;
-        return fail(GL_ERR_INVALID, "conv2d_plan_create: transform too large for one shared-memory residency");
-    }
+    p->G = (p->Q / 2 + 1 + 1) / 2;
+    p->rows = (p->H + 1) / 2 * 2;
+    p->k_rows = (p->P + 1) / 2 * 2;
+    p->dq = make_dims(p->Q);
+    p->dp = make_dims(p->P);
+    p->dpi = reversed(p->dp);
+    p->pp_row = p->Q <= kShort;
+    p->pp_col = p->P <= kShort;
+    p->smem_row = (p->pp_row ? 2 : 1) * kPairs * padded((size_t)p->Q) * sizeof(float2);
+    p->smem_col = (p->pp_col ? 2 : 1) * padded((size_t)p->P * kColsPerCta) * sizeof(float2);
+    p->thr_row = fft_threads(p->Q, kPairs, p->pp_row);
+    p->thr_col = fft_threads(p->P, kColsPerCta, p->pp_col);
     cudaStream_t st = (cudaStream_t)stream;
     // Kernel placed with its centre at the origin, wrapped (so the circular
     // convolution lands 'same'-aligned), as a P x Q real plane, 1/(PQ) folded in.
@@ -324,35 +431,33 @@ extern "C" int gl_conv2d_plan_create(int width, int height, const float* h_kerne
             const int yy = ((u - cy) % p->P + p->P) % p->P, xx = ((v - cx) % p->Q + p->Q) % p->Q;
             kplane[(size_t)yy * p->Q + xx] = h_kernel[(size_t)u * kw + v] * norm;
         }
-    const std::vector<float2> twq = twiddles(p->Q);
-    const std::vector<float2> twp = p->P == p->Q ? std::vector<float2>() : twiddles(p->P);
+    const std::vector<float2> twq = stage_twiddles(p->dq), twp = stage_twiddles(p->dp), twi = stage_twiddles(p->dpi);
     float* kdev = nullptr;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-    chk(cudaMalloc(&p->khat, sizeof(float2) * (size_t)p->G * 4 * p->P));
-    chk(cudaMalloc(&p->buf, sizeof(float2) * 2 * (size_t)p->G * 4 * p->H));
-    chk(cudaMalloc(&p->tw_q, sizeof(float2) * (size_t)p->Q));
-    if (p->P != p->Q) chk(cudaMalloc(&p->tw_p, sizeof(float2) * (size_t)p->P));
-    else p->tw_p = p->tw_q;
+    chk(cudaMalloc(&p->khat, sizeof(float2) * 2 * (size_t)p->G * p->k_rows));
+    chk(cudaMalloc(&p->buf, sizeof(float2) * 3 * 2 * (size_t)p->G * p->rows));
+    chk(cudaMalloc(&p->tw_q, sizeof(float2) * twq.size()));
+    chk(cudaMalloc(&p->tw_p, sizeof(float2) * twp.size()));
+    chk(cudaMalloc(&p->tw_pi, sizeof(float2) * twi.size()));
     chk(cudaMalloc(&kdev, sizeof(float) * kplane.size()));
-    chk((cudaError_t)raise_smem_limit((const void*)conv_cols, p->smem_col));
-    chk((cudaError_t)raise_smem_limit((const void*)conv_rows_fwd, p->smem_row));
-    chk((cudaError_t)raise_smem_limit((const void*)conv_rows_inv, p->smem_row));
+    chk((cudaError_t)raise_smem_limit(p->pp_col ? (const void*)conv_cols<false, true> : (const void*)conv_cols<false, false>, p->smem_col));
+    chk((cudaError_t)raise_smem_limit(p->pp_col ? (const void*)conv_cols<true, true> : (const void*)conv_cols<true, false>, p->smem_col));
+    chk((cudaError_t)raise_smem_limit(p->pp_row ? (const void*)conv_rows_fwd<true> : (const void*)conv_rows_fwd<false>, p->smem_row));
+    chk((cudaError_t)raise_smem_limit(p->pp_row ? (const void*)conv_rows_inv<true> : (const void*)conv_rows_inv<false>, p->smem_row));
     if (e == cudaSuccess)
     {
         chk(cudaMemcpyAsync(p->tw_q, twq.data(), sizeof(float2) * twq.size(), cudaMemcpyHostToDevice, st));
-        if (p->P != p->Q)
-            chk(cudaMemcpyAsync(p->tw_p, twp.data(), sizeof(float2) * twp.size(), cudaMemcpyHostToDevice, st));
+        chk(cudaMemcpyAsync(p->tw_p, twp.data(), sizeof(float2) * twp.size(), cudaMemcpyHostToDevice, st));
+        chk(cudaMemcpyAsync(p->tw_pi, twi.data(), sizeof(float2) * twi.size(), cudaMemcpyHostToDevice, st));
         chk(cudaMemcpyAsync(kdev, kplane.data(), sizeof(float) * kplane.size(), cudaMemcpyHostToDevice, st));
-        const FftDims dq = make_dims(p->Q), dp = make_dims(p->P);
         if (e == cudaSuccess)
         {
-            // kernel spectrum: row FFTs of the real plane into tiles, then forward column FFTs in place
-            conv_rows_fwd<<<dim3((p->P + kRowsPerCta - 1) / kRowsPerCta, 1), p->thr_row, p->smem_row, st>>>(kdev, nullptr, nullptr, nullptr, nullptr,
-                                                                            nullptr, p->Q, p->P, p->khat, dq,
-                                                                            p->tw_q);
-            conv_cols<<<dim3(2 * p->G, 1), p->thr_col, p->smem_col, st>>>(p->khat, nullptr, p->P, p->P, dp, p->Q, 1,
-                                                                       p->tw_p);
+            // kernel spectrum: row FFTs of the real plane, then forward column FFTs in place
+            ConvPlanes K{};
+            K.in[0] = kdev;
+            conv_fwd(p, K, 1, p->Q, p->P, p->k_rows, p->khat, st);
+            conv_mid<true>(p, 1, p->khat, nullptr, p->P, p->k_rows, st);
             chk(cudaGetLastError());
         }
         chk(cudaStreamSynchronize(st));
@@ -378,13 +483,12 @@ extern "C" int gl_conv2d_plan_execute2(gl_conv_plan* plan, const float* d_in_r, 
         return fail(GL_ERR_INVALID, "conv2d_plan_execute: the added layer needs all three planes or none");
     ConvPlan* p = plan->p;
     cudaStream_t st = (cudaStream_t)stream;
-    const FftDims dq = make_dims(p->Q), dp = make_dims(p->P);
-    const unsigned rb = (unsigned)((p->H + kRowsPerCta - 1) / kRowsPerCta);
-    conv_rows_fwd<<<dim3(rb, 2), p->thr_row, p->smem_row, st>>>(d_in_r, d_in_g, d_in_b, d_add_r, d_add_g, d_add_b,
-                                                                    p->W, p->H, p->buf, dq, p->tw_q);
-    conv_cols<<<dim3(2 * p->G, 2), p->thr_col, p->smem_col, st>>>(p->buf, p->khat, p->H, p->H, dp, p->Q, 0, p->tw_p);
-    conv_rows_inv<<<dim3(rb, 2), p->thr_row, p->smem_row, st>>>(p->buf, p->W, p->H, d_out_r, d_out_g, d_out_b, dq,
-                                                                    p->tw_q);
+    const ConvPlanes A{{d_in_r, d_in_g, d_in_b}, {d_add_r, d_add_g, d_add_b}, {d_out_r, d_out_g, d_out_b}};
+    conv_fwd(p, A, 3, p->W, p->H, p->rows, p->buf, st);
+    conv_mid<false>(p, 3, p->buf, p->khat, p->H, p->rows, st);
+    const dim3 rb((unsigned)((p->rows + 2 * kPairs - 1) / (2 * kPairs)), 3);
+    if (p->pp_row) conv_rows_inv<true><<<rb, p->thr_row, p->smem_row, st>>>(p->buf, A, p->W, p->H, p->rows, p->G, p->dq, p->tw_q);
+    else conv_rows_inv<false><<<rb, p->thr_row, p->smem_row, st>>>(p->buf, A, p->W, p->H, p->rows, p->G, p->dq, p->tw_q);
     GL_CUDA_TRY(cudaGetLastError());
     g_last_launches = 3;
     return GL_OK;

@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <vector>
@@ -13,15 +14,17 @@
 namespace gl {
 
 // Radix plan of one transform length n = 2^a 3^b: per stage its radix r, the
-// span Ls of the sub-transforms done before it, ceil(2^32 / Ls) for an exact
-// division by multiply-high (indices < 2^14), and the twiddle-table stride
-// n / (Ls r).
+// span Ls of the sub-transforms done before it, ceil(2^32 / Ls) and
+// ceil(2^32 / (n / r)) for exact divisions by multiply-high (indices < 2^16),
+// the stride n / (Ls r) in a whole-circle twiddle table, and the stage's place
+// in the stage tables (stage_twiddles).
 struct FftDims {
-    int n, nrad;
-    int rad[16];
-    int ls[16];
-    uint32_t lmag[16];
-    int twstep[16];
+    int n, nrad;                       // at most five radices below 2^14
+    int rad[6];
+    int ls[6];
+    uint32_t lmag[6], mmag[6];
+    int twstep[6];
+    int twoff[7];
 };
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
@@ -217,6 +220,192 @@ __device__ float2* stockham(float2* x, float2* y, const FftDims& d, const float2
     return x;
 }
 
+// ---- stages between registers and shared memory ---------------------------------
+// Two forms.  In place (PP = false): every thread holds 16 elements (one
+// radix-16 butterfly, two of radix 8 or 9, ...), reads a stage's inputs, waits,
+// and writes the outputs to the same shared buffer: one buffer per transform
+// where ping-pong needs two, so twice the CTAs fit an SM; blockDim >= n NB / 16.
+// Ping-pong (PP = true): a loop over butterflies from one buffer to the other,
+// a fraction of the code, for short transforms, whose time is latency and
+// instruction fetch.  The first stage can read its inputs straight from global
+// memory, the last write its outputs there (both are in natural order across
+// threads).  Twiddles come from per-stage tables in the order the threads read
+// them (a whole-circle table is read with strides that take a line per lane).
+// NB sequences; INTER: element i of sequence s at pad(i NB + s), else at
+// s padded(n) + pad(i).
+template <int NB, bool INTER>
+__device__ __forceinline__ int fft_slot(int i, int s, int n)
+{
+    return INTER ? pad(i * NB + s) : s * (int)padded((size_t)n) + pad(i);
+}
+
+struct FftNone {
+    __device__ float2 operator()(int, int) const { return make_float2(0.0f, 0.0f); }
+    __device__ void operator()(int, int, float2) const {}
+};
+
+// What one stage needs of the dims.
+struct FftStage {
+    int n, Ls;
+    uint32_t lmag, mmag;
+    const float2* tw;
+};
+
+__device__ __forceinline__ FftStage fft_stage_of(const FftDims& d, int stage, const float2* tws)
+{
+    return {d.n, d.ls[stage], d.lmag[stage], d.mmag[stage], tws + d.twoff[stage]};
+}
+
+// The item `it` of a stage with m = n / R butterflies per sequence: its
+// sequence and butterfly.
+template <int NB, bool INTER>
+__device__ __forceinline__ void fft_item(int it, int m, uint32_t mmag, int& s, int& j)
+{
+    if (INTER) { s = it % NB; j = it / NB; }
+    else if (NB == 1) { s = 0; j = it; }
+    else
+    {
+        s = m > 1 ? (int)__umulhi((uint32_t)it, mmag) : it;
+        j = it - s * m;
+    }
+}
+
+// v[q] *= w^q, w = exp(-+2 pi i k / (Ls R)): the powers 1, 2, 4, 8 from the
+// table, the others as products of two or three of them (15 table reads per
+// radix-16 butterfly cost more than the extra multiplications; the transform's
+// error does not change).
+template <int R>
+__device__ __forceinline__ void fft_twiddle(float2 (&v)[R], int k, int Ls, const float2* __restrict__ tw, bool inv)
+{
+    float2 w[R];
+    #pragma unroll
+    for (int q = 1; q < R; q <<= 1)
+    {
+        w[q] = __ldg(tw + (q - 1) * Ls + k);
+        if (inv) w[q].y = -w[q].y;
+        v[q] = cmul(v[q], w[q]);
+        #pragma unroll
+        for (int r = 1; r < q; ++r)
+            if (q + r < R)
+            {
+                w[q + r] = cmul(w[q], w[r]);
+                v[q + r] = cmul(v[q + r], w[q + r]);
+            }
+    }
+}
+
+// The butterfly of item `it`: inputs from ld (FIRST) or shared memory, twiddled, transformed.
+template <int R, int NB, bool INTER, bool INV, bool FIRST, class LD>
+__device__ __forceinline__ void fft_take(float2 (&v)[R], const float2* x, int it, const FftStage& d, const LD& ld)
+{
+    const int n = d.n, m = n / R;
+    int s, j;
+    fft_item<NB, INTER>(it, m, d.mmag, s, j);
+    #pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = FIRST ? ld(s, j + q * m) : x[fft_slot<NB, INTER>(j + q * m, s, n)];
+    if (d.Ls > 1) fft_twiddle<R>(v, j - (int)__umulhi((uint32_t)j, d.lmag) * d.Ls, d.Ls, d.tw, INV);
+    dft<R>(v, INV ? 1.0f : -1.0f);
+}
+
+// Its outputs, to st (LAST) or shared memory.
+template <int R, int NB, bool INTER, bool LAST, class ST>
+__device__ __forceinline__ void fft_put(const float2 (&v)[R], float2* y, int it, const FftStage& d, const ST& st)
+{
+    const int n = d.n, m = n / R;
+    int s, j;
+    fft_item<NB, INTER>(it, m, d.mmag, s, j);
+    const int g = d.Ls > 1 ? (int)__umulhi((uint32_t)j, d.lmag) : j;
+    const int ob = g * d.Ls * R + (j - g * d.Ls);
+    #pragma unroll
+    for (int p = 0; p < R; ++p)
+    {
+        if (LAST) st(s, ob + p * d.Ls, v[p]);
+        else y[fft_slot<NB, INTER>(ob + p * d.Ls, s, n)] = v[p];
+    }
+}
+
+// One stage, x -> y (in place: the same buffer).  FIRST: inputs from ld(s, i);
+// LAST: outputs to st(s, i, value).  Ends on a barrier unless LAST.  In place,
+// the elements start as zeros: set under a condition only, they count as live
+// from the kernel's start and every radix's stage adds to the spills.
+template <int R, int NB, bool INTER, bool INV, bool PP, bool FIRST, bool LAST, class LD, class ST>
+__device__ __forceinline__ void fft_stage(const float2* x, float2* y, const FftStage& d, const LD& ld, const ST& st)
+{
+    const int items = d.n / R * NB;
+    if (PP)
+    {
+        for (int it = threadIdx.x; it < items; it += blockDim.x)
+        {
+            float2 v[R];
+            fft_take<R, NB, INTER, INV, FIRST>(v, x, it, d, ld);
+            fft_put<R, NB, INTER, LAST>(v, y, it, d, st);
+        }
+    }
+    else
+    {
+        constexpr int I = (16 + R - 1) / R;
+        float2 v[I][R] = {};
+        #pragma unroll
+        for (int u = 0; u < I; ++u)
+        {
+            const int it = threadIdx.x + u * blockDim.x;
+            if (it < items) fft_take<R, NB, INTER, INV, FIRST>(v[u], x, it, d, ld);
+        }
+        if (!FIRST) __syncthreads();
+        #pragma unroll
+        for (int u = 0; u < I; ++u)
+        {
+            const int it = threadIdx.x + u * blockDim.x;
+            if (it < items) fft_put<R, NB, INTER, LAST>(v[u], y, it, d, st);
+        }
+    }
+    if (!LAST) __syncthreads();
+}
+
+// The stage of whatever radix; leaves the result's buffer in x (in place: y == x).
+template <int NB, bool INTER, bool INV, bool PP, bool FIRST, bool LAST, class LD, class ST>
+__device__ __forceinline__ void fft_any(float2*& x, float2*& y, const FftDims& d, int stage,
+                                        const float2* __restrict__ tws, const LD& ld, const ST& st)
+{
+    const FftStage f = fft_stage_of(d, stage, tws);
+    switch (d.rad[stage])
+    {
+    case 16: fft_stage<16, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
+    case 9: fft_stage<9, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
+    case 8: fft_stage<8, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
+    case 4: fft_stage<4, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
+    case 3: fft_stage<3, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
+    default: fft_stage<2, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
+    }
+    float2* t = x;
+    x = y;
+    y = t;
+}
+
+// Threads of a CTA that holds NB transforms of n points.
+inline int fft_threads(int n, int nb, bool pp)
+{
+    return std::min(pp ? 512 : 1024, std::max(pp ? 64 : 32, pp ? (n * nb / 4 + 31) / 32 * 32 : (n * nb + 511) / 512 * 32));
+}
+
+// Spans, division constants and table places of the radices in d.
+inline void set_spans(FftDims& d)
+{
+    int Ls = 1, off = 0;
+    for (int s = 0; s < d.nrad; ++s)
+    {
+        const int m = d.n / d.rad[s];
+        d.ls[s] = Ls;
+        d.lmag[s] = Ls > 1 ? (uint32_t)((((uint64_t)1 << 32) + Ls - 1) / Ls) : 0u;
+        d.mmag[s] = m > 1 ? (uint32_t)((((uint64_t)1 << 32) + m - 1) / m) : 0u;
+        d.twstep[s] = d.n / (Ls * d.rad[s]);
+        d.twoff[s] = off;
+        if (Ls > 1) off += (d.rad[s] - 1) * Ls;
+        Ls *= d.rad[s];
+    }
+    d.twoff[d.nrad] = off;
+}
+
 inline FftDims make_dims(int n)
 {
     FftDims d{};
@@ -228,15 +417,35 @@ inline FftDims make_dims(int n)
     if (m % 2 == 0) { d.rad[d.nrad++] = 2; m /= 2; }
     while (m % 9 == 0) { d.rad[d.nrad++] = 9; m /= 9; }
     if (m % 3 == 0) { d.rad[d.nrad++] = 3; m /= 3; }
-    int Ls = 1;
+    set_spans(d);
+    return d;
+}
+
+// The same stages in the opposite order.
+inline FftDims reversed(FftDims d)
+{
+    std::reverse(d.rad, d.rad + d.nrad);
+    set_spans(d);
+    return d;
+}
+
+// Per-stage twiddles exp(-2 pi i q k / (Ls r)), entry (q - 1) Ls + k of the
+// stage's table at twoff, in double then rounded (at least one entry).
+inline std::vector<float2> stage_twiddles(const FftDims& d)
+{
+    std::vector<float2> t((size_t)std::max(1, d.twoff[d.nrad]));
+    const double pi = 3.14159265358979323846;
     for (int s = 0; s < d.nrad; ++s)
     {
-        d.ls[s] = Ls;
-        d.lmag[s] = Ls > 1 ? (uint32_t)((((uint64_t)1 << 32) + Ls - 1) / Ls) : 0u;
-        d.twstep[s] = n / (Ls * d.rad[s]);
-        Ls *= d.rad[s];
+        if (d.ls[s] == 1) continue;
+        for (int q = 1; q < d.rad[s]; ++q)
+            for (int k = 0; k < d.ls[s]; ++k)
+            {
+                const double a = 2.0 * pi * (double)(q * k) / (double)(d.ls[s] * d.rad[s]);
+                t[(size_t)d.twoff[s] + (size_t)(q - 1) * d.ls[s] + k] = make_float2((float)std::cos(a), (float)-std::sin(a));
+            }
     }
-    return d;
+    return t;
 }
 
 // exp(-2 pi i t / n), t < n, in double then rounded

@@ -6,7 +6,8 @@ outside the image) by a mixed-radix FFT route on the device: the padded
 transform sizes P, Q are the smallest 2^a 3^b >= image + kernel - 1, the kernel
 spectrum is built once per plan and stays resident, and one execute is three
 HBM passes (rows forward; columns forward x K-hat x inverse; rows inverse and
-crop).  Two colour planes share one complex transform.
+crop).  Two rows of a plane share one complex transform; the spectra are
+Hermitian halves.
 
 The reference has no image convolution on its flare path; its nearest pieces
 are the analytic veil sprite (ghostlight/src/veil_render.cu:243) and the PSF
@@ -73,11 +74,11 @@ class ConvPlan:
 
     def traffic_bytes(self) -> int:
         """HBM bytes of one execute by the three-pass schedule: planes in and
-        out, the two-pair complex intermediate written and read twice, the
-        kernel spectrum read once."""
+        out, the planes' complex half spectra written and read twice, the
+        kernel's half spectrum read once."""
         planes = 3 * self.width * self.height * 4
-        inter = 2 * self.height * self.Q * 8
-        return 2 * planes + 4 * inter + self.P * self.Q * 8
+        half = self.Q // 2 + 1
+        return 2 * planes + 4 * 3 * self.height * half * 8 + self.P * half * 8
 
     def close(self):
         if getattr(self, "_h", None):
