@@ -16,14 +16,12 @@ namespace gl {
 // Radix plan of one transform length n = 2^a 3^b: per stage its radix r, the
 // span Ls of the sub-transforms done before it, ceil(2^32 / Ls) and
 // ceil(2^32 / (n / r)) for exact divisions by multiply-high (indices < 2^16),
-// the stride n / (Ls r) in a whole-circle twiddle table, and the stage's place
-// in the stage tables (stage_twiddles).
+// and the stage's place in the stage tables (stage_twiddles).
 struct FftDims {
     int n, nrad;                       // at most five radices below 2^14
     int rad[6];
     int ls[6];
     uint32_t lmag[6], mmag[6];
-    int twstep[6];
     int twoff[7];
 };
 
@@ -157,67 +155,6 @@ __device__ __forceinline__ void dft<9>(float2 (&v)[9], float sign)
         for (int p2 = 0; p2 < 3; ++p2) x[p1 + 3 * p2] = v[3 * p1 + p2];
     #pragma unroll
     for (int i = 0; i < 9; ++i) v[i] = x[i];
-}
-
-// One Stockham stage of radix R over NB interleaved sequences (element i of
-// sequence s at logical index i * NB + s, stored at pad()), x -> y.
-template <int R, int NB>
-__device__ __forceinline__ void radix_stage(const float2* __restrict__ x, float2* __restrict__ y, int n, int Ls,
-                                            uint32_t lmag, int twstep, const float2* __restrict__ tw, bool inv)
-{
-    const int m = n / R;
-    const int items = m * NB;
-    const float sign = inv ? 1.0f : -1.0f;
-    for (int it = threadIdx.x; it < items; it += blockDim.x)
-    {
-        const int s = it % NB, j = it / NB;
-        int g = j, k = 0;
-        if (Ls > 1)
-        {
-            g = (int)__umulhi((uint32_t)j, lmag);
-            k = j - g * Ls;
-        }
-        float2 v[R];
-        #pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = x[pad((j + q * m) * NB + s)];
-        if (k > 0)
-        {
-            #pragma unroll
-            for (int q = 1; q < R; ++q)
-            {
-                float2 w = __ldg(&tw[q * k * twstep]);   // q k < R Ls: index < n
-                if (inv) w.y = -w.y;
-                v[q] = cmul(v[q], w);
-            }
-        }
-        dft<R>(v, sign);
-        const int ob = g * Ls * R + k;
-        #pragma unroll
-        for (int p = 0; p < R; ++p) y[pad((ob + p * Ls) * NB + s)] = v[p];
-    }
-}
-
-// Full transform; returns the buffer holding the result (x or y).
-template <int NB>
-__device__ float2* stockham(float2* x, float2* y, const FftDims& d, const float2* __restrict__ tw, bool inv)
-{
-    for (int st = 0; st < d.nrad; ++st)
-    {
-        const int n = d.n, L = d.ls[st], ts = d.twstep[st];
-        const uint32_t lm = d.lmag[st];
-        switch (d.rad[st])
-        {
-        case 16: radix_stage<16, NB>(x, y, n, L, lm, ts, tw, inv); break;
-        case 9: radix_stage<9, NB>(x, y, n, L, lm, ts, tw, inv); break;
-        case 8: radix_stage<8, NB>(x, y, n, L, lm, ts, tw, inv); break;
-        case 4: radix_stage<4, NB>(x, y, n, L, lm, ts, tw, inv); break;
-        case 3: radix_stage<3, NB>(x, y, n, L, lm, ts, tw, inv); break;
-        default: radix_stage<2, NB>(x, y, n, L, lm, ts, tw, inv); break;
-        }
-        __syncthreads();
-        float2* t = x; x = y; y = t;
-    }
-    return x;
 }
 
 // ---- stages between registers and shared memory ---------------------------------
@@ -398,7 +335,6 @@ inline void set_spans(FftDims& d)
         d.ls[s] = Ls;
         d.lmag[s] = Ls > 1 ? (uint32_t)((((uint64_t)1 << 32) + Ls - 1) / Ls) : 0u;
         d.mmag[s] = m > 1 ? (uint32_t)((((uint64_t)1 << 32) + m - 1) / m) : 0u;
-        d.twstep[s] = d.n / (Ls * d.rad[s]);
         d.twoff[s] = off;
         if (Ls > 1) off += (d.rad[s] - 1) * Ls;
         Ls *= d.rad[s];
@@ -444,19 +380,6 @@ inline std::vector<float2> stage_twiddles(const FftDims& d)
                 const double a = 2.0 * pi * (double)(q * k) / (double)(d.ls[s] * d.rad[s]);
                 t[(size_t)d.twoff[s] + (size_t)(q - 1) * d.ls[s] + k] = make_float2((float)std::cos(a), (float)-std::sin(a));
             }
-    }
-    return t;
-}
-
-// exp(-2 pi i t / n), t < n, in double then rounded
-inline std::vector<float2> twiddles(int n)
-{
-    std::vector<float2> t((size_t)n);
-    const double pi = 3.14159265358979323846;
-    for (int i = 0; i < n; ++i)
-    {
-        const double a = 2.0 * pi * (double)i / (double)n;
-        t[i] = make_float2((float)std::cos(a), (float)-std::sin(a));
     }
     return t;
 }

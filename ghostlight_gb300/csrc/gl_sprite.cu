@@ -11,11 +11,13 @@
 //   resample), times the source colour and the gain.
 //
 // GB300 layout (one GPU, everything resident in the plan):
-//   * 2-D FFT as two shared-memory Stockham passes (gl_fft.cuh): row FFTs,
-//     one CTA per row, skipping rows the pupil leaves dark (the pupil fills a
-//     centred disc of `fill` of the grid, so most rows are zero); column FFTs
-//     over groups of NB adjacent columns whose epilogue writes |X|^2 straight
-//     to its fftshifted place and adds the block's energy to one FP64 sum;
+//   * 2-D FFT of the real pupil as two shared-memory passes (gl_fft.cuh): (1)
+//     column transforms, two real columns per complex transform, split into
+//     their half spectra ky <= N / 2; a CTA whose columns the pupil leaves dark
+//     only says so (the pupil fills a centred disc of `fill` of the grid, so
+//     most are); (2) two rows ky per CTA over the lit columns, whose last stage
+//     writes |X|^2 straight to its fftshifted place and, the pupil being real,
+//     to the mirrored one, and adds the CTA's energy to one FP64 sum;
 //   * the wavelength bake and the ds x ds box sum fused in one kernel, so the
 //     N x N x 3 fine sprite (805 MB at N = 8192) never exists in HBM; the
 //     1 / energy normalisation is read on the device (no host round trip);
@@ -40,64 +42,140 @@ constexpr int kMaxSpriteGrid = 8192;   // a complex row pair fits the 227 KB of 
 
 struct StarSource { float px, py, r, g, b; };
 
-// columns per CTA in the column pass, so the interleaved pair of shared
-// buffers stays within 8192 complex each
-__host__ __device__ inline int col_group(int N) { return N >= 8192 ? 1 : (N >= 4096 ? 2 : 4); }
+// ---- 2-D transform of a real grid ------------------------------------------------
+// N = 2048 with a pupil of 0.3 of it: rows then columns of the full complex
+// spectrum took 28 + 110 us (139 KB of shared memory and 8 warps per CTA, one
+// CTA per SM, 16-byte pieces of each row), the half spectrum's two passes
+// 17 + 18 us.
+constexpr int kShortGrid = 1024;    // ping-pong stages up to here, in place above (gl_fft.cuh)
 
-__global__ void __launch_bounds__(kSpriteThreads) sprite_rows(const float* __restrict__ pupil, int N, FftDims d,
-                                                              const float2* __restrict__ tw, float2* __restrict__ work)
+// Half spectrum of the first pass: column x, row ky <= N / 2 at
+// ((ky / 2) N + x) 2 + ky % 2, so a pair of rows is one contiguous block.
+__device__ __forceinline__ size_t half_index(int N, int pair, int x) { return ((size_t)pair * N + x) * 2; }
+
+// Pass 1: columns 4 blockIdx.x .. + 3, two real ones per complex sequence; rows
+// ky < 2 pairs kept.  lit[blockIdx.x]
+// = 0 where all are zero (nothing is written then).
+template <bool PP>
+__global__ void __launch_bounds__(1024) grid_cols(const float* __restrict__ in, int N, int pairs,
+                                                  const __grid_constant__ FftDims d, const float2* __restrict__ tw,
+                                                  float2* __restrict__ half, unsigned char* __restrict__ lit)
 {
     extern __shared__ float2 sm[];
     float2* x = sm;
-    float2* y = sm + padded((size_t)N);
-    const int j = blockIdx.x;
-    const float* row = pupil + (size_t)j * N;
-    float2* out = work + (size_t)j * N;
-    int lit = 0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x)
+    float2* y = PP ? sm + padded((size_t)N * 2) : sm;
+    const int c0 = blockIdx.x * 4;
+    int any = 0;
+    for (int i = threadIdx.x; i < 2 * N; i += blockDim.x)
     {
-        const float a = row[i];
-        lit |= (a != 0.0f);
-        x[pad(i)] = make_float2(a, 0.0f);
+        const float2 v = *reinterpret_cast<const float2*>(in + (size_t)(i >> 1) * N + c0 + 2 * (i & 1));
+        any |= (v.x != 0.0f) | (v.y != 0.0f);
+        x[fft_slot<2, true>(i >> 1, i & 1, N)] = v;
     }
-    if (!__syncthreads_or(lit))
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) lit[blockIdx.x] = any ? 1 : 0;
+    if (!any) return;
+    for (int st = 0; st < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    // Z = FFT(a + i b): FFT(a)[k] = (Z[k] + conj Z[N - k]) / 2, FFT(b)[k] = (Z[k] - conj Z[N - k]) / 2i;
+    // per pair of rows: 2 x 2 columns x 2 rows, one 64-byte piece
+    for (int t = threadIdx.x; t < pairs * 2; t += blockDim.x)
     {
-        for (int i = threadIdx.x; i < N; i += blockDim.x) out[i] = make_float2(0.0f, 0.0f);
-        return;
+        const int pr = t >> 1, s = t & 1;
+        float2 a[2], b[2];
+        #pragma unroll
+        for (int c = 0; c < 2; ++c)
+        {
+            const int k = 2 * pr + c;
+            a[c] = b[c] = make_float2(0.0f, 0.0f);
+            if (k <= N / 2)
+            {
+                const float2 z = x[fft_slot<2, true>(k, s, N)], w = x[fft_slot<2, true>((N - k) & (N - 1), s, N)];
+                a[c] = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
+                b[c] = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
+            }
+        }
+        float4* o = reinterpret_cast<float4*>(half + half_index(N, pr, c0 + 2 * s));
+        o[0] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
+        o[1] = make_float4(b[0].x, b[0].y, b[1].x, b[1].y);
     }
-    const float2* r = stockham<1>(x, y, d, tw, false);
-    for (int i = threadIdx.x; i < N; i += blockDim.x) out[i] = r[pad(i)];
 }
 
-template <int NB>
-__global__ void __launch_bounds__(kSpriteThreads) sprite_cols(const float2* __restrict__ work, int N, FftDims d,
-                                                              const float2* __restrict__ tw, float* __restrict__ psf,
-                                                              double* __restrict__ energy)
+// Rows ky = 2 pair + s of the half spectrum; dark columns are zero.
+struct HalfRows {
+    const float2* half;            // the pair's block
+    const unsigned char* lit;      // shared memory
+    __device__ __forceinline__ float2 operator()(int s, int x) const
+    {
+        return lit[x >> 2] ? half[2 * x + s] : make_float2(0.0f, 0.0f);
+    }
+};
+
+// |X|^2 at its fftshifted place and at the mirrored one.
+struct PsfStore {
+    float* psf;
+    float* sum;                    // this thread's energy
+    int N, pair;
+    __device__ __forceinline__ void operator()(int s, int kx, float2 z) const
+    {
+        const int ky = 2 * pair + s, h = N / 2, m = N - 1;
+        if (ky > h) return;
+        const float p = z.x * z.x + z.y * z.y;
+        psf[(size_t)((ky + h) & m) * N + ((kx + h) & m)] = p;
+        *sum += p;
+        if (ky == 0 || ky == h) return;                  // these rows hold their own mirror
+        psf[(size_t)((h - ky) & m) * N + ((h - kx) & m)] = p;
+        *sum += p;
+    }
+};
+
+// The matrix-DFT engine's compact autocorrelation (mdft_render.cu:88-99,
+// 247-262), from the transform of the fftshifted PSF: lags within +-mc,
+// C[a][b] (a = y lag + mc, b = x lag + mc) = (-1)^(lx + ly) Re X[ly][lx] /
+// (energy N^2).  The sign undoes the fftshift of the PSF (a shift by N/2
+// multiplies the transform by (-1)^l); energy = sum |FFT A|^2 = G[0][0].  A real
+// pupil has a real, point-symmetric autocorrelation: the imaginary part is
+// rounding, and C[-ly][-lx] is C[ly][lx].
+struct LagStore {
+    float* C;
+    int N, pair, mc, ldc;
+    float scale;
+    __device__ __forceinline__ void operator()(int s, int kx, float2 z) const
+    {
+        const int ly = 2 * pair + s, lx = kx <= N / 2 ? kx : kx - N;
+        if (ly > mc || lx < -mc || lx > mc) return;
+        const float v = ((lx + ly) & 1) ? -z.x * scale : z.x * scale;
+        C[(size_t)(mc + ly) * ldc + (mc + lx)] = v;
+        if (ly > 0) C[(size_t)(mc - ly) * ldc + (mc - lx)] = v;
+    }
+};
+
+// Pass 2: rows ky of pair blockIdx.x.  LAGS: the autocorrelation's lags, else
+// the PSF and its energy.
+template <bool PP, bool LAGS>
+__global__ void __launch_bounds__(1024) grid_rows(const float2* __restrict__ half, const unsigned char* __restrict__ lit,
+                                                  int N, const __grid_constant__ FftDims d, const float2* __restrict__ tw,
+                                                  float* __restrict__ out, double* __restrict__ energy, int mc, int ldc)
 {
     extern __shared__ float2 sm[];
+    __shared__ float red[32];
     float2* x = sm;
-    float2* y = sm + padded((size_t)N * NB);
-    __shared__ float red[kSpriteThreads / 32];
-    const int c0 = blockIdx.x * NB;
-    for (int it = threadIdx.x; it < N * NB; it += blockDim.x)
-    {
-        const int r = it / NB, s = it % NB;
-        x[pad(r * NB + s)] = work[(size_t)r * N + c0 + s];
-    }
+    float2* y = PP ? sm + padded((size_t)N * 2) : sm;
+    unsigned char* flags = reinterpret_cast<unsigned char*>(sm + (PP ? 2 : 1) * padded((size_t)N * 2));
+    const int pair = blockIdx.x;
+    for (int i = threadIdx.x; i < N / 4; i += blockDim.x) flags[i] = lit[i];
     __syncthreads();
-    const float2* X = stockham<NB>(x, y, d, tw, false);
-    // fftshift: transform row k, column c lands at ((k + N/2) % N, (c + N/2) % N)
-    const int h = N / 2;
-    float part = 0.0f;
-    for (int it = threadIdx.x; it < N * NB; it += blockDim.x)
+    const HalfRows load{half + half_index(N, pair, 0), flags};
+    fft_any<2, true, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
+    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    if (LAGS)
     {
-        const int k = it / NB, s = it % NB;
-        const float2 z = X[pad(k * NB + s)];
-        const float p = z.x * z.x + z.y * z.y;
-        part += p;
-        const int jj = (k + h) & (N - 1), ii = (c0 + s + h) & (N - 1);
-        psf[(size_t)jj * N + ii] = p;
+        const double e = *energy;
+        const float scale = e > 0.0 ? (float)(1.0 / (e * (double)N * (double)N)) : 0.0f;
+        fft_any<2, true, false, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, LagStore{out, N, pair, mc, ldc, scale});
+        return;
     }
+    float part = 0.0f;
+    fft_any<2, true, false, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, PsfStore{out, &part, N, pair});
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
     __syncthreads();
@@ -106,54 +184,6 @@ __global__ void __launch_bounds__(kSpriteThreads) sprite_cols(const float2* __re
         double t = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += (double)red[w];
         atomicAdd(energy, t);
-    }
-}
-
-// Column pass of the second transform of the matrix-DFT engine's compact
-// autocorrelation (mdft_render.cu:88-99, 247-262): after the row pass of the
-// fftshifted PSF, transform the columns whose x lag lies within +-mc of zero
-// and write C[a][b] (a = y lag + mc, b = x lag + mc) = (-1)^(lx + ly)
-// Re X[ly][lx] / (energy N^2).  The sign undoes the fftshift of the PSF
-// (a shift by N/2 multiplies the transform by (-1)^l); energy = sum |FFT A|^2
-// = G[0][0], summed on the device by the first column pass.  A real pupil has
-// a real, point-symmetric autocorrelation: the imaginary part is rounding.
-template <int NB>
-__global__ void __launch_bounds__(kSpriteThreads) autocorr_cols(const float2* __restrict__ work, int N, FftDims d,
-                                                                const float2* __restrict__ tw, int mc,
-                                                                const double* __restrict__ energy,
-                                                                float* __restrict__ C, int ldc)
-{
-    extern __shared__ float2 sm[];
-    const int c0 = blockIdx.x * NB;
-    const int h = N / 2;
-    bool any = false;
-    #pragma unroll
-    for (int s = 0; s < NB; ++s)
-    {
-        const int c = c0 + s, lag = c <= h ? c : c - N;
-        any |= (lag >= -mc && lag <= mc);
-    }
-    if (!any) return;                          // uniform over the block
-    float2* x = sm;
-    float2* y = sm + padded((size_t)N * NB);
-    for (int it = threadIdx.x; it < N * NB; it += blockDim.x)
-    {
-        const int r = it / NB, s = it % NB;
-        x[pad(r * NB + s)] = work[(size_t)r * N + c0 + s];
-    }
-    __syncthreads();
-    const float2* X = stockham<NB>(x, y, d, tw, false);
-    const double e = *energy;
-    const float scale = e > 0.0 ? (float)(1.0 / (e * (double)N * (double)N)) : 0.0f;
-    const int Mc = 2 * mc + 1;
-    for (int it = threadIdx.x; it < Mc * NB; it += blockDim.x)
-    {
-        const int a = it / NB, s = it % NB;
-        const int c = c0 + s, lx = c <= h ? c : c - N;
-        if (lx < -mc || lx > mc) continue;
-        const int ly = a - mc, r = (ly + N) & (N - 1);
-        const float v = X[pad(r * NB + s)].x * scale;
-        C[(size_t)a * ldc + (lx + mc)] = ((lx + ly) & 1) ? -v : v;
     }
 }
 
@@ -168,18 +198,26 @@ __global__ void __launch_bounds__(kSpriteThreads) autocorr_cols(const float2* __
 // the next: about 2.5 loads per texel and wavelength where separate samples
 // take 4, and all loads of a thread's rows are in flight at once (carrying the
 // blend from row to row behind a branch left each row waiting for its own
-// load: 228 us).
+// load).
 // The box sum goes over the thread's rows, then lanes, then (d > T) warps, in
 // a fixed order.  Every fine texel is a thread's, so a strongly minified sprite
 // (few coarse texels) still fills the chip.  Bound by load latency and issue in
-// equal parts (issue slots 56% busy, L1 49%); 16 rows per thread or more CTAs
-// per SM at fewer registers are slower.
-// N = 2048, 31 wavelengths, d = 2: 221 -> 183 us; N = 1024, 16 wavelengths,
-// d = 16 (one thread per coarse texel: 16 CTAs): 1404 -> 37 us.
+// equal parts (issue slots 56% busy, L1 49%); eight rows per thread, or more
+// CTAs per SM at fewer registers, are slower.
+// N = 2048, 31 wavelengths, d = 2: 221 -> 157 us; N = 1024, 16 wavelengths,
+// d = 16 (one thread per coarse texel: 16 CTAs): 1404 -> 28 us.
 constexpr int kBakeSpec = 32;      // wavelengths staged at a time
 
-// A fine row's source row at one wavelength: y N (negative: outside), blend.
-struct __align__(8) RowAt { int off; float t; };
+// A fine row's source rows at one wavelength: byte offset of the lower one, its
+// lowest bit set where the upper one is the lower one of the fine row before
+// (offsets are multiples of 4 N), and the blend of the two (zero outside).
+struct __align__(16) RowAt { uint32_t lower; float up, lo, pad; };
+
+// A float of the grid by its byte offset (a grid has at most 2^28 bytes).
+__device__ __forceinline__ float grid_at(const float* g, uint32_t byte)
+{
+    return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(g) + byte));
+}
 
 template <int T>
 __global__ void __launch_bounds__(kSpriteThreads) sprite_bake(const float* __restrict__ psf, int N,
@@ -212,13 +250,19 @@ __global__ void __launch_bounds__(kSpriteThreads) sprite_bake(const float* __res
             const float fy = half + dy * k;
             const bool in = fy >= 0.0f && fy < top;
             const int y0 = in ? (int)floorf(fy) : 0;
+            // the row before, of the same thread
+            const float fz = half + (dy - 1.0f) * k;
+            const bool carried = r % T != 0 && in && fz >= 0.0f && y0 == (int)floorf(fz) + 1;
             RowAt at;
-            at.off = in ? y0 * N : -1;
-            at.t = fy - (float)y0;
+            at.lower = (uint32_t)(y0 + 1) * (uint32_t)N * 4u | (carried ? 1u : 0u);
+            at.lo = in ? fy - (float)y0 : 0.0f;
+            at.up = in ? 1.0f - at.lo : 0.0f;
+            at.pad = 0.0f;
             row_at[l][r] = at;
             if (r == 0) lam[l] = make_float4(k, s.y * (k * k * scale), s.z * (k * k * scale), s.w * (k * k * scale));
         }
         __syncthreads();
+        #pragma unroll 2
         for (int l = 0; l < nl; ++l)
         {
             const float4 s = lam[l];
@@ -229,32 +273,32 @@ __global__ void __launch_bounds__(kSpriteThreads) sprite_bake(const float* __res
             const float tx = fx - (float)x0;
             // a column outside blends to zero
             const float b0 = in ? 1.0f - tx : 0.0f, b1 = in ? tx : 0.0f;
-            const float* col = psf + x0;
-            RowAt at[T];
-            #pragma unroll
-            for (int r = 0; r < T; ++r) at[r] = row_at[l][warp * T + r];
+            const uint32_t x4 = 4u * (uint32_t)x0, n4 = 4u * (uint32_t)N;
             // lower source row of each fine row; the upper one where it is not
             // the row before's (the same for the whole warp)
             float lo[T], up[T];
             #pragma unroll
             for (int r = 0; r < T; ++r)
             {
-                const int y = max(at[r].off, 0);
-                lo[r] = __ldg(col + (y + N)) * b0 + __ldg(col + (y + N + 1)) * b1;
+                const uint32_t o = (row_at[l][warp * T + r].lower & ~1u) + x4;
+                lo[r] = grid_at(psf, o) * b0 + grid_at(psf, o + 4) * b1;
             }
             #pragma unroll
             for (int r = 0; r < T; ++r)
             {
-                const int y = max(at[r].off, 0);
-                const bool carried = r > 0 && at[r].off == at[max(r - 1, 0)].off + N && at[max(r - 1, 0)].off >= 0;
-                up[r] = 0.0f;
-                if (!carried) up[r] = __ldg(col + y) * b0 + __ldg(col + (y + 1)) * b1;
-                else up[r] = lo[max(r - 1, 0)];
+                const uint32_t f = row_at[l][warp * T + r].lower;
+                up[r] = lo[max(r - 1, 0)];
+                if (!(f & 1u))
+                {
+                    const uint32_t o = f + x4 - n4;
+                    up[r] = grid_at(psf, o) * b0 + grid_at(psf, o + 4) * b1;
+                }
             }
             #pragma unroll
             for (int r = 0; r < T; ++r)
             {
-                const float v = at[r].off < 0 ? 0.0f : up[r] * (1.0f - at[r].t) + lo[r] * at[r].t;
+                const RowAt& at = row_at[l][warp * T + r];
+                const float v = up[r] * at.up + lo[r] * at.lo;
                 acc[r][0] += s.y * v;
                 acc[r][1] += s.z * v;
                 acc[r][2] += s.w * v;
@@ -393,8 +437,9 @@ struct SpritePlan {
     int N = 0, n_spec = 0, M = 0, device = 0;
     float lambda_ref = 550.0f;
     FftDims dims{};
-    float2* tw = nullptr;
-    float2* work = nullptr;
+    float2* tw = nullptr;        // stage twiddles
+    float2* half = nullptr;      // half spectrum, N / 4 + 1 row pairs x N columns
+    unsigned char* lit = nullptr;   // per four columns: anything lit
     float* psf = nullptr;
     float* sprite = nullptr;
     size_t sprite_cap = 0;       // floats; grown by the bake to 3 M^2 (and the scratch of a large box sum)
@@ -402,7 +447,9 @@ struct SpritePlan {
     double* energy = nullptr;
     StarSource* src = nullptr;
     int src_cap = 0;
-    size_t smem_rows = 0, smem_cols = 0;
+    bool pp = false;
+    int threads = 0;
+    size_t smem = 0;
 };
 
 }  // namespace gl
@@ -414,7 +461,8 @@ using namespace gl;
 static void sprite_free(SpritePlan* p)
 {
     cudaFree(p->tw);
-    cudaFree(p->work);
+    cudaFree(p->half);
+    cudaFree(p->lit);
     cudaFree(p->psf);
     cudaFree(p->sprite);
     cudaFree(p->spec);
@@ -439,30 +487,36 @@ extern "C" int gl_sprite_plan_create(int N, const gl_spectral_sample* spec, int 
     p->dims = make_dims(N);
     cudaGetDevice(&p->device);
     const size_t NN = (size_t)N * N;
-    const int nb = col_group(N);
-    p->smem_rows = 2 * padded((size_t)N) * sizeof(float2);
-    p->smem_cols = 2 * padded((size_t)N * nb) * sizeof(float2);
+    p->pp = N <= kShortGrid;
+    p->threads = fft_threads(N, 2, p->pp);
+    p->smem = (p->pp ? 2 : 1) * padded((size_t)N * 2) * sizeof(float2) + N / 4;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-    chk(cudaMalloc(&p->tw, sizeof(float2) * N));
-    chk(cudaMalloc(&p->work, sizeof(float2) * NN));
+    const std::vector<float2> tw = stage_twiddles(p->dims);
+    chk(cudaMalloc(&p->tw, sizeof(float2) * tw.size()));
+    chk(cudaMalloc(&p->half, sizeof(float2) * 2 * (size_t)N * (N / 4 + 1)));
+    chk(cudaMalloc(&p->lit, N / 4));
     chk(cudaMalloc(&p->psf, sizeof(float) * NN));
     chk(cudaMalloc(&p->spec, sizeof(float4) * n_spec));
     chk(cudaMalloc(&p->energy, sizeof(double)));
     if (e == cudaSuccess)
     {
-        const std::vector<float2> tw = twiddles(N);
         std::vector<float4> sp((size_t)n_spec);
         for (int l = 0; l < n_spec; ++l) sp[l] = make_float4(spec[l].lambda, spec[l].cmf_r, spec[l].cmf_g, spec[l].cmf_b);
-        chk(cudaMemcpy(p->tw, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+        chk(cudaMemcpy(p->tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
         chk(cudaMemcpy(p->spec, sp.data(), sizeof(float4) * n_spec, cudaMemcpyHostToDevice));
-        chk((cudaError_t)raise_smem_limit((const void*)sprite_rows, p->smem_rows));
-        if (nb == 4) chk((cudaError_t)raise_smem_limit((const void*)sprite_cols<4>, p->smem_cols));
-        if (nb == 2) chk((cudaError_t)raise_smem_limit((const void*)sprite_cols<2>, p->smem_cols));
-        if (nb == 1) chk((cudaError_t)raise_smem_limit((const void*)sprite_cols<1>, p->smem_cols));
-        if (nb == 4) chk((cudaError_t)raise_smem_limit((const void*)autocorr_cols<4>, p->smem_cols));
-        if (nb == 2) chk((cudaError_t)raise_smem_limit((const void*)autocorr_cols<2>, p->smem_cols));
-        if (nb == 1) chk((cudaError_t)raise_smem_limit((const void*)autocorr_cols<1>, p->smem_cols));
+        if (p->pp)
+        {
+            chk((cudaError_t)raise_smem_limit((const void*)grid_cols<true>, p->smem));
+            chk((cudaError_t)raise_smem_limit((const void*)grid_rows<true, false>, p->smem));
+            chk((cudaError_t)raise_smem_limit((const void*)grid_rows<true, true>, p->smem));
+        }
+        else
+        {
+            chk((cudaError_t)raise_smem_limit((const void*)grid_cols<false>, p->smem));
+            chk((cudaError_t)raise_smem_limit((const void*)grid_rows<false, false>, p->smem));
+            chk((cudaError_t)raise_smem_limit((const void*)grid_rows<false, true>, p->smem));
+        }
     }
     if (e != cudaSuccess)
     {
@@ -472,6 +526,22 @@ extern "C" int gl_sprite_plan_create(int N, const gl_spectral_sample* spec, int 
     }
     *out = new gl_sprite_plan{p};
     return GL_OK;
+}
+
+// The fftshifted |FFT(grid)|^2 into p->psf, its sum added to p->energy.
+static void sprite_psf(SpritePlan* p, const float* d_grid, cudaStream_t st)
+{
+    const int N = p->N, pairs = N / 4 + 1;
+    if (p->pp)
+    {
+        grid_cols<true><<<N / 4, p->threads, p->smem, st>>>(d_grid, N, pairs, p->dims, p->tw, p->half, p->lit);
+        grid_rows<true, false><<<pairs, p->threads, p->smem, st>>>(p->half, p->lit, N, p->dims, p->tw, p->psf, p->energy, 0, 0);
+    }
+    else
+    {
+        grid_cols<false><<<N / 4, p->threads, p->smem, st>>>(d_grid, N, pairs, p->dims, p->tw, p->half, p->lit);
+        grid_rows<false, false><<<pairs, p->threads, p->smem, st>>>(p->half, p->lit, N, p->dims, p->tw, p->psf, p->energy, 0, 0);
+    }
 }
 
 extern "C" int gl_sprite_plan_bake(gl_sprite_plan* plan, const float* d_pupil, int ds, void* stream)
@@ -496,24 +566,16 @@ extern "C" int gl_sprite_plan_bake(gl_sprite_plan* plan, const float* d_pupil, i
     }
     p->M = N / ds;
     GL_CUDA_TRY(cudaMemsetAsync(p->energy, 0, sizeof(double), st));
-    sprite_rows<<<N, kSpriteThreads, p->smem_rows, st>>>(d_pupil, N, p->dims, p->tw, p->work);
-    const int nb = col_group(N);
-    if (nb == 4)
-        sprite_cols<4><<<N / 4, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
-    else if (nb == 2)
-        sprite_cols<2><<<N / 2, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
-    else
-        sprite_cols<1><<<N, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
-    // rows per thread: eight share the most loads; small grids take fewer, for
-    // enough warps (256 CTAs at least)
+    sprite_psf(p, d_pupil, st);
+    // rows per thread: four and two wavelengths in flight measured best at 1024
+    // and 2048; the smallest grid takes one, for enough warps (256 CTAs)
     const int d = std::min(ds, 32), m1 = N / d;
     float* fine = ds > 32 ? p->sprite + 3 * (size_t)p->M * p->M : p->sprite;
     auto bake = [&](auto kernel, int T) {
         kernel<<<dim3(N / 32, N / (8 * T)), kSpriteThreads, 0, st>>>(p->psf, N, p->spec, p->n_spec, p->lambda_ref, d, m1,
                                                                      p->energy, fine);
     };
-    if (N >= 1024) bake(sprite_bake<8>, 8);
-    else if (N >= 512 || d > 8) bake(sprite_bake<4>, 4);      // a CTA's 8 T rows hold whole box sums
+    if (N >= 512 || d > 8) bake(sprite_bake<4>, 4);          // a CTA's 8 T rows hold whole box sums
     else bake(sprite_bake<1>, 1);
     if (ds > 32)
         sprite_box<<<(3 * p->M * p->M + kSpriteThreads - 1) / kSpriteThreads, kSpriteThreads, 0, st>>>(fine, ds / 32, p->M,
@@ -592,23 +654,20 @@ extern "C" int gl_sprite_plan_autocorr(gl_sprite_plan* plan, const float* d_pupi
     cudaStream_t st = (cudaStream_t)stream;
     GL_CUDA_TRY(cudaMemsetAsync(d_C, 0, sizeof(float) * (size_t)ldc * rows, st));
     GL_CUDA_TRY(cudaMemsetAsync(p->energy, 0, sizeof(double), st));
-    const int nb = col_group(N);
     // |FFT A|^2 (fftshifted) and its sum, as the sprite bake computes them
-    sprite_rows<<<N, kSpriteThreads, p->smem_rows, st>>>(d_pupil, N, p->dims, p->tw, p->work);
-    if (nb == 4)
-        sprite_cols<4><<<N / 4, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
-    else if (nb == 2)
-        sprite_cols<2><<<N / 2, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
-    else
-        sprite_cols<1><<<N, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, p->psf, p->energy);
+    sprite_psf(p, d_pupil, st);
     // the second transform, kept only at lags within +-mc
-    sprite_rows<<<N, kSpriteThreads, p->smem_rows, st>>>(p->psf, N, p->dims, p->tw, p->work);
-    if (nb == 4)
-        autocorr_cols<4><<<N / 4, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, mc, p->energy, d_C, ldc);
-    else if (nb == 2)
-        autocorr_cols<2><<<N / 2, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, mc, p->energy, d_C, ldc);
+    const int pairs = mc / 2 + 1;
+    if (p->pp)
+    {
+        grid_cols<true><<<N / 4, p->threads, p->smem, st>>>(p->psf, N, pairs, p->dims, p->tw, p->half, p->lit);
+        grid_rows<true, true><<<pairs, p->threads, p->smem, st>>>(p->half, p->lit, N, p->dims, p->tw, d_C, p->energy, mc, ldc);
+    }
     else
-        autocorr_cols<1><<<N, kSpriteThreads, p->smem_cols, st>>>(p->work, N, p->dims, p->tw, mc, p->energy, d_C, ldc);
+    {
+        grid_cols<false><<<N / 4, p->threads, p->smem, st>>>(p->psf, N, pairs, p->dims, p->tw, p->half, p->lit);
+        grid_rows<false, true><<<pairs, p->threads, p->smem, st>>>(p->half, p->lit, N, p->dims, p->tw, d_C, p->energy, mc, ldc);
+    }
     GL_CUDA_TRY(cudaGetLastError());
     // the bake's sprite no longer matches the PSF buffer's contents
     p->M = 0;

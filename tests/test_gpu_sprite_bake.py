@@ -10,7 +10,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
-# rows per thread 1 (256), 4 (512), 8 (1024); box sums within the rows, across
+# rows per thread 1 (256) and 4; box sums within the rows, across
 # lanes, across warps (above the rows) and above 32 (second pass); more
 # wavelengths than one staging (64).  1e-4: a float32 sample position at 1000
 # texels is known to 6e-5 of a texel.
