@@ -3,8 +3,19 @@
 // Replaces filter_ghost_pairs (ghostlight/src/ghost.cpp:105-138).  One block
 // per enumerated pair traces the reference's probes — three axial rays at
 // 650/550/450 nm for the intensity estimate (ghost.cpp:34-50) and the 8x8
-// green probe for the area boost (ghost.cpp:53-102) — in one launch instead of
-// 67 host traces per pair.
+// green probe for the area boost (ghost.cpp:53-102; the 52 of its points inside
+// the unit disc) — in one launch instead of 55 host traces per pair.
+//
+// The launch is one wave whose time is one trace of up to three passes over the
+// lens by IEEE-exact steps, so what is in that chain counts:
+//   * all of a block's rays walk together through one call site, geometry only:
+//     whether a probe lands and where does not depend on its weight;
+//   * the axial rays note each bend; their coating weights are worked out
+//     afterwards, all bends in parallel, and multiplied in path order;
+//   * the graze test's three silhouettes (below) are checks along one walk,
+//     with a mask of the variants still alive, not three walks.
+// 24 surfaces, 253 pairs: 442 -> 107 us (three variants of three warps each,
+// the weights in the chain and the axial rays walked apart from the probe).
 //
 // This translation unit is compiled IEEE-exact (-fmad=false, IEEE division
 // and square root, no flush-to-zero), so its float arithmetic equals the
@@ -25,6 +36,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -34,7 +46,7 @@ namespace gl {
 
 namespace {
 
-constexpr int kProbeThreads = 96;   // 3 intensity rays + 64 spread probes, padded
+constexpr int kProbeThreads = 64;   // 3 intensity rays + 52 spread probes, padded
 
 using ProbeOut = FilterProbe;
 constexpr float kGraze = 1e-6f;     // relative clear-radius perturbation of the graze test
@@ -51,72 +63,186 @@ bool same_probe(const ProbeOut& x, const ProbeOut& y)
     return std::memcmp(&x, &y, sizeof(ProbeOut)) == 0;
 }
 
-// One out-of-line copy of the trace for both kinds of probe ray: the IEEE
-// general step is large, and the launch is one wave whose time is one
-// divergent trace, so a single copy keeps its code in the instruction cache.
-__device__ __noinline__ TraceOut probe_trace(const SurfRec* lens, int n, const float* at, const float* bf, V3 o,
-                                              float lam, int a, int b)
+// One bend of an axial ray: what its weight needs (surface_weight and
+// surface_attenuator of step(), gl_trace.cuh).
+struct Bend {
+    V3 d, nrm, hit;
+    float n1, n2;
+    int surf_refl;                  // surface, bit 16: reflected
+};
+
+// Shared memory of a block for n surfaces and walks of up to L bends.
+size_t probe_smem(int n, int L)
 {
-    return trace_ghost(lens, n, at, bf, o, v3(0.0f, 0.0f, 1.0f), lam, a, b);
+    return sizeof(SurfRec) * n + sizeof(float) * 6 * n + (sizeof(Bend) + sizeof(float2)) * 3 * L + 16;
 }
 
+// recs: nv variants of n records (exact, then the widened and narrowed
+// silhouettes of the graze test); open: the exact records with the silhouette
+// surfaces' apertures opened; silhouettes: bit per such surface (none: nv = 1).
 __global__ void __launch_bounds__(kProbeThreads)
-filter_probe_kernel(const SurfRec* __restrict__ recs, int n, const float* __restrict__ ior_at3,
-                    const float* __restrict__ ior_bf3, const int2* __restrict__ pairs,
-                    float front_R, float start_z, ProbeOut* __restrict__ out)
+filter_probe_kernel(const SurfRec* __restrict__ recs, const SurfRec* __restrict__ open, int n, int nv,
+                    uint64_t silhouettes, const float* __restrict__ ior_at3, const float* __restrict__ ior_bf3,
+                    const int2* __restrict__ pairs, float front_R, float start_z, int lmax, ProbeOut* __restrict__ out)
 {
-    // blockIdx.y: the record variant (exact, then the widened and narrowed
-    // silhouettes of the graze test)
-    recs += (size_t)blockIdx.y * n;
-    out += (size_t)blockIdx.y * gridDim.x;
-    __shared__ SurfRec lens[kMaxSurfaces];
-    __shared__ float at[3 * kMaxSurfaces], bf[3 * kMaxSurfaces];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Bend* bends = reinterpret_cast<Bend*>(smem_raw);                 // [axial ray][lmax]
+    float2* factors = reinterpret_cast<float2*>(bends + 3 * lmax);   // weight, attenuator
+    SurfRec* lens = reinterpret_cast<SurfRec*>(factors + 3 * lmax);
+    float* at = reinterpret_cast<float*>(lens + n);
+    float* bf = at + 3 * n;
     __shared__ float px[64], py[64];
-    __shared__ int ok[64];
+    __shared__ int ok[64];                                           // variants that land
+    __shared__ int points[64];                                       // probe points inside the disc
+    __shared__ int n_points[2];
+    __shared__ int n_bends[3], axial_ok[3], end[3][3];               // [ray], [ray], [ray][variant]
     const int tid = threadIdx.x;
     {
         const int words = n * (int)(sizeof(SurfRec) / 4);
-        const int* src = reinterpret_cast<const int*>(recs);
+        const int* src = reinterpret_cast<const int*>(open);
         int* dst = reinterpret_cast<int*>(lens);
-        for (int i = tid; i < words; i += blockDim.x) dst[i] = src[i];
-        for (int i = tid; i < 3 * n; i += blockDim.x) { at[i] = ior_at3[i]; bf[i] = ior_bf3[i]; }
+        for (int i = tid; i < words; i += kProbeThreads) dst[i] = src[i];
+        for (int i = tid; i < 3 * n; i += kProbeThreads) { at[i] = ior_at3[i]; bf[i] = ior_bf3[i]; }
     }
+    const float gu = ((tid % 8 + 0.5f) / 8) * 2.0f - 1.0f, gv = ((tid / 8 + 0.5f) / 8) * 2.0f - 1.0f;
+    const bool inside = !(gu * gu + gv * gv > 1.0f);
+    const unsigned m = __ballot_sync(0xffffffffu, inside);
+    if ((tid & 31) == 0) n_points[tid >> 5] = __popc(m);
+    ok[tid] = 0;
+    __syncthreads();
+    if (inside) points[(tid >= 32 ? n_points[0] : 0) + __popc(m & ((1u << (tid & 31)) - 1u))] = tid;
     __syncthreads();
     const int2 p = pairs[blockIdx.x];
-    const float lams[3] = {650.0f, 550.0f, 450.0f};
-    ProbeOut* o = out + blockIdx.x;
-    if (tid < 3)
+    const int a = p.x, b = p.y, L1 = b + 1, L2 = L1 + (b - a), L = L2 + (n - 1 - a);
+    const bool axial = tid < 3;
+    if (tid < 3 + n_points[0] + n_points[1])
     {
-        TraceOut r = probe_trace(lens, n, at + tid * n, bf + tid * n, v3(0.0f, 0.0f, start_z), lams[tid], p.x, p.y);
-        o->w[tid] = r.w;
-        o->wok[tid] = (r.status == 0);
-    }
-    else if (tid < 67)
-    {
-        const int k = tid - 3, gx = k % 8, gy = k / 8;
-        const float u = ((gx + 0.5f) / 8) * 2.0f - 1.0f;
-        const float v = ((gy + 0.5f) / 8) * 2.0f - 1.0f;
-        int good = 0;
-        if (!(u * u + v * v > 1.0f))
+        const int k = axial ? 0 : points[tid - 3], li = axial ? tid : 1;
+        const float u = ((k % 8 + 0.5f) / 8) * 2.0f - 1.0f;
+        const float v = ((k / 8 + 0.5f) / 8) * 2.0f - 1.0f;
+        V3 o = axial ? v3(0.0f, 0.0f, start_z) : v3(u * front_R, v * front_R, start_z);
+        V3 d = v3(0.0f, 0.0f, 1.0f);
+        const float* la = at + li * n;
+        const float* lb = bf + li * n;
+        float cur = 1.0f;
+        int alive = (1 << nv) - 1, cnt = 0;
+        #pragma unroll 1
+        for (int q = 0; q < L && alive; ++q)
         {
-            TraceOut r = probe_trace(lens, n, at + n, bf + n, v3(u * front_R, v * front_R, start_z), 550.0f, p.x, p.y);
-            if (r.status == 0) { px[k] = r.x; py[k] = r.y; good = 1; }
+            // the three legs of trace_ghost
+            int s; bool refl, back = false;
+            if (q < L1)      { s = q;                refl = (s == b); }
+            else if (q < L2) { s = 2 * b - q;        refl = (s == a); back = true; }
+            else             { s = a + 1 + (q - L2); refl = false; }
+            const SurfRec& S = lens[s];
+            if (!(S.flags & SF_ACTIVE)) continue;
+            const float n1 = cur, n2 = back ? lb[s] : la[s];
+            float t = 0.0f;
+            V3 nrm, nd;
+            int left = 0;
+            if (intersect(o, d, S, t, nrm))
+            {
+                left = alive;
+                if ((silhouettes >> s) & 1)
+                {
+                    // the hit in the surface's frame, as intersect() forms it
+                    V3 lo = o, ld = d;
+                    if (S.flags & SF_TRANSFORMED)
+                    {
+                        lo = m3tmul(S.rot, o - v3(S.dec_x, S.dec_y, S.z)) + v3(0.0f, 0.0f, S.z);
+                        ld = m3tmul(S.rot, d);
+                    }
+                    const V3 hit = lo + ld * t;
+                    for (int w = 0; w < nv; ++w)
+                        if (((left >> w) & 1) && !check_aperture(hit, recs[w * n + s])) left &= ~(1 << w);
+                }
+                if (!refl && left && !refract(d, nrm, n1, n2, nd)) left = 0;
+            }
+            // a variant that ends here has the weight of the bends so far
+            if (axial)
+                for (int w = 0; w < nv; ++w)
+                    if (((alive & ~left) >> w) & 1) end[tid][w] = cnt;
+            alive = left;
+            if (!alive) break;
+            const V3 hit = o + d * t;
+            if (axial)
+            {
+                Bend B;
+                B.d = d; B.nrm = nrm; B.hit = hit; B.n1 = n1; B.n2 = n2;
+                B.surf_refl = s | (refl ? 1 << 16 : 0);
+                bends[tid * lmax + cnt] = B;
+            }
+            ++cnt;
+            o = hit;
+            if (refl)
+            {
+                d = reflect(d, nrm);
+                cur = back ? la[a] : cur;
+            }
+            else
+            {
+                d = nd;
+                cur = n2;
+            }
         }
-        ok[k] = good;
+        TraceOut r;
+        r.status = 1;
+        if (alive) to_sensor(o, d, r);
+        const int landed = r.status == 0 ? alive : 0;
+        if (axial)
+        {
+            n_bends[tid] = cnt;
+            axial_ok[tid] = landed;
+            for (int w = 0; w < nv; ++w)
+                if ((alive >> w) & 1) end[tid][w] = cnt;
+        }
+        else
+        {
+            ok[k] = landed;
+            if (landed) { px[k] = r.x; py[k] = r.y; }
+        }
     }
     __syncthreads();
-    if (tid == 0)
+    // the bends' weights, all at once
+    const float lams[3] = {650.0f, 550.0f, 450.0f};
+    for (int i = tid; i < 3 * lmax; i += kProbeThreads)
     {
+        const int r = i / lmax;
+        if (i - r * lmax >= n_bends[r]) continue;
+        const Bend B = bends[i];
+        const SurfRec& S = lens[B.surf_refl & 0xffff];
+        factors[i] = make_float2(surface_weight(B.d, B.nrm, B.n1, B.n2, S, lams[r], (B.surf_refl >> 16) != 0),
+                                 surface_attenuator(B.hit, S));
+    }
+    __syncthreads();
+    if (tid < 3 * nv)
+    {
+        const int w = tid / 3, r = tid - 3 * w;
+        ProbeOut* q = out + (size_t)w * gridDim.x + blockIdx.x;
+        float weight = 1.0f;
+        for (int i = 0; i < end[r][w]; ++i)
+        {
+            const float2 f = factors[r * lmax + i];
+            weight *= f.x;
+            weight *= f.y;
+        }
+        q->w[r] = weight;
+        q->wok[r] = (axial_ok[r] >> w) & 1;
+    }
+    else if (tid >= 32 && tid < 32 + nv)
+    {
+        const int w = tid - 32;
+        ProbeOut* q = out + (size_t)w * gridDim.x + blockIdx.x;
         float mnx = 1e30f, mxx = -1e30f, mny = 1e30f, mxy = -1e30f;
         int valid = 0;
         for (int k = 0; k < 64; ++k)
         {
-            if (!ok[k]) continue;
+            if (!((ok[k] >> w) & 1)) continue;
             mnx = fminf(mnx, px[k]); mxx = fmaxf(mxx, px[k]);
             mny = fminf(mny, py[k]); mxy = fmaxf(mxy, py[k]);
             ++valid;
         }
-        o->mnx = mnx; o->mxx = mxx; o->mny = mny; o->mxy = mxy; o->valid = valid;
+        q->mnx = mnx; q->mxx = mxx; q->mny = mny; q->mxy = mxy; q->valid = valid;
     }
 }
 
@@ -176,14 +302,18 @@ extern "C" int gl_filter_ghost_pairs(const gl_surface* surfaces, int n, float hw
         std::vector<ProbeOut> res((size_t)np * nv);
         cudaError_t e = cudaSuccess;
         auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-        const size_t o_at = align256(sizeof(SurfRec) * n * nv), o_bf = o_at + align256(sizeof(float) * 3 * n);
+        // one block: records of the variants and the opened set, tables, pairs; then the results
+        const size_t o_at = align256(sizeof(SurfRec) * n * (nv + 1)), o_bf = o_at + align256(sizeof(float) * 3 * n);
         const size_t o_pairs = o_bf + align256(sizeof(float) * 3 * n);
         const size_t o_out = o_pairs + align256(sizeof(int2) * np);
         const size_t need = o_out + align256(sizeof(ProbeOut) * np * nv);
         int dev = 0;
         chk(cudaGetDevice(&dev));
         if (e == cudaSuccess && (dev < 0 || dev >= 64)) e = cudaErrorInvalidDevice;
-        std::vector<SurfRec> drecs((size_t)n * nv);                 // the device probes' records
+        std::vector<SurfRec> drecs((size_t)n * (nv + 1));           // the device probes' records
+        uint64_t silhouettes = 0;
+        int lmax = 0;
+        for (const int2& c : cand) lmax = std::max(lmax, (c.y + 1) + (c.y - c.x) + (n - 1 - c.x));
         if (e == cudaSuccess)
         {
             rc = pack_lens(surfaces, n, drecs.data(), dev);
@@ -196,6 +326,15 @@ extern "C" int gl_filter_ghost_pairs(const gl_surface* surfaces, int n, float hw
                     if (g.aperture_shape == GL_APERTURE_POLYGON && g.aperture_blades >= 3) g.semi_aperture *= f;
                 rc = pack_lens(moved.data(), n, drecs.data() + (size_t)v * n, dev);
                 if (rc) return rc;
+            }
+            for (int i = 0; i < n; ++i)
+            {
+                SurfRec& open = drecs[(size_t)nv * n + i];
+                open = drecs[i];
+                if (nv == 1 || surfaces[i].aperture_shape != GL_APERTURE_POLYGON || surfaces[i].aperture_blades < 3) continue;
+                silhouettes |= (uint64_t)1 << i;
+                open.shape = 0;
+                open.semi_ap = INFINITY;
             }
         }
         std::unique_lock<std::mutex> lock(g_scratch_mu);
@@ -216,17 +355,22 @@ extern "C" int gl_filter_ghost_pairs(const gl_surface* surfaces, int n, float hw
         ProbeOut* d_out = reinterpret_cast<ProbeOut*>(base + o_out);
         if (e == cudaSuccess)
         {
-            chk(cudaMemcpy(d_recs, drecs.data(), sizeof(SurfRec) * n * nv, cudaMemcpyHostToDevice));
-            chk(cudaMemcpy(d_at, at.data(), sizeof(float) * 3 * n, cudaMemcpyHostToDevice));
-            chk(cudaMemcpy(d_bf, bf.data(), sizeof(float) * 3 * n, cudaMemcpyHostToDevice));
-            chk(cudaMemcpy(d_pairs, cand.data(), sizeof(int2) * np, cudaMemcpyHostToDevice));
+            std::vector<char> host(o_out);
+            std::memcpy(host.data(), drecs.data(), sizeof(SurfRec) * drecs.size());
+            std::memcpy(host.data() + o_at, at.data(), sizeof(float) * 3 * n);
+            std::memcpy(host.data() + o_bf, bf.data(), sizeof(float) * 3 * n);
+            std::memcpy(host.data() + o_pairs, cand.data(), sizeof(int2) * np);
+            chk(cudaMemcpy(base, host.data(), o_out, cudaMemcpyHostToDevice));
+            const size_t smem = probe_smem(n, lmax);
+            if (e == cudaSuccess && smem > 46 * 1024) chk((cudaError_t)raise_smem_limit((const void*)filter_probe_kernel, smem));
         }
         if (e == cudaSuccess)
         {
             const float front_R = surfaces[0].semi_aperture;
             const float start_z = surfaces[0].z - kSpawnOffset;
-            filter_probe_kernel<<<dim3(np, nv), kProbeThreads>>>(d_recs, n, d_at, d_bf, d_pairs, front_R, start_z,
-                                                                  d_out);
+            filter_probe_kernel<<<np, kProbeThreads, probe_smem(n, lmax)>>>(d_recs, d_recs + (size_t)nv * n, n, nv,
+                                                                          silhouettes, d_at, d_bf, d_pairs, front_R,
+                                                                          start_z, lmax, d_out);
             chk(cudaGetLastError());
             chk(cudaMemcpy(res.data(), d_out, sizeof(ProbeOut) * np * nv, cudaMemcpyDeviceToHost));
         }
