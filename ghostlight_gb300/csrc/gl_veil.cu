@@ -23,33 +23,58 @@ constexpr int kVeilGrid = 1024;       // sprite side (texels)
 constexpr int kVeilCoreDiv = 32;      // core radius = grid / 32 texels: the sprite spans 16 core radii
 constexpr int kSpriteOversample = 3;  // sprite texels kept per output pixel after the downsample
 
-__global__ void veil_bake_kernel(float* __restrict__ ref, int N, float a_texels, float p)
+// Bake, and normalise to unit sum, in two launches over kVeilBlocks blocks: the
+// first leaves its block's FP64 sum, the second adds all blocks' sums in a fixed
+// order (each block for itself, 8 KB from L2) and scales its own texels.  One
+// block summing and scaling the whole grid took 777 us of render_veil's call;
+// the two take 23 us.
+constexpr int kVeilBlocks = 1024, kVeilThreads = 256;
+
+__device__ __forceinline__ double veil_block_sum(double s)
 {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= N * N) return;
-    const int i = idx % N, j = idx / N;
-    const float dx = (float)(i - N / 2), dy = (float)(j - N / 2);
-    const float a2 = a_texels * a_texels;
-    ref[idx] = powf(a2 / (dx * dx + dy * dy + a2), p);
+    __shared__ double part[kVeilThreads / 32];
+    __shared__ double total;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        double t = 0.0;
+        for (int w = 0; w < kVeilThreads / 32; ++w) t += part[w];
+        total = t;
+    }
+    __syncthreads();
+    return total;
 }
 
-// One block: FP64 sum of the grid (deterministic order), then scale to unit sum.
-__global__ void __launch_bounds__(1024) veil_normalise_kernel(float* __restrict__ ref, int n)
+__global__ void __launch_bounds__(kVeilThreads) veil_bake_kernel(float* __restrict__ ref, int N, float a_texels, float p,
+                                                                 double* __restrict__ sums)
 {
-    __shared__ double part[1024];
+    const int per = N * N / kVeilBlocks, base = blockIdx.x * per;
+    const float a2 = a_texels * a_texels;
     double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s += (double)ref[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1)
+    for (int q = threadIdx.x; q < per; q += kVeilThreads)
     {
-        if ((int)threadIdx.x < h) part[threadIdx.x] += part[threadIdx.x + h];
-        __syncthreads();
+        const int idx = base + q, i = idx % N, j = idx / N;
+        const float dx = (float)(i - N / 2), dy = (float)(j - N / 2);
+        const float v = powf(a2 / (dx * dx + dy * dy + a2), p);
+        ref[idx] = v;
+        s += (double)v;
     }
-    const double total = part[0];
+    s = veil_block_sum(s);
+    if (threadIdx.x == 0) sums[blockIdx.x] = s;
+}
+
+__global__ void __launch_bounds__(kVeilThreads) veil_normalise_kernel(float* __restrict__ ref, int N,
+                                                                      const double* __restrict__ sums)
+{
+    double s = 0.0;
+    for (int q = threadIdx.x; q < kVeilBlocks; q += kVeilThreads) s += sums[q];
+    const double total = veil_block_sum(s);
     if (!(total > 0.0)) return;
     const float k = (float)(1.0 / total);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ref[i] *= k;
+    const int per = N * N / kVeilBlocks, base = blockIdx.x * per;
+    for (int q = threadIdx.x; q < per; q += kVeilThreads) ref[base + q] *= k;
 }
 
 // Box-sum the N x N sprite into M x M (M = N / ds): summing keeps the deposit
@@ -162,8 +187,10 @@ extern "C" int gl_veil_plan_create(float falloff, void* stream, gl_veil_plan** o
     if (e == cudaSuccess) e = cudaMalloc(&v->coarse, (NN / 4) * sizeof(float));
     if (e == cudaSuccess)
     {
-        veil_bake_kernel<<<(int)((NN + 255) / 256), 256, 0, st>>>(v->ref, N, (float)N / (float)kVeilCoreDiv, p);
-        veil_normalise_kernel<<<1, 1024, 0, st>>>(v->ref, (int)NN);
+        // the block sums borrow the coarse buffer, which an execute fills before it reads it
+        double* sums = reinterpret_cast<double*>(v->coarse);
+        veil_bake_kernel<<<kVeilBlocks, kVeilThreads, 0, st>>>(v->ref, N, (float)N / (float)kVeilCoreDiv, p, sums);
+        veil_normalise_kernel<<<kVeilBlocks, kVeilThreads, 0, st>>>(v->ref, N, sums);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
