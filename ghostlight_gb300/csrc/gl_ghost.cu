@@ -752,7 +752,7 @@ struct GhostPlan {
     int* counter = nullptr;
     float4* accum = nullptr;            // RGBA scratch, width x height
     size_t smem = 0;
-    int grid_persistent = 0;
+    int queue_ctas = 0;                 // CTAs of the persistent queue when there is work for all
     int per_sm = 0, n_sm = 0;           // resident render CTAs per SM, SM count
     int launch_ipw = 0;                 // 0: persistent queue; > 0: static chunks of this many items per warp
     int l_chunks = 1;                   // wavelength ranges per item (tasks per item)
@@ -1141,8 +1141,21 @@ int plan_create(const gl_surface* surfaces, int n_surf, const gl_ghost_pair* pai
     const int warps_per_block = kRenderThreads / 32;
     p->per_sm = std::max(1, per_sm);
     p->n_sm = n_sm;
-    p->grid_persistent = std::max(1, std::min((p->n_items + warps_per_block - 1) / warps_per_block,
-                                              p->per_sm * n_sm));
+    p->queue_ctas = p->per_sm * n_sm;
+    // A plan of few items splits its wavelengths further, to about 20 tasks per
+    // resident warp: a task's chain of steps is what such a frame waits for.
+    // 66 pairs: 32^2 x 8 wavelengths 158 -> 64 us, 64^2 x 8 232 -> 139; 120 pairs x
+    // 5 sources, 42^2 x 8 621 -> 463; above (180850 items x 31) the default's
+    // eight wavelengths per task stay best (6128 us, 6326 with four).
+    if (!prm->plain_per_pair && p->n_items > 0)
+    {
+        const long long want = (20LL * p->queue_ctas * warps_per_block + p->n_items - 1) / p->n_items;
+        if (want > p->l_chunks)
+        {
+            const int l_size = std::max(1, (int)(n_spec / std::min<long long>(want, n_spec)));
+            p->l_chunks = std::max(p->l_chunks, (n_spec + l_size - 1) / l_size);
+        }
+    }
     *out = p;
     return GL_OK;
 }
@@ -1154,10 +1167,17 @@ int plan_set_launch(GhostPlan* p, int items_per_warp, int ctas_per_sm)
 {
     if (items_per_warp < 0 || ctas_per_sm < 0) return fail(GL_ERR_INVALID, "ghost_plan_set_launch: negative value");
     const int cps = ctas_per_sm == 0 ? p->per_sm : std::min(ctas_per_sm, p->per_sm);
-    const int warps_per_block = kRenderThreads / 32;
     p->launch_ipw = items_per_warp;
-    p->grid_persistent = std::max(1, std::min((p->n_items + warps_per_block - 1) / warps_per_block, cps * p->n_sm));
+    p->queue_ctas = cps * p->n_sm;
     return GL_OK;
+}
+
+// CTAs of the persistent queue for `items` items of `chunks` tasks.
+static int queue_grid(const GhostPlan* p, long long items, int chunks)
+{
+    const int warps_per_block = kRenderThreads / 32;
+    const long long tasks = items * std::max(1, chunks);
+    return (int)std::max<long long>(1, std::min<long long>((tasks + warps_per_block - 1) / warps_per_block, p->queue_ctas));
 }
 
 // An event recorded inside a stream capture becomes an event-record node
@@ -1211,21 +1231,20 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
         B.traced = p->traced + 1;
         B.hw2 = 2.0f * (p->prm.sensor_half_w * 1.25f);
         B.hh2 = 2.0f * (p->prm.sensor_half_h * 1.25f);
-        const int warps_per_block = kRenderThreads / 32;
         const int n_it = p->probe_begin[3];
         if (n_it > 0)
         {
             B.items = p->probe_items;
             B.n_items = n_it;
             B.counter = p->probe_counters;
-            const int grid = std::max(1, std::min((n_it + warps_per_block - 1) / warps_per_block, p->grid_persistent));
+            const int grid = queue_grid(p, n_it, B.l_chunks);
             if (p->probe_perm != nullptr)
             {
                 // stage 1: every probe ray's first wavelength, recording where it died
                 RenderArgs B1 = B;
                 B1.lam_lo = 0; B1.lam_hi = 1; B1.l_chunks = 1;
                 B1.death = p->probe_death; B1.perm_stride = p->probe_samples_n;
-                ghost_render_kernel<true><<<grid, kRenderThreads, p->smem, st>>>(B1);
+                ghost_render_kernel<true><<<queue_grid(p, n_it, 1), kRenderThreads, p->smem, st>>>(B1);
                 const int* sb = p->probe_sample_begin;
                 probe_sort_kernel<<<dim3((unsigned)p->n_pairs, 3), 32, 0, st>>>(
                     p->probe_death, p->probe_perm, p->pair_hits, p->probe_samples_n, sb[0], sb[1], sb[2], sb[3]);
@@ -1276,7 +1295,7 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
         {
             GL_CUDA_TRY(cudaMemsetAsync(p->counter, 0, sizeof(int), st));
             A.counter = p->counter;
-            ghost_render_kernel<false><<<p->grid_persistent, kRenderThreads, p->smem, st>>>(A);
+            ghost_render_kernel<false><<<queue_grid(p, p->n_items, A.l_chunks), kRenderThreads, p->smem, st>>>(A);
             GL_CUDA_TRY(cudaGetLastError());
             ++launches;
         }
@@ -1426,7 +1445,7 @@ int gl_ghost_plan_info(const gl_ghost_plan* plan, long long* rays, int* n_items,
     if (!plan) return fail(GL_ERR_INVALID, "ghost_plan_info: null plan");
     if (rays) *rays = plan->p->rays + plan->p->probe_rays;
     if (n_items) *n_items = plan->p->n_items;
-    if (grid) *grid = plan->p->grid_persistent;
+    if (grid) *grid = queue_grid(plan->p, plan->p->n_items, plan->p->l_chunks);
     return GL_OK;
 }
 
