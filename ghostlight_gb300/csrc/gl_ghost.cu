@@ -7,18 +7,18 @@
 //     grids (one per pair; grids may differ in size), per-source beam data and
 //     a list of work items = (pair, source, 256-sample tile).
 //   * ONE persistent launch covers every pair x source: each CTA stages the
-//     lens table and IOR slices in shared memory once, then pops work items
-//     from a global counter until the list is empty.  Launch-bound
-//     per-ghost loops and their tail effects disappear; the plan executes with
-//     kernel launches only, so it can be captured in a CUDA graph.
+//     lens table and IOR slices in shared memory once, then pops tasks from a
+//     global counter until none is left.  The pairs that sample one grid are
+//     walked as a tree that shares their common legs (ghost_tree_kernel).
+//     Launch-bound per-ghost loops and their tail effects disappear; the plan
+//     executes with kernel launches only, so it can be captured in a CUDA graph.
 //   * The reference's per-pair launch loop (ghost_render.cu:1544-1557) is kept
 //     as `plain_per_pair` — the same kernel, one launch per pair, no queue.
 //   * Splat: the reference issues 12 scalar float atomics per surviving
-//     ray-wavelength.  Here the accumulator is RGBA float4 and each thread
-//     carries its current 2x2 footprint in registers across the wavelength
-//     loop (dispersion moves a ghost by a fraction of a pixel between
-//     neighbouring wavelengths), flushing with one 16-byte vector atomic per
-//     tap only when the footprint moves.
+//     ray-wavelength.  Here the accumulator is RGBA float4, one 16-byte vector
+//     atomic per tap; a warp whose landings share one footprint sums them first.
+//     The pair-by-pair walk carries its current 2x2 footprint across the
+//     wavelength loop and flushes it when it moves.
 //   * The flush kernel reads the RGBA accumulator once, applies the 3x3
 //     spectral correction (ghost_render.cu:610-622, same rounding order) and
 //     writes the three planar float32 outputs with coalesced vector stores.
@@ -44,6 +44,7 @@ constexpr unsigned kFull = 0xffffffffu;
 // Per-lane splat footprint kept in shared memory (12 floats, stride 13 so the
 // lanes of a warp fall in distinct banks) together with its 2x2 origin.
 constexpr int kAccStride = 13;
+constexpr int kLaneFloats = 14;      // a lane's shared memory: the footprint, or two ray states of the tree walk
 
 __device__ __forceinline__ void flush_taps(float4* accum, int W, int H, int cx, int cy, const float* acc)
 {
@@ -547,37 +548,52 @@ __device__ __forceinline__ void trace_warp(const RenderArgs& A, const SurfRec* l
         atomicAdd(A.stats + 3 * pair, (unsigned long long)n_lanes * n_lambda);
 }
 
+// A render CTA's tables in shared memory.
+struct Staged {
+    HotRec* hot;
+    float4* spec;
+    float2* ab;        // per (wavelength, surface): (IOR after the surface, IOR before it), one
+                       // 8-byte shared load for either direction of the walk
+    float* kdel;
+    SurfRec* lens;
+    float* lanes;      // kLaneFloats per lane
+};
+
+__device__ __forceinline__ Staged stage_tables(const RenderArgs& A, unsigned char* smem_raw)
+{
+    Staged T;
+    T.hot = reinterpret_cast<HotRec*>(smem_raw);
+    T.spec = reinterpret_cast<float4*>(T.hot + A.n_surf);
+    T.ab = reinterpret_cast<float2*>(T.spec + A.n_spec);
+    T.kdel = reinterpret_cast<float*>(T.ab + A.n_spec * A.n_surf);
+    T.lens = reinterpret_cast<SurfRec*>(T.kdel + A.n_spec);
+    T.lanes = reinterpret_cast<float*>(T.lens + A.n_surf);
+    const int tid = threadIdx.x;
+    const int words = A.n_surf * (int)(sizeof(SurfRec) / 4);
+    const int* src = reinterpret_cast<const int*>(A.recs);
+    int* dst = reinterpret_cast<int*>(T.lens);
+    for (int i = tid; i < words; i += blockDim.x) dst[i] = src[i];
+    for (int i = tid; i < A.n_spec; i += blockDim.x)
+    {
+        T.spec[i] = A.spec[i];
+        // film phase factor of the MgF2 quarter-wave layer (fresnel.h:103, 168)
+        T.kdel[i] = 2.0f * kPi * 1.38f * (550.0f / (4.0f * 1.38f)) / A.spec[i].x;
+    }
+    const int nt = A.n_spec * A.n_surf;
+    for (int i = tid; i < nt; i += blockDim.x) T.ab[i] = make_float2(A.ior_at[i], A.ior_bf[i]);
+    __syncthreads();
+    for (int i = tid; i < A.n_surf; i += blockDim.x) T.hot[i] = make_hot(T.lens[i]);
+    __syncthreads();
+    return T;
+}
+
 template <bool PROBE>
 __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_render_kernel(const RenderArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HotRec* hot = reinterpret_cast<HotRec*>(smem_raw);
-    float4* spec = reinterpret_cast<float4*>(hot + A.n_surf);
-    // per (wavelength, surface): (IOR after the surface, IOR before it), one
-    // 8-byte shared load for either direction of the walk
-    float2* ab = reinterpret_cast<float2*>(spec + A.n_spec);
-    float* kdel = reinterpret_cast<float*>(ab + A.n_spec * A.n_surf);
-    SurfRec* lens = reinterpret_cast<SurfRec*>(kdel + A.n_spec);
-    float* acc_base = reinterpret_cast<float*>(lens + A.n_surf);
+    const Staged T = stage_tables(A, smem_raw);
     const int tid = threadIdx.x;
-    float* acc = acc_base + tid * kAccStride;   // 13 floats per lane: conflict-free banks
-    {
-        const int words = A.n_surf * (int)(sizeof(SurfRec) / 4);
-        const int* src = reinterpret_cast<const int*>(A.recs);
-        int* dst = reinterpret_cast<int*>(lens);
-        for (int i = tid; i < words; i += blockDim.x) dst[i] = src[i];
-        for (int i = tid; i < A.n_spec; i += blockDim.x)
-        {
-            spec[i] = A.spec[i];
-            // film phase factor of the MgF2 quarter-wave layer (fresnel.h:103, 168)
-            kdel[i] = 2.0f * kPi * 1.38f * (550.0f / (4.0f * 1.38f)) / A.spec[i].x;
-        }
-        const int nt = A.n_spec * A.n_surf;
-        for (int i = tid; i < nt; i += blockDim.x) ab[i] = make_float2(A.ior_at[i], A.ior_bf[i]);
-    }
-    __syncthreads();
-    for (int i = tid; i < A.n_surf; i += blockDim.x) hot[i] = make_hot(lens[i]);
-    __syncthreads();
+    float* acc = T.lanes + tid * kAccStride;   // 13 floats per lane: conflict-free banks
     // Warp-granular work: each warp takes one task at a time — a (pair,
     // source, 32-sample) item and one of its l_chunks wavelength ranges — so
     // no CTA-wide barrier sits inside the loop, and splitting the wavelengths
@@ -642,7 +658,218 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_render
         int sidx = w.z + lane;
         if (PROBE && A.perm != nullptr && active) sidx = A.perm[(size_t)w.x * A.perm_stride + sidx];
         const float2 uv = active ? A.samples[sidx] : make_float2(0.0f, 0.0f);
-        trace_warp<PROBE>(A, lens, hot, ab, spec, kdel, P, S, uv, active, acc, w.x, li0, li1, sidx);
+        trace_warp<PROBE>(A, T.lens, T.hot, T.ab, T.spec, T.kdel, P, S, uv, active, acc, w.x, li0, li1, sidx);
+    }
+}
+
+// ---- shared legs ---------------------------------------------------------------
+// Rays of one pupil sample, source and wavelength that belong to different
+// pairs walk the same way as long as their pairs agree: every pair (a, b) goes
+// forward through 0 .. b - 1, and every pair of one b turns there and comes back
+// through b - 1, b - 2, ....  The pairs that sample the same grid are therefore
+// walked as one tree: forward once, at each b back once, and from each a its
+// own last leg to the sensor.  Each ray still sees the operations of its own
+// walk in their order, so its landing and weight are the same.  All pairs of 24
+// surfaces are 4924 steps that way against 11224 pair by pair.
+//
+// The tree is cut into segments of a few hundred steps (which repeat the
+// forward leg up to their first b), a task is one segment of one 32-sample tile,
+// source and wavelength.  A segment is a list of runs, each a straight walk over
+// neighbouring surfaces with one step site; the ray states to come back to, before
+// the last b and before the last a, wait in the lane's shared-memory slot
+// (which the pair-by-pair walk uses for its splat footprint: a task has one
+// wavelength, so there is nothing to carry).
+// Bound by instruction issue, as the pair-by-pair walk.  24 surfaces, 253 pairs
+// on adaptive grids, 31 wavelengths: the frame 6.14 -> 2.61 ms (the render 5.15 ->
+// 1.65); 120 pairs x 5 sources, 64^2 x 16 wavelengths: 1.66 -> 0.52.
+enum RunFlags { RUN_REFLECT = 1, RUN_BACK = 2, RUN_LOAD_F = 4, RUN_LOAD_B = 8, RUN_SAVE_F = 16, RUN_SAVE_B = 32,
+                RUN_FORWARD = 64, RUN_LAST = 128 };
+
+// A run is an int4 {s0 | s1 << 8, flags, pair, skip}.  Walk from s0 to s1 (one surface at a time, backward with RUN_BACK), the first
+// step reflecting with RUN_REFLECT.  RUN_LAST: pair's last leg, splatted at its
+// end; skip: the run to go on with when every ray died on the way.
+struct TreeSegment { int run_begin, run_end, pair_begin, pair_end; };
+struct TreeGrid { int task_begin, sample_base, n_samples, tiles, seg_base, pad; };
+
+struct TreeArgs {
+    const TreeGrid* grids;          // n_grids + 1 (the last: the task count)
+    const TreeSegment* segments;
+    const int4* runs;
+    const int* pairs;               // pairs of the segments, in order
+    int n_grids, n_src;
+};
+
+// splat_ray for a single ray-wavelength: straight to the accumulator.  Called by
+// the whole warp; lanes whose ray did not land have valid = false.  Where all
+// landings of the warp share one 2 x 2 footprint (a focused ghost) they are
+// summed first, so that its pixels take one addition instead of 32.
+__device__ __forceinline__ void splat_now(const RenderArgs& A, const PairDev& P, const SourceDev& S, const float4& sp,
+                                          V3 o, V3 d, float w, bool valid)
+{
+    int x0 = 0, y0 = 0;
+    float v[12];
+    #pragma unroll
+    for (int q = 0; q < 12; ++q) v[q] = 0.0f;
+    const float ts = -o.z / d.z;
+    const float rx = o.x + d.x * ts, ry = o.y + d.y * ts;
+    const float base = w * P.w_ray * A.gain * P.boost;
+    float px = (rx / A.hw2 + 0.5f) * A.fmt_w + A.fmt_x0;
+    float py = (ry / A.hh2 + 0.5f) * A.fmt_h + A.fmt_y0;
+    valid = valid && fabsf(d.z) >= 1e-12f && ts >= 0.0f && isfinite(rx) && isfinite(ry) && !(base < 1e-14f) &&
+            isfinite(px) && isfinite(py);
+    if (valid)
+    {
+        px = fmaxf(-2.0e9f, fminf(2.0e9f, px));
+        py = fmaxf(-2.0e9f, fminf(2.0e9f, py));
+        x0 = (int)floorf(px - 0.5f);
+        y0 = (int)floorf(py - 0.5f);
+        // off the frame altogether: nothing to add
+        valid = x0 >= -1 && x0 < A.width && y0 >= -1 && y0 < A.height;
+    }
+    const unsigned m = __ballot_sync(kFull, valid);
+    if (m == 0) return;
+    if (valid)
+    {
+        const float fx = (px - 0.5f) - (float)x0, fy = (py - 0.5f) - (float)y0;
+        const float power = (S.r * sp.y + S.g * sp.z + S.b * sp.w) * base;
+        const float c0 = power * sp.y, c1 = power * sp.z, c2 = power * sp.w;
+        const float wt[4] = {(1.0f - fx) * (1.0f - fy), fx * (1.0f - fy), (1.0f - fx) * fy, fx * fy};
+        #pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            v[3 * q] = c0 * wt[q];
+            v[3 * q + 1] = c1 * wt[q];
+            v[3 * q + 2] = c2 * wt[q];
+        }
+    }
+    const int lead = __ffs(m) - 1;
+    const int lx = __shfl_sync(kFull, x0, lead), ly = __shfl_sync(kFull, y0, lead);
+    if (__popc(m) > 3 && __all_sync(kFull, !valid || (x0 == lx && y0 == ly)))
+    {
+        #pragma unroll
+        for (int q = 0; q < 12; ++q)
+            for (int k = 16; k > 0; k >>= 1) v[q] += __shfl_xor_sync(kFull, v[q], k);
+        if ((int)(threadIdx.x & 31) == lead) flush_taps(A.accum, A.width, A.height, lx, ly, v);
+        return;
+    }
+    if (valid) flush_taps(A.accum, A.width, A.height, x0, y0, v);
+}
+
+__global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_tree_kernel(const RenderArgs A, const TreeArgs G)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Staged T = stage_tables(A, smem_raw);
+    const int lane = threadIdx.x & 31;
+    // the lane's slot: the state before the last b, then (7 fields on) before the last a
+    float* slot = T.lanes + threadIdx.x;
+    const int n_tasks = G.grids[G.n_grids].task_begin;
+    for (;;)
+    {
+        int task = 0;
+        if (lane == 0) task = atomicAdd(A.counter, 1);
+        task = __shfl_sync(kFull, task, 0);
+        if (task >= n_tasks) break;
+        int lo = 0, hi = G.n_grids;
+        while (hi - lo > 1)
+        {
+            const int mid = (lo + hi) >> 1;
+            if (G.grids[mid].task_begin <= task) lo = mid;
+            else hi = mid;
+        }
+        // tiles fastest: neighbouring tasks land on different pixels
+        const TreeGrid g = G.grids[lo];
+        int r = task - g.task_begin;
+        const int tile = r % g.tiles;
+        r /= g.tiles;
+        const int si = r % G.n_src;
+        r /= G.n_src;
+        const int li = r % A.n_spec;
+        const TreeSegment seg = G.segments[g.seg_base + r / A.n_spec];
+        const bool active = tile * kTile + lane < g.n_samples;
+        const unsigned n_lanes = (unsigned)min(kTile, g.n_samples - tile * kTile);
+        // pairs found off the sensor are not walked; the others count as traced
+        unsigned live_pairs = 0;
+        for (int q = seg.pair_begin; q < seg.pair_end; q += 32)
+        {
+            const bool on = q + lane < seg.pair_end && (A.pair_hits == nullptr || A.pair_hits[G.pairs[q + lane]] != 0);
+            live_pairs += __popc(__ballot_sync(kFull, on));
+        }
+        if (live_pairs == 0) continue;
+        if (A.traced && lane == 0) atomicAdd(A.traced, (unsigned long long)n_lanes * live_pairs);
+        const SourceDev S = A.sources[si];
+        const float2 uv = active ? A.samples[g.sample_base + tile * kTile + lane] : make_float2(0.0f, 0.0f);
+        const float4 sp = T.spec[li];
+        const float kdelta = T.kdel[li];
+        const float2* abl = T.ab + li * A.n_surf;
+        V3 o = v3(uv.x * A.front_R + S.sdx, uv.y * A.front_R + S.sdy, A.start_z);
+        V3 d = v3(S.dx, S.dy, S.dz);
+        float w = 1.0f, cur = 1.0f, cur_f = 1.0f, cur_b = 1.0f;
+        bool alive = active;
+        unsigned alive_f = 0, alive_b = 0;
+        #pragma unroll 1
+        for (int ri = seg.run_begin; ri < seg.run_end; ++ri)
+        {
+            const int4 run = __ldg(G.runs + ri);
+            const int flags = run.y;
+            if ((flags & RUN_LAST) && A.pair_hits != nullptr && A.pair_hits[run.z] == 0) continue;
+            if (flags & (RUN_LOAD_F | RUN_LOAD_B))
+            {
+                const bool f = (flags & RUN_LOAD_F) != 0;
+                const float* q = slot + (f ? 0 : 7 * kRenderThreads);
+                o = v3(q[0], q[kRenderThreads], q[2 * kRenderThreads]);
+                d = v3(q[3 * kRenderThreads], q[4 * kRenderThreads], q[5 * kRenderThreads]);
+                w = q[6 * kRenderThreads];
+                cur = f ? cur_f : cur_b;
+                alive = (((f ? alive_f : alive_b) >> lane) & 1u) != 0;
+            }
+            const int s0 = run.x & 0xff, s1 = (run.x >> 8) & 0xff;
+            const int dir = (flags & RUN_BACK) ? -1 : 1;
+            int left = (flags & RUN_BACK) ? s0 - s1 : s1 - s0;
+            bool refl = (flags & RUN_REFLECT) != 0;
+            #pragma unroll 1
+            for (int s = s0; left >= 0; s += dir, --left, refl = false)
+            {
+                if (!__any_sync(kFull, alive)) break;
+                // a turn is met in the direction before it
+                const bool back = ((flags & RUN_BACK) != 0) != refl;
+                const HotRec hr = T.hot[s];
+                const float2 io = abl[s];
+                const float n2 = back ? io.y : io.x;
+                const float rior = (back && refl) ? io.x : cur;
+                bool ok;
+                if (hr.bits & HB_ROUND)
+                    ok = surface_step_fast<true, true>(o, d, hr, kdelta, n2, refl, back, abl + s, cur, w, alive);
+                else if (hr.bits & HB_FAST)
+                    ok = surface_step_fast<true, false>(o, d, hr, kdelta, n2, refl, back, abl + s, cur, w, alive);
+                else if (hr.bits & HB_ACTIVE)
+                    ok = surface_step<true>(o, d, hr, T.lens[s], sp.x, kdelta, n2, refl, rior, cur, w, alive);
+                else continue;
+                alive = ok;
+            }
+            const unsigned left_alive = __ballot_sync(kFull, alive);
+            if (flags & RUN_LAST)
+            {
+                if (left_alive) splat_now(A, A.pairs[run.z], S, sp, o, d, w, alive);
+                continue;
+            }
+            if (left_alive == 0)
+            {
+                // nothing comes of the runs that start from here
+                if (flags & RUN_FORWARD) break;
+                ri = run.w - 1;
+                continue;
+            }
+            if (flags & (RUN_SAVE_F | RUN_SAVE_B))
+            {
+                const bool f = (flags & RUN_SAVE_F) != 0;
+                float* q = slot + (f ? 0 : 7 * kRenderThreads);
+                q[0] = o.x; q[kRenderThreads] = o.y; q[2 * kRenderThreads] = o.z;
+                q[3 * kRenderThreads] = d.x; q[4 * kRenderThreads] = d.y; q[5 * kRenderThreads] = d.z;
+                q[6 * kRenderThreads] = w;
+                if (f) { cur_f = cur; alive_f = left_alive; }
+                else { cur_b = cur; alive_b = left_alive; }
+            }
+        }
     }
 }
 
@@ -756,6 +983,12 @@ struct GhostPlan {
     int per_sm = 0, n_sm = 0;           // resident render CTAs per SM, SM count
     int launch_ipw = 0;                 // 0: persistent queue; > 0: static chunks of this many items per warp
     int l_chunks = 1;                   // wavelength ranges per item (tasks per item)
+    // shared legs: pairs of one grid walked as a tree (n_tree_tasks > 0: used by the persistent queue)
+    int n_tree_tasks = 0, n_tree_grids = 0, n_src = 0;
+    TreeGrid* tree_grids = nullptr;
+    TreeSegment* tree_segments = nullptr;
+    int4* tree_runs = nullptr;
+    int* tree_pairs = nullptr;
     long long rays = 0;                 // ray-wavelength traces per execute
     float front_R = 0.0f, start_z = 0.0f;
     // off-sensor cull (probe passes)
@@ -803,7 +1036,8 @@ static void plan_free(GhostPlan* p)
     else if (p->executed && p->done) cudaEventSynchronize(p->done);
     void* blocks[] = {p->recs, p->ior_at, p->ior_bf, p->spec, p->items, p->pairs, p->sources, p->samples,
                       p->counter, p->accum, p->probe_items, p->probe_samples, p->pair_hits, p->probe_counters,
-                      p->traced, p->pair_hits_init, p->probe_death, p->probe_perm};
+                      p->traced, p->pair_hits_init, p->probe_death, p->probe_perm, p->tree_grids, p->tree_segments,
+                      p->tree_runs, p->tree_pairs};
     for (void* b : blocks)
     {
         if (!b) continue;
@@ -833,7 +1067,7 @@ static cudaError_t alloc(T** dst, size_t bytes, cudaMemPool_t pool, cudaStream_t
 size_t render_smem(int n_surf, int n_spec)
 {
     return (size_t)n_surf * 32 + (size_t)n_spec * 16 + (size_t)n_spec * 4 + 2 * (size_t)n_spec * n_surf * 4 +
-           (size_t)n_surf * sizeof(SurfRec) + (size_t)kRenderThreads * kAccStride * 4;
+           (size_t)n_surf * sizeof(SurfRec) + (size_t)kRenderThreads * kLaneFloats * 4;
 }
 
 // The opt-in only grows (per device and kernel), so a plan created earlier
@@ -856,6 +1090,7 @@ int raise_smem_limit(const void* kernel, size_t bytes)
 cudaError_t render_prepare(size_t smem, int* per_sm, int* n_sm)
 {
     cudaError_t e = (cudaError_t)raise_smem_limit((const void*)ghost_render_kernel<false>, smem);
+    if (e == cudaSuccess) e = (cudaError_t)raise_smem_limit((const void*)ghost_tree_kernel, smem);
     if (e == cudaSuccess) e = (cudaError_t)raise_smem_limit((const void*)ghost_render_kernel<true>, smem);
     if (e == cudaSuccess && per_sm) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, ghost_render_kernel<false>, kRenderThreads, smem);
     int dev = 0;
@@ -961,6 +1196,127 @@ int probe_grids(const gl_surface* surfaces, int n_surf, int blades_override, flo
 int default_lambda_split(int n_spec)
 {
     return std::max(1, std::min(n_spec, (n_spec + 4) / 8));
+}
+
+// The tree walk's tables (see "shared legs").  tasks = 0: the pair-by-pair walk
+// it is (a pair that turns at an inactive surface, or more tasks than a counter
+// holds).  Otherwise the tree is taken even where little is shared: one pair
+// alone, 128^2 x 31 wavelengths 51 us pair by pair, 48 as a tree; four pairs of
+// one b 166 / 123; 66 pairs 16^2 x 8 45 / 46, 96^2 x 16 542 / 343.
+struct TreeBuild {
+    std::vector<TreeGrid> grids;
+    std::vector<TreeSegment> segments;
+    std::vector<int4> runs;
+    std::vector<int> pairs;
+    int tasks = 0;
+};
+
+static TreeBuild build_tree(const SurfRec* recs, int n, const gl_ghost_pair* pairs, const int32_t* pair_grid,
+                            int n_pairs, const int32_t* grid_offsets, int n_grids, int n_src, int n_spec,
+                            long long warps)
+{
+    // active surfaces before each
+    std::vector<int> act((size_t)n + 1, 0);
+    for (int i = 0; i < n; ++i) act[i + 1] = act[i] + ((recs[i].flags & SF_ACTIVE) ? 1 : 0);
+    auto steps = [&](int from, int to) { return to >= from ? act[to + 1] - act[from] : 0; };     // surfaces from .. to
+    std::vector<std::vector<int>> of((size_t)n_grids);
+    for (int i = 0; i < n_pairs; ++i)
+    {
+        // the turn must be a step (an inactive surface is passed by unturned)
+        if (!(recs[pairs[i].surf_a].flags & SF_ACTIVE) || !(recs[pairs[i].surf_b].flags & SF_ACTIVE)) return {};
+        of[pair_grid ? pair_grid[i] : 0].push_back(i);
+    }
+    // steps of the whole tree over all tiles, sources and wavelengths
+    double whole = 0.0;
+    for (int g = 0; g < n_grids; ++g)
+    {
+        std::sort(of[g].begin(), of[g].end(), [&](int x, int y) {
+            return pairs[x].surf_b != pairs[y].surf_b ? pairs[x].surf_b < pairs[y].surf_b : pairs[x].surf_a > pairs[y].surf_a;
+        });
+        const double rays = (double)((grid_offsets[g + 1] - grid_offsets[g] + kTile - 1) / kTile) * n_src * n_spec;
+        int b0 = -1, a0 = 0, f = 0;
+        for (int i : of[g])
+        {
+            const int a = pairs[i].surf_a, b = pairs[i].surf_b;
+            if (b != b0)
+            {
+                whole += rays * (steps(f, b - 1) + 1);
+                f = b;
+                b0 = b;
+                a0 = b - 1;
+            }
+            whole += rays * (steps(a + 1, a0) + steps(a, n - 1));
+            a0 = a;
+        }
+    }
+    // about 20 tasks per resident warp, of a few hundred steps
+    const int target = (int)std::min(400.0, std::max(40.0, whole / (20.0 * (double)warps)));
+    TreeBuild T;
+    long long tasks = 0;
+    for (int g = 0; g < n_grids; ++g)
+    {
+        const int ng = grid_offsets[g + 1] - grid_offsets[g];
+        if (ng <= 0 || of[g].empty()) continue;
+        const TreeGrid G{(int)std::min<long long>(tasks, 1LL << 30), grid_offsets[g], ng, (ng + kTile - 1) / kTile, (int)T.segments.size(), 0};
+        int cost = 0, b0 = -1, a0 = 0, f = 0, last_f = -1, last_b = -1;
+        // the runs after an outer run that died: up to the next forward run, or the segment's end
+        auto close = [&] {
+            if (T.segments.size() == (size_t)G.seg_base || T.segments.back().run_end >= 0) return;
+            T.segments.back().run_end = (int)T.runs.size();
+            T.segments.back().pair_end = (int)T.pairs.size();
+            int next = (int)T.runs.size();
+            for (int r = (int)T.runs.size() - 1; r >= T.segments.back().run_begin; --r)
+            {
+                T.runs[r].w = next;
+                if (T.runs[r].y & RUN_FORWARD) next = r;
+            }
+        };
+        for (int i : of[g])
+        {
+            const int a = pairs[i].surf_a, b = pairs[i].surf_b;
+            if (b0 < 0 || cost >= target)
+            {
+                close();
+                T.segments.push_back({(int)T.runs.size(), -1, (int)T.pairs.size(), 0});
+                cost = 0;
+                b0 = -1;
+                f = 0;
+                last_f = -1;
+            }
+            if (b != b0)
+            {
+                // forward from the last b (or the start) to b - 1
+                if (last_f >= 0) T.runs[last_f].y |= RUN_SAVE_F;
+                T.runs.push_back(make_int4(f | ((b - 1) << 8), RUN_FORWARD | (last_f >= 0 ? RUN_LOAD_F : 0), -1, 0));
+                last_f = (int)T.runs.size() - 1;
+                cost += steps(f, b - 1);
+                // turn at b, back through b - 1 .. a + 1
+                T.runs.push_back(make_int4(b | ((a + 1) << 8), RUN_REFLECT | RUN_BACK, -1, 0));
+                cost += 1 + steps(a + 1, b - 1);
+                f = b;
+            }
+            else
+            {
+                // on from the last a: back through a0 .. a + 1
+                T.runs[last_b].y |= RUN_SAVE_B;
+                T.runs.push_back(make_int4(a0 | ((a + 1) << 8), RUN_BACK | RUN_LOAD_B, -1, 0));
+                cost += steps(a + 1, a0);
+            }
+            last_b = (int)T.runs.size() - 1;
+            T.runs.push_back(make_int4(a | ((n - 1) << 8), RUN_REFLECT | RUN_LAST, i, 0));
+            T.pairs.push_back(i);
+            cost += steps(a, n - 1);
+            b0 = b;
+            a0 = a;
+        }
+        close();
+        T.grids.push_back(G);
+        tasks += (long long)((int)T.segments.size() - G.seg_base) * G.tiles * n_src * n_spec;
+    }
+    if (tasks <= 0 || tasks >= (1LL << 30)) return {};
+    T.grids.push_back({(int)tasks, 0, 0, 1, (int)T.segments.size(), 0});
+    T.tasks = (int)tasks;
+    return T;
 }
 
 int plan_create(const gl_surface* surfaces, int n_surf, const gl_ghost_pair* pairs, const float* boosts,
@@ -1125,6 +1481,24 @@ int plan_create(const gl_surface* surfaces, int n_surf, const gl_ghost_pair* pai
             chk(upload(&p->probe_perm, ident.data(), ident.size(), pool, ost));
         }
     }
+    TreeBuild tree;
+    if (e == cudaSuccess && !prm->plain_per_pair && p->n_items > 0)
+    {
+        int n_sm = 0;
+        chk(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, p->device));
+        tree = build_tree(recs.data(), n_surf, pairs, pair_grid, n_pairs, grid_offsets, n_grids, n_src, n_spec,
+                          (long long)n_sm * kRenderMinBlocks * (kRenderThreads / 32));
+        if (tree.tasks > 0)
+        {
+            p->n_tree_tasks = tree.tasks;
+            p->n_tree_grids = (int)tree.grids.size() - 1;
+            p->n_src = n_src;
+            chk(upload(&p->tree_grids, tree.grids.data(), tree.grids.size(), pool, ost));
+            chk(upload(&p->tree_segments, tree.segments.data(), tree.segments.size(), pool, ost));
+            chk(upload(&p->tree_runs, tree.runs.data(), tree.runs.size(), pool, ost));
+            chk(upload(&p->tree_pairs, tree.pairs.data(), tree.pairs.size(), pool, ost));
+        }
+    }
     chk(alloc(&p->accum, (size_t)prm->width * prm->height * sizeof(float4), pool, ost));
     if (e == cudaSuccess) chk(cudaMemsetAsync(p->accum, 0, (size_t)prm->width * prm->height * sizeof(float4), ost));
     // the host vectors above go out of scope: the uploads must have landed
@@ -1142,11 +1516,12 @@ int plan_create(const gl_surface* surfaces, int n_surf, const gl_ghost_pair* pai
     p->per_sm = std::max(1, per_sm);
     p->n_sm = n_sm;
     p->queue_ctas = p->per_sm * n_sm;
-    // A plan of few items splits its wavelengths further, to about 20 tasks per
-    // resident warp: a task's chain of steps is what such a frame waits for.
-    // 66 pairs: 32^2 x 8 wavelengths 158 -> 64 us, 64^2 x 8 232 -> 139; 120 pairs x
-    // 5 sources, 42^2 x 8 621 -> 463; above (180850 items x 31) the default's
-    // eight wavelengths per task stay best (6128 us, 6326 with four).
+    // The pair-by-pair walk and the probes: a plan of few items splits its
+    // wavelengths further, to about 20 tasks per resident warp; a task's chain of
+    // steps is what such a frame waits for.  66 pairs pair by pair: 32^2 x 8
+    // wavelengths 158 -> 64 us, 64^2 x 8 232 -> 139; 120 pairs x 5 sources, 42^2 x 8
+    // 621 -> 463; above (180850 items x 31) the default's eight wavelengths per task
+    // stay best (6128 us, 6326 with four).
     if (!prm->plain_per_pair && p->n_items > 0)
     {
         const long long want = (20LL * p->queue_ctas * warps_per_block + p->n_items - 1) / p->n_items;
@@ -1295,7 +1670,13 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
         {
             GL_CUDA_TRY(cudaMemsetAsync(p->counter, 0, sizeof(int), st));
             A.counter = p->counter;
-            ghost_render_kernel<false><<<queue_grid(p, p->n_items, A.l_chunks), kRenderThreads, p->smem, st>>>(A);
+            if (p->n_tree_tasks > 0)
+            {
+                const TreeArgs G{p->tree_grids, p->tree_segments, p->tree_runs, p->tree_pairs, p->n_tree_grids, p->n_src};
+                ghost_tree_kernel<<<queue_grid(p, p->n_tree_tasks, 1), kRenderThreads, p->smem, st>>>(A, G);
+            }
+            else
+                ghost_render_kernel<false><<<queue_grid(p, p->n_items, A.l_chunks), kRenderThreads, p->smem, st>>>(A);
             GL_CUDA_TRY(cudaGetLastError());
             ++launches;
         }
