@@ -444,8 +444,7 @@ template <bool PROBE>
 __device__ __forceinline__ void trace_warp(const RenderArgs& A, const SurfRec* lens, const HotRec* hot,
                                            const float2* ab, const float4* spec,
                                            const float* kdel, const PairDev& P, const SourceDev& S,
-                                           float2 uv, bool active, float* acc, int pair, int li0, int li1,
-                                           int sidx)
+                                           float2 uv, bool active, float* acc, int pair, int li0, int li1)
 {
     const int n = A.n_surf, a = P.a, b = P.b;
     const int L1 = b + 1, L2 = L1 + (b - a), L = L2 + (n - 1 - a);
@@ -467,7 +466,6 @@ __device__ __forceinline__ void trace_warp(const RenderArgs& A, const SurfRec* l
         V3 d = v3(S.dx, S.dy, S.dz);
         float w = 1.0f, cur = 1.0f;
         bool alive = active;
-        int kdead = L;                          // the step the ray died at (L: it left the lens)
         #pragma unroll 1
         for (int k = 0; k < L; ++k)
         {
@@ -490,11 +488,8 @@ __device__ __forceinline__ void trace_warp(const RenderArgs& A, const SurfRec* l
             else if (hr.bits & HB_ACTIVE)
                 ok = surface_step<!PROBE>(o, d, hr, lens[s], sp.x, kdelta, n2, refl, rior, cur, w, alive);
             else continue;
-            if (PROBE && alive && !ok) kdead = k;
             alive = ok;
         }
-        if (PROBE && A.death != nullptr && active)
-            A.death[(size_t)pair * A.perm_stride + sidx] = (unsigned char)min(kdead, 255);
         if (PROBE)
         {
             // Off-sensor probe (the STATS pass of ghost_render.cu:402-415 with
@@ -623,11 +618,6 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_render
         const int item = (int)(task / chunks);
         const int chunk = (int)(task - (long long)item * chunks);
         int li0 = chunk * l_size, li1 = min(A.n_spec, li0 + l_size);
-        if (PROBE && A.lam_hi > 0)
-        {
-            li0 = max(li0, A.lam_lo);
-            li1 = min(li1, A.lam_hi);
-        }
         if (li0 >= li1) continue;
         int4 w;
         if (A.items != nullptr) w = A.items[item];
@@ -655,10 +645,8 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_render
         if (A.items == nullptr) P.w_ray = A.w_uniform;
         const SourceDev S = A.sources[w.y];
         const bool active = lane < w.w;
-        int sidx = w.z + lane;
-        if (PROBE && A.perm != nullptr && active) sidx = A.perm[(size_t)w.x * A.perm_stride + sidx];
-        const float2 uv = active ? A.samples[sidx] : make_float2(0.0f, 0.0f);
-        trace_warp<PROBE>(A, T.lens, T.hot, T.ab, T.spec, T.kdel, P, S, uv, active, acc, w.x, li0, li1, sidx);
+        const float2 uv = active ? A.samples[w.z + lane] : make_float2(0.0f, 0.0f);
+        trace_warp<PROBE>(A, T.lens, T.hot, T.ab, T.spec, T.kdel, P, S, uv, active, acc, w.x, li0, li1);
     }
 }
 
@@ -679,17 +667,23 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_render
 // the last b and before the last a, wait in the lane's shared-memory slot
 // (which the pair-by-pair walk uses for its splat footprint: a task has one
 // wavelength, so there is nothing to carry).
-// Bound by instruction issue, as the pair-by-pair walk.  24 surfaces, 253 pairs
-// on adaptive grids, 31 wavelengths: the frame 6.14 -> 2.61 ms (the render 5.15 ->
-// 1.65); 120 pairs x 5 sources, 64^2 x 16 wavelengths: 1.66 -> 0.52.
+// Bound by instruction issue (74% of the slots, the rest mostly waits for
+// instructions: the warps of an SM stand at different surfaces, and the code of
+// all kinds of step is larger than the first instruction cache, so the round-stop
+// copy of the common step is left out here, 2%).  24 surfaces, 253 pairs on
+// adaptive grids, 31 wavelengths: the render 5.15 -> 1.60 ms; 120 pairs x 5
+// sources, 64^2 x 16 wavelengths: 1.66 -> 0.50.
 enum RunFlags { RUN_REFLECT = 1, RUN_BACK = 2, RUN_LOAD_F = 4, RUN_LOAD_B = 8, RUN_SAVE_F = 16, RUN_SAVE_B = 32,
                 RUN_FORWARD = 64, RUN_LAST = 128 };
 
-// A run is an int4 {s0 | s1 << 8, flags, pair, skip}.  Walk from s0 to s1 (one surface at a time, backward with RUN_BACK), the first
-// step reflecting with RUN_REFLECT.  RUN_LAST: pair's last leg, splatted at its
-// end; skip: the run to go on with when every ray died on the way.
+// A run is an int4 {s0 | s1 << 8, flags, pairs, skip}.  Walk from s0 to s1 (one
+// surface at a time, backward with RUN_BACK), the first step reflecting with
+// RUN_REFLECT.  pairs: the pairs of the segment (at most
+// 32) that hang on the run, as their mask; skip: the run to go on with when none
+// of them is wanted any more or every ray died on the way.  RUN_LAST: the last
+// leg of one pair, splatted at its end.
 struct TreeSegment { int run_begin, run_end, pair_begin, pair_end; };
-struct TreeGrid { int task_begin, sample_base, n_samples, tiles, seg_base, pad; };
+struct TreeGrid { int task_begin, sample_base, n_samples, tiles, seg_base, n_segs; };
 
 struct TreeArgs {
     const TreeGrid* grids;          // n_grids + 1 (the last: the task count)
@@ -749,12 +743,29 @@ __device__ __forceinline__ void splat_now(const RenderArgs& A, const PairDev& P,
         #pragma unroll
         for (int q = 0; q < 12; ++q)
             for (int k = 16; k > 0; k >>= 1) v[q] += __shfl_xor_sync(kFull, v[q], k);
-        if ((int)(threadIdx.x & 31) == lead) flush_taps(A.accum, A.width, A.height, lx, ly, v);
-        return;
+        valid = (int)(threadIdx.x & 31) == lead;
     }
     if (valid) flush_taps(A.accum, A.width, A.height, x0, y0, v);
 }
 
+// Whether the lane's ray landed inside the inflated frame (see trace_warp).
+__device__ __forceinline__ bool probe_hit(const RenderArgs& A, V3 o, V3 d, bool alive)
+{
+    if (!alive || !(fabsf(d.z) >= 1e-12f)) return false;
+    const float ts = -o.z / d.z;
+    if (!(ts >= 0.0f)) return false;
+    const float sx = o.x + d.x * ts, sy = o.y + d.y * ts;
+    const float spx = (sx / A.hw2 + 0.5f) * A.fmt_w + A.fmt_x0;
+    const float spy = (sy / A.hh2 + 0.5f) * A.fmt_h + A.fmt_y0;
+    return isfinite(spx) && isfinite(spy) && spx >= 0.0f && spx < (float)A.width && spy >= 0.0f && spy < (float)A.height;
+}
+
+// PROBE: the off-sensor probe (see trace_warp).  Pairs with a hit are not wanted
+// any more; wavelengths are the slowest index, so that the first finds most of
+// them.  The frame above: the probe pair by pair in two stages (the second with
+// its samples sorted by where the first wavelength's ray died) 0.95 ms, as a tree
+// 0.44.
+template <bool PROBE>
 __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_tree_kernel(const RenderArgs A, const TreeArgs G)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -783,19 +794,21 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_tree_k
         r /= g.tiles;
         const int si = r % G.n_src;
         r /= G.n_src;
-        const int li = r % A.n_spec;
-        const TreeSegment seg = G.segments[g.seg_base + r / A.n_spec];
+        const int li = PROBE ? r / g.n_segs : r % A.n_spec;
+        const TreeSegment seg = G.segments[g.seg_base + (PROBE ? r % g.n_segs : r / A.n_spec)];
         const bool active = tile * kTile + lane < g.n_samples;
         const unsigned n_lanes = (unsigned)min(kTile, g.n_samples - tile * kTile);
-        // pairs found off the sensor are not walked; the others count as traced
-        unsigned live_pairs = 0;
-        for (int q = seg.pair_begin; q < seg.pair_end; q += 32)
+        // the pairs to walk: probe, those without a hit yet (read through L2,
+        // where the other warps' atomics land); render, those with one
+        bool on = seg.pair_begin + lane < seg.pair_end;
+        if (on && A.pair_hits != nullptr)
         {
-            const bool on = q + lane < seg.pair_end && (A.pair_hits == nullptr || A.pair_hits[G.pairs[q + lane]] != 0);
-            live_pairs += __popc(__ballot_sync(kFull, on));
+            const int* hit = A.pair_hits + G.pairs[seg.pair_begin + lane];
+            on = PROBE ? __ldcg(hit) == 0 : *hit != 0;
         }
-        if (live_pairs == 0) continue;
-        if (A.traced && lane == 0) atomicAdd(A.traced, (unsigned long long)n_lanes * live_pairs);
+        unsigned want = __ballot_sync(kFull, on);
+        if (want == 0) continue;
+        if (A.traced && lane == 0) atomicAdd(A.traced, (unsigned long long)n_lanes * __popc(want));
         const SourceDev S = A.sources[si];
         const float2 uv = active ? A.samples[g.sample_base + tile * kTile + lane] : make_float2(0.0f, 0.0f);
         const float4 sp = T.spec[li];
@@ -811,7 +824,12 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_tree_k
         {
             const int4 run = __ldg(G.runs + ri);
             const int flags = run.y;
-            if ((flags & RUN_LAST) && A.pair_hits != nullptr && A.pair_hits[run.z] == 0) continue;
+            if (((unsigned)run.z & want) == 0)
+            {
+                if (flags & RUN_FORWARD) break;          // nor anything after it
+                if (!(flags & RUN_LAST)) ri = run.w - 1;
+                continue;
+            }
             if (flags & (RUN_LOAD_F | RUN_LOAD_B))
             {
                 const bool f = (flags & RUN_LOAD_F) != 0;
@@ -837,19 +855,26 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_tree_k
                 const float n2 = back ? io.y : io.x;
                 const float rior = (back && refl) ? io.x : cur;
                 bool ok;
-                if (hr.bits & HB_ROUND)
-                    ok = surface_step_fast<true, true>(o, d, hr, kdelta, n2, refl, back, abl + s, cur, w, alive);
-                else if (hr.bits & HB_FAST)
-                    ok = surface_step_fast<true, false>(o, d, hr, kdelta, n2, refl, back, abl + s, cur, w, alive);
+                if (hr.bits & HB_FAST)          // (a round stop's aspect factor is exactly 1)
+                    ok = surface_step_fast<!PROBE, false>(o, d, hr, kdelta, n2, refl, back, abl + s, cur, w, alive);
                 else if (hr.bits & HB_ACTIVE)
-                    ok = surface_step<true>(o, d, hr, T.lens[s], sp.x, kdelta, n2, refl, rior, cur, w, alive);
+                    ok = surface_step<!PROBE>(o, d, hr, T.lens[s], sp.x, kdelta, n2, refl, rior, cur, w, alive);
                 else continue;
                 alive = ok;
             }
             const unsigned left_alive = __ballot_sync(kFull, alive);
             if (flags & RUN_LAST)
             {
-                if (left_alive) splat_now(A, A.pairs[run.z], S, sp, o, d, w, alive);
+                const int pair = G.pairs[seg.pair_begin + __ffs(run.z) - 1];
+                if (PROBE)
+                {
+                    if (__any_sync(kFull, probe_hit(A, o, d, alive)))
+                    {
+                        if (lane == 0) atomicAdd(A.pair_hits + pair, 1);
+                        want &= ~(unsigned)run.z;
+                    }
+                }
+                else if (left_alive) splat_now(A, A.pairs[pair], S, sp, o, d, w, alive);
                 continue;
             }
             if (left_alive == 0)
@@ -870,51 +895,6 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_tree_k
                 else { cur_b = cur; alive_b = left_alive; }
             }
         }
-    }
-}
-
-// Between the probe's two stages: each (pair, pass) still without a hit gets
-// its samples sorted by the death step of their first-wavelength ray (stable
-// counting sort, one warp), so the second stage's warps hold rays that leave
-// the lens together.  The set of samples is unchanged; only their order.
-__global__ void __launch_bounds__(32) probe_sort_kernel(const unsigned char* __restrict__ death,
-                                                        unsigned short* __restrict__ perm,
-                                                        const int* __restrict__ pair_hits, int stride, int b0,
-                                                        int b1, int b2, int b3)
-{
-    __shared__ int off[257];
-    const int pair = blockIdx.x, pass = blockIdx.y, lane = threadIdx.x;
-    if (pair_hits[pair] > 0) return;              // found on the sensor: stage 2 skips it
-    const int lo = pass == 0 ? b0 : (pass == 1 ? b1 : b2);
-    const int hi = pass == 0 ? b1 : (pass == 1 ? b2 : b3);
-    const unsigned char* d = death + (size_t)pair * stride;
-    unsigned short* out = perm + (size_t)pair * stride;
-    for (int b = lane; b < 257; b += 32) off[b] = 0;
-    __syncwarp();
-    for (int i = lo + lane; i < hi; i += 32) atomicAdd(&off[d[i]], 1);
-    __syncwarp();
-    if (lane == 0)
-    {
-        int run = lo;
-        for (int b = 0; b < 256; ++b)
-        {
-            const int c = off[b];
-            off[b] = run;
-            run += c;
-        }
-    }
-    __syncwarp();
-    for (int c0 = lo; c0 < hi; c0 += 32)
-    {
-        const int i = c0 + lane;
-        const bool v = i < hi;
-        const int key = v ? (int)d[i] : 256;
-        const unsigned m = __match_any_sync(kFull, key);
-        const int rank = __popc(m & ((1u << lane) - 1u));
-        if (v) out[off[key] + rank] = (unsigned short)i;
-        __syncwarp();
-        if (v && rank == 0) off[key] += __popc(m);
-        __syncwarp();
     }
 }
 
@@ -961,6 +941,15 @@ __global__ void ghost_flush_kernel(const float4* __restrict__ accum, size_t n_px
 // ---------------------------------------------------------------------------
 // Plan: resident device state of one ghost render request.
 // ---------------------------------------------------------------------------
+// A tree of shared legs (TreeArgs) on the device.
+struct TreeDev {
+    int n_tasks = 0, n_grids = 0;
+    TreeGrid* grids = nullptr;
+    TreeSegment* segments = nullptr;
+    int4* runs = nullptr;
+    int* pairs = nullptr;
+};
+
 struct GhostPlan {
     int device = 0;
     int n_surf = 0, n_spec = 0, n_pairs = 0, n_items = 0;
@@ -983,22 +972,15 @@ struct GhostPlan {
     int per_sm = 0, n_sm = 0;           // resident render CTAs per SM, SM count
     int launch_ipw = 0;                 // 0: persistent queue; > 0: static chunks of this many items per warp
     int l_chunks = 1;                   // wavelength ranges per item (tasks per item)
-    // shared legs: pairs of one grid walked as a tree (n_tree_tasks > 0: used by the persistent queue)
-    int n_tree_tasks = 0, n_tree_grids = 0, n_src = 0;
-    TreeGrid* tree_grids = nullptr;
-    TreeSegment* tree_segments = nullptr;
-    int4* tree_runs = nullptr;
-    int* tree_pairs = nullptr;
+    // shared legs (n_tasks > 0: used by the persistent queue, and by the probe)
+    int n_src = 0;
+    TreeDev tree, probe_tree;
     long long rays = 0;                 // ray-wavelength traces per execute
     float front_R = 0.0f, start_z = 0.0f;
     // off-sensor cull (probe passes)
     bool cull = false;
     int4* probe_items = nullptr;
     float2* probe_samples = nullptr;
-    unsigned char* probe_death = nullptr;     // two-stage probe (one source): death steps
-    unsigned short* probe_perm = nullptr;     // and the sorted sample order, per pair
-    int probe_samples_n = 0;
-    int probe_sample_begin[4] = {0, 0, 0, 0}; // sample range of each pass
     int probe_begin[4] = {0, 0, 0, 0};   // item range of each pass
     int* pair_hits = nullptr;
     int* probe_counters = nullptr;
@@ -1036,8 +1018,8 @@ static void plan_free(GhostPlan* p)
     else if (p->executed && p->done) cudaEventSynchronize(p->done);
     void* blocks[] = {p->recs, p->ior_at, p->ior_bf, p->spec, p->items, p->pairs, p->sources, p->samples,
                       p->counter, p->accum, p->probe_items, p->probe_samples, p->pair_hits, p->probe_counters,
-                      p->traced, p->pair_hits_init, p->probe_death, p->probe_perm, p->tree_grids, p->tree_segments,
-                      p->tree_runs, p->tree_pairs};
+                      p->traced, p->pair_hits_init, p->tree.grids, p->tree.segments, p->tree.runs, p->tree.pairs,
+                      p->probe_tree.grids, p->probe_tree.segments, p->probe_tree.runs, p->probe_tree.pairs};
     for (void* b : blocks)
     {
         if (!b) continue;
@@ -1090,7 +1072,8 @@ int raise_smem_limit(const void* kernel, size_t bytes)
 cudaError_t render_prepare(size_t smem, int* per_sm, int* n_sm)
 {
     cudaError_t e = (cudaError_t)raise_smem_limit((const void*)ghost_render_kernel<false>, smem);
-    if (e == cudaSuccess) e = (cudaError_t)raise_smem_limit((const void*)ghost_tree_kernel, smem);
+    if (e == cudaSuccess) e = (cudaError_t)raise_smem_limit((const void*)ghost_tree_kernel<false>, smem);
+    if (e == cudaSuccess) e = (cudaError_t)raise_smem_limit((const void*)ghost_tree_kernel<true>, smem);
     if (e == cudaSuccess) e = (cudaError_t)raise_smem_limit((const void*)ghost_render_kernel<true>, smem);
     if (e == cudaSuccess && per_sm) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, ghost_render_kernel<false>, kRenderThreads, smem);
     int dev = 0;
@@ -1211,31 +1194,29 @@ struct TreeBuild {
     int tasks = 0;
 };
 
-static TreeBuild build_tree(const SurfRec* recs, int n, const gl_ghost_pair* pairs, const int32_t* pair_grid,
-                            int n_pairs, const int32_t* grid_offsets, int n_grids, int n_src, int n_spec,
-                            long long warps)
+// Groups of pairs with the samples [base, base + n) that each is traced on.
+struct TreeGroup { std::vector<int> pairs; int base, n; };
+
+static TreeBuild build_tree(const SurfRec* recs, int n, const gl_ghost_pair* pairs, std::vector<TreeGroup> groups,
+                            int n_src, int n_spec, long long warps)
 {
     // active surfaces before each
     std::vector<int> act((size_t)n + 1, 0);
     for (int i = 0; i < n; ++i) act[i + 1] = act[i] + ((recs[i].flags & SF_ACTIVE) ? 1 : 0);
     auto steps = [&](int from, int to) { return to >= from ? act[to + 1] - act[from] : 0; };     // surfaces from .. to
-    std::vector<std::vector<int>> of((size_t)n_grids);
-    for (int i = 0; i < n_pairs; ++i)
-    {
-        // the turn must be a step (an inactive surface is passed by unturned)
-        if (!(recs[pairs[i].surf_a].flags & SF_ACTIVE) || !(recs[pairs[i].surf_b].flags & SF_ACTIVE)) return {};
-        of[pair_grid ? pair_grid[i] : 0].push_back(i);
-    }
+    for (const TreeGroup& g : groups)
+        for (int i : g.pairs)       // the turn must be a step (an inactive surface is passed by unturned)
+            if (!(recs[pairs[i].surf_a].flags & SF_ACTIVE) || !(recs[pairs[i].surf_b].flags & SF_ACTIVE)) return {};
     // steps of the whole tree over all tiles, sources and wavelengths
     double whole = 0.0;
-    for (int g = 0; g < n_grids; ++g)
+    for (TreeGroup& g : groups)
     {
-        std::sort(of[g].begin(), of[g].end(), [&](int x, int y) {
+        std::sort(g.pairs.begin(), g.pairs.end(), [&](int x, int y) {
             return pairs[x].surf_b != pairs[y].surf_b ? pairs[x].surf_b < pairs[y].surf_b : pairs[x].surf_a > pairs[y].surf_a;
         });
-        const double rays = (double)((grid_offsets[g + 1] - grid_offsets[g] + kTile - 1) / kTile) * n_src * n_spec;
+        const double rays = (double)((g.n + kTile - 1) / kTile) * n_src * n_spec;
         int b0 = -1, a0 = 0, f = 0;
-        for (int i : of[g])
+        for (int i : g.pairs)
         {
             const int a = pairs[i].surf_a, b = pairs[i].surf_b;
             if (b != b0)
@@ -1253,28 +1234,40 @@ static TreeBuild build_tree(const SurfRec* recs, int n, const gl_ghost_pair* pai
     const int target = (int)std::min(400.0, std::max(40.0, whole / (20.0 * (double)warps)));
     TreeBuild T;
     long long tasks = 0;
-    for (int g = 0; g < n_grids; ++g)
+    for (const TreeGroup& g : groups)
     {
-        const int ng = grid_offsets[g + 1] - grid_offsets[g];
-        if (ng <= 0 || of[g].empty()) continue;
-        const TreeGrid G{(int)std::min<long long>(tasks, 1LL << 30), grid_offsets[g], ng, (ng + kTile - 1) / kTile, (int)T.segments.size(), 0};
+        if (g.n <= 0 || g.pairs.empty()) continue;
+        TreeGrid G{(int)std::min<long long>(tasks, 1LL << 30), g.base, g.n, (g.n + kTile - 1) / kTile, (int)T.segments.size(), 0};
         int cost = 0, b0 = -1, a0 = 0, f = 0, last_f = -1, last_b = -1;
-        // the runs after an outer run that died: up to the next forward run, or the segment's end
+        // A segment's end: which pairs hang on each run (a forward run: all from
+        // its b on; a backward run: those of its b from its a on), and where to
+        // go on without it (the next forward run, or the end).
         auto close = [&] {
             if (T.segments.size() == (size_t)G.seg_base || T.segments.back().run_end >= 0) return;
-            T.segments.back().run_end = (int)T.runs.size();
-            T.segments.back().pair_end = (int)T.pairs.size();
-            int next = (int)T.runs.size();
-            for (int r = (int)T.runs.size() - 1; r >= T.segments.back().run_begin; --r)
+            TreeSegment& seg = T.segments.back();
+            seg.run_end = (int)T.runs.size();
+            seg.pair_end = (int)T.pairs.size();
+            int next = seg.run_end;
+            unsigned after = 0, of_b = 0;
+            for (int r = seg.run_end - 1; r >= seg.run_begin; --r)
             {
-                T.runs[r].w = next;
-                if (T.runs[r].y & RUN_FORWARD) next = r;
+                int4& run = T.runs[r];
+                run.w = next;
+                if (run.y & RUN_LAST) of_b |= (unsigned)run.z;
+                else if (run.y & RUN_FORWARD)
+                {
+                    after |= of_b;
+                    of_b = 0;
+                    run.z = (int)after;
+                    next = r;
+                }
+                else run.z = (int)of_b;
             }
         };
-        for (int i : of[g])
+        for (int i : g.pairs)
         {
             const int a = pairs[i].surf_a, b = pairs[i].surf_b;
-            if (b0 < 0 || cost >= target)
+            if (b0 < 0 || cost >= target || (int)T.pairs.size() - T.segments.back().pair_begin >= 32)
             {
                 close();
                 T.segments.push_back({(int)T.runs.size(), -1, (int)T.pairs.size(), 0});
@@ -1287,11 +1280,11 @@ static TreeBuild build_tree(const SurfRec* recs, int n, const gl_ghost_pair* pai
             {
                 // forward from the last b (or the start) to b - 1
                 if (last_f >= 0) T.runs[last_f].y |= RUN_SAVE_F;
-                T.runs.push_back(make_int4(f | ((b - 1) << 8), RUN_FORWARD | (last_f >= 0 ? RUN_LOAD_F : 0), -1, 0));
+                T.runs.push_back(make_int4(f | ((b - 1) << 8), RUN_FORWARD | (last_f >= 0 ? RUN_LOAD_F : 0), 0, 0));
                 last_f = (int)T.runs.size() - 1;
                 cost += steps(f, b - 1);
                 // turn at b, back through b - 1 .. a + 1
-                T.runs.push_back(make_int4(b | ((a + 1) << 8), RUN_REFLECT | RUN_BACK, -1, 0));
+                T.runs.push_back(make_int4(b | ((a + 1) << 8), RUN_REFLECT | RUN_BACK, 0, 0));
                 cost += 1 + steps(a + 1, b - 1);
                 f = b;
             }
@@ -1299,19 +1292,21 @@ static TreeBuild build_tree(const SurfRec* recs, int n, const gl_ghost_pair* pai
             {
                 // on from the last a: back through a0 .. a + 1
                 T.runs[last_b].y |= RUN_SAVE_B;
-                T.runs.push_back(make_int4(a0 | ((a + 1) << 8), RUN_BACK | RUN_LOAD_B, -1, 0));
+                T.runs.push_back(make_int4(a0 | ((a + 1) << 8), RUN_BACK | RUN_LOAD_B, 0, 0));
                 cost += steps(a + 1, a0);
             }
             last_b = (int)T.runs.size() - 1;
-            T.runs.push_back(make_int4(a | ((n - 1) << 8), RUN_REFLECT | RUN_LAST, i, 0));
+            T.runs.push_back(make_int4(a | ((n - 1) << 8), RUN_REFLECT | RUN_LAST,
+                                       (int)(1u << ((int)T.pairs.size() - T.segments.back().pair_begin)), 0));
             T.pairs.push_back(i);
             cost += steps(a, n - 1);
             b0 = b;
             a0 = a;
         }
         close();
+        G.n_segs = (int)T.segments.size() - G.seg_base;
         T.grids.push_back(G);
-        tasks += (long long)((int)T.segments.size() - G.seg_base) * G.tiles * n_src * n_spec;
+        tasks += (long long)G.n_segs * G.tiles * n_src * n_spec;
     }
     if (tasks <= 0 || tasks >= (1LL << 30)) return {};
     T.grids.push_back({(int)tasks, 0, 0, 1, (int)T.segments.size(), 0});
@@ -1415,8 +1410,6 @@ int plan_create(const gl_surface* surfaces, int n_surf, const gl_ghost_pair* pai
             if (rcs) { plan_free(p); return rcs; }
         }
         const int n_probe_samples = pbeg[3];
-        p->probe_samples_n = n_probe_samples;
-        for (int q = 0; q < 4; ++q) p->probe_sample_begin[q] = pbeg[q];
         for (int i = 0; i < n_pairs; ++i)
         {
             const int gi = pair_grid ? pair_grid[i] : 0;
@@ -1471,32 +1464,37 @@ int plan_create(const gl_surface* surfaces, int n_surf, const gl_ghost_pair* pai
         chk(alloc(&p->pair_hits, sizeof(int) * std::max(1, n_pairs), pool, ost));
         chk(upload(&p->pair_hits_init, hits_init.data(), hits_init.size(), pool, ost));
         chk(alloc(&p->probe_counters, sizeof(int) * 4, pool, ost));
-        if (n_src == 1 && n_spec > 1 && p->probe_samples_n > 0 && p->probe_samples_n < 65536)
-        {
-            const size_t cells = (size_t)std::max(1, n_pairs) * p->probe_samples_n;
-            chk(alloc(&p->probe_death, cells, pool, ost));
-            // the identity order to start from: every entry a valid sample of its own pass
-            std::vector<unsigned short> ident(cells);
-            for (size_t c = 0; c < cells; ++c) ident[c] = (unsigned short)(c % (size_t)p->probe_samples_n);
-            chk(upload(&p->probe_perm, ident.data(), ident.size(), pool, ost));
-        }
     }
-    TreeBuild tree;
-    if (e == cudaSuccess && !prm->plain_per_pair && p->n_items > 0)
+    TreeBuild trees[2];
+    if (e == cudaSuccess && p->n_items > 0)
     {
         int n_sm = 0;
         chk(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, p->device));
-        tree = build_tree(recs.data(), n_surf, pairs, pair_grid, n_pairs, grid_offsets, n_grids, n_src, n_spec,
-                          (long long)n_sm * kRenderMinBlocks * (kRenderThreads / 32));
-        if (tree.tasks > 0)
+        const long long warps = (long long)n_sm * kRenderMinBlocks * (kRenderThreads / 32);
+        p->n_src = n_src;
+        auto put = [&](TreeBuild& t, TreeDev& d, std::vector<TreeGroup> groups) {
+            t = build_tree(recs.data(), n_surf, pairs, std::move(groups), n_src, n_spec, warps);
+            if (t.tasks <= 0) return;
+            d.n_tasks = t.tasks;
+            d.n_grids = (int)t.grids.size() - 1;
+            chk(upload(&d.grids, t.grids.data(), t.grids.size(), pool, ost));
+            chk(upload(&d.segments, t.segments.data(), t.segments.size(), pool, ost));
+            chk(upload(&d.runs, t.runs.data(), t.runs.size(), pool, ost));
+            chk(upload(&d.pairs, t.pairs.data(), t.pairs.size(), pool, ost));
+        };
+        if (!prm->plain_per_pair)
         {
-            p->n_tree_tasks = tree.tasks;
-            p->n_tree_grids = (int)tree.grids.size() - 1;
-            p->n_src = n_src;
-            chk(upload(&p->tree_grids, tree.grids.data(), tree.grids.size(), pool, ost));
-            chk(upload(&p->tree_segments, tree.segments.data(), tree.segments.size(), pool, ost));
-            chk(upload(&p->tree_runs, tree.runs.data(), tree.runs.size(), pool, ost));
-            chk(upload(&p->tree_pairs, tree.pairs.data(), tree.pairs.size(), pool, ost));
+            std::vector<TreeGroup> groups((size_t)n_grids);
+            for (int g = 0; g < n_grids; ++g) groups[g] = {{}, grid_offsets[g], grid_offsets[g + 1] - grid_offsets[g]};
+            for (int i = 0; i < n_pairs; ++i) groups[pair_grid ? pair_grid[i] : 0].pairs.push_back(i);
+            put(trees[0], p->tree, std::move(groups));
+        }
+        if (p->cull)
+        {
+            TreeGroup probed{{}, 0, (int)psamples.size()};
+            for (int i = 0; i < n_pairs; ++i)
+                if (hits_init[i] == 0) probed.pairs.push_back(i);
+            put(trees[1], p->probe_tree, {std::move(probed)});
         }
     }
     chk(alloc(&p->accum, (size_t)prm->width * prm->height * sizeof(float4), pool, ost));
@@ -1555,6 +1553,11 @@ static int queue_grid(const GhostPlan* p, long long items, int chunks)
     return (int)std::max<long long>(1, std::min<long long>((tasks + warps_per_block - 1) / warps_per_block, p->queue_ctas));
 }
 
+static TreeArgs tree_args(const GhostPlan* p, const TreeDev& t)
+{
+    return {t.grids, t.segments, t.runs, t.pairs, t.n_grids, p->n_src};
+}
+
 // An event recorded inside a stream capture becomes an event-record node
 // (external), so a replayed graph records it too.
 static cudaError_t record_event(cudaEvent_t ev, cudaStream_t st)
@@ -1601,7 +1604,6 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
         GL_CUDA_TRY(cudaMemsetAsync(p->probe_counters, 0, sizeof(int) * 4, st));
         RenderArgs B = A;
         B.samples = p->probe_samples;
-        B.items = p->probe_items;
         B.pair_hits = p->pair_hits;
         B.traced = p->traced + 1;
         B.hw2 = 2.0f * (p->prm.sensor_half_w * 1.25f);
@@ -1612,30 +1614,12 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
             B.items = p->probe_items;
             B.n_items = n_it;
             B.counter = p->probe_counters;
-            const int grid = queue_grid(p, n_it, B.l_chunks);
-            if (p->probe_perm != nullptr)
-            {
-                // stage 1: every probe ray's first wavelength, recording where it died
-                RenderArgs B1 = B;
-                B1.lam_lo = 0; B1.lam_hi = 1; B1.l_chunks = 1;
-                B1.death = p->probe_death; B1.perm_stride = p->probe_samples_n;
-                ghost_render_kernel<true><<<queue_grid(p, n_it, 1), kRenderThreads, p->smem, st>>>(B1);
-                const int* sb = p->probe_sample_begin;
-                probe_sort_kernel<<<dim3((unsigned)p->n_pairs, 3), 32, 0, st>>>(
-                    p->probe_death, p->probe_perm, p->pair_hits, p->probe_samples_n, sb[0], sb[1], sb[2], sb[3]);
-                // stage 2: the other wavelengths of the pairs still without a hit, samples in sorted order
-                RenderArgs B2 = B;
-                B2.lam_lo = 1; B2.lam_hi = p->n_spec;
-                B2.perm = p->probe_perm; B2.perm_stride = p->probe_samples_n;
-                B2.counter = p->probe_counters + 1;
-                ghost_render_kernel<true><<<grid, kRenderThreads, p->smem, st>>>(B2);
-                launches += 3;
-            }
+            if (p->probe_tree.n_tasks > 0)
+                ghost_tree_kernel<true><<<queue_grid(p, p->probe_tree.n_tasks, 1), kRenderThreads, p->smem, st>>>(
+                    B, tree_args(p, p->probe_tree));
             else
-            {
-                ghost_render_kernel<true><<<grid, kRenderThreads, p->smem, st>>>(B);
-                ++launches;
-            }
+                ghost_render_kernel<true><<<queue_grid(p, n_it, B.l_chunks), kRenderThreads, p->smem, st>>>(B);
+            ++launches;
         }
         GL_CUDA_TRY(cudaGetLastError());
         A.pair_hits = p->pair_hits;
@@ -1670,11 +1654,9 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
         {
             GL_CUDA_TRY(cudaMemsetAsync(p->counter, 0, sizeof(int), st));
             A.counter = p->counter;
-            if (p->n_tree_tasks > 0)
-            {
-                const TreeArgs G{p->tree_grids, p->tree_segments, p->tree_runs, p->tree_pairs, p->n_tree_grids, p->n_src};
-                ghost_tree_kernel<<<queue_grid(p, p->n_tree_tasks, 1), kRenderThreads, p->smem, st>>>(A, G);
-            }
+            if (p->tree.n_tasks > 0)
+                ghost_tree_kernel<false><<<queue_grid(p, p->tree.n_tasks, 1), kRenderThreads, p->smem, st>>>(
+                    A, tree_args(p, p->tree));
             else
                 ghost_render_kernel<false><<<queue_grid(p, p->n_items, A.l_chunks), kRenderThreads, p->smem, st>>>(A);
             GL_CUDA_TRY(cudaGetLastError());

@@ -80,3 +80,31 @@ def test_focused_ghost_sums_in_the_warp():
     want = render()
     assert float(want.sum()) > 0
     assert float((got - want).abs().max()) <= 624 * 2.0 ** -24 * float(want.max())
+
+
+@pytest.mark.parametrize("lens,sources,spectral,off", [("wide_angle_24", 1, 31, 7), ("wide_angle_24", 3, 4, 7),
+                                                        ("anamorphic_18", 2, 9, 6), ("anamorphic_18", 1, 5, 6)])
+def test_probe_culls_the_same_pairs(lens, sources, spectral, off):
+    """A plan with a pair that turns at an inactive surface is probed pair by pair:
+    the other pairs must come out the same as from the tree."""
+    import ghostlight_gb300 as gl
+    from ghostlight_gb300 import prescriptions as P
+    lens = gl.OpticalSystem(getattr(P, lens)())
+    lens.surfaces[off].is_active = False
+    n = len(lens.surfaces)
+    pairs = [(a, b) for b in range(n) for a in range(b) if off not in (a, b)]
+    src = np.array([[0.3 + 0.02 * i, 0.2 * i, 1.0, 0.8, 0.6] for i in range(sources)], np.float32)
+    spec, corr = gl.spectral_table(spectral)
+
+    def culled(pairs):
+        plan = gl.GhostRenderPlan(lens, pairs, np.ones(len(pairs), np.float32), src, [gl.pupil_grid(lens, 160)], None, spec,
+                                  corr, 64, 48, 1.2, 0.9, 1000.0, cull_dead_pairs=True)
+        out = [torch.empty((48, 64), device="cuda") for _ in range(3)]
+        plan.execute(*out)
+        return [int(h) > 0 for h in plan.pair_hits()], out
+
+    got, image = culled(pairs)
+    want, _ = culled(pairs + [(off, n - 1)])
+    assert got[:len(pairs)] == want[:len(pairs)]
+    assert 0 < sum(got[:len(pairs)]) < len(pairs)
+    assert all(bool(torch.isfinite(c).all()) for c in image)
