@@ -28,11 +28,14 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 HOST_FLAGS = ["-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-I", str(REPO / "include"), "-I", str(CSRC)]
 FAST = ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"]
+# no value changes: only errno and the exception flags are given up, which keep
+# a loop with a square root or a selection from becoming vector instructions
+VECTOR = ["-Xcompiler", "-fno-math-errno", "-Xcompiler", "-fno-trapping-math"]
 EXACT = ["-fmad=false", "-ftz=false", "-prec-div=true", "-prec-sqrt=true"]
 
 UNITS = {
     "gl_host.cpp": [],
-    "gl_setup.cpp": [],
+    "gl_setup.cpp": VECTOR,
     "gl_coat.cpp": [],
     "gl_filter.cu": EXACT,
     "gl_ghost.cu": FAST,

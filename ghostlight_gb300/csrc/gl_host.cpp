@@ -207,6 +207,7 @@ bool pupil_contains(const PupilMask& m, float u, float v)
     if (m.n_blades >= 3)
     {
         if (m.blade.deformed) return sqrtf(r2) <= blade_radius_at(m.blade, atan2f(v, ux));
+        if (sqrtf(r2) <= m.apothem) return true;         // the inscribed circle: a cosine does not make it larger
         float angle = atan2f(v, ux) - m.rot_rad;
         float sector = fmodf(angle, m.sector);
         if (sector < 0.0f) sector += m.sector;

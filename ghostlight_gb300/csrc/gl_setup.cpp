@@ -68,17 +68,27 @@ void shoot(const SetupLens<T>& L, T ah, T av, const std::vector<Shot<T>>& shots,
     const T bx = Math<T>::tan(ah), by = Math<T>::tan(av);
     const T sdx = -T(kSpawnOffset) * bx, sdy = -T(kSpawnOffset) * by;   // the disc follows the beam
     const T R = L.front_R();
-    out.resize(shots.size());
+    out.assign(shots.size(), Hit<T>{T(0), T(0), false});
+    std::vector<T> hx, hy;
+    std::vector<size_t> at;
+    hx.reserve(shots.size());
+    hy.reserve(shots.size());
+    at.reserve(shots.size());
     for (size_t k = 0; k < shots.size(); ++k)
     {
         const Shot<T>& s = shots[k];
-        Hit<T> h{T(0), T(0), false};
-        if (L.pupil_has(s.u, s.v))
-        {
-            h = L.trace(s.u * R + sdx, s.v * R + sdy, ah, av);
-            h.ok = h.ok && std::isfinite(h.x) && std::isfinite(h.y);
-        }
-        out[k] = h;
+        if (!L.pupil_has(s.u, s.v)) continue;
+        hx.push_back(s.u * R + sdx);
+        hy.push_back(s.v * R + sdy);
+        at.push_back(k);
+    }
+    std::vector<Hit<T>> hits(at.size());
+    L.trace_beam(hx.data(), hy.data(), at.size(), ah, av, hits.data());
+    for (size_t q = 0; q < at.size(); ++q)
+    {
+        Hit<T> h = hits[q];
+        h.ok = h.ok && std::isfinite(h.x) && std::isfinite(h.y);
+        out[at[q]] = h;
     }
 }
 
@@ -734,31 +744,34 @@ template <class T> struct PupilCloud { int hits = 0; T frac = T(0), mx = T(0), m
 
 template <class T> PupilCloud<T> pupil_cloud(SetupLens<T>& L, T ax, T ay, int N)
 {
-    std::vector<Shot<T>> shots;
+    const T bx = Math<T>::tan(ax), by = Math<T>::tan(ay);
+    const T sdx = -T(kSpawnOffset) * bx, sdy = -T(kSpawnOffset) * by;
+    const T R = L.front_R();
+    std::vector<T> hx, hy;
     for (int iy = 0; iy < N; ++iy)
     {
         const T v = T(-1) + (T(iy) + T(0.5)) * (T(2) / T(N));
         for (int ix = 0; ix < N; ++ix)
         {
             const T u = T(-1) + (T(ix) + T(0.5)) * (T(2) / T(N));
-            if (u * u + v * v <= T(1)) shots.push_back(Shot<T>{u, v});
+            if (u * u + v * v > T(1)) continue;
+            hx.push_back(u * R + sdx);
+            hy.push_back(v * R + sdy);
         }
     }
     L.set_lambda(T(kChiefLambda));
-    const T bx = Math<T>::tan(ax), by = Math<T>::tan(ay);
-    const T sdx = -T(kSpawnOffset) * bx, sdy = -T(kSpawnOffset) * by;
-    const T R = L.front_R();
+    std::vector<Hit<T>> hits(hx.size());
+    L.trace_beam(hx.data(), hy.data(), hx.size(), ax, ay, hits.data());
     PupilCloud<T> p;
     T sx = T(0), sy = T(0);
-    for (const Shot<T>& s : shots)
+    for (const Hit<T>& h : hits)
     {
-        const Hit<T> h = L.trace(s.u * R + sdx, s.v * R + sdy, ax, ay);
         if (!h.ok || !std::isfinite(h.x) || !std::isfinite(h.y)) continue;
         sx += h.x;
         sy += h.y;
         ++p.hits;
     }
-    p.frac = shots.empty() ? T(0) : T(p.hits) / T(shots.size());
+    p.frac = hits.empty() ? T(0) : T(p.hits) / T(hits.size());
     p.mx = p.hits > 0 ? sx / T(p.hits) : T(0);
     p.my = p.hits > 0 ? sy / T(p.hits) : T(0);
     return p;
@@ -767,8 +780,8 @@ template <class T> PupilCloud<T> pupil_cloud(SetupLens<T>& L, T ax, T ay, int N)
 // The chief ray of a cell aimed at its target: the u = v = 0 ray first, then
 // the mean of a 9 x 9 pupil cloud, then (deep pupils) the tracked disc probe;
 // a cell with no light keeps its seed and is reported dark.
-template <class T>
-void aim_tile(SetupLens<T>& L, bool axial_ok, const Frame<T>& axial_win, T sx, T sy, T tx, T ty, gl_psf_cell& c)
+template <class T, class Axial>
+void aim_tile(SetupLens<T>& L, Axial&& axial, const Frame<T>& axial_win, T sx, T sy, T tx, T ty, gl_psf_cell& c)
 {
     const int kSteps_ = 8, kCloudN = 9, kFracN = 17, kMinHits = 4;
     const T kFd = T(1e-4f), kTol = T(1e-4f), kTolSoft = T(5e-3f), kDeepFd = T(1e-3f);
@@ -805,7 +818,7 @@ void aim_tile(SetupLens<T>& L, bool axial_ok, const Frame<T>& axial_win, T sx, T
         return true;
     };
     if (try_aim(cloud, kFd, kTolSoft, GL_PSF_CELL_CHIEF_VIGNETTED, false)) return;
-    if (axial_ok)
+    if (axial())
     {
         Frame<T> track = axial_win;
         auto deep = [&](T ax, T ay, T& x, T& y) {
@@ -844,9 +857,20 @@ int psf_anchors(const gl_surface* s, int n, const float* src7, int n_src, int mo
     if (rc) return rc;
     // where the pupil sits on axis: the deep-stop searches start there
     L.set_lambda(T(kChiefLambda));
-    const Coverage<T> ax0 = cover(L, T(0), T(0), Frame<T>{}, kDiscSampling);
-    const bool axial_ok = ax0.area > T(0);
-    const Frame<T> axial_win = ax0.fit;
+    // (measured when the first one asks for it)
+    bool measured = false, axial_ok = false;
+    Frame<T> axial_win;
+    auto axial = [&] {
+        if (!measured)
+        {
+            L.set_lambda(T(kChiefLambda));
+            const Coverage<T> c = cover(L, T(0), T(0), Frame<T>{}, kDiscSampling);
+            axial_ok = c.area > T(0);
+            axial_win = c.fit;
+            measured = true;
+        }
+        return axial_ok;
+    };
     for (int i = 0; i < n_src; ++i)
     {
         const float* q = src7 + 7 * (size_t)i;
@@ -856,7 +880,7 @@ int psf_anchors(const gl_surface* s, int n, const float* src7, int n_src, int mo
         c.status = GL_PSF_CELL_OK;
         if (mode == GL_PSF_CENTER_FIXED_TARGET)
         {
-            aim_tile(L, axial_ok, axial_win, sx, sy, T(q[5]), T(q[6]), c);
+            aim_tile(L, axial, axial_win, sx, sy, T(q[5]), T(q[6]), c);
         }
         else
         {
@@ -866,7 +890,7 @@ int psf_anchors(const gl_surface* s, int n, const float* src7, int n_src, int mo
             c.chief_x_mm = (float)p.mx; c.chief_y_mm = (float)p.my;
             c.status = p.hits > 0 ? GL_PSF_CELL_OK : GL_PSF_CELL_DARK;
             c.pupil_fraction = (float)p.frac;
-            if (p.hits == 0 && axial_ok)
+            if (p.hits == 0 && axial())
             {
                 Frame<T> w = axial_win;
                 const T mag = Math<T>::sqrt(sx * sx + sy * sy);
