@@ -22,6 +22,7 @@
 //   * The flush kernel reads the RGBA accumulator once, applies the 3x3
 //     spectral correction (ghost_render.cu:610-622, same rounding order) and
 //     writes the three planar float32 outputs with coalesced vector stores.
+#include "gl_disp.cuh"
 #include "gl_render.h"
 
 #include <cuda_runtime.h>
@@ -1691,34 +1692,6 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
 // with an arbitrary wavelength per ray: the IOR of every surface is
 // evaluated per ray from the dispersion data.
 // ---------------------------------------------------------------------------
-struct DispRec {
-    int model;
-    float nd, vd, pad;
-    float B[3], C[3];
-};
-
-__device__ __forceinline__ float disp_ior(const DispRec& d, float lam)
-{
-    if (d.model == GL_DISP_SELLMEIER)
-    {
-        float l = lam * 1e-3f;
-        float l2 = l * l;
-        float n2 = 1.0f;
-        n2 += d.B[0] * l2 / (l2 - d.C[0]);
-        n2 += d.B[1] * l2 / (l2 - d.C[1]);
-        n2 += d.B[2] * l2 / (l2 - d.C[2]);
-        return (n2 > 0.0f) ? sqrtf(n2) : 1.0f;
-    }
-    const float n_d = d.nd, V_d = d.vd;
-    if (V_d < 0.1f || n_d <= 1.0001f) return n_d;
-    const float lF = 486.13f, lC = 656.27f, ld = 587.56f;
-    float dn = (n_d - 1.0f) / V_d;
-    float iF = 1.0f / (lF * lF), iC = 1.0f / (lC * lC), id = 1.0f / (ld * ld);
-    float B = dn / (iF - iC);
-    float Aa = n_d - B * id;
-    return Aa + B / (lam * lam);
-}
-
 __global__ void __launch_bounds__(128) trace_rays_kernel(const SurfRec* __restrict__ recs,
                                                          const DispRec* __restrict__ disp, int n,
                                                          int a, int b, const float* __restrict__ rays,
@@ -1932,13 +1905,7 @@ int gl_trace_rays(const gl_surface* surfaces, int n, int bounce_a, int bounce_b,
     std::vector<SurfRec> recs((size_t)n);
     int rc = pack_lens(surfaces, n, recs.data(), dev);
     if (rc) return rc;
-    std::vector<DispRec> disp((size_t)n);
-    for (int i = 0; i < n; ++i)
-    {
-        disp[i].model = surfaces[i].disp_model;
-        disp[i].nd = surfaces[i].ior; disp[i].vd = surfaces[i].abbe_v; disp[i].pad = 0.0f;
-        for (int k = 0; k < 3; ++k) { disp[i].B[k] = surfaces[i].sellmeier_B[k]; disp[i].C[k] = surfaces[i].sellmeier_C[k]; }
-    }
+    const std::vector<DispRec> disp = disp_records(surfaces, n);
     cudaStream_t st = (cudaStream_t)stream;
     // one block of the device's pool (kept, where the default pool gives its
     // memory back at every synchronisation: 0.2 ms of each call), one copy

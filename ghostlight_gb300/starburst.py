@@ -492,7 +492,7 @@ def effective_pupil_info(lens, config, g, field) -> dict:
     if not any_surv:
         return {"pupil": None, "T": 0.0, "chief": (0.0, 0.0), "survivors": False}
     me = min(max(int(dc.survivor_grid), 16), 1024)
-    env = survivor_envelope(lens, g["ep_x"], g["ep_y"], cx, cy, float(ax), float(ay), me)
+    env = _survivor_envelope_device(lens, g["ep_x"], g["ep_y"], cx, cy, float(ax), float(ay), me)
     plain = build_pupil2(lens, g["N"], g["fill"], bo, rot)
     pupil = build_pupil2(lens, g["N"], g["fill"], bo, rot, envelope=env)
     s_ref = float((plain.double() ** 2).sum())
@@ -728,9 +728,9 @@ def survivor_center(lens, ax: float, ay: float, survives=None):
     """Centroid of the spawn-plane launches whose ray reaches the sensor at
     field (ax, ay) (solve_survivor_center, starburst_render.cu:503-583):
     an 81 x 81 scan over the front element's reach, boundary cells
-    supersampled 8 x 8.  Returns (cx, cy, any_survivor)."""
+    supersampled 8 x 8.  Returns (cx, cy, any_survivor).  survives: the trace to
+    ask instead of the device (x, y, z, d -> survived)."""
     f = np.float32
-    survives = survives or (lambda x, y, z, d: _survives_device(lens, x, y, z, d))
     front_R = f(lens.surfaces[0].semi_aperture) if lens.surfaces else f(0.0)
     if front_R <= 0:
         return 0.0, 0.0, False
@@ -739,6 +739,16 @@ def survivor_center(lens, ax: float, ay: float, survives=None):
     span_x = f(f(f(1.1) * front_R) + f(f(20.0) * f(abs(bx))))
     span_y = f(f(f(1.1) * front_R) + f(f(20.0) * f(abs(by))))
     S = SURVIVOR_SCAN
+    if survives is None:
+        import torch
+        from . import _native
+        arr = lens.to_array()
+        out = (C.c_double * 3)()
+        _native.check(_native.load().gl_survivor_center(
+            arr, len(arr), LAMBDA_REF_NM, (C.c_float * 3)(*map(float, d)), float(z), float(span_x), float(span_y), S, SURVIVOR_CENTER_SS, out,
+            torch.cuda.current_stream().cuda_stream), "survivor_center")
+        sx, sy, w = out
+        return (float(f(sx / w)), float(f(sy / w)), True) if w > 0 else (0.0, 0.0, False)
     t = (f(2.0) * np.arange(S, dtype=np.float32) / f(S - 1) - f(1.0)).astype(np.float32)
     lx = (span_x * t).astype(np.float32)
     ly = (span_y * t).astype(np.float32)
@@ -766,6 +776,22 @@ def survivor_center(lens, ax: float, ay: float, survives=None):
     return 0.0, 0.0, False
 
 
+def _survivor_envelope_device(lens, ep_x, ep_y, cx, cy, ax, ay, ME: int):
+    """survivor_envelope as a device tensor."""
+    import torch
+    from . import _native
+    env = torch.ones((ME, ME), dtype=torch.float32, device="cuda")
+    if lens.surfaces:
+        _, _, d = _launch_dir(ax, ay)
+        arr = lens.to_array()
+        _native.check(_native.load().gl_survivor_envelope(
+            arr, len(arr), LAMBDA_REF_NM, (C.c_float * 3)(*map(float, d)),
+            float(np.float32(lens.surfaces[0].z) - np.float32(20.0)), float(cx), float(cy),
+            float(ep_x), float(ep_y), ME, SURVIVOR_EDGE_SS, C.c_void_p(env.data_ptr()), torch.cuda.current_stream().cuda_stream),
+            "survivor_envelope")
+    return env
+
+
 def survivor_envelope(lens, ep_x, ep_y, cx, cy, ax, ay, ME: int, survives=None, contains=None):
     """Cat's-eye rim-vignetting envelope over pupil [-1, 1]^2, ME x ME
     (build_survivor_envelope, starburst_render.cu:393-491): 1 where a primary
@@ -775,6 +801,8 @@ def survivor_envelope(lens, ep_x, ep_y, cx, cy, ax, ay, ME: int, survives=None, 
     f = np.float32
     from ._abi import surface_array
     from . import _native
+    if survives is None and contains is None:
+        return _survivor_envelope_device(lens, ep_x, ep_y, cx, cy, ax, ay, ME).cpu().numpy()
     survives = survives or (lambda x, y, z, d: _survives_device(lens, x, y, z, d))
     if contains is None:
         arr = surface_array(lens.records())

@@ -462,6 +462,17 @@ int gl_build_pupil2(const gl_surface* surfaces, int n_surfaces, int N, float pup
  * points uv[2 k], uv[2 k + 1] -> out[k] (host float arithmetic). */
 int gl_pupil_contains(const gl_surface* surfaces, int n, int blades_override, float rotation_deg, int aspect_one,
                       const float* uv, int n_pts, uint8_t* out);
+/* The surviving part of an off-axis beam (starburst_render.cu:393-583): primary
+ * launches from plane launch_z along dir[3] at one wavelength.  center: out =
+ * {sum x, sum y, weight} of the survivors of a scan x scan grid over +-span, its
+ * border cells taken apart into ss x ss launches.  envelope: d_env (device, me x
+ * me over pupil [-1, 1]^2) = the surviving fraction of the launches at (cx + u
+ * ep_x, cy + v ep_y) inside the stop, filled two cells outward.  Both
+ * synchronise the stream. */
+int gl_survivor_center(const gl_surface* surfaces, int n, float lambda, const float* dir, float launch_z, float span_x,
+                       float span_y, int scan, int ss, double* out, void* stream);
+int gl_survivor_envelope(const gl_surface* surfaces, int n, float lambda, const float* dir, float launch_z, float cx, float cy,
+                         float ep_x, float ep_y, int me, int ss, float* d_env, void* stream);
 
 /* PSF / veil image convolution: out_c = in_c (*) k ('same' size, kernel
  * centred, odd kw x kh, float32).  The reference has no such operation on
