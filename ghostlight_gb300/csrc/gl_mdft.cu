@@ -220,9 +220,7 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 // registers) throughout.
 //
 // 512^2 pupil to 2048^2, 31 wavelengths, split BF16: step 1 233 -> 109 us, step
-// 2 1093 -> 550 us.  Step 2 issues 1536 cycles of MMA per 96 KB stage, two
-// stages deep, and runs its tensor pipe at about 60%: bound by the operand
-// stream from L2 (62 bytes per cycle and SM at full rate).
+// 2 1093 -> 480 us (in pairs of CTAs; 88% of the measured dense BF16 rate).
 //
 // Storage (Kp = 2 nh bf16, or nh floats; rows of Kp; unfolded: nh = n):
 //   W'  [lam][C | S][k]                                  TF32: [Wr | Wi]
@@ -292,14 +290,15 @@ __device__ __forceinline__ void store_split16(__nv_bfloat16* row, int nh, int i0
 // Shared-memory stages of one CTA and its accumulators.  A stage holds two A
 // tiles of 128 rows (folded: hi and lo; TF32: Wr and Wi) and the row blocks of
 // B (folded: hi and lo of each), as many stages as fit, four at most.
-template <int FORM, int STEP, int TN, bool BOX>
+template <int FORM, int STEP, int TN, bool BOX, int CL>
 struct MdftShape {
     static constexpr bool kFold = FORM != kTf32;
     static constexpr int kBSets = kFold ? 2 : 1;
     static constexpr int kBlocks = kFold ? (BOX ? 1 : 2) : STEP;    // row blocks of B per unit and set
     static constexpr int kRows = STEP == 2 ? TN : 128;              // rows of one block
     static constexpr int kN = (!kFold && STEP == 2 && BOX) ? TN : kBlocks * kRows;   // MMA N
-    static constexpr int kBBytes = kBlocks * kRows * 128;
+    static constexpr int kOwn = kBlocks / CL;                       // of them this CTA loads (a pair: one each)
+    static constexpr int kBBytes = kOwn * kRows * 128;
     static constexpr int kStageBytes = 2 * kOpTile + kBSets * kBBytes;
     static constexpr int kStages = 212992 / kStageBytes < 4 ? 212992 / kStageBytes : 4;
     static constexpr int kAccCols = kFold ? kN : 2 * kN;            // TMEM columns of a unit (TF32: D1 and D2)
@@ -315,12 +314,22 @@ struct MdftShape {
 
 // TN (step 2): complex output columns per unit, 128 or 64 (the autotuner's
 // tile-shape knob); twice the units spread a small frame over more SMs.
-template <int FORM, int STEP, int TN, bool BOX>
+// CL = 2 (split BF16, field form): a pair of CTAs takes two neighbouring row blocks
+// of one column block as one product of 256 rows (cta_group::2): each loads its
+// own rows of A and one of the two row blocks of B, the first one issues, and each
+// finds its 128 rows in its own TMEM.  Half of B per CTA is 64 KB a stage instead
+// of 96, so three stages fit, and half the shared-memory reads for B, which with
+// one CTA are the bound (36 KB of operands and 24 KB of fill per 384 cycles of MMA,
+// at 128 bytes a cycle).  512^2 -> 2048^2 x 31: step 2 550 -> 480 us.  (Two CTAs that
+// only shared B's tiles by multicast: 540.)
+template <int FORM, int STEP, int TN, bool BOX, int CL>
 __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_constant__ CUtensorMap tA,
                                                               const __grid_constant__ CUtensorMap tB, MdftArgs args)
 {
     static_assert(TN == 128 || TN == 64, "tile width");
-    using Sh = MdftShape<FORM, STEP, TN, BOX>;
+    static_assert(CL == 1 || (CL == 2 && FORM == 0 && !BOX && TN == 128), "pairs");
+    const int rank = CL == 2 ? (int)(blockIdx.x & 1) : 0;
+    using Sh = MdftShape<FORM, STEP, TN, BOX, CL>;
     constexpr int kStagesM = Sh::kStages;
     constexpr int kbe = (FORM == 0) ? 64 : 32;                   // reduction elements per 128-byte row
     constexpr int kStep = (FORM == 0) ? 16 : 8;                  // and per MMA
@@ -331,11 +340,17 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int* err = args.err;
 
-    if (warp == 5) tc::tmem_alloc(&tmem_base, 512);
+    if (warp == 5)
+    {
+        if (CL == 2) tc::tmem_alloc_pair(&tmem_base, 512);
+        else tc::tmem_alloc(&tmem_base, 512);
+    }
     if (threadIdx.x == 128)
     {
+        // a pair's full and acc_empty are the first CTA's; empty and acc_full are
+        // signalled in both
         for (int s = 0; s < kStagesM; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], 128); }
+        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], 128 * CL); }
         tc::mbar_init(&mma_done, 1);
         tc::fence_mbar_init();
         tc::tma_prefetch(&tA);
@@ -345,32 +360,33 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base;
+    if (CL == 2) tc::cluster_sync();           // the other's barriers are set up
 
     // Units are dealt round-robin (unit u to CTA u mod G), so the units in
     // flight at any moment are consecutive: with wavelength-major unit order
     // they share one wavelength's operands, which then stay in L2.
-    const int G = gridDim.x;
-    const int u0 = blockIdx.x, u1 = args.n_units;
+    const int G = gridDim.x / CL;
+    const int u0 = blockIdx.x / CL, u1 = args.n_units / CL;       // CL = 2: pairs of units
 
     auto decode = [&](int u, int& lam, int& mb, int& xb, int& part) {
         part = 0;
         if (STEP == 2)
         {
             // wavelength-major: all output tiles of one wavelength, then the next
-            const int tiles = args.NBm * args.NBt;
+            const int tiles = args.NBm / CL * args.NBt;
             const int lr = u / tiles;               // wavelength within this launch's range
             lam = args.lam_base + lr;
             const int tile = u - lr * tiles;
-            mb = tile / args.NBt;
+            mb = tile / args.NBt * CL + rank;
             xb = tile % args.NBt;
         }
         else
         {
-            const int per = args.NBm * args.NI * Sh::kParts;
+            const int per = args.NBm / CL * args.NI * Sh::kParts;
             lam = args.lam_base + u / per;
             const int r = u % per;
             part = r % Sh::kParts;                  // C, then S
-            mb = (r / Sh::kParts) / args.NI;
+            mb = (r / Sh::kParts) / args.NI * CL + rank;
             xb = (r / Sh::kParts) % args.NI;
         }
     };
@@ -393,17 +409,22 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                         const int s = it % kStagesM, r = it / kStagesM;
                         if (it >= kStagesM && !tc::mbar_wait(&empty[s], (r - 1) & 1, err, tc::TC_TIMEOUT_EMPTY)) { stop = true; break; }
                         uint8_t* st = smem + s * Sh::kStageBytes;
-                        tc::mbar_expect_tx(&full[s], Sh::kStageBytes);
+                        if (rank == 0) tc::mbar_expect_tx(&full[s], CL * Sh::kStageBytes);
                         const int x = kb * kbe;
-                        tc::tma_load_2d(st, &tA, x, rowA, &full[s]);
-                        if (Sh::kFold) tc::tma_load_2d(st + kOpTile, &tA, args.nh + x, rowA, &full[s]);
-                        else tc::tma_load_2d(st + kOpTile, &tA, x, rowA + args.KA, &full[s]);
+                        const uint32_t bar = CL == 2 ? tc::leader_u32(&full[s]) : 0u;
+                        auto load = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1) {
+                            if (CL == 2) tc::tma_load_2d_pair(dst, map, c0, c1, bar);
+                            else tc::tma_load_2d(dst, map, c0, c1, &full[s]);
+                        };
+                        load(st, &tA, x, rowA);
+                        if (Sh::kFold) load(st + kOpTile, &tA, args.nh + x, rowA);
+                        else load(st + kOpTile, &tA, x, rowA + args.KA);
                         #pragma unroll
                         for (int t = 0; t < Sh::kBSets; ++t)
                             #pragma unroll
-                            for (int j = 0; j < Sh::kBlocks; ++j)
+                            for (int j = 0; j < Sh::kOwn; ++j)
                             {
-                                const int q = cs * Sh::kBlocks + j;
+                                const int q = cs * Sh::kBlocks + j + rank;
                                 int rowB;
                                 if (STEP == 2)
                                 {
@@ -415,23 +436,32 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                                 }
                                 else
                                     rowB = q * args.nhr + xb * 128;
-                                tc::tma_load_2d(st + 2 * kOpTile + t * Sh::kBBytes + j * Sh::kRows * 128, &tB,
-                                                t * args.nh + x, rowB, &full[s]);
+                                load(st + 2 * kOpTile + t * Sh::kBBytes + j * Sh::kRows * 128, &tB, t * args.nh + x, rowB);
                             }
                         ++issued;
                     }
                 }
             }
+            // this thread's copies have landed (a pair: have been used, which both CTAs are told)
             for (int q = (issued > kStagesM ? issued - kStagesM : 0); q < issued; ++q)
-                tc::mbar_wait(&full[q % kStagesM], (q / kStagesM) & 1, err, tc::TC_TIMEOUT_FULL);
+                tc::mbar_wait(CL == 2 ? &empty[q % kStagesM] : &full[q % kStagesM], (q / kStagesM) & 1, err,
+                              CL == 2 ? tc::TC_TIMEOUT_EMPTY : tc::TC_TIMEOUT_FULL);
         }
         __syncwarp();
     }
     else if (warp == 5)
     {
-        if (lane == 0)
+        if (lane == 0 && rank == 0)
         {
-            const uint32_t id = idesc_any<FORM>(128, Sh::kN);
+            const uint32_t id = idesc_any<FORM>(128 * CL, Sh::kN);
+            auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+                if (CL == 2) tc::mma_f16_pair(d, a, b, id, acc);
+                else mma_any<FORM>(d, a, b, id, acc);
+            };
+            auto commit = [&](uint64_t* bar) {
+                if (CL == 2) tc::mma_commit_pair(bar);
+                else tc::mma_commit(bar);
+            };
             int it = 0, ui = 0;
             bool stop = false;
             for (int u = u0; u < u1 && !stop; u += G, ++ui)
@@ -459,21 +489,21 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                     {
                         if (kk >= left) break;
                         const uint32_t acc = (kk0 | kk) != 0;
-                        mma_any<FORM>(d, a0 + 2 * kk, b0 + 2 * kk, id, acc);
+                        mma(d, a0 + 2 * kk, b0 + 2 * kk, acc);
                         if (Sh::kFold)
                         {
-                            mma_any<FORM>(d, a0 + 2 * kk, b1 + 2 * kk, id, 1);
-                            mma_any<FORM>(d, a1 + 2 * kk, b0 + 2 * kk, id, 1);
+                            mma(d, a0 + 2 * kk, b1 + 2 * kk, 1);
+                            mma(d, a1 + 2 * kk, b0 + 2 * kk, 1);
                         }
                         else
-                            mma_any<FORM>(d + Sh::kN, a1 + 2 * kk, (STEP == 2 && BOX ? b1 : b0) + 2 * kk, id, acc);
+                            mma(d + Sh::kN, a1 + 2 * kk, (STEP == 2 && BOX ? b1 : b0) + 2 * kk, acc);
                     }
-                    tc::mma_commit(&empty[s]);
+                    commit(&empty[s]);
                 }
-                tc::mma_commit(&acc_full[b]);
+                commit(&acc_full[b]);
             }
             // every MMA this thread issued must be complete before TMEM is freed
-            tc::mma_commit(&mma_done);
+            commit(&mma_done);
             tc::mbar_wait(&mma_done, 0, err, tc::TC_TIMEOUT_ACC);
         }
         __syncwarp();
@@ -612,12 +642,23 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                 }
             }
             tc::tc_fence_before();
-            tc::mbar_arrive(&acc_empty[b]);
+            if (CL == 2) tc::mbar_arrive_cluster(tc::leader_u32(&acc_empty[b]));
+            else tc::mbar_arrive(&acc_empty[b]);
         }
+        // the arrival that the first CTA's last commit makes here too
+        if (CL == 2 && rank == 1 && threadIdx.x == 0) tc::mbar_wait(&mma_done, 0, err, tc::TC_TIMEOUT_ACC);
+        __syncwarp();
     }
     tc::tc_fence_before();
     __syncthreads();
-    if (warp == 5) tc::tmem_dealloc(tmem, 512);
+    // a pair's MMAs read and write both CTAs, and arrive in both: neither leaves
+    // before the other is done (every wait above ends, so both get here)
+    if (CL == 2) tc::cluster_sync();
+    if (warp == 5)
+    {
+        if (CL == 2) tc::tmem_dealloc_pair(tmem, 512);
+        else tc::tmem_dealloc(tmem, 512);
+    }
 }
 
 // DFT matrices W'[lam][C | S][k][Kp]: cos and sin of 2 pi s(lam) d (k - ck) at
@@ -1051,6 +1092,7 @@ struct MdftPlan {
     int* err = nullptr;
     CUtensorMap t_wx, t_wy, t_mask, t_tp, t_tp64;
     int sms = 0;
+    int pairs = 0;              // clusters of two CTAs resident at once (split BF16)
 };
 
 static void mdft_free(MdftPlan* p)
@@ -1087,30 +1129,85 @@ static cudaError_t mdft_build_matrices(MdftPlan* p, cudaStream_t st)
 }
 
 // Opt one GEMM instance in to its shared memory.
-template <int FORM, int STEP, int TN, bool BOX>
+template <int FORM, int STEP, int TN, bool BOX, int CL>
 static cudaError_t mdft_prepare()
 {
-    return cudaFuncSetAttribute(mdft_kernel<FORM, STEP, TN, BOX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                MdftShape<FORM, STEP, TN, BOX>::kSmem);
+    return cudaFuncSetAttribute(mdft_kernel<FORM, STEP, TN, BOX, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                MdftShape<FORM, STEP, TN, BOX, CL>::kSmem);
 }
 
+struct MdftLaunch {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    MdftLaunch(int grid, int cl, int smem, cudaStream_t st)
+    {
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(kMdftThreads);
+        cfg.dynamicSmemBytes = (size_t)smem;
+        cfg.stream = st;
+        if (cl == 1) return;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)cl;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+    }
+};
+
+// *pairs: pairs of CTAs that are resident at once (0: the form has none).
 template <int FORM, bool BOX>
-static cudaError_t mdft_prepare_all()
+static cudaError_t mdft_prepare_all(int* pairs)
 {
-    cudaError_t e = mdft_prepare<FORM, 1, 128, BOX>();
-    if (e == cudaSuccess) e = mdft_prepare<FORM, 2, 128, BOX>();
-    if (e == cudaSuccess) e = mdft_prepare<FORM, 2, 64, BOX>();
+    cudaError_t e = mdft_prepare<FORM, 1, 128, BOX, 1>();
+    if (e == cudaSuccess) e = mdft_prepare<FORM, 2, 128, BOX, 1>();
+    if (e == cudaSuccess) e = mdft_prepare<FORM, 2, 64, BOX, 1>();
+    *pairs = 0;
+    if constexpr (FORM == 0 && !BOX)
+    {
+        if (e == cudaSuccess) e = mdft_prepare<0, 1, 128, false, 2>();
+        if (e == cudaSuccess) e = mdft_prepare<0, 2, 128, false, 2>();
+        int n1 = 0, n2 = 0;
+        const MdftLaunch L1(2, 2, MdftShape<0, 1, 128, false, 2>::kSmem, nullptr);
+        const MdftLaunch L2(2, 2, MdftShape<0, 2, 128, false, 2>::kSmem, nullptr);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n1, mdft_kernel<0, 1, 128, false, 2>, &L1.cfg);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n2, mdft_kernel<0, 2, 128, false, 2>, &L2.cfg);
+        if (e == cudaSuccess) *pairs = std::min(n1, n2);
+    }
     return e;
 }
 
-template <int FORM, bool BOX>
-static void mdft_gemms(const MdftPlan* p, const MdftArgs& a1, int g1, const MdftArgs& a2, int g2, cudaStream_t st)
+// One step over its units.  The field form in split BF16 runs in pairs where the
+// row blocks come in pairs, a unit's reduction is long and there are many units: a
+// cluster's launch costs 2 us more, and a short reduction is bound by its epilogue.
+// Measured, whole plan, step in single CTAs -> in pairs: step 2 at 8 stages a unit
+// 682 -> 621 us (7936 units), 95.5 -> 92.3 (496), 37.0 -> 38.9 (128), at 4 stages
+// 148 -> 152; step 1 at 16 stages 137 -> 125 (512 units), at 8 stages 141 -> 137 and
+// 355 -> 379, at 4 stages 219 -> 224.
+template <int FORM, int STEP, int TN, bool BOX>
+static cudaError_t mdft_step(const CUtensorMap& tA, const CUtensorMap& tB, const MdftArgs& a, int gmax, int pairs, cudaStream_t st)
 {
-    mdft_kernel<FORM, 1, 128, BOX><<<g1, kMdftThreads, MdftShape<FORM, 1, 128, BOX>::kSmem, st>>>(p->t_wx, p->t_mask, a1);
-    if (p->tile_n == 64)
-        mdft_kernel<FORM, 2, 64, BOX><<<g2, kMdftThreads, MdftShape<FORM, 2, 64, BOX>::kSmem, st>>>(p->t_wy, p->t_tp64, a2);
-    else
-        mdft_kernel<FORM, 2, 128, BOX><<<g2, kMdftThreads, MdftShape<FORM, 2, 128, BOX>::kSmem, st>>>(p->t_wy, p->t_tp, a2);
+    if constexpr (FORM == 0 && !BOX && TN == 128)
+    {
+        pairs = std::min(std::min(a.n_units, gmax) / 2, pairs);
+        const int stages = MdftShape<FORM, STEP, TN, BOX, 2>::kPhases * a.nkb;
+        const bool worth = stages >= (STEP == 1 ? 16 : 8) && (long long)stages * a.n_units >= 3000;
+        if ((a.NBm & 1) == 0 && pairs > 0 && worth)
+        {
+            const MdftLaunch L(2 * pairs, 2, MdftShape<FORM, STEP, TN, BOX, 2>::kSmem, st);
+            return cudaLaunchKernelEx(&L.cfg, mdft_kernel<FORM, STEP, TN, BOX, 2>, tA, tB, a);
+        }
+    }
+    const MdftLaunch L(std::min(a.n_units, gmax), 1, MdftShape<FORM, STEP, TN, BOX, 1>::kSmem, st);
+    return cudaLaunchKernelEx(&L.cfg, mdft_kernel<FORM, STEP, TN, BOX, 1>, tA, tB, a);
+}
+
+template <int FORM, bool BOX>
+static cudaError_t mdft_gemms(const MdftPlan* p, const MdftArgs& a1, const MdftArgs& a2, int gmax, cudaStream_t st)
+{
+    cudaError_t e = mdft_step<FORM, 1, 128, BOX>(p->t_wx, p->t_mask, a1, gmax, p->pairs, st);
+    if (e != cudaSuccess) return e;
+    return p->tile_n == 64 ? mdft_step<FORM, 2, 64, BOX>(p->t_wy, p->t_tp64, a2, gmax, p->pairs, st)
+                           : mdft_step<FORM, 2, 128, BOX>(p->t_wy, p->t_tp, a2, gmax, p->pairs, st);
 }
 
 template <bool BOX>
@@ -1203,8 +1300,8 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     }
     chk(cudaStreamSynchronize(st));
     // shared-memory opt-in once here, so execute enqueues kernels only (graph capture)
-    if (form == 0) chk(box ? mdft_prepare_all<0, true>() : mdft_prepare_all<0, false>());
-    else if (form == 1) chk(box ? mdft_prepare_all<1, true>() : mdft_prepare_all<1, false>());
+    if (form == 0) chk(box ? mdft_prepare_all<0, true>(&p->pairs) : mdft_prepare_all<0, false>(&p->pairs));
+    else if (form == 1) chk(box ? mdft_prepare_all<1, true>(&p->pairs) : mdft_prepare_all<1, false>(&p->pairs));
     const CUtensorMapDataType dt = form == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const uint32_t bc = form == 0 ? 64 : 32;
     int rc = GL_OK;
@@ -1294,12 +1391,10 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     a.lam_base = l0;
     a.n_units = nl * NBx * a.NI * (p->form == kTf32 ? 1 : 2);   // step 1: (lambda, k block, pupil-row block, C / S)
     const int gmax = p->ctas > 0 ? p->ctas : p->sms;
-    const int g1 = std::min(a.n_units, gmax);
     MdftArgs a2 = a;
     a2.KA = p->Ky; a2.NBm = NBy;
     a2.NBt = p->Kx / p->tile_n;
     a2.n_units = NBy * a2.NBt * nl;                     // step 2: (lambda, output tile)
-    const int g2 = std::min(a2.n_units, gmax);
     if (p->form == 2)
     {
         if (p->box) mdft_simt<true>(p, a, a2, l1, st);
@@ -1307,13 +1402,11 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     }
     else if (p->form == 0)
     {
-        if (p->box) mdft_gemms<0, true>(p, a, g1, a2, g2, st);
-        else mdft_gemms<0, false>(p, a, g1, a2, g2, st);
+        GL_CUDA_TRY(p->box ? (mdft_gemms<0, true>(p, a, a2, gmax, st)) : (mdft_gemms<0, false>(p, a, a2, gmax, st)));
     }
     else
     {
-        if (p->box) mdft_gemms<1, true>(p, a, g1, a2, g2, st);
-        else mdft_gemms<1, false>(p, a, g1, a2, g2, st);
+        GL_CUDA_TRY(p->box ? (mdft_gemms<1, true>(p, a, a2, gmax, st)) : (mdft_gemms<1, false>(p, a, a2, gmax, st)));
     }
     GL_CUDA_TRY(cudaGetLastError());
     launches += 2;

@@ -1,6 +1,6 @@
 // gl_tc.cuh — Blackwell (sm_103a) tensor-core primitives in inline PTX:
 // TMA tiled loads, mbarriers with bounded waits, TMEM allocation,
-// tcgen05.mma (kind::f16 / kind::tf32, cta_group::1) and tcgen05.ld / st.
+// tcgen05.mma (kind::f16 / kind::tf32, one CTA or a pair) and tcgen05.ld / st.
 //
 // Shared-memory operands use the canonical K-major SWIZZLE_128B layout that a
 // TMA tiled load with CU_TENSOR_MAP_SWIZZLE_128B produces: rows of 128 bytes,
@@ -101,8 +101,53 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 
+// ---- pairs of CTAs (cta_group::2) ---------------------------------------------
+// The address of this CTA's shared-memory word in the pair's first CTA.
+__device__ __forceinline__ uint32_t leader_u32(const void* p)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+    return a;
+}
+
+// A load into this CTA whose bytes are counted by a barrier of the pair (its
+// shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, int c0, int c1, uint32_t bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
+            "r"(smem_u32(smem_dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Every thread of every CTA of the cluster.
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ---- TMEM -------------------------------------------------------------------
-// Allocation by one full warp; the TMEM base address lands in *dst (smem).
+// Allocation by one full warp (of a pair: one in each CTA); the TMEM base
+// address lands in *dst (smem).
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst, uint32_t ncols)
+{
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)),
+                 "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols)
+{
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols)
 {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)),
@@ -189,6 +234,29 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint6
         "}\n" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+// The pair's MMA: 256 rows, each CTA's own 128 of A and half of B's rows.
+__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// mma_commit for the pair's MMAs, on the barrier at this offset in both CTAs.
+__device__ __forceinline__ void mma_commit_pair(uint64_t* bar)
+{
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                     smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
 }
 
 // Arrive on an mbarrier when every previously issued MMA of this thread is done.
