@@ -531,7 +531,8 @@ def run_cfg3(args, dev, stream, flush, timed):
         if plan.status() != 0:
             raise RuntimeError("mdft %s: device wait timed out" % form)
         sec = sum(ts) / len(ts)
-        ach = flops / sec / 1e12
+        # the folded forms need half of the direct form's products
+        ach = (flops if form == "tf32" else 0.5 * flops) / sec / 1e12
         forms[form] = dict(ms=1e3 * sec, tflops_algorithmic=ach, launch=getattr(plan, "launch", None),
                            **_errs(sb, ref),
                            roofline={"bound": "tensor" if form != "fp32" else "fp32", "achieved": ach,
@@ -1269,7 +1270,7 @@ def main():
 
 
 def roofline(res, plan):
-    """Dominant kernel: ghost_render_kernel (render launch), bound by FP32
+    """Dominant kernel: ghost_tree_kernel (render launch), bound by FP32
     issue on the CUDA cores (the trace is sequential FP32 arithmetic; the
     splat is a small share).  Algorithmic FLOPs per launch = the launch's
     traced ray-wavelengths x the per-trace FP32 operation count measured once
@@ -1281,7 +1282,7 @@ def roofline(res, plan):
     achieved = res["traces_render"] * flops_per_trace / sec / 1e12 if (flops_per_trace and sec > 0) else None
     return {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": (achieved / peak) if (achieved and peak) else None, "traffic": RENDER_DRAM_BYTES,
-            "kernel": "ghost_render_kernel", "kernel_ms": res["kernel_ms"]["render"],
+            "kernel": "ghost_tree_kernel", "kernel_ms": res["kernel_ms"]["render"],
             "flop_per_launch": res["traces_render"] * flops_per_trace,
             "peak_note": "GB300 FP32 CUDA-core peak: 152 SMs x 128 lanes x 2 FLOP x max SM clock",
             "traffic_note": "DRAM bytes of one render launch from ncu (dram__bytes_read.sum + "
@@ -1289,17 +1290,15 @@ def roofline(res, plan):
 
 
 # FP32 operations per traced ray-wavelength (FADD + FMUL + 2 x FFMA, thread
-# level, predicated on) of the render kernel on this workload, measured with
-# ncu on one launch of the tuned shape while only the lanes of live rays ran
-# the step (smsp__sass_thread_inst_executed_op_{fadd,fmul,ffma}_pred_on.sum:
-# 4.926e9 + 20.971e9 + 2 x 18.993e9 = 6.388e10 FLOP over 6.007e7 traces),
-# and frozen as the algorithmic count.  The branch-free step now also runs
-# on the lanes of dead rays (work nobody reads: 7.5e10 counted FLOP per
-# launch), which the algorithmic count leaves out.
-FLOPS_PER_RAY_LAMBDA = 1063.5
+# level, predicated on) of the render launch on this workload, measured with
+# ncu on one launch of the tree walk, whose pairs share their legs
+# (smsp__sass_thread_inst_executed_op_{fadd,fmul,ffma}_pred_on.sum:
+# 2.19e9 + 7.17e9 + 2 x 6.27e9 = 2.190e10 FLOP over 6.007e7 traces).  Pair by
+# pair the same traces took 6.388e10.
+FLOPS_PER_RAY_LAMBDA = 364.6
 # DRAM bytes (read + write) of one render launch on this frame, from the same
-# capture (dram__bytes_read.sum + dram__bytes_write.sum: 40.99 + 4.94 MB).
-RENDER_DRAM_BYTES = 45.93e6
+# capture (dram__bytes_read.sum + dram__bytes_write.sum: 39.53 + 1.30 MB).
+RENDER_DRAM_BYTES = 40.84e6
 FP32_PEAK_TFLOPS = 152 * 128 * 2 * 2.070e9 / 1e12
 
 

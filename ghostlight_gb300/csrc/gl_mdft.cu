@@ -220,7 +220,7 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 // registers) throughout.
 //
 // 512^2 pupil to 2048^2, 31 wavelengths, split BF16: step 1 233 -> 109 us, step
-// 2 1093 -> 480 us (in pairs of CTAs; 88% of the measured dense BF16 rate).
+// 2 1093 -> 460 us (in pairs of CTAs; 91% of the measured dense BF16 rate).
 //
 // Storage (Kp = 2 nh bf16, or nh floats; rows of Kp; unfolded: nh = n):
 //   W'  [lam][C | S][k]                                  TF32: [Wr | Wi]
@@ -320,7 +320,7 @@ struct MdftShape {
 // finds its 128 rows in its own TMEM.  Half of B per CTA is 64 KB a stage instead
 // of 96, so three stages fit, and half the shared-memory reads for B, which with
 // one CTA are the bound (36 KB of operands and 24 KB of fill per 384 cycles of MMA,
-// at 128 bytes a cycle).  512^2 -> 2048^2 x 31: step 2 550 -> 480 us.  (Two CTAs that
+// at 128 bytes a cycle).  512^2 -> 2048^2 x 31: step 2 550 -> 460 us.  (Two CTAs that
 // only shared B's tiles by multicast: 540.)
 template <int FORM, int STEP, int TN, bool BOX, int CL>
 __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_constant__ CUtensorMap tA,
