@@ -83,7 +83,8 @@ template <bool LAND>
 __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* lens, const float* at, float* tile,
                                               int si, int gi);
 
-// LAND: the landings go to A.land instead of the tiles (the dense path).
+// LAND: the landings go to A.land instead of the tiles (the dense path), the
+// wavelengths split over grid.z.
 template <bool LAND>
 __global__ void __launch_bounds__(kPsfThreads) psf_kernel(PsfArgs A)
 {
@@ -139,13 +140,15 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
     const V3 dir = normalized(v3(bx, by, 1.0f));
     const V3 org = v3(uv.x * A.front_R - kSpawnOffset * bx, uv.y * A.front_R - kSpawnOffset * by, A.start_z);
     const int tx_min = S.tile_x0, ty_min = S.tile_y0, tx_max = S.tile_x0 + A.tile_w, ty_max = S.tile_y0 + A.tile_h;
-    const int l0 = LAND ? A.l_base : 0, l1 = LAND ? A.l_base + A.n_land : A.n_spec;
+    const int per = LAND ? (A.n_land + (int)gridDim.z - 1) / (int)gridDim.z : A.n_spec;
+    const int l0 = LAND ? A.l_base + (int)blockIdx.z * per : 0;
+    const int l1 = LAND ? min(A.l_base + A.n_land, l0 + per) : A.n_spec;
     for (int l = l0; l < l1; ++l)
     {
         float4* land = nullptr;
         if (LAND)
         {
-            land = A.land + ((size_t)(si - A.s_base) * A.n_land + (l - l0)) * A.n_grid + gi;
+            land = A.land + ((size_t)(si - A.s_base) * A.n_land + (l - A.l_base)) * A.n_grid + gi;
             land->z = -1.0f;
         }
         const float4 sp = A.spec[l];
@@ -232,7 +235,7 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
 //      wavelength's colour weights, to the composite.
 // Bound by the FP32 pipes in step 2 (64 FMA per 4 shared 16-byte loads); the
 // trace before it is most of the time left.  8 x 8 tiles of 64^2, 16
-// wavelengths, radius 13 (the default settings): 3.96 -> 0.44 ms for both
+// wavelengths, radius 13 (the default settings): 3.96 -> 0.35 ms for both
 // kernels.  The trace stays a kernel of its own (landings through a scratch
 // that fits L2): inlined here it rounded some landings differently.
 constexpr int kDenseChunk = 32;       // landings per outer-product step
@@ -503,7 +506,15 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
                 const unsigned ns = (unsigned)std::min(land_s, n_sources - s0);
                 A.s_base = s0; A.l_base = l0;
                 A.n_land = std::min(land_l, n_spec - l0);
-                psf_kernel<true><<<dim3(ns, blocks), kPsfThreads, smem, st>>>(A);
+                // wavelengths over grid.z until there are about eight CTAs per
+                // resident slot (four of 58 registers x 256 per SM): 64 cells of
+                // 2816 samples are 704 CTAs, a second wave of 96 with all 16
+                // wavelengths in each: landings 330 -> 256 us in eight parts
+                // (0.96 -> 0.88 ms a call; in two 0.92, four 0.89, sixteen 0.89)
+                const long long ctas = (long long)ns * blocks, want = 32LL * n_sm;
+                const int parts = (int)std::min<long long>(A.n_land, std::max(1LL, (want + ctas - 1) / ctas));
+                const int per = (A.n_land + parts - 1) / parts;
+                psf_kernel<true><<<dim3(ns, blocks, (unsigned)((A.n_land + per - 1) / per)), kPsfThreads, smem, st>>>(A);
                 psf_dense_kernel<<<dim3(ns, (unsigned)A.n_land, (unsigned)dense_z(rounds)), kPsfThreads, dense_smem, st>>>(A);
                 launches += 2;
             }

@@ -34,3 +34,24 @@ def test_psf_dense_tiles(pins, tile_w, tile_h, grid, sigma_px):
                      tile_w, tile_h, 2, 2 * tile_w, 2 * tile_h, mm_pp, False, sigma, radius)
     assert want.sum() > 0
     assert rel_l2(got, want) < 2e-3
+
+
+def test_wavelengths_split_into_uneven_parts(pins):
+    """25 sources of 13 blocks: the landings' 31 wavelengths go in parts of 3, the
+    last one shorter.  The same atlas without the splat's Gaussian being dense
+    (bilinear) carries the same energy into each tile: the Gaussian is normalised
+    and 2 px wide here, and the landings stay clear of the 64 px tiles' borders.
+    Float32 sums of ~80,000 weights: 80,000 x 2^-24 apart at most, and the
+    Gaussian's taps below 1e-6 of its sum are left out (25 x 25 of them at most)."""
+    import ghostlight_gb300 as gl
+    lens = gl.OpticalSystem.from_records(lens_from_pins(pins, "cfg1_double_gauss_12"))
+    src = np.array([[0.02 * i, 0.02 * j, 1.0, 0.8, 0.6, 0.0, 0.0] for j in range(5) for i in range(5)], np.float32)
+    energy = []
+    for sigma_um in (0.0, 25.0):
+        cfg = gl.PSFConfig(grid_nx=5, grid_ny=5, tile_w=64, tile_h=64, tile_extent_mm=0.8, ray_grid=64, spectral_samples=31,
+                           splat_sigma_um=sigma_um)
+        out = gl.render_psf(src, lens, cfg)
+        a = np.stack([out[k].cpu().numpy() for k in ("r", "g", "b")]).astype(np.float64)
+        energy.append(a.reshape(3, 5, 64, 5, 64).sum((2, 4)))
+    assert energy[0].min() > 0
+    assert np.abs(energy[1] / energy[0] - 1.0).max() <= 80000 * 2.0 ** -24 + 625e-6
