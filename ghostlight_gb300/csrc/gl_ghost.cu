@@ -164,8 +164,9 @@ struct __align__(16) HotRec {
 // elliptical stop, single-layer coating with at least one layer, no
 // attenuator — whose step is one straight-line path behind one test.
 // HB_ROUND: an HB_FAST surface whose stop is round (aspect 1).
+// HB_COMMON: a surface of any form and stop with HB_FAST's coating.
 enum HotBits { HB_ACTIVE = 1, HB_GENERAL = 2, HB_POLYGON = 4, HB_SIMPLE = 8, HB_ATTEN = 16, HB_IMAGE = 32,
-               HB_FAST = 64, HB_ROUND = 128 };
+               HB_FAST = 64, HB_ROUND = 128, HB_COMMON = 256 };
 
 __device__ __forceinline__ HotRec make_hot(const SurfRec& s)
 {
@@ -179,6 +180,7 @@ __device__ __forceinline__ HotRec make_hot(const SurfRec& s)
              ((s.shape == 1) ? HB_POLYGON : 0) | ((s.coating == 0) ? HB_SIMPLE : 0) |
              ((s.coating == 4) ? HB_ATTEN : 0) | ((s.shape == 2) ? HB_IMAGE : 0);
     if (h.bits == (HB_ACTIVE | HB_SIMPLE) && s.ar_layers >= 1) h.bits |= HB_FAST | (s.aspect == 1.0f ? HB_ROUND : 0);
+    if ((h.bits & (HB_ACTIVE | HB_SIMPLE | HB_ATTEN)) == (HB_ACTIVE | HB_SIMPLE) && s.ar_layers >= 1) h.bits |= HB_COMMON;
     h.ar_layers = s.ar_layers;
     h.ar_scale = 1.0f;
     for (int i = 1; i < s.ar_layers; ++i) h.ar_scale *= 0.25f;
@@ -261,25 +263,52 @@ __device__ __forceinline__ float refract_unit(V3& d, V3 nrm, float ci, float n1,
 // ROUND: the stop is round (no aspect scaling).  reflect_ior is read only
 // on a reflecting step: through ior_a (the IOR after surface a) when the walk
 // runs backward, else it is the current medium.
-template <bool WEIGHT, bool ROUND>
+// COMMON: any HB_COMMON surface (s: its record).  Other forms and stops take
+// their own way to the hit and the normal and join the path there.
+template <bool WEIGHT, bool ROUND, bool COMMON = false>
 __device__ __forceinline__ bool surface_step_fast(V3& o, V3& d, const HotRec& h, float kdelta, float n2,
                                                   bool reflecting, bool back, const float2* ior_a, float& cur,
-                                                  float& w, bool alive)
+                                                  float& w, bool alive, const SurfRec* s = nullptr)
 {
-    const float c = h.c;
-    V3 q;
-    float t;
-    bool ok = alive & sphere_hit(o, d, h.z, c, t, q);
-    const float hx = ROUND ? q.x : q.x * h.inv_aspect, hy = q.y;
-    ok = ok & (hx * hx + hy * hy <= h.sa2);
+    bool ok;
+    V3 nrm;
+    if (!COMMON || (h.bits & HB_FAST))
+    {
+        const float c = h.c;
+        V3 q;
+        float t;
+        ok = alive & sphere_hit(o, d, h.z, c, t, q);
+        const float hx = ROUND ? q.x : q.x * h.inv_aspect, hy = q.y;
+        ok = ok & (hx * hx + hy * hy <= h.sa2);
+        nrm = v3(c * q.x, c * q.y, c * q.z - 1.0f);
+        o = v3(q.x, q.y, q.z + h.z);
+    }
+    else if (h.bits & HB_GENERAL)
+    {
+        float t = 0.0f;
+        ok = alive && intersect_general(o, d, *s, t, nrm);
+        o = o + d * t;
+    }
+    else
+    {
+        const float c = h.c;
+        V3 q;
+        float t;
+        ok = alive & sphere_hit(o, d, h.z, c, t, q);
+        const float hx = q.x * h.inv_aspect, hy = q.y;
+        const float h2 = hx * hx + hy * hy;
+        ok = ok & (h2 <= h.sa2);
+        if (h.bits & HB_POLYGON) ok = ok & check_polygon(hx, hy, h2, *s);
+        else if ((h.bits & HB_IMAGE) && ok) ok = image_aperture_ok(q.x, q.y, *s);
+        nrm = v3(c * q.x, c * q.y, c * q.z - 1.0f);
+        o = v3(q.x, q.y, q.z + h.z);
+    }
     // The normal is not turned to oppose the ray: with cr = -nrm.d, ci = |cr|
     // and sg the sign of cr, reflection d + (sg nrm)(2 ci) = d + nrm (2 cr)
     // and Snell's nr d + (sg nrm)(nr ci - ct) = nr d + nrm (nr cr - sg ct),
     // the signs cancelling exactly.
-    const V3 nrm = v3(c * q.x, c * q.y, c * q.z - 1.0f);
     const float cr = -dot(nrm, d);
     const float ci = fabsf(cr);
-    o = v3(q.x, q.y, q.z + h.z);
     const float n1 = cur;
     if (reflecting)
     {
@@ -668,12 +697,14 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_render
 // the last b and before the last a, wait in the lane's shared-memory slot
 // (which the pair-by-pair walk uses for its splat footprint: a task has one
 // wavelength, so there is nothing to carry).
-// Bound by instruction issue (74% of the slots, the rest mostly waits for
-// instructions: the warps of an SM stand at different surfaces, and the code of
-// all kinds of step is larger than the first instruction cache, so the round-stop
-// copy of the common step is left out here, 2%).  24 surfaces, 253 pairs on
-// adaptive grids, 31 wavelengths: the render 5.15 -> 1.60 ms; 120 pairs x 5
-// sources, 64^2 x 16 wavelengths: 1.66 -> 0.50.
+// Bound by instruction issue and fetch: the warps of an SM stand at different
+// surfaces, and with a copy of the step per kind of surface their instructions
+// came from the cache of the whole GPC at 97% of its rate (82% hits in the SM's,
+// 74% of the issue slots used; the probe, whose step has no weights, 98% and
+// 87%).  So the round-stop copy is left out here and surfaces of other forms and
+// stops join the common step behind their intersection (HB_COMMON).  24 surfaces,
+// 253 pairs on adaptive grids, 31 wavelengths: the render 5.15 -> 1.50 ms; 120
+// pairs x 5 sources, 64^2 x 16 wavelengths: 1.66 -> 0.47.
 enum RunFlags { RUN_REFLECT = 1, RUN_BACK = 2, RUN_LOAD_F = 4, RUN_LOAD_B = 8, RUN_SAVE_F = 16, RUN_SAVE_B = 32,
                 RUN_FORWARD = 64, RUN_LAST = 128 };
 
@@ -856,8 +887,8 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderMinBlocks) ghost_tree_k
                 const float n2 = back ? io.y : io.x;
                 const float rior = (back && refl) ? io.x : cur;
                 bool ok;
-                if (hr.bits & HB_FAST)          // (a round stop's aspect factor is exactly 1)
-                    ok = surface_step_fast<!PROBE, false>(o, d, hr, kdelta, n2, refl, back, abl + s, cur, w, alive);
+                if (hr.bits & HB_COMMON)        // (a round stop's aspect factor is exactly 1)
+                    ok = surface_step_fast<!PROBE, false, true>(o, d, hr, kdelta, n2, refl, back, abl + s, cur, w, alive, T.lens + s);
                 else if (hr.bits & HB_ACTIVE)
                     ok = surface_step<!PROBE>(o, d, hr, T.lens[s], sp.x, kdelta, n2, refl, rior, cur, w, alive);
                 else continue;
