@@ -303,7 +303,7 @@ int gl_survivor_center(const gl_surface* surfaces, int n, float lambda, const fl
 int gl_survivor_envelope(const gl_surface* surfaces, int n, float lambda, const float* dir, float launch_z, float cx, float cy,
                          float ep_x, float ep_y, int me, int ss, float* d_env, void* stream)
 {
-    if (!surfaces || n <= 0 || !dir || !d_env || me < 1 || me > 4096 || ss < 1 || ss > 64)
+    if (!surfaces || n <= 0 || !dir || !d_env || me < 1 || me > 32768 || ss < 1 || ss > 64)
         return fail(GL_ERR_INVALID, "survivor_envelope: bad arguments");
     SurviveArgs A{};
     A.m = me; A.ss = ss;

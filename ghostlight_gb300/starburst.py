@@ -801,7 +801,7 @@ def survivor_envelope(lens, ep_x, ep_y, cx, cy, ax, ay, ME: int, survives=None, 
     f = np.float32
     from ._abi import surface_array
     from . import _native
-    if survives is None and contains is None:
+    if survives is None and contains is None and 0 < ME <= 32768:
         return _survivor_envelope_device(lens, ep_x, ep_y, cx, cy, ax, ay, ME).cpu().numpy()
     survives = survives or (lambda x, y, z, d: _survives_device(lens, x, y, z, d))
     if contains is None:
