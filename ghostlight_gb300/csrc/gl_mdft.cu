@@ -912,26 +912,30 @@ __global__ void __launch_bounds__(128) mdft_fold_kernel(const float* __restrict_
 
 // ---- FP32 CUDA-core form -------------------------------------------------------
 // The same folded products in FP32 FMAs over the TF32 form's storage.  A CTA
-// makes a 64 x 64 tile of every row block of a unit (step 1: one parity of T;
-// step 2: Re E and Im E over both), 256 threads of 4 x 4 per block, reduction
-// chunks of 16 staged in shared memory one chunk ahead.  Step 2 adds its
-// wavelengths' colours up in registers; a frame of few tiles is also split over
-// wavelength ranges (n_ranges), whose CTAs add into the planes with atomics.
-// Bound by the FP32 pipes: 32 FMA per three 16-byte shared loads (box: 16 per
-// two).  256^2 pupil to 512^2, 8 wavelengths: both steps 1.75 -> 0.09 ms (the
-// unfolded form looped over the wavelengths in 16 CTAs of 128 x 128 tiles).
+// makes a tile of 16 P x 64 of every row block of a unit (step 1: one parity of T;
+// step 2: Re E and Im E over both), 256 threads of P x 4 per block, reduction
+// chunks of 16 staged in shared memory one chunk ahead.  In step 2 the wavelengths
+// are split over CTAs (n_ranges), which add into the planes with atomics; P = 4
+// adds its wavelengths' colours up in registers, P = 8 has none left for that.
+// Bound by shared-memory reads and the FP32 pipes: P = 4 32 FMA per three 16-byte
+// loads (box: 16 per two), P = 8 64 per four (32 per three).  256^2 pupil to 512^2,
+// 8 wavelengths: step 2 79 -> 58 us, both steps 1.75 -> 0.07 ms (the unfolded form
+// looped over the wavelengths in 16 CTAs of 128 x 128 tiles); 512^2 to 2048^2, 8:
+// 1.88 -> 1.73 ms.
 constexpr int kSB = 64, kSK = 16;
 
-template <int STEP, bool BOX>
+template <int STEP, bool BOX, int P>
 __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restrict__ W, const float* __restrict__ B,
                                                            MdftArgs args, int lam1, int n_ranges)
 {
+    static_assert(P == 4 || (P == 8 && STEP == 2), "rows per thread");
     constexpr int NBLK = BOX ? 1 : 2;
-    __shared__ __align__(16) float sA[kSK][kSB + 4];
+    constexpr int kRows = 16 * P, kLoads = P / 4;              // rows of the tile, staging loads of them per thread
+    __shared__ __align__(16) float sA[kSK][kRows + 4];
     __shared__ __align__(16) float sB[NBLK][kSK][kSB + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int lr = tid >> 2, lc = (tid & 3) * 4;               // row and first column of this thread's staging loads
-    const int nh = args.nh, xb = blockIdx.x, mb = blockIdx.y;  // 64-wide tiles
+    const int nh = args.nh, xb = blockIdx.x, mb = blockIdx.y;  // tiles of kRows x 64
     int l0, l1, part = 0;
     if (STEP == 1)
     {
@@ -945,14 +949,15 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
         l0 = args.lam_base + (int)blockIdx.z * per;
         l1 = min(lam1, l0 + per);
     }
-    float rgb[STEP == 2 ? 3 : 1][4][4] = {};
+    constexpr bool kSum = STEP == 2 && P == 4;                 // colours summed in registers
+    float rgb[kSum ? 3 : 1][4][4] = {};
     for (int lam = l0; lam < l1; ++lam)
     {
-        float acc[NBLK][4][4] = {};
+        float acc[NBLK][P][4] = {};
         {
             // chunks of C and S in turn (step 2), like the tensor-core forms
             constexpr int kPh = STEP == 2 ? 2 : 1;
-            const float* Ar = W + ((size_t)(lam * 2 + part) * args.KA + mb * kSB + lr) * nh + lc;
+            const float* Ar = W + ((size_t)(lam * 2 + part) * args.KA + mb * kRows + lr) * nh + lc;
             const size_t step_a = (size_t)args.KA * nh, step_b = (size_t)NBLK * (STEP == 2 ? 128 : args.nhr) * nh;
             const float* Br[NBLK];
             #pragma unroll
@@ -964,14 +969,21 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                     : (size_t)(part * NBLK + j) * args.nhr + xb * kSB + lr;
                 Br[j] = B + row * nh + lc;
             }
-            float4 pa = *reinterpret_cast<const float4*>(Ar), pb[NBLK];
+            float4 pa[kLoads], pb[NBLK];
+            #pragma unroll
+            for (int h = 0; h < kLoads; ++h) pa[h] = *reinterpret_cast<const float4*>(Ar + (size_t)h * 64 * nh);
             #pragma unroll
             for (int j = 0; j < NBLK; ++j) pb[j] = *reinterpret_cast<const float4*>(Br[j]);
             const int chunks = kPh * (nh / kSK);
             for (int ch = 0; ch < chunks; ++ch)
             {
                 __syncthreads();
-                sA[lc][lr] = pa.x; sA[lc + 1][lr] = pa.y; sA[lc + 2][lr] = pa.z; sA[lc + 3][lr] = pa.w;
+                #pragma unroll
+                for (int h = 0; h < kLoads; ++h)
+                {
+                    const int r = lr + h * 64;
+                    sA[lc][r] = pa[h].x; sA[lc + 1][r] = pa[h].y; sA[lc + 2][r] = pa[h].z; sA[lc + 3][r] = pa[h].w;
+                }
                 #pragma unroll
                 for (int j = 0; j < NBLK; ++j)
                 {
@@ -982,22 +994,28 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                 if (ch + 1 < chunks)
                 {
                     const int k0 = ((ch + 1) / kPh) * kSK, cs = (ch + 1) % kPh;
-                    pa = *reinterpret_cast<const float4*>(Ar + cs * step_a + k0);
+                    #pragma unroll
+                    for (int h = 0; h < kLoads; ++h) pa[h] = *reinterpret_cast<const float4*>(Ar + cs * step_a + (size_t)h * 64 * nh + k0);
                     #pragma unroll
                     for (int j = 0; j < NBLK; ++j) pb[j] = *reinterpret_cast<const float4*>(Br[j] + cs * step_b + k0);
                 }
                 #pragma unroll
                 for (int kk = 0; kk < kSK; ++kk)
                 {
-                    const float4 a4 = *reinterpret_cast<const float4*>(&sA[kk][ty * 4]);
-                    const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+                    float av[P];
+                    #pragma unroll
+                    for (int h = 0; h < kLoads; ++h)
+                    {
+                        const float4 a4 = *reinterpret_cast<const float4*>(&sA[kk][h * 64 + ty * 4]);
+                        av[4 * h] = a4.x; av[4 * h + 1] = a4.y; av[4 * h + 2] = a4.z; av[4 * h + 3] = a4.w;
+                    }
                     #pragma unroll
                     for (int j = 0; j < NBLK; ++j)
                     {
                         const float4 b4 = *reinterpret_cast<const float4*>(&sB[j][kk][tx * 4]);
                         const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
                         #pragma unroll
-                        for (int p = 0; p < 4; ++p)
+                        for (int p = 0; p < P; ++p)
                             #pragma unroll
                             for (int q = 0; q < 4; ++q) acc[j][p][q] = fmaf(av[p], bv[q], acc[j][p][q]);
                     }
@@ -1017,7 +1035,7 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                 const int dst = BOX ? part : (part == 0 ? (j == 0 ? 0 : 3) : (j == 0 ? 1 : 2));
                 const float sign = (part == 0 && j == 0) ? 1.0f : -1.0f;
                 #pragma unroll
-                for (int p = 0; p < 4; ++p)
+                for (int p = 0; p < P; ++p)
                     *reinterpret_cast<float4*>(T + (blk + dst * 128 + (mb & 1) * kSB + ty * 4 + p) * nh + i0) =
                         make_float4(sign * acc[j][p][0], sign * acc[j][p][1], sign * acc[j][p][2], sign * acc[j][p][3]);
             }
@@ -1027,19 +1045,47 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
             const float4 w = args.weights[lam];
             const float wr = w.x * args.tint.x, wg = w.y * args.tint.y, wb = w.z * args.tint.z;
             #pragma unroll
-            for (int p = 0; p < 4; ++p)
+            for (int p = 0; p < P; ++p)
+            {
+                float I[4];
                 #pragma unroll
                 for (int q = 0; q < 4; ++q)
                 {
                     const float re = acc[0][p][q], im = BOX ? 0.0f : acc[NBLK - 1][p][q];
-                    const float I = BOX ? re : re * re + im * im;
-                    rgb[0][p][q] += wr * I;
-                    rgb[1 % (STEP == 2 ? 3 : 1)][p][q] += wg * I;
-                    rgb[2 % (STEP == 2 ? 3 : 1)][p][q] += wb * I;
+                    I[q] = BOX ? re : re * re + im * im;
                 }
+                if (kSum)
+                {
+                    #pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                    {
+                        rgb[0][p & 3][q] += wr * I[q];
+                        rgb[1 % (kSum ? 3 : 1)][p & 3][q] += wg * I[q];
+                        rgb[2 % (kSum ? 3 : 1)][p & 3][q] += wb * I[q];
+                    }
+                    continue;
+                }
+                const int l = mb * kRows + (p >> 2) * 64 + ty * 4 + (p & 3), c0 = xb * kSB + tx * 4;
+                if (l >= args.win_h) continue;
+                const size_t o = (size_t)(args.y0 + l) * args.out_w + args.x0 + c0;
+                float* outs[3] = {args.out_r + o, args.out_g + o, args.out_b + o};
+                const float wc[3] = {wr, wg, wb};
+                #pragma unroll
+                for (int c = 0; c < 3; ++c)
+                {
+                    if (c0 + 3 < args.win_w && ((uintptr_t)outs[c] & 15) == 0)
+                        atomicAdd(reinterpret_cast<float4*>(outs[c]), make_float4(wc[c] * I[0], wc[c] * I[1], wc[c] * I[2], wc[c] * I[3]));
+                    else
+                    {
+                        #pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (c0 + q < args.win_w) atomicAdd(outs[c] + q, wc[c] * I[q]);
+                    }
+                }
+            }
         }
     }
-    if (STEP == 2)
+    if (kSum)
     {
         float* outs[3] = {args.out_r, args.out_g, args.out_b};
         #pragma unroll
@@ -1055,7 +1101,7 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                 #pragma unroll
                 for (int c = 0; c < 3; ++c)
                 {
-                    const float v = rgb[c % (STEP == 2 ? 3 : 1)][p][q];
+                    const float v = rgb[c % (kSum ? 3 : 1)][p][q];
                     if (n_ranges > 1) atomicAdd(outs[c] + row + q, v);
                     else outs[c][row + q] += v;                // this block owns the tile
                 }
@@ -1215,12 +1261,21 @@ static void mdft_simt(const MdftPlan* p, const MdftArgs& a1, const MdftArgs& a2,
 {
     const int nl = l1 - a1.lam_base;
     const dim3 t1((p->nh + kSB - 1) / kSB, p->Kx / kSB, 2 * nl);
-    mdft_simt_kernel<1, BOX><<<t1, 256, 0, st>>>(static_cast<const float*>(p->wx), static_cast<const float*>(p->mask), a1, l1, 1);
-    // wavelength ranges until about three CTAs per SM are in flight
+    mdft_simt_kernel<1, BOX, 4><<<t1, 256, 0, st>>>(static_cast<const float*>(p->wx), static_cast<const float*>(p->mask), a1, l1, 1);
+    // wavelength ranges until about three CTAs per SM are in flight (tall tiles,
+    // twice the work each: two)
     const int tiles = (p->Kx / kSB) * (p->Ky / kSB);
-    const int ranges = std::min(nl, std::max(1, (3 * p->sms + tiles - 1) / tiles));
-    const dim3 t2(p->Kx / kSB, p->Ky / kSB, ranges);
-    mdft_simt_kernel<2, BOX><<<t2, 256, 0, st>>>(static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime), a2, l1, ranges);
+    // Tall tiles read a third less shared memory per FMA, but halve the CTAs: 256^2
+    // to 512^2, 64 x 64 -> 128 x 64, whole plan: 96.3 -> 75.9 us (256 tall CTAs),
+    // 55.4 -> 49.2 (96), 41.0 -> 49.2 (64), 29.0 -> 30.8 (24).
+    const bool tall = (long long)tiles * nl > p->sms;          // tiles / 2 tall ones: half of the SMs or more
+    const int rows = tall ? 128 : kSB;
+    const int ranges = std::min(nl, std::max(1, ((tall ? 2 : 3) * p->sms + tiles * kSB / rows - 1) / (tiles * kSB / rows)));
+    const dim3 t2(p->Kx / kSB, p->Ky / rows, ranges);
+    if (tall)
+        mdft_simt_kernel<2, BOX, 8><<<t2, 256, 0, st>>>(static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime), a2, l1, ranges);
+    else
+        mdft_simt_kernel<2, BOX, 4><<<t2, 256, 0, st>>>(static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime), a2, l1, ranges);
 }
 
 }  // namespace gl
