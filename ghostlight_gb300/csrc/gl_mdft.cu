@@ -216,6 +216,10 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 // its roundings.  Step 1 makes [Tr | Ti] = [Wr | Wi] A, step 2 accumulates
 // D1 = Wr [Tr | Ti], D2 = Wi [Tr | Ti] and combines them (Re E = D1[Tr] -
 // D2[Ti], Im E = D1[Ti] + D2[Tr]); the box form makes D1[Tr] and D2[Ti] only.
+// The pixel-integrated form in split BF16 is not folded either: its images are a
+// small window of dim pixels around a peak, where the order of the additions
+// shows.  It runs like TF32, with the reduction in three passes (hi hi, hi lo,
+// lo hi) over the same [hi | lo] rows.
 // FORM 2 (FP32 on the CUDA cores) is folded.  Accumulation is FP32 in TMEM (or
 // registers) throughout.
 //
@@ -232,7 +236,10 @@ namespace gl {
 namespace {
 
 constexpr int kMdftThreads = 192;     // warps 0-3 epilogue, warp 4 TMA, warp 5 MMA
-constexpr int kTf32 = 1;              // the form that is not folded
+constexpr int kTf32 = 1;              // not folded
+constexpr int kSplitBox = 3;          // split BF16, pixel-integrated: not folded, three passes (a plan's form 0 with box)
+__host__ __device__ constexpr bool is_bf16(int form) { return form == 0 || form == kSplitBox; }
+__host__ __device__ constexpr bool is_folded(int form) { return form == 0 || form == 2; }
 constexpr int kOpTile = 128 * 128;    // bytes of one 128-row x 128-byte operand tile
 
 struct MdftArgs {
@@ -258,14 +265,14 @@ struct MdftArgs {
 template <int FORM>
 __device__ __forceinline__ void mma_any(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
 {
-    if (FORM == 0) tc::mma_f16(d, a, b, idesc, acc);
+    if (is_bf16(FORM)) tc::mma_f16(d, a, b, idesc, acc);
     else tc::mma_tf32(d, a, b, idesc, acc);
 }
 
 template <int FORM>
 __host__ __device__ constexpr uint32_t idesc_any(int M, int N)
 {
-    return FORM == 0 ? tc::idesc_bf16(M, N, false) : tc::idesc_tf32(M, N, false);
+    return is_bf16(FORM) ? tc::idesc_bf16(M, N, false) : tc::idesc_tf32(M, N, false);
 }
 
 __device__ __forceinline__ void store_split16(__nv_bfloat16* row, int nh, int i0, const float (&v)[16], float sign)
@@ -292,7 +299,7 @@ __device__ __forceinline__ void store_split16(__nv_bfloat16* row, int nh, int i0
 // B (folded: hi and lo of each), as many stages as fit, four at most.
 template <int FORM, int STEP, int TN, bool BOX, int CL>
 struct MdftShape {
-    static constexpr bool kFold = FORM != kTf32;
+    static constexpr bool kFold = is_folded(FORM);
     static constexpr int kBSets = kFold ? 2 : 1;
     static constexpr int kBlocks = kFold ? (BOX ? 1 : 2) : STEP;    // row blocks of B per unit and set
     static constexpr int kRows = STEP == 2 ? TN : 128;              // rows of one block
@@ -331,8 +338,8 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
     const int rank = CL == 2 ? (int)(blockIdx.x & 1) : 0;
     using Sh = MdftShape<FORM, STEP, TN, BOX, CL>;
     constexpr int kStagesM = Sh::kStages;
-    constexpr int kbe = (FORM == 0) ? 64 : 32;                   // reduction elements per 128-byte row
-    constexpr int kStep = (FORM == 0) ? 16 : 8;                  // and per MMA
+    constexpr int kbe = is_bf16(FORM) ? 64 : 32;                   // reduction elements per 128-byte row
+    constexpr int kStep = is_bf16(FORM) ? 16 : 8;                  // and per MMA
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align1024(smem_raw);
     __shared__ uint64_t full[kStagesM], empty[kStagesM], acc_full[2], acc_empty[2], mma_done;
@@ -410,7 +417,10 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                         if (it >= kStagesM && !tc::mbar_wait(&empty[s], (r - 1) & 1, err, tc::TC_TIMEOUT_EMPTY)) { stop = true; break; }
                         uint8_t* st = smem + s * Sh::kStageBytes;
                         if (rank == 0) tc::mbar_expect_tx(&full[s], CL * Sh::kStageBytes);
-                        const int x = kb * kbe;
+                        // three passes: hi hi, hi lo, lo hi
+                        const int pass = FORM == kSplitBox ? kb / (args.nkb / 3) : 0;
+                        const int x = (FORM == kSplitBox ? kb % (args.nkb / 3) : kb) * kbe + (pass == 2 ? args.nh : 0);
+                        const int xB = FORM == kSplitBox ? (kb % (args.nkb / 3)) * kbe + (pass == 1 ? args.nh : 0) : x;
                         const uint32_t bar = CL == 2 ? tc::leader_u32(&full[s]) : 0u;
                         auto load = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1) {
                             if (CL == 2) tc::tma_load_2d_pair(dst, map, c0, c1, bar);
@@ -436,7 +446,7 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                                 }
                                 else
                                     rowB = q * args.nhr + xb * 128;
-                                load(st + 2 * kOpTile + t * Sh::kBBytes + j * Sh::kRows * 128, &tB, t * args.nh + x, rowB);
+                                load(st + 2 * kOpTile + t * Sh::kBBytes + j * Sh::kRows * 128, &tB, t * args.nh + xB, rowB);
                             }
                         ++issued;
                     }
@@ -483,7 +493,7 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                     // folded: the lo set; TF32 box: the Ti block
                     const uint64_t b1 = tc::sw128_desc(tc::smem_u32(st + 2 * kOpTile + (Sh::kFold ? Sh::kBBytes : Sh::kRows * 128)));
                     // the last step of a reduction may be partly past nh (whatever lies there is not multiplied)
-                    const int left = (args.nh - kb * kbe) / kStep;
+                    const int left = FORM == kSplitBox ? 4 : (args.nh - kb * kbe) / kStep;
                     #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
                     {
@@ -626,7 +636,7 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                         tc::tmem_ld16(ta + (uint32_t)(j * 128 + c * 16), v);
                         const int i0 = xb * 128 + c * 16;
                         if (!ok || i0 >= args.nh) continue;
-                        if (FORM == 0)
+                        if (is_bf16(FORM))
                         {
                             __nv_bfloat16* T = static_cast<__nv_bfloat16*>(args.tprime);
                             store_split16(T + (blk + dst * 128 + row) * (size_t)(2 * args.nh), args.nh, i0, v, sign);
@@ -719,7 +729,7 @@ __global__ void __launch_bounds__(256) mdft_dft_kernel(DftRows R, int n_lambda, 
     const float bh = kf - R.ck_hi;
     const float bb = bh - kf;
     const float bl = ((kf - (bh - bb)) + (-R.ck_hi - bb)) - R.ck_lo;
-    const int Kp = FORM == 0 ? 2 * nh : nh;
+    const int Kp = is_bf16(FORM) ? 2 * nh : nh;
     const size_t rc = ((size_t)(lam * 2 + 0) * R.K + k) * Kp, rs = ((size_t)(lam * 2 + 1) * R.K + k) * Kp;
     for (int m = 2 * threadIdx.x; m < nh; m += 2 * blockDim.x)
     {
@@ -739,9 +749,9 @@ __global__ void __launch_bounds__(256) mdft_dft_kernel(DftRows R, int n_lambda, 
             sincospif(2.0f * fr, &sv[q], &cv[q]);
             const float amp = amps[m + q];
             cv[q] *= amp;
-            sv[q] = FORM == kTf32 ? -amp * sv[q] : amp * sv[q];
+            sv[q] = is_folded(FORM) ? amp * sv[q] : -amp * sv[q];
         }
-        if (FORM == 0)
+        if (is_bf16(FORM))
         {
             __nv_bfloat16* W = static_cast<__nv_bfloat16*>(R.out);
             __nv_bfloat162 ch, cl, sh, sl;
@@ -839,10 +849,19 @@ template <int FORM>
 __device__ __forceinline__ void mdft_fold_one(const float* __restrict__ a, void* out, int n, int nh, int nhr, int nf,
                                               int h2, int box, int x, int y)
 {
-    const int Kp = FORM == 0 ? 2 * nh : nh;
-    if (FORM == kTf32)                               // not folded: nh = n
+    const int Kp = is_bf16(FORM) ? 2 * nh : nh;
+    if (!is_folded(FORM))                            // nh = n
     {
-        static_cast<float*>(out)[(size_t)y * Kp + x] = a[(size_t)y * n + x];
+        const float w = a[(size_t)y * n + x];
+        if (!is_bf16(FORM))
+        {
+            static_cast<float*>(out)[(size_t)y * Kp + x] = w;
+            return;
+        }
+        __nv_bfloat16* M = static_cast<__nv_bfloat16*>(out) + (size_t)y * Kp + x;
+        const __nv_bfloat16 h = __float2bfloat16_rn(w);
+        M[0] = h;
+        M[nh] = __float2bfloat16_rn(w - __bfloat162float(h));
         return;
     }
     const int base = (h2 + 1) >> 1;                  // index at the smallest distance
@@ -1115,11 +1134,14 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
 // ---- MDFT plan ----------------------------------------------------------------
 constexpr double kMaxCentre = 12288.0;   // pattern centre range (pixels)
 
+// The kernels' form of a plan.
+static int mdft_kernel_form(int form, int box) { return form == 0 && box ? kSplitBox : form; }
+
 struct MdftPlan {
     int n = 0, Kx = 0, Ky = 0, n_lambda = 0, form = 0, Kp = 0, elem = 2;
     // folded reduction: nf distances |j - cj|, padded to nh (16); nhr rows per
     // part of A' (128); h2 = 2 cj
-    // (TF32, not folded: nf = nh = n); d0 = smallest distance (TF32: -cj)
+    // (not folded: nf = nh = n); d0 = smallest distance (not folded: -cj)
     int nf = 0, nh = 0, nhr = 0, h2 = 0;
     float d0 = 0.0f;
     void* wx = nullptr;     // W_x' [lam][C | S][Kx][Kp]
@@ -1167,7 +1189,8 @@ static cudaError_t mdft_build_matrices(MdftPlan* p, cudaStream_t st)
     for (const DftRows& r : R)
     {
         const int grid = (p->n_lambda * r.K + (int)block.y - 1) / (int)block.y;
-        if (p->form == 0) mdft_dft_kernel<0><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
+        if (p->form == 0 && p->box) mdft_dft_kernel<kSplitBox><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
+        else if (p->form == 0) mdft_dft_kernel<0><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
         else if (p->form == kTf32) mdft_dft_kernel<kTf32><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
         else mdft_dft_kernel<2><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
     }
@@ -1305,14 +1328,15 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     p->cx = center_x; p->cy = center_y;
     p->box = box; p->cj = red_center;
     p->h2 = (int)(2.0f * red_center);
-    p->nf = form == kTf32 ? n : (int)std::floor(std::max((double)red_center, (double)(n - 1) - (double)red_center)) + 1;
-    p->d0 = form == kTf32 ? -red_center : ((p->h2 & 1) ? 0.5f : 0.0f);
+    const bool folded = is_folded(mdft_kernel_form(form, box));
+    p->nf = !folded ? n : (int)std::floor(std::max((double)red_center, (double)(n - 1) - (double)red_center)) + 1;
+    p->d0 = !folded ? -red_center : ((p->h2 & 1) ? 0.5f : 0.0f);
     p->nh = (p->nf + 15) / 16 * 16;
     p->nhr = (p->nh + 127) / 128 * 128;
     p->Kp = form == 0 ? 2 * p->nh : p->nh;
     p->elem = form == 0 ? 2 : 4;
-    const int NBx = Kx / 128, parts = (box || form == kTf32) ? 2 : 4;      // of T'
-    const int mparts = form == kTf32 ? 1 : parts;                          // of A'
+    const int NBx = Kx / 128, parts = (box || !folded) ? 2 : 4;            // of T'
+    const int mparts = !folded ? 1 : parts;                          // of A'
     const size_t wxbytes = (size_t)n_lambda * 2 * Kx * p->Kp * p->elem;
     const size_t wybytes = (size_t)n_lambda * 2 * Ky * p->Kp * p->elem;
     const size_t mbytes = (size_t)mparts * p->nhr * p->Kp * p->elem;
@@ -1355,7 +1379,7 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     }
     chk(cudaStreamSynchronize(st));
     // shared-memory opt-in once here, so execute enqueues kernels only (graph capture)
-    if (form == 0) chk(box ? mdft_prepare_all<0, true>(&p->pairs) : mdft_prepare_all<0, false>(&p->pairs));
+    if (form == 0) chk(box ? mdft_prepare_all<kSplitBox, true>(&p->pairs) : mdft_prepare_all<0, false>(&p->pairs));
     else if (form == 1) chk(box ? mdft_prepare_all<1, true>(&p->pairs) : mdft_prepare_all<1, false>(&p->pairs));
     const CUtensorMapDataType dt = form == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const uint32_t bc = form == 0 ? 64 : 32;
@@ -1428,7 +1452,8 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
         kernel<<<fold, 128, 0, st>>>(d_pupil, p->mask, p->n, p->nh, p->nhr, p->nf, p->h2, p->box, d_out_r, d_out_g,
                                      d_out_b, zero, p->err);
     };
-    if (p->form == 0) run_fold(mdft_fold_kernel<0>);
+    if (p->form == 0 && p->box) run_fold(mdft_fold_kernel<kSplitBox>);
+    else if (p->form == 0) run_fold(mdft_fold_kernel<0>);
     else if (p->form == kTf32) run_fold(mdft_fold_kernel<kTf32>);
     else run_fold(mdft_fold_kernel<2>);
     ++launches;
@@ -1436,7 +1461,8 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     a.KA = p->Kx; a.NBm = NBx; a.NBt = NBx;
     a.nh = p->nh; a.nhr = p->nhr;
     const int kbe = p->form == 0 ? 64 : 32;
-    a.nkb = (p->nh + kbe - 1) / kbe;
+    const bool folded = is_folded(mdft_kernel_form(p->form, p->box));
+    a.nkb = (p->nh + kbe - 1) / kbe * (p->form == 0 && p->box ? 3 : 1);
     a.NB = NBx; a.NI = p->nhr / 128;
     a.tprime = p->tprime; a.out_r = d_out_r; a.out_g = d_out_g; a.out_b = d_out_b;
     a.weights = p->weights; a.err = p->err;
@@ -1444,7 +1470,7 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     a.tint = tint_rgb ? make_float4(tint_rgb[0], tint_rgb[1], tint_rgb[2], 0.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     const int l0 = p->lam0, l1 = p->lam1 < 0 ? p->n_lambda : p->lam1, nl = l1 - l0;
     a.lam_base = l0;
-    a.n_units = nl * NBx * a.NI * (p->form == kTf32 ? 1 : 2);   // step 1: (lambda, k block, pupil-row block, C / S)
+    a.n_units = nl * NBx * a.NI * (folded ? 2 : 1);   // step 1: (lambda, k block, pupil-row block, C / S)
     const int gmax = p->ctas > 0 ? p->ctas : p->sms;
     MdftArgs a2 = a;
     a2.KA = p->Ky; a2.NBm = NBy;
@@ -1457,7 +1483,7 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     }
     else if (p->form == 0)
     {
-        GL_CUDA_TRY(p->box ? (mdft_gemms<0, true>(p, a, a2, gmax, st)) : (mdft_gemms<0, false>(p, a, a2, gmax, st)));
+        GL_CUDA_TRY(p->box ? (mdft_gemms<kSplitBox, true>(p, a, a2, gmax, st)) : (mdft_gemms<0, false>(p, a, a2, gmax, st)));
     }
     else
     {

@@ -138,11 +138,12 @@ class MdftPlan:
         over the distances from the reduction centre), the operand's parity
         parts and the intermediate T' in the form's element type (split-BF16:
         two bf16 terms per element)."""
-        tf32 = self.form == "tf32"          # not folded
-        nh = self.n if tf32 else (int(max(self._red_center, self.n - 1 - self._red_center)) + 16) // 16 * 16
+        tf32 = self.form == "tf32"
+        folded = not tf32 and not (self.form == "split_bf16" and self.box)
+        nh = self.n if not folded else (int(max(self._red_center, self.n - 1 - self._red_center)) + 16) // 16 * 16
         row = nh * 4                        # two bf16 terms or one float
         parts, nl = (2 if self.box or tf32 else 4), self.n_lambda
-        return (nl * 2 * (self.Kx + self.Ky) * row + (1 if tf32 else parts) * ((nh + 127) // 128 * 128) * row +
+        return (nl * 2 * (self.Kx + self.Ky) * row + (parts if folded else 1) * ((nh + 127) // 128 * 128) * row +
                 nl * parts * self.Kx * row + 32 * nl + 4)
 
     def close(self):
