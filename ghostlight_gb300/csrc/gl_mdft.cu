@@ -220,7 +220,9 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 // small window of dim pixels around a peak, where the order of the additions
 // shows.  It runs like TF32, with the reduction in three passes (hi hi, hi lo,
 // lo hi) over the same [hi | lo] rows.
-// FORM 2 (FP32 on the CUDA cores) is folded.  Accumulation is FP32 in TMEM (or
+// FORM 2 (FP32 on the CUDA cores) is folded in the field form; its
+// pixel-integrated form makes the folded products over all signed distances, with
+// the operand in both parts (Te_r = C A, To_i = -S A).  Accumulation is FP32 in TMEM (or
 // registers) throughout.
 //
 // 512^2 pupil to 2048^2, 31 wavelengths, split BF16: step 1 233 -> 109 us, step
@@ -864,6 +866,12 @@ __device__ __forceinline__ void mdft_fold_one(const float* __restrict__ a, void*
         M[nh] = __float2bfloat16_rn(w - __bfloat162float(h));
         return;
     }
+    if (FORM == 2 && box)                            // all signed distances: both parts are the operand
+    {
+        const float w = a[(size_t)y * n + x];
+        for (int k = 0; k < 2; ++k) static_cast<float*>(out)[((size_t)k * nhr + y) * Kp + x] = w;
+        return;
+    }
     const int base = (h2 + 1) >> 1;                  // index at the smallest distance
     auto at = [&](int r, int c) {
         return (r >= 0 && r < n && c >= 0 && c < n) ? a[(size_t)r * n + c] : 0.0f;
@@ -933,18 +941,18 @@ __global__ void __launch_bounds__(128) mdft_fold_kernel(const float* __restrict_
 // The same folded products in FP32 FMAs over the TF32 form's storage.  A CTA
 // makes a tile of 16 P x 64 of every row block of a unit (step 1: one parity of T;
 // step 2: Re E and Im E over both), 256 threads of P x 4 per block, reduction
-// chunks of 16 staged in shared memory one chunk ahead.  In step 2 the wavelengths
-// are split over CTAs (n_ranges), which add into the planes with atomics; P = 4
-// adds its wavelengths' colours up in registers, P = 8 has none left for that.
+// chunks of 16 staged in shared memory one chunk ahead, sums in two levels (32
+// terms, then their sums): one long sum rounded the pattern's peak 0.3 to 1.7e-6 off
+// 64 bits, two levels 0.1 to 0.3e-6.  In step 2 the wavelengths are split over CTAs
+// (n_ranges), which add into the planes with atomics.
 // Bound by shared-memory reads and the FP32 pipes: P = 4 32 FMA per three 16-byte
 // loads (box: 16 per two), P = 8 64 per four (32 per three).  256^2 pupil to 512^2,
-// 8 wavelengths: step 2 79 -> 58 us, both steps 1.75 -> 0.07 ms (the unfolded form
-// looped over the wavelengths in 16 CTAs of 128 x 128 tiles); 512^2 to 2048^2, 8:
-// 1.88 -> 1.73 ms.
+// 8 wavelengths: both steps 1.75 -> 0.08 ms (the unfolded form looped over the
+// wavelengths in 16 CTAs of 128 x 128 tiles).
 constexpr int kSB = 64, kSK = 16;
 
 template <int STEP, bool BOX, int P>
-__global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restrict__ W, const float* __restrict__ B,
+__global__ void __launch_bounds__(256, P == 8 ? 1 : 2) mdft_simt_kernel(const float* __restrict__ W, const float* __restrict__ B,
                                                            MdftArgs args, int lam1, int n_ranges)
 {
     static_assert(P == 4 || (P == 8 && STEP == 2), "rows per thread");
@@ -968,11 +976,10 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
         l0 = args.lam_base + (int)blockIdx.z * per;
         l1 = min(lam1, l0 + per);
     }
-    constexpr bool kSum = STEP == 2 && P == 4;                 // colours summed in registers
-    float rgb[kSum ? 3 : 1][4][4] = {};
     for (int lam = l0; lam < l1; ++lam)
     {
-        float acc[NBLK][P][4] = {};
+        // two levels: a long sum of one sign (the pattern's peak) would round at every step
+        float total[NBLK][P][4] = {}, acc[NBLK][P][4] = {};
         {
             // chunks of C and S in turn (step 2), like the tensor-core forms
             constexpr int kPh = STEP == 2 ? 2 : 1;
@@ -1039,6 +1046,19 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                             for (int q = 0; q < 4; ++q) acc[j][p][q] = fmaf(av[p], bv[q], acc[j][p][q]);
                     }
                 }
+                if ((ch & 1) == 1 || ch + 1 == chunks)
+                {
+                    #pragma unroll
+                    for (int j = 0; j < NBLK; ++j)
+                        #pragma unroll
+                        for (int p = 0; p < P; ++p)
+                            #pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                            {
+                                total[j][p][q] += acc[j][p][q];
+                                acc[j][p][q] = 0.0f;
+                            }
+                }
             }
         }
         if (STEP == 1)
@@ -1056,7 +1076,7 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                 #pragma unroll
                 for (int p = 0; p < P; ++p)
                     *reinterpret_cast<float4*>(T + (blk + dst * 128 + (mb & 1) * kSB + ty * 4 + p) * nh + i0) =
-                        make_float4(sign * acc[j][p][0], sign * acc[j][p][1], sign * acc[j][p][2], sign * acc[j][p][3]);
+                        make_float4(sign * total[j][p][0], sign * total[j][p][1], sign * total[j][p][2], sign * total[j][p][3]);
             }
         }
         else
@@ -1070,19 +1090,8 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                 #pragma unroll
                 for (int q = 0; q < 4; ++q)
                 {
-                    const float re = acc[0][p][q], im = BOX ? 0.0f : acc[NBLK - 1][p][q];
+                    const float re = total[0][p][q], im = BOX ? 0.0f : total[NBLK - 1][p][q];
                     I[q] = BOX ? re : re * re + im * im;
-                }
-                if (kSum)
-                {
-                    #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                    {
-                        rgb[0][p & 3][q] += wr * I[q];
-                        rgb[1 % (kSum ? 3 : 1)][p & 3][q] += wg * I[q];
-                        rgb[2 % (kSum ? 3 : 1)][p & 3][q] += wb * I[q];
-                    }
-                    continue;
                 }
                 const int l = mb * kRows + (p >> 2) * 64 + ty * 4 + (p & 3), c0 = xb * kSB + tx * 4;
                 if (l >= args.win_h) continue;
@@ -1100,29 +1109,6 @@ __global__ void __launch_bounds__(256, 2) mdft_simt_kernel(const float* __restri
                         for (int q = 0; q < 4; ++q)
                             if (c0 + q < args.win_w) atomicAdd(outs[c] + q, wc[c] * I[q]);
                     }
-                }
-            }
-        }
-    }
-    if (kSum)
-    {
-        float* outs[3] = {args.out_r, args.out_g, args.out_b};
-        #pragma unroll
-        for (int p = 0; p < 4; ++p)
-        {
-            const int l = mb * kSB + ty * 4 + p;
-            if (l >= args.win_h) continue;
-            const size_t row = (size_t)(args.y0 + l) * args.out_w + args.x0 + xb * kSB + tx * 4;
-            #pragma unroll
-            for (int q = 0; q < 4; ++q)
-            {
-                if (xb * kSB + tx * 4 + q >= args.win_w) continue;
-                #pragma unroll
-                for (int c = 0; c < 3; ++c)
-                {
-                    const float v = rgb[c % (kSum ? 3 : 1)][p][q];
-                    if (n_ranges > 1) atomicAdd(outs[c] + row + q, v);
-                    else outs[c][row + q] += v;                // this block owns the tile
                 }
             }
         }
@@ -1289,8 +1275,9 @@ static void mdft_simt(const MdftPlan* p, const MdftArgs& a1, const MdftArgs& a2,
     // twice the work each: two)
     const int tiles = (p->Kx / kSB) * (p->Ky / kSB);
     // Tall tiles read a third less shared memory per FMA, but halve the CTAs: 256^2
-    // to 512^2, 64 x 64 -> 128 x 64, whole plan: 96.3 -> 75.9 us (256 tall CTAs),
-    // 55.4 -> 49.2 (96), 41.0 -> 49.2 (64), 29.0 -> 30.8 (24).
+    // to 512^2, 64 x 64 -> 128 x 64, whole plan (sums in one level, which are 6 us
+    // faster): 96.3 -> 75.9 us (256 tall CTAs), 55.4 -> 49.2 (96), 41.0 -> 49.2 (64),
+    // 29.0 -> 30.8 (24).
     const bool tall = (long long)tiles * nl > p->sms;          // tiles / 2 tall ones: half of the SMs or more
     const int rows = tall ? 128 : kSB;
     const int ranges = std::min(nl, std::max(1, ((tall ? 2 : 3) * p->sms + tiles * kSB / rows - 1) / (tiles * kSB / rows)));
@@ -1328,9 +1315,9 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     p->cx = center_x; p->cy = center_y;
     p->box = box; p->cj = red_center;
     p->h2 = (int)(2.0f * red_center);
-    const bool folded = is_folded(mdft_kernel_form(form, box));
-    p->nf = !folded ? n : (int)std::floor(std::max((double)red_center, (double)(n - 1) - (double)red_center)) + 1;
-    p->d0 = !folded ? -red_center : ((p->h2 & 1) ? 0.5f : 0.0f);
+    const bool folded = is_folded(mdft_kernel_form(form, box)), distances = folded && !box;
+    p->nf = !distances ? n : (int)std::floor(std::max((double)red_center, (double)(n - 1) - (double)red_center)) + 1;
+    p->d0 = !distances ? -red_center : ((p->h2 & 1) ? 0.5f : 0.0f);
     p->nh = (p->nf + 15) / 16 * 16;
     p->nhr = (p->nh + 127) / 128 * 128;
     p->Kp = form == 0 ? 2 * p->nh : p->nh;

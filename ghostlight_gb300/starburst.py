@@ -140,7 +140,7 @@ class MdftPlan:
         two bf16 terms per element)."""
         tf32 = self.form == "tf32"
         folded = not tf32 and not (self.form == "split_bf16" and self.box)
-        nh = self.n if not folded else (int(max(self._red_center, self.n - 1 - self._red_center)) + 16) // 16 * 16
+        nh = self.n if self.box or not folded else (int(max(self._red_center, self.n - 1 - self._red_center)) + 16) // 16 * 16
         row = nh * 4                        # two bf16 terms or one float
         parts, nl = (2 if self.box or tf32 else 4), self.n_lambda
         return (nl * 2 * (self.Kx + self.Ky) * row + (parts if folded else 1) * ((nh + 127) // 128 * 128) * row +
