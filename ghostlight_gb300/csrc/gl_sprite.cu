@@ -55,7 +55,9 @@ __device__ __forceinline__ size_t half_index(int N, int pair, int x) { return ((
 
 // Pass 1: columns 4 blockIdx.x .. + 3, two real ones per complex sequence; rows
 // ky < 2 pairs kept.  lit[blockIdx.x]
-// = 0 where all are zero (nothing is written then).
+// = 0 where all are zero (nothing is written then).  The grid may be a caller's
+// that starts at an odd float: pairs of columns are read as such only from 8-byte
+// boundaries (N is even, so the base decides for all rows).
 template <bool PP>
 __global__ void __launch_bounds__(1024) grid_cols(const float* __restrict__ in, int N, int pairs,
                                                   const __grid_constant__ FftDims d, const float2* __restrict__ tw,
@@ -65,10 +67,18 @@ __global__ void __launch_bounds__(1024) grid_cols(const float* __restrict__ in, 
     float2* x = sm;
     float2* y = PP ? sm + padded((size_t)N * 2) : sm;
     const int c0 = blockIdx.x * 4;
+    const bool pairwise = (reinterpret_cast<uintptr_t>(in) & 7) == 0;
     int any = 0;
     for (int i = threadIdx.x; i < 2 * N; i += blockDim.x)
     {
-        const float2 v = *reinterpret_cast<const float2*>(in + (size_t)(i >> 1) * N + c0 + 2 * (i & 1));
+        const float* q = in + (size_t)(i >> 1) * N + c0 + 2 * (i & 1);
+        float2 v;
+        if (pairwise) v = *reinterpret_cast<const float2*>(q);
+        else
+        {
+            v.x = q[0];
+            v.y = q[1];
+        }
         any |= (v.x != 0.0f) | (v.y != 0.0f);
         x[fft_slot<2, true>(i >> 1, i & 1, N)] = v;
     }
