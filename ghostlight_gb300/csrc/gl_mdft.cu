@@ -259,6 +259,7 @@ struct MdftArgs {
     // step-2 output placement: plan pixel (l, k) -> frame (y0 + l, x0 + k) of
     // planes out_w wide, kept when l < win_h and k < win_w
     int out_w, x0, y0, win_w, win_h;
+    int vec;                          // 1: every row piece of a tile starts on a 16-byte boundary in all three planes
     float4 tint;                      // per-launch colour factor on the weights
     int lam_base;                     // first wavelength of this launch's range
     int NBt;                          // step 2: output tiles per row of the frame (Kx / tile width)
@@ -547,7 +548,6 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                 float* turn = reinterpret_cast<float*>(smem + kStagesM * Sh::kStageBytes) + warp * (32 * 33);
                 const int lrow = mb * 128 + warp * 32;
                 const size_t o0 = (size_t)(args.y0 + lrow) * (size_t)args.out_w + (size_t)args.x0 + (size_t)xb * TN;
-                const bool vec = ((args.out_w | args.x0) & 3) == 0;
                 const int rows = min(32, args.win_h - lrow);
                 #pragma unroll 1
                 for (int c = 0; c < TN / 32; ++c)
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                     }
                     __syncwarp();
                     const int kc = xb * TN + c * 32;
-                    if (ok && vec)
+                    if (ok && args.vec)
                     {
                         const int col = (lane & 7) * 4;
                         for (int r = lane >> 3; r < rows; r += 4)
@@ -1454,6 +1454,9 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     a.tprime = p->tprime; a.out_r = d_out_r; a.out_g = d_out_g; a.out_b = d_out_b;
     a.weights = p->weights; a.err = p->err;
     a.out_w = out_w; a.x0 = x0; a.y0 = y0; a.win_w = win_w; a.win_h = win_h;
+    // the planes may be views that start at any float
+    a.vec = ((out_w | x0) & 3) == 0 && ((reinterpret_cast<uintptr_t>(d_out_r) | reinterpret_cast<uintptr_t>(d_out_g) |
+                                         reinterpret_cast<uintptr_t>(d_out_b)) & 15) == 0;
     a.tint = tint_rgb ? make_float4(tint_rgb[0], tint_rgb[1], tint_rgb[2], 0.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     const int l0 = p->lam0, l1 = p->lam1 < 0 ? p->n_lambda : p->lam1, nl = l1 - l0;
     a.lam_base = l0;

@@ -44,3 +44,31 @@ def test_sprite_pupil(N):
         for a, b in zip(got[1:3], want[1:3]):
             assert float((a - b).abs().max()) <= 2.0 ** -22 * float(b.abs().max())
     plan.close()
+
+
+# field and pixel form, both tiles of the second product, a pair of CTAs (2560)
+@pytest.mark.parametrize("form,K,box", [("split_bf16", 256, False), ("split_bf16", 256, True), ("split_bf16", 2560, False),
+                                        ("tf32", 256, False), ("tf32", 256, True), ("fp32", 256, False), ("fp32", 256, True)])
+def test_mdft_planes(form, K, box):
+    """One wavelength: one addition to a pixel, so equal bit for bit.  Planes that
+    start at different offsets, too, and the pupil at one."""
+    import ghostlight_gb300 as gl
+    n = 512 if K == 2560 else 128
+    r = np.random.default_rng(K)
+    A = torch.from_numpy(r.random((n, n)).astype(np.float32)).cuda()
+    plan = gl.MdftPlan(n, K, [0.9 / K], [0.8 / K], r.random((1, 3)).astype(np.float32), form, center_x=K / 2 - 0.7,
+                       center_y=K / 2 + 0.3, box=box)
+    for tile in (128,) if K == 2560 else (128, 64):
+        plan.set_launch(0, tile)
+        want = [torch.empty((K, K), device="cuda") for _ in range(3)]
+        plan.execute(A, *want)
+        assert float(want[0].abs().max()) > 0
+        for offs in [(1, 1, 1), (2, 2, 2), (3, 3, 3), (0, 1, 0), (0, 0, 2)]:
+            got = [_at_offset(torch.full((K, K), 7.0), o) for o in offs]
+            plan.execute(_at_offset(A, offs[1]), *got)
+            assert plan.status() == 0
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+        frame = [_at_offset(torch.zeros((K + 3, K + 8)), o) for o in (3, 0, 1)]
+        plan.execute_window(A, *frame, 4, 2, K - 5, K - 9)
+        for f, w in zip(frame, want):
+            assert torch.equal(f[2:2 + K - 9, 4:4 + K - 5], w[:K - 9, :K - 5])
