@@ -1432,8 +1432,18 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     const int NBx = p->Kx / 128, NBy = p->Ky / 128;
     const size_t npx = (size_t)out_w * out_h;
     int launches = 0;
-    // zeroing blocks: two waves of the chip at most, one at least (the error word)
-    const size_t zero = accumulate ? 0 : npx;
+    // zeroing blocks: one wave of the chip at most, one block at least (the error
+    // word).  A pupil that shares memory with a plane is read before the plane is
+    // zeroed, by memsets behind the fold.
+    float* planes[3] = {d_out_r, d_out_g, d_out_b};
+    const uintptr_t pupil0 = reinterpret_cast<uintptr_t>(d_pupil), pupil1 = pupil0 + sizeof(float) * (size_t)p->n * p->n;
+    bool shared = false;
+    for (float* c : planes)
+    {
+        const uintptr_t c0 = reinterpret_cast<uintptr_t>(c);
+        shared = shared || (pupil0 < c0 + sizeof(float) * npx && c0 < pupil1);
+    }
+    const size_t zero = accumulate || shared ? 0 : npx;
     const int fold = p->nh + (int)std::max<size_t>(1, std::min<size_t>((3 * zero / 4 + 1023) / 1024, 16 * (size_t)p->sms));
     auto run_fold = [&](auto kernel) {
         kernel<<<fold, 128, 0, st>>>(d_pupil, p->mask, p->n, p->nh, p->nhr, p->nf, p->h2, p->box, d_out_r, d_out_g,
@@ -1444,6 +1454,8 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     else if (p->form == kTf32) run_fold(mdft_fold_kernel<kTf32>);
     else run_fold(mdft_fold_kernel<2>);
     ++launches;
+    if (shared && !accumulate)
+        for (float* c : planes) GL_CUDA_TRY(cudaMemsetAsync(c, 0, sizeof(float) * npx, st));
     MdftArgs a;
     a.KA = p->Kx; a.NBm = NBx; a.NBt = NBx;
     a.nh = p->nh; a.nhr = p->nhr;
