@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_rows
         __syncthreads();
     }
     else
-        fft_any<kPairs, false, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
-    for (int st = 1; st < d.nrad; ++st) fft_any<kPairs, false, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+        fft_any<kPairs, false, false, PP, true, false, PP>(x, y, d, 0, tw, load, FftNone{});
+    for (int st = 1; st < d.nrad; ++st) fft_any<kPairs, false, false, PP, false, false, PP>(x, y, d, st, tw, FftNone{}, FftNone{});
     // Z = FFT(a + i b): FFT(a)[q] = (Z[q] + conj Z[Q - q]) / 2, FFT(b)[q] = (Z[q] - conj Z[Q - q]) / 2i;
     // the pairs of one column pair are neighbouring sectors, so they go to neighbouring threads
     for (int t = threadIdx.x; t < G * kPairs; t += blockDim.x)
@@ -174,13 +174,13 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_rows
 // The middle of a column: last forward stage, times the kernel spectrum, first
 // inverse stage, all on the same registers (that stage's outputs j + p m are
 // the inputs of the inverse's first stage of the same radix).
-template <int R, class MUL>
+template <int R, bool FINE, class MUL>
 __device__ __forceinline__ void conv_turn(float2 (&v)[R], int it, const FftStage& d, const MUL& mul)
 {
     const int m = d.n / R, s = it % kColsPerCta, j = it / kColsPerCta;
     #pragma unroll
     for (int p = 0; p < R; ++p) v[p] = mul(s, j + p * m, v[p]);
-    dft<R>(v, 1.0f);
+    dft<R, FINE>(v, 1.0f);
 }
 
 template <int R, bool PP, bool FIRST, bool LAST, class LD, class MUL, class ST>
@@ -196,8 +196,8 @@ __device__ __forceinline__ void conv_middle(const float2* x, float2* y, const Ff
         for (int it = threadIdx.x; it < items; it += blockDim.x)
         {
             float2 v[R];
-            fft_take<R, NB, true, false, FIRST>(v, x, it, d, ld);
-            conv_turn<R>(v, it, d, mul);
+            fft_take<R, NB, true, false, FIRST, PP>(v, x, it, d, ld);
+            conv_turn<R, PP>(v, it, d, mul);
             fft_put<R, NB, true, LAST>(v, y, it, back, st);
         }
     }
@@ -210,8 +210,8 @@ __device__ __forceinline__ void conv_middle(const float2* x, float2* y, const Ff
         {
             const int it = threadIdx.x + u * blockDim.x;
             if (it >= items) continue;
-            fft_take<R, NB, true, false, FIRST>(v[u], x, it, d, ld);
-            conv_turn<R>(v[u], it, d, mul);
+            fft_take<R, NB, true, false, FIRST, PP>(v[u], x, it, d, ld);
+            conv_turn<R, PP>(v[u], it, d, mul);
         }
         if (!FIRST) __syncthreads();
         #pragma unroll
@@ -263,12 +263,12 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_cols
     {
         if (d.nrad < 2)
         {
-            if (d.nrad == 1) fft_any<2, true, false, PP, true, true>(x, y, d, 0, tw, load, store);
+            if (d.nrad == 1) fft_any<2, true, false, PP, true, true, PP>(x, y, d, 0, tw, load, store);
             return;                                    // one point: its own transform
         }
-        fft_any<2, true, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
-        for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
-        fft_any<2, true, false, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
+        fft_any<2, true, false, PP, true, false, PP>(x, y, d, 0, tw, load, FftNone{});
+        for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false, PP>(x, y, d, st, tw, FftNone{}, FftNone{});
+        fft_any<2, true, false, PP, false, true, PP>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
         return;
     }
     const ColMul mul{khat + pair_index(0, G, k_rows, g, 0)};
@@ -278,11 +278,11 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_cols
         else if (threadIdx.x < 2) store(threadIdx.x, 0, mul(threadIdx.x, 0, load(threadIdx.x, 0)));
         return;
     }
-    fft_any<2, true, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
-    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    fft_any<2, true, false, PP, true, false, PP>(x, y, d, 0, tw, load, FftNone{});
+    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false, PP>(x, y, d, st, tw, FftNone{}, FftNone{});
     conv_middle_any<PP, false, false>(x, y, d, tw, FftNone{}, mul, FftNone{});
-    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, true, PP, false, false>(x, y, di, st, twi, FftNone{}, FftNone{});
-    fft_any<2, true, true, PP, false, true>(x, y, di, d.nrad - 1, twi, FftNone{}, store);
+    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, true, PP, false, false, PP>(x, y, di, st, twi, FftNone{}, FftNone{});
+    fft_any<2, true, true, PP, false, true, PP>(x, y, di, d.nrad - 1, twi, FftNone{}, store);
 }
 
 // Pass 3: the row pairs' transforms Z = FFT(a) + i FFT(b) from the half
@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_rows
         if (threadIdx.x < kPairs) store(threadIdx.x, 0, x[fft_slot<kPairs, false>(0, threadIdx.x, Q)]);
         return;
     }
-    for (int st = 0; st + 1 < d.nrad; ++st) fft_any<kPairs, false, true, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
-    fft_any<kPairs, false, true, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
+    for (int st = 0; st + 1 < d.nrad; ++st) fft_any<kPairs, false, true, PP, false, false, PP>(x, y, d, st, tw, FftNone{}, FftNone{});
+    fft_any<kPairs, false, true, PP, false, true, PP>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
 }
 
 int good_size(int need)

@@ -34,6 +34,21 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(
 // (sign i) * a
 __device__ __forceinline__ float2 cis(float2 a, float sign) { return make_float2(-sign * a.y, sign * a.x); }
 
+// a times the constant c + sign i s.  FINE: the constant in two floats each; one
+// rounded to one float is off by up to 3e-8 in every product with it, the same way
+// every time.  Error of a transform of 1024^2 noise against 64 bits 2.0e-7, FINE
+// 1.65e-7.  The sprite's transforms take it at no cost in time, so do short ones
+// (latency); the convolution's long ones would be 4 % slower (161 -> 168 us).
+template <bool FINE>
+__device__ __forceinline__ float2 cmul_const(float2 a, double c, double s, float sign)
+{
+    const float ch = (float)c, sh = sign * (float)s;
+    if (!FINE) return cmul(a, make_float2(ch, sh));
+    const float cl = (float)(c - (double)(float)c), sl = sign * (float)(s - (double)(float)s);
+    return make_float2(fmaf(a.x, ch, fmaf(-a.y, sh, fmaf(a.x, cl, -a.y * sl))),
+                       fmaf(a.x, sh, fmaf(a.y, ch, fmaf(a.x, sl, a.y * cl))));
+}
+
 // Padded shared-memory index: one spare word per 16 elements, so a warp
 // writing 16-element runs at a stride of 16 hits 16 different banks.
 __device__ __forceinline__ int pad(int i) { return i + (i >> 4); }
@@ -56,43 +71,30 @@ __device__ __forceinline__ void dft4(float2& v0, float2& v1, float2& v2, float2&
     v3 = csub(t1, t3);
 }
 
+template <bool FINE>
 __device__ __forceinline__ void dft3(float2& v0, float2& v1, float2& v2, float sign)
 {
-    const float c = 0.86602540378443864676f;   // sqrt(3)/2
+    constexpr double c = 0.86602540378443864676;   // sqrt(3)/2
+    constexpr float ch = (float)c, cl = FINE ? (float)(c - (double)ch) : 0.0f;
     const float2 t1 = cadd(v1, v2);
     const float2 t2 = csub(v1, v2);
     const float2 base = make_float2(v0.x - 0.5f * t1.x, v0.y - 0.5f * t1.y);
-    const float2 rot = cis(make_float2(c * t2.x, c * t2.y), sign);
+    const float2 rot = cis(FINE ? make_float2(fmaf(ch, t2.x, cl * t2.x), fmaf(ch, t2.y, cl * t2.y)) : make_float2(ch * t2.x, ch * t2.y), sign);
     v0 = cadd(v0, t1);
     v1 = cadd(base, rot);
     v2 = csub(base, rot);
 }
 
-// w_N^k = (cos 2 pi k / N, sign sin 2 pi k / N) for the in-register twiddles
-__device__ __forceinline__ float2 wk(float c, float s, float sign) { return make_float2(c, sign * s); }
-
-template <int R>
-__device__ __forceinline__ void dft(float2 (&v)[R], float sign);
-
-template <>
-__device__ __forceinline__ void dft<2>(float2 (&v)[2], float) { dft2(v[0], v[1]); }
-
-template <>
-__device__ __forceinline__ void dft<3>(float2 (&v)[3], float sign) { dft3(v[0], v[1], v[2], sign); }
-
-template <>
-__device__ __forceinline__ void dft<4>(float2 (&v)[4], float sign) { dft4(v[0], v[1], v[2], v[3], sign); }
-
 // 8 = 2 x 4: q = q1 + 2 q2; inner DFT4 over q2, twiddle w8^(q1 p1), outer DFT2.
-template <>
-__device__ __forceinline__ void dft<8>(float2 (&v)[8], float sign)
+template <bool FINE>
+__device__ __forceinline__ void dft8(float2 (&v)[8], float sign)
 {
-    const float h = 0.70710678118654752440f;
+    constexpr double h = 0.70710678118654752440;
     dft4(v[0], v[2], v[4], v[6], sign);   // q1 = 0 -> A0[p1] at v[0], v[2], v[4], v[6]
     dft4(v[1], v[3], v[5], v[7], sign);   // q1 = 1 -> A1[p1]
-    v[3] = cmul(v[3], wk(h, h, sign));
+    v[3] = cmul_const<FINE>(v[3], h, h, sign);
     v[5] = cis(v[5], sign);
-    v[7] = cmul(v[7], wk(-h, h, sign));
+    v[7] = cmul_const<FINE>(v[7], -h, h, sign);
     float2 x[8];
     #pragma unroll
     for (int p1 = 0; p1 < 4; ++p1)
@@ -105,22 +107,22 @@ __device__ __forceinline__ void dft<8>(float2 (&v)[8], float sign)
 }
 
 // 16 = 4 x 4: q = q1 + 4 q2; inner DFT4 over q2, twiddle w16^(q1 p1), outer DFT4 over q1.
-template <>
-__device__ __forceinline__ void dft<16>(float2 (&v)[16], float sign)
+template <bool FINE>
+__device__ __forceinline__ void dft16(float2 (&v)[16], float sign)
 {
-    const float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, h = 0.70710678118654752440f;
+    constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173, h = 0.70710678118654752440;
     #pragma unroll
     for (int q1 = 0; q1 < 4; ++q1) dft4(v[q1], v[q1 + 4], v[q1 + 8], v[q1 + 12], sign);
     // v[q1 + 4 p1] = A[q1][p1]; multiply by w16^(q1 p1)
-    v[5] = cmul(v[5], wk(c1, s1, sign));     // q1 1, p1 1: k 1
-    v[9] = cmul(v[9], wk(h, h, sign));       // 1,2: k 2
-    v[13] = cmul(v[13], wk(s1, c1, sign));   // 1,3: k 3
-    v[6] = cmul(v[6], wk(h, h, sign));       // 2,1: k 2
+    v[5] = cmul_const<FINE>(v[5], c1, s1, sign);     // q1 1, p1 1: k 1
+    v[9] = cmul_const<FINE>(v[9], h, h, sign);       // 1,2: k 2
+    v[13] = cmul_const<FINE>(v[13], s1, c1, sign);   // 1,3: k 3
+    v[6] = cmul_const<FINE>(v[6], h, h, sign);       // 2,1: k 2
     v[10] = cis(v[10], sign);                // 2,2: k 4
-    v[14] = cmul(v[14], wk(-h, h, sign));    // 2,3: k 6
-    v[7] = cmul(v[7], wk(s1, c1, sign));     // 3,1: k 3
-    v[11] = cmul(v[11], wk(-h, h, sign));    // 3,2: k 6
-    v[15] = cmul(v[15], wk(-c1, -s1, sign)); // 3,3: k 9
+    v[14] = cmul_const<FINE>(v[14], -h, h, sign);    // 2,3: k 6
+    v[7] = cmul_const<FINE>(v[7], s1, c1, sign);     // 3,1: k 3
+    v[11] = cmul_const<FINE>(v[11], -h, h, sign);    // 3,2: k 6
+    v[15] = cmul_const<FINE>(v[15], -c1, -s1, sign); // 3,3: k 9
     #pragma unroll
     for (int p1 = 0; p1 < 4; ++p1) dft4(v[4 * p1], v[4 * p1 + 1], v[4 * p1 + 2], v[4 * p1 + 3], sign);
     // now v[4 p1 + p2] = X[p1 + 4 p2]: transpose the 4 x 4 index
@@ -134,20 +136,20 @@ __device__ __forceinline__ void dft<16>(float2 (&v)[16], float sign)
 }
 
 // 9 = 3 x 3: q = q1 + 3 q2; inner DFT3 over q2, twiddle w9^(q1 p1), outer DFT3 over q1.
-template <>
-__device__ __forceinline__ void dft<9>(float2 (&v)[9], float sign)
+template <bool FINE>
+__device__ __forceinline__ void dft9(float2 (&v)[9], float sign)
 {
-    const float c1 = 0.76604444311897803520f, s1 = 0.64278760968653932632f;   // 2 pi / 9
-    const float c2 = 0.17364817766693034885f, s2 = 0.98480775301220805936f;   // 4 pi / 9
-    const float c4 = -0.93969262078590838405f, s4 = 0.34202014332566873304f; // 8 pi / 9
+    constexpr double c1 = 0.76604444311897803520, s1 = 0.64278760968653932632;   // 2 pi / 9
+    constexpr double c2 = 0.17364817766693034885, s2 = 0.98480775301220805936;   // 4 pi / 9
+    constexpr double c4 = -0.93969262078590838405, s4 = 0.34202014332566873304; // 8 pi / 9
     #pragma unroll
-    for (int q1 = 0; q1 < 3; ++q1) dft3(v[q1], v[q1 + 3], v[q1 + 6], sign);
-    v[4] = cmul(v[4], wk(c1, s1, sign));   // q1 1, p1 1: k 1
-    v[7] = cmul(v[7], wk(c2, s2, sign));   // 1,2: k 2
-    v[5] = cmul(v[5], wk(c2, s2, sign));   // 2,1: k 2
-    v[8] = cmul(v[8], wk(c4, s4, sign));   // 2,2: k 4
+    for (int q1 = 0; q1 < 3; ++q1) dft3<FINE>(v[q1], v[q1 + 3], v[q1 + 6], sign);
+    v[4] = cmul_const<FINE>(v[4], c1, s1, sign);   // q1 1, p1 1: k 1
+    v[7] = cmul_const<FINE>(v[7], c2, s2, sign);   // 1,2: k 2
+    v[5] = cmul_const<FINE>(v[5], c2, s2, sign);   // 2,1: k 2
+    v[8] = cmul_const<FINE>(v[8], c4, s4, sign);   // 2,2: k 4
     #pragma unroll
-    for (int p1 = 0; p1 < 3; ++p1) dft3(v[3 * p1], v[3 * p1 + 1], v[3 * p1 + 2], sign);
+    for (int p1 = 0; p1 < 3; ++p1) dft3<FINE>(v[3 * p1], v[3 * p1 + 1], v[3 * p1 + 2], sign);
     float2 x[9];
     #pragma unroll
     for (int p1 = 0; p1 < 3; ++p1)
@@ -155,6 +157,17 @@ __device__ __forceinline__ void dft<9>(float2 (&v)[9], float sign)
         for (int p2 = 0; p2 < 3; ++p2) x[p1 + 3 * p2] = v[3 * p1 + p2];
     #pragma unroll
     for (int i = 0; i < 9; ++i) v[i] = x[i];
+}
+
+template <int R, bool FINE>
+__device__ __forceinline__ void dft(float2 (&v)[R], float sign)
+{
+    if constexpr (R == 2) dft2(v[0], v[1]);
+    else if constexpr (R == 3) dft3<FINE>(v[0], v[1], v[2], sign);
+    else if constexpr (R == 4) dft4(v[0], v[1], v[2], v[3], sign);
+    else if constexpr (R == 8) dft8<FINE>(v, sign);
+    else if constexpr (R == 9) dft9<FINE>(v, sign);
+    else dft16<FINE>(v, sign);
 }
 
 // ---- stages between registers and shared memory ---------------------------------
@@ -207,32 +220,25 @@ __device__ __forceinline__ void fft_item(int it, int m, uint32_t mmag, int& s, i
     }
 }
 
-// v[q] *= w^q, w = exp(-+2 pi i k / (Ls R)): the powers 1, 2, 4, 8 from the
-// table, the others as products of two or three of them (15 table reads per
-// radix-16 butterfly cost more than the extra multiplications; the transform's
-// error does not change).
+// v[q] *= w^q, w = exp(-+2 pi i k / (Ls R)), every power from the table (a
+// product of two entries carries twice the error of one), two of them in each
+// 16-byte read.
 template <int R>
 __device__ __forceinline__ void fft_twiddle(float2 (&v)[R], int k, int Ls, const float2* __restrict__ tw, bool inv)
 {
-    float2 w[R];
+    const float4* t = reinterpret_cast<const float4*>(tw) + k;
     #pragma unroll
-    for (int q = 1; q < R; q <<= 1)
+    for (int p = 0; p < R / 2; ++p)
     {
-        w[q] = __ldg(tw + (q - 1) * Ls + k);
-        if (inv) w[q].y = -w[q].y;
-        v[q] = cmul(v[q], w[q]);
-        #pragma unroll
-        for (int r = 1; r < q; ++r)
-            if (q + r < R)
-            {
-                w[q + r] = cmul(w[q], w[r]);
-                v[q + r] = cmul(v[q + r], w[q + r]);
-            }
+        const float4 w = __ldg(t + p * Ls);
+        const int q = 2 * p + 1;
+        v[q] = cmul(v[q], make_float2(w.x, inv ? -w.y : w.y));
+        if (q + 1 < R) v[q + 1] = cmul(v[q + 1], make_float2(w.z, inv ? -w.w : w.w));
     }
 }
 
 // The butterfly of item `it`: inputs from ld (FIRST) or shared memory, twiddled, transformed.
-template <int R, int NB, bool INTER, bool INV, bool FIRST, class LD>
+template <int R, int NB, bool INTER, bool INV, bool FIRST, bool FINE, class LD>
 __device__ __forceinline__ void fft_take(float2 (&v)[R], const float2* x, int it, const FftStage& d, const LD& ld)
 {
     const int n = d.n, m = n / R;
@@ -241,7 +247,7 @@ __device__ __forceinline__ void fft_take(float2 (&v)[R], const float2* x, int it
     #pragma unroll
     for (int q = 0; q < R; ++q) v[q] = FIRST ? ld(s, j + q * m) : x[fft_slot<NB, INTER>(j + q * m, s, n)];
     if (d.Ls > 1) fft_twiddle<R>(v, j - (int)__umulhi((uint32_t)j, d.lmag) * d.Ls, d.Ls, d.tw, INV);
-    dft<R>(v, INV ? 1.0f : -1.0f);
+    dft<R, FINE>(v, INV ? 1.0f : -1.0f);
 }
 
 // Its outputs, to st (LAST) or shared memory.
@@ -265,7 +271,7 @@ __device__ __forceinline__ void fft_put(const float2 (&v)[R], float2* y, int it,
 // LAST: outputs to st(s, i, value).  Ends on a barrier unless LAST.  In place,
 // the elements start as zeros: set under a condition only, they count as live
 // from the kernel's start and every radix's stage adds to the spills.
-template <int R, int NB, bool INTER, bool INV, bool PP, bool FIRST, bool LAST, class LD, class ST>
+template <int R, int NB, bool INTER, bool INV, bool PP, bool FIRST, bool LAST, bool FINE, class LD, class ST>
 __device__ __forceinline__ void fft_stage(const float2* x, float2* y, const FftStage& d, const LD& ld, const ST& st)
 {
     const int items = d.n / R * NB;
@@ -274,7 +280,7 @@ __device__ __forceinline__ void fft_stage(const float2* x, float2* y, const FftS
         for (int it = threadIdx.x; it < items; it += blockDim.x)
         {
             float2 v[R];
-            fft_take<R, NB, INTER, INV, FIRST>(v, x, it, d, ld);
+            fft_take<R, NB, INTER, INV, FIRST, FINE>(v, x, it, d, ld);
             fft_put<R, NB, INTER, LAST>(v, y, it, d, st);
         }
     }
@@ -286,7 +292,7 @@ __device__ __forceinline__ void fft_stage(const float2* x, float2* y, const FftS
         for (int u = 0; u < I; ++u)
         {
             const int it = threadIdx.x + u * blockDim.x;
-            if (it < items) fft_take<R, NB, INTER, INV, FIRST>(v[u], x, it, d, ld);
+            if (it < items) fft_take<R, NB, INTER, INV, FIRST, FINE>(v[u], x, it, d, ld);
         }
         if (!FIRST) __syncthreads();
         #pragma unroll
@@ -300,19 +306,19 @@ __device__ __forceinline__ void fft_stage(const float2* x, float2* y, const FftS
 }
 
 // The stage of whatever radix; leaves the result's buffer in x (in place: y == x).
-template <int NB, bool INTER, bool INV, bool PP, bool FIRST, bool LAST, class LD, class ST>
+template <int NB, bool INTER, bool INV, bool PP, bool FIRST, bool LAST, bool FINE, class LD, class ST>
 __device__ __forceinline__ void fft_any(float2*& x, float2*& y, const FftDims& d, int stage,
                                         const float2* __restrict__ tws, const LD& ld, const ST& st)
 {
     const FftStage f = fft_stage_of(d, stage, tws);
     switch (d.rad[stage])
     {
-    case 16: fft_stage<16, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
-    case 9: fft_stage<9, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
-    case 8: fft_stage<8, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
-    case 4: fft_stage<4, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
-    case 3: fft_stage<3, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
-    default: fft_stage<2, NB, INTER, INV, PP, FIRST, LAST>(x, y, f, ld, st); break;
+    case 16: fft_stage<16, NB, INTER, INV, PP, FIRST, LAST, FINE>(x, y, f, ld, st); break;
+    case 9: fft_stage<9, NB, INTER, INV, PP, FIRST, LAST, FINE>(x, y, f, ld, st); break;
+    case 8: fft_stage<8, NB, INTER, INV, PP, FIRST, LAST, FINE>(x, y, f, ld, st); break;
+    case 4: fft_stage<4, NB, INTER, INV, PP, FIRST, LAST, FINE>(x, y, f, ld, st); break;
+    case 3: fft_stage<3, NB, INTER, INV, PP, FIRST, LAST, FINE>(x, y, f, ld, st); break;
+    default: fft_stage<2, NB, INTER, INV, PP, FIRST, LAST, FINE>(x, y, f, ld, st); break;
     }
     float2* t = x;
     x = y;
@@ -336,7 +342,7 @@ inline void set_spans(FftDims& d)
         d.lmag[s] = Ls > 1 ? (uint32_t)((((uint64_t)1 << 32) + Ls - 1) / Ls) : 0u;
         d.mmag[s] = m > 1 ? (uint32_t)((((uint64_t)1 << 32) + m - 1) / m) : 0u;
         d.twoff[s] = off;
-        if (Ls > 1) off += (d.rad[s] - 1) * Ls;
+        if (Ls > 1) off += d.rad[s] / 2 * 2 * Ls;
         Ls *= d.rad[s];
     }
     d.twoff[d.nrad] = off;
@@ -365,8 +371,9 @@ inline FftDims reversed(FftDims d)
     return d;
 }
 
-// Per-stage twiddles exp(-2 pi i q k / (Ls r)), entry (q - 1) Ls + k of the
-// stage's table at twoff, in double then rounded (at least one entry).
+// Per-stage twiddles exp(-2 pi i q k / (Ls r)), entry ((q - 1) / 2 Ls + k) 2 +
+// (q - 1) % 2 of the stage's table at twoff, in double then rounded (at least
+// one entry; an even radix leaves the last power's neighbour unused).
 inline std::vector<float2> stage_twiddles(const FftDims& d)
 {
     std::vector<float2> t((size_t)std::max(1, d.twoff[d.nrad]));
@@ -378,7 +385,7 @@ inline std::vector<float2> stage_twiddles(const FftDims& d)
             for (int k = 0; k < d.ls[s]; ++k)
             {
                 const double a = 2.0 * pi * (double)(q * k) / (double)(d.ls[s] * d.rad[s]);
-                t[(size_t)d.twoff[s] + (size_t)(q - 1) * d.ls[s] + k] = make_float2((float)std::cos(a), (float)-std::sin(a));
+                t[(size_t)d.twoff[s] + ((size_t)((q - 1) / 2) * d.ls[s] + k) * 2 + (q - 1) % 2] = make_float2((float)std::cos(a), (float)-std::sin(a));
             }
     }
     return t;

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(1024) grid_cols(const float* __restrict__ in, 
     any = __syncthreads_or(any);
     if (threadIdx.x == 0) lit[blockIdx.x] = any ? 1 : 0;
     if (!any) return;
-    for (int st = 0; st < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    for (int st = 0; st < d.nrad; ++st) fft_any<2, true, false, PP, false, false, true>(x, y, d, st, tw, FftNone{}, FftNone{});
     // Z = FFT(a + i b): FFT(a)[k] = (Z[k] + conj Z[N - k]) / 2, FFT(b)[k] = (Z[k] - conj Z[N - k]) / 2i;
     // per pair of rows: 2 x 2 columns x 2 rows, one 64-byte piece
     for (int t = threadIdx.x; t < pairs * 2; t += blockDim.x)
@@ -120,10 +120,21 @@ struct HalfRows {
     }
 };
 
+// A sum in two floats: a thread's dozens of terms lie many powers of two apart.
+struct Sum2 {
+    float hi, lo;
+    __device__ __forceinline__ void add(float v)
+    {
+        const float t = hi + v, b = t - hi;
+        lo += (hi - (t - b)) + (v - b);
+        hi = t;
+    }
+};
+
 // |X|^2 at its fftshifted place and at the mirrored one.
 struct PsfStore {
     float* psf;
-    float* sum;                    // this thread's energy
+    Sum2* sum;                     // this thread's energy
     int N, pair;
     __device__ __forceinline__ void operator()(int s, int kx, float2 z) const
     {
@@ -131,10 +142,13 @@ struct PsfStore {
         if (ky > h) return;
         const float p = z.x * z.x + z.y * z.y;
         psf[(size_t)((ky + h) & m) * N + ((kx + h) & m)] = p;
-        *sum += p;
-        if (ky == 0 || ky == h) return;                  // these rows hold their own mirror
+        if (ky == 0 || ky == h)
+        {
+            sum->add(p);                                 // these rows hold their own mirror
+            return;
+        }
         psf[(size_t)((h - ky) & m) * N + ((h - kx) & m)] = p;
-        *sum += p;
+        sum->add(2.0f * p);
     }
 };
 
@@ -148,12 +162,12 @@ struct PsfStore {
 struct LagStore {
     float* C;
     int N, pair, mc, ldc;
-    float scale;
+    float scale, scale_lo;         // the scale in two floats: one rounding would be in every lag
     __device__ __forceinline__ void operator()(int s, int kx, float2 z) const
     {
         const int ly = 2 * pair + s, lx = kx <= N / 2 ? kx : kx - N;
         if (ly > mc || lx < -mc || lx > mc) return;
-        const float v = ((lx + ly) & 1) ? -z.x * scale : z.x * scale;
+        const float x = ((lx + ly) & 1) ? -z.x : z.x, v = fmaf(x, scale, x * scale_lo);
         C[(size_t)(mc + ly) * ldc + (mc + lx)] = v;
         if (ly > 0) C[(size_t)(mc - ly) * ldc + (mc - lx)] = v;
     }
@@ -167,7 +181,7 @@ __global__ void __launch_bounds__(1024) grid_rows(const float2* __restrict__ hal
                                                   float* __restrict__ out, double* __restrict__ energy, int mc, int ldc)
 {
     extern __shared__ float2 sm[];
-    __shared__ float red[32];
+    __shared__ double red[32];
     float2* x = sm;
     float2* y = PP ? sm + padded((size_t)N * 2) : sm;
     unsigned char* flags = reinterpret_cast<unsigned char*>(sm + (PP ? 2 : 1) * padded((size_t)N * 2));
@@ -175,24 +189,26 @@ __global__ void __launch_bounds__(1024) grid_rows(const float2* __restrict__ hal
     for (int i = threadIdx.x; i < N / 4; i += blockDim.x) flags[i] = lit[i];
     __syncthreads();
     const HalfRows load{half + half_index(N, pair, 0), flags};
-    fft_any<2, true, false, PP, true, false>(x, y, d, 0, tw, load, FftNone{});
-    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false>(x, y, d, st, tw, FftNone{}, FftNone{});
+    fft_any<2, true, false, PP, true, false, true>(x, y, d, 0, tw, load, FftNone{});
+    for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false, true>(x, y, d, st, tw, FftNone{}, FftNone{});
     if (LAGS)
     {
         const double e = *energy;
-        const float scale = e > 0.0 ? (float)(1.0 / (e * (double)N * (double)N)) : 0.0f;
-        fft_any<2, true, false, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, LagStore{out, N, pair, mc, ldc, scale});
+        const double k = e > 0.0 ? 1.0 / (e * (double)N * (double)N) : 0.0;
+        const float scale = (float)k, scale_lo = (float)(k - (double)scale);
+        fft_any<2, true, false, PP, false, true, true>(x, y, d, d.nrad - 1, tw, FftNone{}, LagStore{out, N, pair, mc, ldc, scale, scale_lo});
         return;
     }
-    float part = 0.0f;
-    fft_any<2, true, false, PP, false, true>(x, y, d, d.nrad - 1, tw, FftNone{}, PsfStore{out, &part, N, pair});
+    Sum2 own{0.0f, 0.0f};
+    fft_any<2, true, false, PP, false, true, true>(x, y, d, d.nrad - 1, tw, FftNone{}, PsfStore{out, &own, N, pair});
+    double part = isfinite(own.hi) ? (double)own.hi + (double)own.lo : (double)own.hi;
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
     __syncthreads();
     if (threadIdx.x == 0)
     {
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += (double)red[w];
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
         atomicAdd(energy, t);
     }
 }
