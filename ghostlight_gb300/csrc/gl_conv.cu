@@ -245,8 +245,8 @@ __device__ __forceinline__ void conv_middle_any(float2*& x, float2*& y, const Ff
 
 // Pass 2: column pair blockIdx.x of plane blockIdx.y: forward FFT over P rows
 // (rows >= rows_in are zero), times the kernel spectrum, inverse FFT; rows
-// [0, rows_in) back in place.  SETUP (kernel spectrum): forward only, all P rows.
-template <bool SETUP, bool PP>
+// [0, rows_in) back in place.
+template <bool PP>
 __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_cols(float2* __restrict__ buf, const float2* __restrict__ khat,
                                                             int rows_in, int rows, int k_rows, int G, const __grid_constant__ FftDims d,
                                                             const __grid_constant__ FftDims di,
@@ -259,18 +259,6 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_cols
     float2* base = buf + pair_index(blockIdx.y, G, rows, g, 0);
     const ColLoad load{base, rows_in};
     const ColStore store{base, rows_in};
-    if (SETUP)
-    {
-        if (d.nrad < 2)
-        {
-            if (d.nrad == 1) fft_any<2, true, false, PP, true, true, PP>(x, y, d, 0, tw, load, store);
-            return;                                    // one point: its own transform
-        }
-        fft_any<2, true, false, PP, true, false, PP>(x, y, d, 0, tw, load, FftNone{});
-        for (int st = 1; st + 1 < d.nrad; ++st) fft_any<2, true, false, PP, false, false, PP>(x, y, d, st, tw, FftNone{}, FftNone{});
-        fft_any<2, true, false, PP, false, true, PP>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
-        return;
-    }
     const ColMul mul{khat + pair_index(0, G, k_rows, g, 0)};
     if (d.nrad < 2)
     {
@@ -330,6 +318,101 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_rows
     fft_any<kPairs, false, true, PP, false, true, PP>(x, y, d, d.nrad - 1, tw, FftNone{}, store);
 }
 
+// ---- kernel spectrum, once per plan ----------------------------------------------
+// In FP64 and rounded once: a third of the rounding of forward transform, product
+// and inverse was the kernel's own float transform, the same in every call (noise, 2048^2
+// (*) 257^2: 3.7e-7 off 64 bits with it, 2.8e-7 without).  Stockham stages
+// of radix 4, 3, 2 between two arrays in global memory, one thread a butterfly.
+
+// Rows of the kernel, its centre at column 0, wrapped.
+__global__ void spec_place(const float* __restrict__ k, int kw, int kh, int Q, double norm, double2* __restrict__ a)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (size_t)kh * Q) return;
+    const int u = (int)(t / Q), c = (int)(t - (size_t)u * Q), v = (c + kw / 2) % Q;
+    a[t] = make_double2(v < kw ? (double)k[(size_t)u * kw + v] * norm : 0.0, 0.0);
+}
+
+// The rows' spectra to P rows, the centre row at row 0, wrapped; columns past Q / 2 zero.
+__global__ void spec_turn(const double2* __restrict__ a, int kh, int Q, int P, int cols, double2* __restrict__ b)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (size_t)P * cols) return;
+    const int y = (int)(t / cols), q = (int)(t - (size_t)y * cols), u = (y + kh / 2) % P;
+    b[t] = (u < kh && q <= Q / 2) ? a[(size_t)u * Q + q] : make_double2(0.0, 0.0);
+}
+
+// To the column pairs of the intermediate (pair_index).
+__global__ void spec_store(const double2* __restrict__ b, int P, int cols, int k_rows, float2* __restrict__ khat)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (size_t)P * cols) return;
+    const int y = (int)(t / cols), q = (int)(t - (size_t)y * cols);
+    const double2 v = b[t];
+    khat[((size_t)(q >> 1) * k_rows + y) * 2 + (q & 1)] = make_float2((float)v.x, (float)v.y);
+}
+
+// One stage over nseq sequences; element i of sequence s at i es + s ss (one of
+// the strides is 1).  tw: exp(-2 pi i t / n), t < n.
+template <int R>
+__global__ void spec_stage(const double2* __restrict__ x, double2* __restrict__ y, int n, int Ls, int nseq, size_t es, size_t ss,
+                           const double2* __restrict__ tw)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int m = n / R;
+    if (t >= (size_t)m * nseq) return;
+    const int s = es == 1 ? (int)(t / m) : (int)(t % nseq), j = es == 1 ? (int)(t % m) : (int)(t / nseq);
+    const int g = j / Ls, k = j - g * Ls;
+    double2 v[R];
+    #pragma unroll
+    for (int q = 0; q < R; ++q)
+    {
+        const double2 a = x[(j + (size_t)q * m) * es + s * ss], w = tw[q * k * (m / Ls)];
+        v[q] = make_double2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+    }
+    #pragma unroll
+    for (int p = 0; p < R; ++p)
+    {
+        double2 o = v[0];
+        #pragma unroll
+        for (int q = 1; q < R; ++q)
+        {
+            const double2 w = tw[p * q % R * m];
+            o.x += v[q].x * w.x - v[q].y * w.y;
+            o.y += v[q].x * w.y + v[q].y * w.x;
+        }
+        y[((size_t)g * Ls * R + k + (size_t)p * Ls) * es + s * ss] = o;
+    }
+}
+
+inline unsigned spec_blocks(size_t threads) { return (unsigned)((threads + 255) / 256); }
+
+// All stages of one axis; leaves the result's array in x.
+void spec_axis(double2*& x, double2*& y, int n, int nseq, size_t es, size_t ss, const double2* tw, cudaStream_t st)
+{
+    int Ls = 1;
+    while (Ls < n)
+    {
+        const int left = n / Ls, R = left % 4 == 0 ? 4 : (left % 2 == 0 ? 2 : 3);
+        const unsigned blocks = spec_blocks((size_t)(n / R) * nseq);
+        if (R == 4) spec_stage<4><<<blocks, 256, 0, st>>>(x, y, n, Ls, nseq, es, ss, tw);
+        else if (R == 3) spec_stage<3><<<blocks, 256, 0, st>>>(x, y, n, Ls, nseq, es, ss, tw);
+        else spec_stage<2><<<blocks, 256, 0, st>>>(x, y, n, Ls, nseq, es, ss, tw);
+        std::swap(x, y);
+        Ls *= R;
+    }
+}
+
+// exp(-2 pi i t / n), t < n
+__global__ void spec_circle(int n, double2* __restrict__ tw)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    double s, c;
+    sincospi(2.0 * (double)t / (double)n, &s, &c);
+    tw[t] = make_double2(c, -s);
+}
+
 int good_size(int need)
 {
     int best = 1 << 30;
@@ -374,22 +457,36 @@ static void conv_free(ConvPlan* p)
     delete p;
 }
 
-// Passes 1 and 2 over `planes` planes of `rows` intermediate rows.
-static void conv_fwd(const ConvPlan* p, const ConvPlanes& A, int planes, int W, int H, int rows, float2* buf, cudaStream_t st)
+// The kernel's spectrum (centre at the origin, so the circular convolution lands
+// 'same'-aligned; 1 / (P Q) folded in) into p->khat.
+static cudaError_t conv_spectrum(const ConvPlan* p, const float* h_kernel, cudaStream_t st)
 {
-    const dim3 rb((unsigned)((rows + 2 * kPairs - 1) / (2 * kPairs)), planes);
-    if (p->pp_row) conv_rows_fwd<true><<<rb, p->thr_row, p->smem_row, st>>>(A, W, H, rows, p->G, buf, p->dq, p->tw_q);
-    else conv_rows_fwd<false><<<rb, p->thr_row, p->smem_row, st>>>(A, W, H, rows, p->G, buf, p->dq, p->tw_q);
-}
-
-template <bool SETUP>
-static void conv_mid(const ConvPlan* p, int planes, float2* buf, const float2* khat, int rows_in, int rows, cudaStream_t st)
-{
-    const dim3 cb(p->G, planes);
-    if (p->pp_col)
-        conv_cols<SETUP, true><<<cb, p->thr_col, p->smem_col, st>>>(buf, khat, rows_in, rows, p->k_rows, p->G, p->dp, p->dpi, p->tw_p, p->tw_pi);
-    else
-        conv_cols<SETUP, false><<<cb, p->thr_col, p->smem_col, st>>>(buf, khat, rows_in, rows, p->k_rows, p->G, p->dp, p->dpi, p->tw_p, p->tw_pi);
+    const size_t nk = (size_t)p->KH * p->KW, cols = 2 * (size_t)p->G;
+    const size_t cells = std::max((size_t)p->KH * p->Q, (size_t)p->P * cols);
+    const size_t k_at = sizeof(double2) * (2 * cells + (size_t)p->Q + p->P);
+    char* block = nullptr;         // two arrays, the circles of both axes, the kernel
+    cudaError_t e = cudaMalloc(&block, k_at + sizeof(float) * nk);
+    auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    double2 *x = reinterpret_cast<double2*>(block), *y = x + cells, *twq = y + cells, *twp = twq + p->Q;
+    float* k = reinterpret_cast<float*>(block + k_at);
+    if (e == cudaSuccess) chk(cudaMemcpyAsync(k, h_kernel, sizeof(float) * nk, cudaMemcpyHostToDevice, st));
+    if (e == cudaSuccess)
+    {
+        double2 *a = x, *b = y;
+        const double norm = 1.0 / ((double)p->P * (double)p->Q);
+        spec_circle<<<spec_blocks((size_t)p->Q), 256, 0, st>>>(p->Q, twq);
+        spec_circle<<<spec_blocks((size_t)p->P), 256, 0, st>>>(p->P, twp);
+        spec_place<<<spec_blocks((size_t)p->KH * p->Q), 256, 0, st>>>(k, p->KW, p->KH, p->Q, norm, a);
+        spec_axis(a, b, p->Q, p->KH, 1, (size_t)p->Q, twq, st);
+        spec_turn<<<spec_blocks((size_t)p->P * cols), 256, 0, st>>>(a, p->KH, p->Q, p->P, (int)cols, b);
+        std::swap(a, b);
+        spec_axis(a, b, p->P, (int)cols, cols, 1, twp, st);
+        spec_store<<<spec_blocks((size_t)p->P * cols), 256, 0, st>>>(a, p->P, (int)cols, p->k_rows, p->khat);
+        chk(cudaGetLastError());
+    }
+    chk(cudaStreamSynchronize(st));
+    cudaFree(block);
+    return e;
 }
 
 extern "C" int gl_conv2d_plan_create(int width, int height, const float* h_kernel, int kw, int kh, void* stream,
@@ -420,19 +517,7 @@ extern "C" int gl_conv2d_plan_create(int width, int height, const float* h_kerne
     p->thr_row = fft_threads(p->Q, kPairs, p->pp_row);
     p->thr_col = fft_threads(p->P, kColsPerCta, p->pp_col);
     cudaStream_t st = (cudaStream_t)stream;
-    // Kernel placed with its centre at the origin, wrapped (so the circular
-    // convolution lands 'same'-aligned), as a P x Q real plane, 1/(PQ) folded in.
-    std::vector<float> kplane((size_t)p->P * p->Q, 0.0f);
-    const int cy = kh / 2, cx = kw / 2;
-    const float norm = 1.0f / ((float)p->P * (float)p->Q);
-    for (int u = 0; u < kh; ++u)
-        for (int v = 0; v < kw; ++v)
-        {
-            const int yy = ((u - cy) % p->P + p->P) % p->P, xx = ((v - cx) % p->Q + p->Q) % p->Q;
-            kplane[(size_t)yy * p->Q + xx] = h_kernel[(size_t)u * kw + v] * norm;
-        }
     const std::vector<float2> twq = stage_twiddles(p->dq), twp = stage_twiddles(p->dp), twi = stage_twiddles(p->dpi);
-    float* kdev = nullptr;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
     chk(cudaMalloc(&p->khat, sizeof(float2) * 2 * (size_t)p->G * p->k_rows));
@@ -440,9 +525,7 @@ extern "C" int gl_conv2d_plan_create(int width, int height, const float* h_kerne
     chk(cudaMalloc(&p->tw_q, sizeof(float2) * twq.size()));
     chk(cudaMalloc(&p->tw_p, sizeof(float2) * twp.size()));
     chk(cudaMalloc(&p->tw_pi, sizeof(float2) * twi.size()));
-    chk(cudaMalloc(&kdev, sizeof(float) * kplane.size()));
-    chk((cudaError_t)raise_smem_limit(p->pp_col ? (const void*)conv_cols<false, true> : (const void*)conv_cols<false, false>, p->smem_col));
-    chk((cudaError_t)raise_smem_limit(p->pp_col ? (const void*)conv_cols<true, true> : (const void*)conv_cols<true, false>, p->smem_col));
+    chk((cudaError_t)raise_smem_limit(p->pp_col ? (const void*)conv_cols<true> : (const void*)conv_cols<false>, p->smem_col));
     chk((cudaError_t)raise_smem_limit(p->pp_row ? (const void*)conv_rows_fwd<true> : (const void*)conv_rows_fwd<false>, p->smem_row));
     chk((cudaError_t)raise_smem_limit(p->pp_row ? (const void*)conv_rows_inv<true> : (const void*)conv_rows_inv<false>, p->smem_row));
     if (e == cudaSuccess)
@@ -450,19 +533,9 @@ extern "C" int gl_conv2d_plan_create(int width, int height, const float* h_kerne
         chk(cudaMemcpyAsync(p->tw_q, twq.data(), sizeof(float2) * twq.size(), cudaMemcpyHostToDevice, st));
         chk(cudaMemcpyAsync(p->tw_p, twp.data(), sizeof(float2) * twp.size(), cudaMemcpyHostToDevice, st));
         chk(cudaMemcpyAsync(p->tw_pi, twi.data(), sizeof(float2) * twi.size(), cudaMemcpyHostToDevice, st));
-        chk(cudaMemcpyAsync(kdev, kplane.data(), sizeof(float) * kplane.size(), cudaMemcpyHostToDevice, st));
-        if (e == cudaSuccess)
-        {
-            // kernel spectrum: row FFTs of the real plane, then forward column FFTs in place
-            ConvPlanes K{};
-            K.in[0] = kdev;
-            conv_fwd(p, K, 1, p->Q, p->P, p->k_rows, p->khat, st);
-            conv_mid<true>(p, 1, p->khat, nullptr, p->P, p->k_rows, st);
-            chk(cudaGetLastError());
-        }
-        chk(cudaStreamSynchronize(st));
     }
-    cudaFree(kdev);
+    // (waits for the tables' copies too)
+    if (e == cudaSuccess) chk(conv_spectrum(p, h_kernel, st));
     if (e != cudaSuccess)
     {
         conv_free(p);
@@ -484,9 +557,14 @@ extern "C" int gl_conv2d_plan_execute2(gl_conv_plan* plan, const float* d_in_r, 
     ConvPlan* p = plan->p;
     cudaStream_t st = (cudaStream_t)stream;
     const ConvPlanes A{{d_in_r, d_in_g, d_in_b}, {d_add_r, d_add_g, d_add_b}, {d_out_r, d_out_g, d_out_b}};
-    conv_fwd(p, A, 3, p->W, p->H, p->rows, p->buf, st);
-    conv_mid<false>(p, 3, p->buf, p->khat, p->H, p->rows, st);
     const dim3 rb((unsigned)((p->rows + 2 * kPairs - 1) / (2 * kPairs)), 3);
+    const dim3 cb(p->G, 3);
+    if (p->pp_row) conv_rows_fwd<true><<<rb, p->thr_row, p->smem_row, st>>>(A, p->W, p->H, p->rows, p->G, p->buf, p->dq, p->tw_q);
+    else conv_rows_fwd<false><<<rb, p->thr_row, p->smem_row, st>>>(A, p->W, p->H, p->rows, p->G, p->buf, p->dq, p->tw_q);
+    if (p->pp_col)
+        conv_cols<true><<<cb, p->thr_col, p->smem_col, st>>>(p->buf, p->khat, p->H, p->rows, p->k_rows, p->G, p->dp, p->dpi, p->tw_p, p->tw_pi);
+    else
+        conv_cols<false><<<cb, p->thr_col, p->smem_col, st>>>(p->buf, p->khat, p->H, p->rows, p->k_rows, p->G, p->dp, p->dpi, p->tw_p, p->tw_pi);
     if (p->pp_row) conv_rows_inv<true><<<rb, p->thr_row, p->smem_row, st>>>(p->buf, A, p->W, p->H, p->rows, p->G, p->dq, p->tw_q);
     else conv_rows_inv<false><<<rb, p->thr_row, p->smem_row, st>>>(p->buf, A, p->W, p->H, p->rows, p->G, p->dq, p->tw_q);
     GL_CUDA_TRY(cudaGetLastError());

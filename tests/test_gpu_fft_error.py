@@ -36,3 +36,22 @@ def test_sprite_transform(N, bound):
     assert float(lags[mc, mc]) * N * N == pytest.approx(1.0, abs=2e-7)
     assert _off(lags * (N * N), c / c[mc, mc]) < 4e-7
     plan.close()
+
+
+# the error of the same convolution with a kernel spectrum and whole-circle
+# twiddles in float32, its best plane (the smallest size: its worst)
+@pytest.mark.parametrize("W,H,kw,kh,bound", [(100, 100, 7, 7, 2.69e-7), (309, 152, 157, 7, 2.82e-7), (640, 480, 31, 33, 2.70e-7),
+                                             (850, 850, 65, 65, 3.05e-7), (1024, 1024, 129, 129, 2.94e-7)])
+def test_convolution(W, H, kw, kh, bound):
+    import ghostlight_gb300 as gl
+    img = [_noise(i, H, W) for i in range(3)]
+    k = np.random.default_rng(kw).standard_normal((kh, kw)).astype(np.float32)
+    plan = gl.ConvPlan(W, H, k)
+    out = [torch.empty_like(i) for i in img]
+    plan.execute(img, out)
+    s = (H + kh - 1, W + kw - 1)
+    K = torch.fft.rfft2(torch.from_numpy(k).cuda().double(), s=s)
+    for i, o in zip(img, out):
+        want = torch.fft.irfft2(torch.fft.rfft2(i.double(), s=s) * K, s=s)[kh // 2:kh // 2 + H, kw // 2:kw // 2 + W]
+        assert _off(o, want) < bound
+    plan.close()
