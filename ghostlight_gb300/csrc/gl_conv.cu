@@ -27,9 +27,13 @@
 // transform, the third alone, ping-pong buffers, 18 warps per SM before); the
 // passes take 47, 73 and 45 us cold, issue slots half busy: bound by instruction
 // issue and fetch (each CTA runs a long straight line of code once), not by HBM
-// (15%) or shared memory (40%).
+// (15%) or shared memory (40%).  Passes 2 and 3 are launched while the pass before
+// them drains (gl_launch.cuh): 100^2 (*) 7^2, calls back to back, 20.5 -> 16 us (18.5
+// with the passes' form before half spectra), one alone 36 -> 31; 2048^2 (*) 257^2
+// 163 -> 157.
 #include "gl_internal.h"
 #include "gl_fft.cuh"
+#include "gl_launch.cuh"
 
 #include <cuda_runtime.h>
 
@@ -125,13 +129,6 @@ struct ColMul {
     const float2* k;
     __device__ __forceinline__ float2 operator()(int s, int r, float2 v) const { return cmul(v, __ldg(k + 2 * (size_t)r + s)); }
 };
-
-// Passes 2 and 3 are launched while the pass before them drains, so that setting
-// up a launch does not add to a call; each begins here, with that pass complete
-// and its writes visible.  100^2 (*) 7^2, calls back to back: 20.5 -> 16 us (18.5
-// with the passes' form before half spectra), one alone 36 -> 31; 2048^2 (*) 257^2
-// 163 -> 158.
-__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Pass 1: plane blockIdx.y, row pairs blockIdx.x kPairs + s.  Rows of width W,
 // zero-padded to Q.
@@ -464,23 +461,6 @@ static void conv_free(ConvPlan* p)
     cudaFree(p->tw_p);
     cudaFree(p->tw_pi);
     delete p;
-}
-
-// A launch that may be set up before the stream's last kernel is done (after_previous).
-template <class... P, class... V>
-static cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const V&... v)
-{
-    cudaLaunchAttribute early{};
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &early;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(v)...);
 }
 
 // The kernel's spectrum (centre at the origin, so the circular convolution lands

@@ -5,6 +5,7 @@
 // one MMA-issuing thread, four epilogue warps reading TMEM) and the plain
 // BF16 GEMM C = A * B^T that pins the descriptors against torch.
 #include "gl_internal.h"
+#include "gl_launch.cuh"
 #include "gl_tc.cuh"
 
 #include <cuda.h>
@@ -259,6 +260,7 @@ struct MdftArgs {
     // step-2 output placement: plan pixel (l, k) -> frame (y0 + l, x0 + k) of
     // planes out_w wide, kept when l < win_h and k < win_w
     int out_w, x0, y0, win_w, win_h;
+    float* parts;                     // FP32 step 2 in several wavelength ranges: each wavelength's own Re E or |E|^2, Ky x Kx
     int vec;                          // 1: every row piece of a tile starts on a 16-byte boundary in all three planes
     float4 tint;                      // per-launch colour factor on the weights
     int lam_base;                     // first wavelength of this launch's range
@@ -944,7 +946,9 @@ __global__ void __launch_bounds__(128) mdft_fold_kernel(const float* __restrict_
 // chunks of 16 staged in shared memory one chunk ahead, sums in two levels (32
 // terms, then their sums): one long sum rounded the pattern's peak 0.3 to 1.7e-6 off
 // 64 bits, two levels 0.1 to 0.3e-6.  In step 2 the wavelengths are split over CTAs
-// (n_ranges), which add into the planes with atomics.
+// (n_ranges); each wavelength's result then goes to a plane of its own and
+// mdft_simt_sum adds them up in order, so that a call repeats bit for bit (the
+// ranges' additions into the output planes would come in any order).
 // Bound by shared-memory reads and the FP32 pipes: P = 4 32 FMA per three 16-byte
 // loads (box: 16 per two), P = 8 64 per four (32 per three).  256^2 pupil to 512^2,
 // 8 wavelengths: both steps 1.75 -> 0.08 ms (the unfolded form looped over the
@@ -955,6 +959,7 @@ template <int STEP, bool BOX, int P>
 __global__ void __launch_bounds__(256, P == 8 ? 1 : 2) mdft_simt_kernel(const float* __restrict__ W, const float* __restrict__ B,
                                                            MdftArgs args, int lam1, int n_ranges)
 {
+    after_previous();
     static_assert(P == 4 || (P == 8 && STEP == 2), "rows per thread");
     constexpr int NBLK = BOX ? 1 : 2;
     constexpr int kRows = 16 * P, kLoads = P / 4;              // rows of the tile, staging loads of them per thread
@@ -1095,6 +1100,12 @@ __global__ void __launch_bounds__(256, P == 8 ? 1 : 2) mdft_simt_kernel(const fl
                 }
                 const int l = mb * kRows + (p >> 2) * 64 + ty * 4 + (p & 3), c0 = xb * kSB + tx * 4;
                 if (l >= args.win_h) continue;
+                if (n_ranges > 1)
+                {
+                    *reinterpret_cast<float4*>(args.parts + ((size_t)(lam - args.lam_base) * args.KA + l) * (args.NB * 128) + c0) =
+                        make_float4(I[0], I[1], I[2], I[3]);
+                    continue;
+                }
                 const size_t o = (size_t)(args.y0 + l) * args.out_w + args.x0 + c0;
                 float* outs[3] = {args.out_r + o, args.out_g + o, args.out_b + o};
                 const float wc[3] = {wr, wg, wb};
@@ -1111,6 +1122,47 @@ __global__ void __launch_bounds__(256, P == 8 ? 1 : 2) mdft_simt_kernel(const fl
                     }
                 }
             }
+        }
+    }
+}
+
+// The weighted sum of the wavelengths' planes, in their order, added to the output
+// window: a thread four columns of a row.
+__global__ void __launch_bounds__(256) mdft_simt_sum(const MdftArgs args, int nl)
+{
+    after_previous();
+    const int quads = args.NB * 32, idx = blockIdx.x * 256 + threadIdx.x;
+    const int l = idx / quads, c0 = (idx - l * quads) * 4;
+    if (l >= args.win_h || c0 >= args.win_w) return;
+    const float4* part = reinterpret_cast<const float4*>(args.parts) + idx;
+    const size_t plane = (size_t)args.KA * quads;
+    float sum[3][4] = {};
+    #pragma unroll 4
+    for (int k = 0; k < nl; ++k)
+    {
+        const float4 w = args.weights[args.lam_base + k], I = part[k * plane];
+        const float wc[3] = {w.x * args.tint.x, w.y * args.tint.y, w.z * args.tint.z}, v[4] = {I.x, I.y, I.z, I.w};
+        #pragma unroll
+        for (int c = 0; c < 3; ++c)
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) sum[c][q] = fmaf(wc[c], v[q], sum[c][q]);
+    }
+    const size_t o = (size_t)(args.y0 + l) * args.out_w + args.x0 + c0;
+    float* outs[3] = {args.out_r + o, args.out_g + o, args.out_b + o};
+    #pragma unroll
+    for (int c = 0; c < 3; ++c)          // one plane after the other: they may be the same memory
+    {
+        if (args.vec && c0 + 3 < args.win_w)
+        {
+            float4 v = *reinterpret_cast<const float4*>(outs[c]);
+            v.x += sum[c][0]; v.y += sum[c][1]; v.z += sum[c][2]; v.w += sum[c][3];
+            *reinterpret_cast<float4*>(outs[c]) = v;
+        }
+        else
+        {
+            #pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (c0 + q < args.win_w) outs[c][q] += sum[c][q];
         }
     }
 }
@@ -1134,6 +1186,8 @@ struct MdftPlan {
     void* wy = nullptr;     // W_y' [lam][C | S][Ky][Kp]
     void* mask = nullptr;   // A'   [4 parts, box 2][nhr][Kp]
     void* tprime = nullptr; // T'   [lam][Kx/128][4 parts, box 2][128][Kp]
+    float* parts = nullptr; // FP32 form: part_l wavelengths' Ky x Kx planes (where step 2 splits them over CTAs)
+    int part_l = 0;
     float4* weights = nullptr;
     float2* scales = nullptr;   // [2][n_lambda] (s_hi, s_lo) device copy
     float* amp = nullptr;       // [x, y][n_lambda][nh] factors of the matrix entries
@@ -1152,7 +1206,7 @@ struct MdftPlan {
 static void mdft_free(MdftPlan* p)
 {
     if (!p) return;
-    cudaFree(p->wx); cudaFree(p->wy); cudaFree(p->mask); cudaFree(p->tprime);
+    cudaFree(p->wx); cudaFree(p->wy); cudaFree(p->mask); cudaFree(p->tprime); cudaFree(p->parts);
     cudaFree(p->weights); cudaFree(p->scales); cudaFree(p->amp); cudaFree(p->err);
     delete p;
 }
@@ -1265,27 +1319,52 @@ static cudaError_t mdft_gemms(const MdftPlan* p, const MdftArgs& a1, const MdftA
                            : mdft_step<FORM, 2, 128, BOX>(p->t_wy, p->t_tp, a2, gmax, p->pairs, st);
 }
 
+// Wavelengths of the FP32 form whose planes are kept at a time: 64 MB of them,
+// which stay in L2 between step 2 and the sum.  0: the output has tiles enough
+// for every SM without splitting the wavelengths.
+static int mdft_part_lambdas(int Kx, int Ky, int n_lambda, int sms)
+{
+    if (n_lambda < 2 || (long long)(Kx / kSB) * (Ky / kSB) >= 4LL * sms) return 0;
+    return (int)std::max<long long>(2, std::min<long long>(n_lambda, (16LL << 20) / ((long long)Kx * Ky)));
+}
+
+// Both steps; *launches grows by their launches (each set up while the one before
+// drains, gl_launch.cuh).
 template <bool BOX>
-static void mdft_simt(const MdftPlan* p, const MdftArgs& a1, const MdftArgs& a2, int l1, cudaStream_t st)
+static cudaError_t mdft_simt(const MdftPlan* p, const MdftArgs& a1, const MdftArgs& a2, int l1, int* launches, cudaStream_t st)
 {
     const int nl = l1 - a1.lam_base;
     const dim3 t1((p->nh + kSB - 1) / kSB, p->Kx / kSB, 2 * nl);
-    mdft_simt_kernel<1, BOX, 4><<<t1, 256, 0, st>>>(static_cast<const float*>(p->wx), static_cast<const float*>(p->mask), a1, l1, 1);
-    // wavelength ranges until about three CTAs per SM are in flight (tall tiles,
-    // twice the work each: two)
+    cudaError_t e = launch_after(mdft_simt_kernel<1, BOX, 4>, t1, 256, 0, st, static_cast<const float*>(p->wx),
+                                 static_cast<const float*>(p->mask), a1, l1, 1);
+    ++*launches;
     const int tiles = (p->Kx / kSB) * (p->Ky / kSB);
-    // Tall tiles read a third less shared memory per FMA, but halve the CTAs: 256^2
-    // to 512^2, 64 x 64 -> 128 x 64, whole plan (sums in one level, which are 6 us
-    // faster): 96.3 -> 75.9 us (256 tall CTAs), 55.4 -> 49.2 (96), 41.0 -> 49.2 (64),
-    // 29.0 -> 30.8 (24).
-    const bool tall = (long long)tiles * nl > p->sms;          // tiles / 2 tall ones: half of the SMs or more
-    const int rows = tall ? 128 : kSB;
-    const int ranges = std::min(nl, std::max(1, ((tall ? 2 : 3) * p->sms + tiles * kSB / rows - 1) / (tiles * kSB / rows)));
-    const dim3 t2(p->Kx / kSB, p->Ky / rows, ranges);
-    if (tall)
-        mdft_simt_kernel<2, BOX, 8><<<t2, 256, 0, st>>>(static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime), a2, l1, ranges);
-    else
-        mdft_simt_kernel<2, BOX, 4><<<t2, 256, 0, st>>>(static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime), a2, l1, ranges);
+    const int groups = p->part_l > 0 ? (nl + p->part_l - 1) / p->part_l : 1;
+    MdftArgs a = a2;
+    for (int g = 0; g < groups; ++g)
+    {
+        a.lam_base = a2.lam_base + (int)((long long)nl * g / groups);
+        const int lg = a2.lam_base + (int)((long long)nl * (g + 1) / groups), n = lg - a.lam_base;
+        // Tall tiles read a third less shared memory per FMA, but halve the CTAs: 256^2
+        // to 512^2, 64 x 64 -> 128 x 64, whole plan (sums in one level, which are 6 us
+        // faster): 96.3 -> 75.9 us (256 tall CTAs), 55.4 -> 49.2 (96), 41.0 -> 49.2 (64),
+        // 29.0 -> 30.8 (24).
+        const bool tall = (long long)tiles * n > p->sms;          // tiles / 2 tall ones: half of the SMs or more
+        const int rows = tall ? 128 : kSB;
+        // wavelength ranges until about three CTAs per SM are in flight (tall tiles,
+        // twice the work each: two)
+        const int ranges = p->part_l > 0 ? std::min(n, std::max(1, ((tall ? 2 : 3) * p->sms + tiles * kSB / rows - 1) / (tiles * kSB / rows))) : 1;
+        const dim3 t2(p->Kx / kSB, p->Ky / rows, ranges);
+        if (e == cudaSuccess)
+            e = launch_after(tall ? mdft_simt_kernel<2, BOX, 8> : mdft_simt_kernel<2, BOX, 4>, t2, 256, 0, st,
+                             static_cast<const float*>(p->wy), static_cast<const float*>(p->tprime), a, lg, ranges);
+        ++*launches;
+        const int quads = p->Kx / 4 * a2.win_h;
+        if (ranges == 1 || quads == 0) continue;
+        if (e == cudaSuccess) e = launch_after(mdft_simt_sum, (quads + 255) / 256, 256, 0, st, a, n);
+        ++*launches;
+    }
+    return e;
 }
 
 }  // namespace gl
@@ -1343,6 +1422,8 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     int dev = 0;
     chk(cudaGetDevice(&dev));
     chk(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
+    if (e == cudaSuccess && form == 2) p->part_l = mdft_part_lambdas(Kx, Ky, n_lambda, p->sms);
+    if (p->part_l > 0) chk(cudaMalloc(&p->parts, sizeof(float) * (size_t)p->part_l * Kx * Ky));
     if (e != cudaSuccess)
     {
         mdft_free(p);
@@ -1464,7 +1545,7 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     a.nkb = (p->nh + kbe - 1) / kbe * (p->form == 0 && p->box ? 3 : 1);
     a.NB = NBx; a.NI = p->nhr / 128;
     a.tprime = p->tprime; a.out_r = d_out_r; a.out_g = d_out_g; a.out_b = d_out_b;
-    a.weights = p->weights; a.err = p->err;
+    a.weights = p->weights; a.err = p->err; a.parts = p->parts;
     a.out_w = out_w; a.x0 = x0; a.y0 = y0; a.win_w = win_w; a.win_h = win_h;
     // the planes may be views that start at any float
     a.vec = ((out_w | x0) & 3) == 0 && ((reinterpret_cast<uintptr_t>(d_out_r) | reinterpret_cast<uintptr_t>(d_out_g) |
@@ -1480,8 +1561,7 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     a2.n_units = NBy * a2.NBt * nl;                     // step 2: (lambda, output tile)
     if (p->form == 2)
     {
-        if (p->box) mdft_simt<true>(p, a, a2, l1, st);
-        else mdft_simt<false>(p, a, a2, l1, st);
+        GL_CUDA_TRY(p->box ? mdft_simt<true>(p, a, a2, l1, &launches, st) : mdft_simt<false>(p, a, a2, l1, &launches, st));
     }
     else if (p->form == 0)
     {
@@ -1492,7 +1572,7 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
         GL_CUDA_TRY(p->box ? (mdft_gemms<1, true>(p, a, a2, gmax, st)) : (mdft_gemms<1, false>(p, a, a2, gmax, st)));
     }
     GL_CUDA_TRY(cudaGetLastError());
-    launches += 2;
+    if (p->form != 2) launches += 2;
     g_last_launches = launches;
     return GL_OK;
 }

@@ -137,14 +137,20 @@ class MdftPlan:
         """HBM the plan holds: the two folded DFT matrices (cosine and sine
         over the distances from the reduction centre), the operand's parity
         parts and the intermediate T' in the form's element type (split-BF16:
-        two bf16 terms per element)."""
+        two bf16 terms per element), the matrices' factors, and the FP32 form's
+        planes of single wavelengths (at most 64 MB or two)."""
+        import torch
         tf32 = self.form == "tf32"
         folded = not tf32 and not (self.form == "split_bf16" and self.box)
         nh = self.n if self.box or not folded else (int(max(self._red_center, self.n - 1 - self._red_center)) + 16) // 16 * 16
         row = nh * 4                        # two bf16 terms or one float
         parts, nl = (2 if self.box or tf32 else 4), self.n_lambda
+        px, sms = self.Kx * self.Ky, torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+        planes = 0
+        if self.form == "fp32" and nl > 1 and px // 4096 < 4 * sms:
+            planes = max(2, min(nl, (16 << 20) // px))
         return (nl * 2 * (self.Kx + self.Ky) * row + (parts if folded else 1) * ((nh + 127) // 128 * 128) * row +
-                nl * parts * self.Kx * row + 32 * nl + 4)
+                nl * parts * self.Kx * row + planes * px * 4 + 8 * nl * nh + 32 * nl + 4)
 
     def close(self):
         if getattr(self, "_h", None):
