@@ -1345,10 +1345,10 @@ static cudaError_t mdft_simt(const MdftPlan* p, const MdftArgs& a1, const MdftAr
     {
         a.lam_base = a2.lam_base + (int)((long long)nl * g / groups);
         const int lg = a2.lam_base + (int)((long long)nl * (g + 1) / groups), n = lg - a.lam_base;
-        // Tall tiles read a third less shared memory per FMA, but halve the CTAs: 256^2
-        // to 512^2, 64 x 64 -> 128 x 64, whole plan (sums in one level, which are 6 us
-        // faster): 96.3 -> 75.9 us (256 tall CTAs), 55.4 -> 49.2 (96), 41.0 -> 49.2 (64),
-        // 29.0 -> 30.8 (24).
+        // Tall tiles read a third less shared memory per FMA, but halve the CTAs.  256^2
+        // to 512^2, whole call, 64 x 64 -> 128 x 64: 86 -> 78 us (256 tall CTAs), 47 -> 45
+        // (96), 35 -> 43 (64), 35 -> 43 (32); pixel form, half the FMA per load: 117 -> 109,
+        // 64 -> 60, 39 -> 50, 36 -> 49.
         const bool tall = (long long)tiles * n > p->sms;          // tiles / 2 tall ones: half of the SMs or more
         const int rows = tall ? 128 : kSB;
         // wavelength ranges until about three CTAs per SM are in flight (tall tiles,
