@@ -207,7 +207,7 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 // (Te / To the even and odd parts of T over the pupil rows).  Both steps take
 // half the products of the unfolded form, the matrices half the memory, and
 // Re E and Im E accumulate directly.  The pixel-integrated (box) form needs
-// Re E only: Te_r and To_i, a quarter of the products.
+// Re E only, Te_r and To_i; it is not folded in any storage (below).
 //
 // FORM 0 (split BF16): every operand X is stored as X_hi = bf16(X) and
 // X_lo = bf16(X - X_hi), rows [hi | lo]; each 128-byte step of the reduction
@@ -231,9 +231,9 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 //
 // Storage (Kp = 2 nh bf16, or nh floats; rows of Kp; unfolded: nh = n):
 //   W'  [lam][C | S][k]                                  TF32: [Wr | Wi]
-//   A'  [ee | oe | eo | oo][row d]   box: [ee | oo]      (nhr rows each; TF32: A)
-//   T'  [lam][k / 128][Te_r | Te_i | To_i | -To_r][k % 128]   box: [Te_r | To_i]
-//                                                        TF32: [Tr | Ti]
+//   A'  [ee | oe | eo | oo][row d]   FP32 box: A twice   (nhr rows each; TF32: A)
+//   T'  [lam][k / 128][Te_r | Te_i | To_i | -To_r][k % 128]   FP32 box: [Te_r | To_i]
+//                                                        TF32, split BF16 box: [Tr | Ti]
 // ===========================================================================
 namespace gl {
 namespace {
@@ -306,9 +306,10 @@ template <int FORM, int STEP, int TN, bool BOX, int CL>
 struct MdftShape {
     static constexpr bool kFold = is_folded(FORM);
     static constexpr int kBSets = kFold ? 2 : 1;
-    static constexpr int kBlocks = kFold ? (BOX ? 1 : 2) : STEP;    // row blocks of B per unit and set
+    static_assert(!(kFold && BOX), "the pixel form is not folded on the tensor cores");
+    static constexpr int kBlocks = kFold ? 2 : STEP;                // row blocks of B per unit and set
     static constexpr int kRows = STEP == 2 ? TN : 128;              // rows of one block
-    static constexpr int kN = (!kFold && STEP == 2 && BOX) ? TN : kBlocks * kRows;   // MMA N
+    static constexpr int kN = (STEP == 2 && BOX) ? TN : kBlocks * kRows;   // MMA N
     static constexpr int kOwn = kBlocks / CL;                       // of them this CTA loads (a pair: one each)
     static constexpr int kBBytes = kOwn * kRows * 128;
     static constexpr int kStageBytes = 2 * kOpTile + kBSets * kBBytes;
@@ -626,12 +627,11 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                 // T' rows of this k.  The C part gives (Te_r, To_r), the S part
                 // (-Te_i, -To_i); step 2 wants [Te_r | Te_i | To_i | -To_r].  TF32:
                 // (Tr, Ti) as they are.
-                constexpr int kOut = Sh::kFold ? Sh::kBlocks : 2;
-                const size_t blk = (size_t)(lam * args.NB + mb) * (Sh::kParts * kOut) * 128;
+                const size_t blk = (size_t)(lam * args.NB + mb) * (Sh::kParts * 2) * 128;
                 #pragma unroll
-                for (int j = 0; j < kOut; ++j)
+                for (int j = 0; j < 2; ++j)
                 {
-                    const int dst = !Sh::kFold ? j : (BOX ? part : (part == 0 ? (j == 0 ? 0 : 3) : (j == 0 ? 1 : 2)));
+                    const int dst = !Sh::kFold ? j : (part == 0 ? (j == 0 ? 0 : 3) : (j == 0 ? 1 : 2));
                     const float sign = (!Sh::kFold || (part == 0 && j == 0)) ? 1.0f : -1.0f;
                     #pragma unroll 1
                     for (int c = 0; c < 8; ++c)
@@ -890,12 +890,10 @@ __device__ __forceinline__ void mdft_fold_one(const float* __restrict__ a, void*
         v[2] = co ? (p - q) + (s - t) : 0.0f;
         v[3] = ro && co ? (p - q) - (s - t) : 0.0f;
     }
-    const int parts = box ? 2 : 4;
     #pragma unroll
     for (int k = 0; k < 4; ++k)
     {
-        if (k >= parts) break;
-        const float w = box ? (k == 0 ? v[0] : v[3]) : v[k];
+        const float w = v[k];
         const size_t o = ((size_t)k * nhr + y) * Kp + x;
         if (FORM == 0)
         {
@@ -1603,7 +1601,7 @@ extern "C" int gl_mdft_plan_set_launch(gl_mdft_plan* plan, int ctas)
 {
     using namespace gl;
     if (!plan || ctas < 0) return fail(GL_ERR_INVALID, "mdft_plan_set_launch: bad arguments");
-    // one 192-thread CTA with up to ~193 KB of shared memory fits per SM
+    // one 192-thread CTA with up to 210 KB of shared memory fits per SM
     plan->p->ctas = ctas == 0 ? 0 : std::min(ctas, plan->p->sms);
     return GL_OK;
 }
