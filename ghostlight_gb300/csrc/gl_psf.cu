@@ -39,9 +39,9 @@ struct PsfArgs {
     float* out_g;
     float* out_b;
     int tile_smem;       // 1: the CTA's source tile is accumulated in shared memory
-    // dense path: landings [source][wavelength][sample] (weight < 0: none near
-    // the tile), of n_land wavelengths from l_base on; samples per CTA in steps
-    // of the CTA's threads
+    // dense path: landings [source][wavelength][sample] as (x, y, weight, 1), the
+    // last 0 where there is none near the tile, of n_land wavelengths from l_base
+    // on; samples per CTA in steps of the CTA's threads
     float4* land;
     int l_base, n_land, s_base, rounds;
 };
@@ -149,7 +149,7 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
         if (LAND)
         {
             land = A.land + ((size_t)(si - A.s_base) * A.n_land + (l - A.l_base)) * A.n_grid + gi;
-            land->z = -1.0f;
+            land->w = 0.0f;
         }
         const float4 sp = A.spec[l];
         const TraceOut r = trace_primary(lens, A.n_surf, at + l * A.n_surf, org, dir, sp.x);
@@ -162,7 +162,9 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
         const float w = r.w * A.ray_weight;
         if (LAND)
         {
-            *land = make_float4(px, py, w, 0.0f);
+            // (an attenuator's weight may have either sign; one that is not a number
+            // is left out, as the taps leave it out)
+            if (w == w) *land = make_float4(px, py, w, 1.0f);
             continue;
         }
         const float lum = (S.r + S.g + S.b) * (1.0f / 3.0f) * sp.z * w;
@@ -283,9 +285,9 @@ __global__ void __launch_bounds__(kPsfThreads, 2) psf_dense_kernel(PsfArgs A)
     for (int q = 0; q < A.rounds; ++q)
     {
         const int gi = (blockIdx.z * A.rounds + q) * kPsfThreads + tid;
-        float4 e = make_float4(0.0f, 0.0f, -1.0f, 0.0f);
+        float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (gi < A.n_grid) e = land[gi];
-        const bool in = e.z >= 0.0f;
+        const bool in = e.w != 0.0f;
         const unsigned m = __ballot_sync(0xffffffffu, in);
         int base = 0;
         if (lane == 0 && m) base = atomicAdd(&n_list, __popc(m));
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(kPsfThreads, 2) psf_dense_kernel(PsfArgs A)
         const float v = sum[y * W8 + x];
         if (v == 0.0f) continue;
         for (int pl = 0; pl < planes; ++pl)
-            if (c[pl] != 0.0f) atomicAdd(outs[pl] + (size_t)yi * A.comp_w + xi, c[pl] * v);
+            if (fabsf(c[pl]) > 0.0f) atomicAdd(outs[pl] + (size_t)yi * A.comp_w + xi, c[pl] * v);
     }
 }
 
