@@ -118,6 +118,9 @@ def _declare(lib):
     lib.gl_psf_render.argtypes = [P(gl_surface), i, P(gl_psf_source), i, P(gl_pupil_sample), i,
                                   P(gl_spectral_sample), i, i, i, i, i, f, i, f, i, vp, vp, vp, vp]
     lib.gl_psf_render_async.argtypes = lib.gl_psf_render.argtypes
+    lib.gl_psf_render_async2.argtypes = lib.gl_psf_render.argtypes[:-1] + [C.c_longlong, vp]
+    lib.gl_psf_scratch_bytes.argtypes = [i, i, i, i, i, C.c_float, i]
+    lib.gl_psf_scratch_bytes.restype = C.c_longlong
     lib.gl_veil_plan_create.argtypes = [f, vp, P(vp)]
     lib.gl_veil_plan_execute.argtypes = [vp, vp, i, P(gl_veil_params), vp, vp, vp, vp]
     lib.gl_veil_plan_destroy.argtypes = [vp]

@@ -242,6 +242,7 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
 // that fits L2): inlined here it rounded some landings differently.
 constexpr int kDenseChunk = 32;       // landings per outer-product step
 constexpr size_t kDenseLandings = (size_t)4 << 20;   // 64 MB: stays in L2 between the two kernels
+constexpr long long kLandingBytes = (long long)(kDenseLandings * sizeof(float4));
 constexpr int kDenseRoundsMax = 16;   // pupil samples per thread and CTA, at most
 
 struct DenseGeom {
@@ -399,6 +400,20 @@ inline bool dense_tile(int tile_w, int tile_h, float sigma_px, int radius_px)
     return sigma_px > 0.0f && g.groups >= 1 && radius_px >= (64 * g.tx * g.ty <= 8192 ? 3 : 4);
 }
 
+// Landings kept at a time: of as many wavelengths and sources as fit the scratch
+// (0 sources: not one wavelength of one source does).
+struct Landings { int l, s; };
+
+inline Landings landings(int n_sources, int n_grid, int n_spec, long long bytes)
+{
+    const size_t most = std::min<size_t>(kDenseLandings, (size_t)std::max(0LL, bytes) / sizeof(float4));
+    Landings k{0, 0};
+    if (most < (size_t)n_grid) return k;
+    k.l = (int)std::min<size_t>(std::min(n_spec, 65535), most / n_grid);
+    k.s = (int)std::min<size_t>(n_sources, most / ((size_t)n_grid * k.l));
+    return k;
+}
+
 }  // namespace
 }  // namespace gl
 
@@ -412,7 +427,7 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
                            const gl_pupil_sample* grid, int n_grid, const gl_spectral_sample* spec, int n_spec,
                            int tile_w, int tile_h, int composite_w, int composite_h, float mm_per_pixel,
                            int monochromatic, float splat_sigma_px, int splat_radius_px, float* d_out_r,
-                           float* d_out_g, float* d_out_b, void* stream, bool ordered)
+                           float* d_out_g, float* d_out_b, long long landing_bytes, void* stream, bool ordered)
 {
     if (!surfaces || n_surfaces <= 0) return fail(GL_ERR_INVALID, "psf_render: lens has no surfaces");
     if (n_sources < 0 || n_grid < 0 || n_spec < 1 || (n_sources > 0 && !sources) || (n_grid > 0 && !grid) || !spec)
@@ -471,14 +486,22 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
     auto dense_z = [&](int r) { return ((long long)n_grid + r * kPsfThreads - 1) / (r * kPsfThreads); };
     while (rounds > 1 && dense_z(rounds) * n_sources * n_spec < 8LL * n_sm) rounds /= 2;
     const size_t dense_smem = dense_smem_floats(dg, rounds) * sizeof(float);
-    const bool dense = dense_tile(tile_w, tile_h, splat_sigma_px, splat_radius_px) && dense_smem <= 220 * 1024 &&
-                       (size_t)n_grid <= kDenseLandings;
-    // landings of as many sources and wavelengths at a time as fit the scratch
-    const int land_l = dense ? (int)std::min<size_t>(std::min(n_spec, 65535), kDenseLandings / n_grid) : 0;
-    const int land_s = dense ? (int)std::min<size_t>(n_sources, std::max<size_t>(1, kDenseLandings / ((size_t)n_grid * land_l))) : 0;
+    const Landings k = landings(n_sources, n_grid, n_spec, landing_bytes);
+    const int land_l = k.l, land_s = k.s;
+    bool dense = dense_tile(tile_w, tile_h, splat_sigma_px, splat_radius_px) && dense_smem <= 220 * 1024 && land_s > 0;
     float4* d_land = nullptr;
     if (e == cudaSuccess && dense)
+    {
         e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&d_land), sizeof(float4) * (size_t)land_s * land_l * n_grid, pool, st);
+        if (e == cudaErrorMemoryAllocation)
+        {
+            // no room for them: the taps need none
+            cudaGetLastError();
+            d_land = nullptr;
+            dense = false;
+            e = cudaSuccess;
+        }
+    }
     const size_t smem = recs.size() * sizeof(SurfRec) + at.size() * sizeof(float) + (tile_smem && !dense ? tile_bytes + 16 : 0);
     if (e == cudaSuccess && smem > 48 * 1024)
         e = (cudaError_t)raise_smem_limit(dense ? (const void*)psf_kernel<true> : (const void*)psf_kernel<false>, smem);
@@ -540,6 +563,18 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
     return GL_OK;
 }
 
+extern "C" long long gl_psf_scratch_bytes(int n_sources, int n_grid, int n_spec, int tile_w, int tile_h, float splat_sigma_px,
+                                          int splat_radius_px)
+{
+    if (n_sources <= 0 || n_grid <= 0 || n_spec <= 0 || tile_w <= 0 || tile_h <= 0) return 0;
+    // lens records, index table, spectrum, sources and pupil grid, each rounded up
+    const long long tables = (long long)kMaxSurfaces * (sizeof(SurfRec) + sizeof(float) * n_spec) + sizeof(float4) * n_spec +
+                             sizeof(gl_psf_source) * (long long)n_sources + sizeof(float2) * (long long)n_grid + 5 * 256;
+    if (!dense_tile(tile_w, tile_h, splat_sigma_px, splat_radius_px)) return tables;
+    const Landings k = landings(n_sources, n_grid, n_spec, kLandingBytes);
+    return tables + (long long)sizeof(float4) * k.s * k.l * n_grid;
+}
+
 extern "C" int gl_psf_render(const gl_surface* surfaces, int n_surfaces, const gl_psf_source* sources, int n_sources,
                              const gl_pupil_sample* grid, int n_grid, const gl_spectral_sample* spec, int n_spec,
                              int tile_w, int tile_h, int composite_w, int composite_h, float mm_per_pixel,
@@ -548,7 +583,7 @@ extern "C" int gl_psf_render(const gl_surface* surfaces, int n_surfaces, const g
 {
     return psf_render_impl(surfaces, n_surfaces, sources, n_sources, grid, n_grid, spec, n_spec, tile_w, tile_h,
                            composite_w, composite_h, mm_per_pixel, monochromatic, splat_sigma_px, splat_radius_px,
-                           d_out_r, d_out_g, d_out_b, stream, false);
+                           d_out_r, d_out_g, d_out_b, kLandingBytes, stream, false);
 }
 
 extern "C" int gl_psf_render_async(const gl_surface* surfaces, int n_surfaces, const gl_psf_source* sources,
@@ -560,5 +595,17 @@ extern "C" int gl_psf_render_async(const gl_surface* surfaces, int n_surfaces, c
 {
     return psf_render_impl(surfaces, n_surfaces, sources, n_sources, grid, n_grid, spec, n_spec, tile_w, tile_h,
                            composite_w, composite_h, mm_per_pixel, monochromatic, splat_sigma_px, splat_radius_px,
-                           d_out_r, d_out_g, d_out_b, stream, true);
+                           d_out_r, d_out_g, d_out_b, kLandingBytes, stream, true);
+}
+
+extern "C" int gl_psf_render_async2(const gl_surface* surfaces, int n_surfaces, const gl_psf_source* sources,
+                                    int n_sources, const gl_pupil_sample* grid, int n_grid,
+                                    const gl_spectral_sample* spec, int n_spec, int tile_w, int tile_h,
+                                    int composite_w, int composite_h, float mm_per_pixel, int monochromatic,
+                                    float splat_sigma_px, int splat_radius_px, float* d_out_r, float* d_out_g,
+                                    float* d_out_b, long long landing_bytes, void* stream)
+{
+    return psf_render_impl(surfaces, n_surfaces, sources, n_sources, grid, n_grid, spec, n_spec, tile_w, tile_h,
+                           composite_w, composite_h, mm_per_pixel, monochromatic, splat_sigma_px, splat_radius_px,
+                           d_out_r, d_out_g, d_out_b, landing_bytes, stream, true);
 }

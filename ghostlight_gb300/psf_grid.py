@@ -106,18 +106,33 @@ def psf_inputs(sources, lens, config, cache=None) -> dict:
                 tile_w=int(cfg.tile_w), tile_h=int(cfg.tile_h))
 
 
-def psf_launch(inp: dict, out, stream, ordered: bool = False) -> None:
+def psf_scratch_bytes(config, n_sources: int, n_spec: int, landings: bool = True) -> int:
+    """Most device scratch of one render of `config` with `n_sources` sources and
+    `n_spec` wavelengths, with or without a wide splat's landings: every point of
+    the sampling square taken as inside the pupil."""
+    mm_pp = float(np.float32(config.tile_extent_mm) / np.float32(config.tile_w))
+    sigma, radius = splat_footprint(config.splat_sigma_um, mm_pp) if landings else (0.0, 0)
+    return int(_native.load().gl_psf_scratch_bytes(int(n_sources), int(config.ray_grid) ** 2, int(n_spec),
+                                                   int(config.tile_w), int(config.tile_h), sigma, radius))
+
+
+def psf_launch(inp: dict, out, stream, ordered: bool = False, landing_bytes=None) -> None:
     """Enqueue the atlas of psf_inputs into `out` ((3, H, W) zeroed float32
     CUDA tensor) on `stream`: gl_psf_render_async when `ordered` (scratch from
-    the device pool, no wait), else gl_psf_render."""
+    the device pool, no wait), else gl_psf_render.  landing_bytes: most scratch
+    for a wide splat's landings (ordered only; None: the library's own limit)."""
     lib = _native.load()
     P = C.POINTER
-    fn = lib.gl_psf_render_async if ordered else lib.gl_psf_render
-    _native.check(fn(inp["arr"], len(inp["arr"]), inp["sources"], inp["n"],
-                     inp["grid"].ctypes.data_as(P(gl_pupil_sample)), len(inp["grid"]),
-                     inp["spec"].ctypes.data_as(P(gl_spectral_sample)), len(inp["spec"]), inp["tile_w"],
-                     inp["tile_h"], inp["comp_w"], inp["comp_h"], inp["mm_pp"], inp["mono"], inp["sigma"],
-                     inp["radius"], out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr(), stream), "render_psf")
+    args = (inp["arr"], len(inp["arr"]), inp["sources"], inp["n"],
+            inp["grid"].ctypes.data_as(P(gl_pupil_sample)), len(inp["grid"]),
+            inp["spec"].ctypes.data_as(P(gl_spectral_sample)), len(inp["spec"]), inp["tile_w"],
+            inp["tile_h"], inp["comp_w"], inp["comp_h"], inp["mm_pp"], inp["mono"], inp["sigma"],
+            inp["radius"], out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr())
+    if ordered and landing_bytes is not None:
+        rc = lib.gl_psf_render_async2(*args, int(landing_bytes), stream)
+    else:
+        rc = (lib.gl_psf_render_async if ordered else lib.gl_psf_render)(*args, stream)
+    _native.check(rc, "render_psf")
 
 
 def render_psf(sources, lens, config) -> dict:

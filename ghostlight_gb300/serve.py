@@ -58,6 +58,7 @@ class FlareRequest:
     # filled by the server
     est_rays: int = 0
     device_bytes: int = 0
+    landing_bytes: int = 0          # of device_bytes: scratch for a PSF atlas's landings
     priority: int = 0
     start: float = 0.0
     finish: float = 0.0
@@ -313,6 +314,23 @@ def request_bytes(width: int, height: int, n_pairs: int, host_copy: bool = True)
     return px * 16 + px * 12 + 4 * max(1, n_pairs) + 16384
 
 
+def psf_request_config(req: FlareRequest):
+    """The PSFConfig of a PSF request."""
+    from .config import PSFConfig
+    return PSFConfig(grid_nx=req.psf_grid, grid_ny=req.psf_grid, tile_w=req.psf_tile, tile_h=req.psf_tile,
+                     tile_extent_mm=req.psf_extent_mm, spectral_samples=req.n_spec, ray_grid=req.ray_grid)
+
+
+def psf_request_bytes(req: FlareRequest) -> tuple:
+    """(HBM a PSF request holds, of it the landings of a wide splat): planes twice
+    (atlas and copy), tables, landings."""
+    from .psf_grid import psf_scratch_bytes
+    cfg, n = psf_request_config(req), req.psf_grid * req.psf_grid
+    tables = psf_scratch_bytes(cfg, n, max(3, req.n_spec), landings=False)
+    landing = psf_scratch_bytes(cfg, n, max(3, req.n_spec)) - tables
+    return 3 * 4 * req.width * req.height * 2 + max(1 << 20, tables) + landing, landing
+
+
 # ---------------------------------------------------------------------------
 # resident lens
 # ---------------------------------------------------------------------------
@@ -495,7 +513,7 @@ class CudaExecutor:
             req.est_rays = int(req.psf_grid * req.psf_grid * masked * req.n_spec)
             req.priority = max(self.greatest, priority_class(req.est_rays, policy="sjf" if self.policy != "lsf"
                                                              else "lsf"))
-            req.device_bytes = 3 * 4 * req.width * req.height * 2 + (1 << 20)
+            req.device_bytes, req.landing_bytes = psf_request_bytes(req)
             return
         req.est_rays = int(rl.n_pairs * masked * req.n_spec)
         if self.policy == "sjf_fifo":
@@ -571,9 +589,7 @@ class CudaExecutor:
 
     def psf_config(self, req: FlareRequest, rl: ResidentLens):
         """The PSFConfig of a PSF request (and its sources), as render_psf takes them."""
-        from .config import PSFConfig
-        cfg = PSFConfig(grid_nx=req.psf_grid, grid_ny=req.psf_grid, tile_w=req.psf_tile, tile_h=req.psf_tile,
-                        tile_extent_mm=req.psf_extent_mm, spectral_samples=req.n_spec, ray_grid=req.ray_grid)
+        cfg = psf_request_config(req)
         cal = rl.calibration
         f = np.float32
         ax, ay = f(cal.max_half_angle_h) * f(req.psf_field_frac), f(cal.max_half_angle_v) * f(req.psf_field_frac)
@@ -618,7 +634,7 @@ class CudaExecutor:
         stream = run.stream[1]
         with torch.cuda.stream(stream):
             run.psf = torch.zeros((3, inp["comp_h"], inp["comp_w"]), dtype=torch.float32, device=self.device)
-            psf_launch(inp, run.psf, stream.cuda_stream, ordered=True)
+            psf_launch(inp, run.psf, stream.cuda_stream, ordered=True, landing_bytes=req.landing_bytes)
             run.host, run.outs = None, None
             if self.host_output:
                 run.host = self._pinned_buf(tuple(run.psf.shape))
@@ -756,8 +772,12 @@ class FlareServer:
 
     def submit(self, req: FlareRequest):
         """Queue a request; one that needs more than the whole HBM budget is
-        marked rejected and kept out of the queue."""
+        marked rejected and kept out of the queue.  A PSF atlas gives up landings
+        first: it can be made with fewer of them at a time, or with none."""
         self.exec.estimate(req)
+        cut = min(req.landing_bytes, max(0, req.device_bytes - self.sched.budget))
+        req.landing_bytes -= cut
+        req.device_bytes -= cut
         try:
             self.sched.submit(req)
         except ValueError:
