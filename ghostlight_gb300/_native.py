@@ -72,6 +72,7 @@ def _declare(lib):
     lib.gl_ghost_plan_destroy.argtypes = [vp]
     lib.gl_ghost_plan_pair_hits.argtypes = [vp, P(C.c_int32), i]
     lib.gl_ghost_plan_traced.argtypes = [vp, P(C.c_longlong)]
+    lib.gl_ghost_plan_walk.argtypes = [vp, P(i), P(i)]
     lib.gl_ghost_plan_traced_split.argtypes = [vp, P(C.c_longlong), P(C.c_longlong)]
     lib.gl_ghost_plan_set_timing.argtypes = [vp, vp, vp, vp]
     lib.gl_morton_order.argtypes = [P(gl_pupil_sample), i, P(gl_pupil_sample)]

@@ -5,14 +5,16 @@ GPU, and keeps the fastest; choices are cached per (device, workload key) in
 memory and, when GL_TUNE_CACHE names a file (or ``cache_path`` is given), in a
 JSON file so a server starts tuned.  Knobs:
 
-* the ghost render: persistent work queue with 4..8 CTAs per SM, or one-shot
-  CTAs of 1..8 32-sample items per warp (``GhostRenderPlan.set_launch``);
+* the ghost render: persistent work queue with 6 or all resident CTAs per SM, or
+  one-shot CTAs of 1..8 32-sample items per warp (``GhostRenderPlan.set_launch``);
+  the queue's wavelengths per task where it traces pair by pair (the walk that
+  shares the pairs' legs has one in every task);
 * the starburst GEMMs: the persistent grid size and the output tile width of
   the second GEMM, 128 or 64 complex columns per unit (``MdftPlan.set_launch``).
 
-The splat has no tile to tune: each lane keeps its 2x2 footprint across the
-wavelength loop and flushes on change, so there is no shared-memory tile whose
-shape would matter.
+The splat has no tile to tune: a landing goes to its four pixels, or a warp whose
+landings share a footprint sums them first, so there is no shared-memory tile
+whose shape would matter.
 """
 from __future__ import annotations
 
@@ -21,9 +23,25 @@ import os
 import threading
 from typing import Callable, Dict, Hashable, List, Optional, Sequence
 
+# Part of every key: raised when the kernels change so that choices kept in a file
+# no longer say what is fastest.
+KERNELS = "k2"
+
 # (items per warp, CTAs per SM, wavelength chunks per item)
 GHOST_CANDIDATES = [(0, 0, 1), (0, 0, 2), (0, 0, 4), (0, 0, 8), (0, 0, 16), (0, 6, 4), (1, 0, 4), (1, 0, 1),
                     (2, 0, 1), (4, 0, 1), (8, 0, 1)]
+
+
+def ghost_candidates(shared_legs: bool) -> List[tuple]:
+    """The launch shapes worth timing: where the queue's walk shares the pairs'
+    legs, one per number of CTAs, since a task has one wavelength there."""
+    out, seen = [], set()
+    for c in GHOST_CANDIDATES:
+        shape = c[:2] if shared_legs and c[0] == 0 else c
+        if shape not in seen:
+            seen.add(shape)
+            out.append(c)
+    return out
 
 
 def mdft_candidates(sms: int) -> List[tuple]:
@@ -116,14 +134,15 @@ def _device_name() -> str:
 def tune_ghost_plan(plan, outs, stream=None, tuner: Optional[Tuner] = None, candidates=None):
     """Pick and apply the render launch shape of a GhostRenderPlan."""
     t = tuner or default_tuner()
-    key = ("ghost", _device_name(), plan.n_items, plan.rays, plan.width * plan.height)
+    walk = "legs" if plan.walk_tasks > 0 else "pairs"
+    key = ("ghost", KERNELS, walk, _device_name(), plan.n_items, plan.rays, plan.width * plan.height)
     st = stream.cuda_stream if stream is not None else None
 
     def run(c):
         plan.set_launch(*c)
         plan.execute(*outs, stream=st)
 
-    choice = t.best(key, candidates or GHOST_CANDIDATES, run, stream)
+    choice = t.best(key, candidates or ghost_candidates(plan.walk_tasks > 0), run, stream)
     plan.set_launch(*choice)
     return choice
 
@@ -133,7 +152,7 @@ def tune_mdft_plan(plan, pupil, outs, stream=None, tuner: Optional[Tuner] = None
     import torch
     t = tuner or default_tuner()
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    key = ("mdft", _device_name(), plan.form, plan.n, plan.Kx, plan.Ky, plan.n_lambda)
+    key = ("mdft", KERNELS, _device_name(), plan.form, plan.n, plan.Kx, plan.Ky, plan.n_lambda)
     st = stream.cuda_stream if stream is not None else None
 
     def run(c):

@@ -1627,10 +1627,11 @@ int plan_execute(GhostPlan* p, float* d_out_r, float* d_out_g, float* d_out_b, c
     {
         // Probe passes: the frame inflated by CULL_MARGIN = 1.25
         // (ghost_render.cu:148).  The three passes are one persistent launch
-        // over their items in pass order: a pair is culled only when no item
-        // of any pass hits, and an item whose pair already has a hit is
-        // skipped, so a later pass re-probes only the pairs still without one
-        // (the reference's candidate rule) without a launch boundary per pass.
+        // without a boundary per pass: a pair is culled only when no ray of any
+        // pass hits, and a pair that has a hit is not looked at again.  The tree
+        // takes the passes' samples as one grid, wavelength by wavelength; pair
+        // by pair the items come in pass order, so a later pass probes only the
+        // pairs still without a hit (the reference's candidate rule).
         GL_CUDA_TRY(cudaMemcpyAsync(p->pair_hits, p->pair_hits_init, sizeof(int) * p->n_pairs,
                                     cudaMemcpyDeviceToDevice, st));
         GL_CUDA_TRY(cudaMemsetAsync(p->probe_counters, 0, sizeof(int) * 4, st));
@@ -1812,7 +1813,16 @@ int gl_ghost_plan_info(const gl_ghost_plan* plan, long long* rays, int* n_items,
     if (!plan) return fail(GL_ERR_INVALID, "ghost_plan_info: null plan");
     if (rays) *rays = plan->p->rays + plan->p->probe_rays;
     if (n_items) *n_items = plan->p->n_items;
-    if (grid) *grid = queue_grid(plan->p, plan->p->n_items, plan->p->l_chunks);
+    const GhostPlan* p = plan->p;
+    if (grid) *grid = p->tree.n_tasks > 0 ? queue_grid(p, p->tree.n_tasks, 1) : queue_grid(p, p->n_items, p->l_chunks);
+    return GL_OK;
+}
+
+int gl_ghost_plan_walk(const gl_ghost_plan* plan, int* render_tasks, int* probe_tasks)
+{
+    if (!plan) return fail(GL_ERR_INVALID, "ghost_plan_walk: null plan");
+    if (render_tasks) *render_tasks = plan->p->tree.n_tasks;
+    if (probe_tasks) *probe_tasks = plan->p->probe_tree.n_tasks;
     return GL_OK;
 }
 

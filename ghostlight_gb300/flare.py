@@ -274,6 +274,10 @@ class GhostRenderPlan:
         self.rays = int(rays.value)
         self.n_items = int(items.value)
         self.persistent_ctas = int(grid.value)
+        walk, probe = C.c_int(), C.c_int()
+        lib.gl_ghost_plan_walk(h, C.byref(walk), C.byref(probe))
+        # tasks of the walk that shares the pairs' legs (0: pair by pair)
+        self.walk_tasks, self.probe_tasks = int(walk.value), int(probe.value)
 
     def stats(self, stream=None):
         """Per-pair counters of the diagnostic pass (gl_ghost_plan_stats):
@@ -301,7 +305,8 @@ class GhostRenderPlan:
         """Launch shape of the batched render: 0 = persistent work queue over
         ctas_per_sm CTAs per SM (0 = all resident), > 0 = one-shot CTAs of that
         many 32-sample items per warp; lambda_chunks splits each item's
-        wavelengths into that many tasks."""
+        wavelengths into that many tasks where the pairs are traced one by one
+        (one-shot CTAs, or walk_tasks == 0; else a task has one wavelength)."""
         _native.check(self._lib.gl_ghost_plan_set_launch(self._h, int(items_per_warp), int(ctas_per_sm)),
                       "set_launch")
         _native.check(self._lib.gl_ghost_plan_set_lambda_split(self._h, int(lambda_chunks)), "set_launch")

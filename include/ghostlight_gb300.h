@@ -324,16 +324,24 @@ int gl_ghost_plan_info(const gl_ghost_plan* plan, long long* rays, int* n_items,
 /* Launch shape of the batched render (the autotuner's knob; no counterpart in
  * the reference, whose launch shape is fixed at ghost_render.cu:1544):
  * items_per_warp = 0 -> persistent work queue over ctas_per_sm CTAs per SM
- * (0 = all resident); > 0 -> one-shot CTAs of that many 32-sample items per warp. */
+ * (0 = all resident); > 0 -> one-shot CTAs of that many 32-sample items per warp,
+ * which trace pair by pair. */
 int gl_ghost_plan_set_launch(gl_ghost_plan* plan, int items_per_warp, int ctas_per_sm);
-/* Wavelength split of the render and probe work (the autotuner's other knob;
- * no counterpart in the reference): each 32-sample item becomes `chunks`
- * tasks over consecutive wavelength ranges, so the tasks left at the end of
- * the queue are shorter.  >= 1, clamped to n_spec; the default is about eight
- * wavelengths per task (31 -> 4, 16 -> 2, 8 -> 1). */
+/* Wavelength split of the pair-by-pair walk (the autotuner's other knob; no
+ * counterpart in the reference): each 32-sample item becomes `chunks` tasks over
+ * consecutive wavelength ranges, so the tasks left at the end of the queue are
+ * shorter.  >= 1, clamped to n_spec; the default is about eight wavelengths per
+ * task (31 -> 4, 16 -> 2, 8 -> 1), fewer where a plan has few items.  It holds
+ * for one-shot CTAs and for queues that trace pair by pair; the walk that shares
+ * the pairs' legs has one wavelength in every task whatever is set here. */
 int gl_ghost_plan_set_lambda_split(gl_ghost_plan* plan, int chunks);
-/* Ray-wavelength traces the last execute ran (render + cull probes; a probe
- * warp stops at its first on-sensor hit).  Synchronous. */
+/* How the persistent queue and the off-sensor probe trace: tasks of the walk that
+ * shares the pairs' common legs, 0 where they trace pair by pair (a pair turns at
+ * an inactive surface; the plan renders pair by pair; nothing to probe). */
+int gl_ghost_plan_walk(const gl_ghost_plan* plan, int* render_tasks, int* probe_tasks);
+/* Ray-wavelength traces the last execute ran (render + cull probes): every ray of
+ * every pair that a task took up, whether it shared its first legs with another
+ * pair's or not.  Pairs with an on-sensor hit are not taken up again.  Synchronous. */
 int gl_ghost_plan_traced(const gl_ghost_plan* plan, long long* out);
 /* The pupil-sample order the batched render traces in: a stable sort along a
  * Morton curve over the pupil square, so the 32 samples of a warp are
