@@ -91,6 +91,7 @@ def _declare(lib):
     lib.gl_sprite_plan_autocorr.argtypes = [vp, vp, i, vp, i, i, vp]
     lib.gl_mdft_plan_set_launch.argtypes = [vp, i]
     lib.gl_mdft_plan_set_tile.argtypes = [vp, i]
+    lib.gl_mdft_plan_pairs.argtypes = [vp, P(i), P(i)]
     lib.gl_mdft_plan_set_lambda_range.argtypes = [vp, i, i]
     lib.gl_mdft_plan_execute2.argtypes = [vp, vp, vp, vp, vp, i, vp]
     lib.gl_build_pupil.argtypes = [P(gl_surface), i, i, f, i, f, vp, vp]

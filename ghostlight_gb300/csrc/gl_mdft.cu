@@ -1291,16 +1291,26 @@ static cudaError_t mdft_prepare_all(int* pairs)
 // 148 -> 152; step 1 at 16 stages 137 -> 125 (512 units), at 8 stages 141 -> 137 and
 // 355 -> 379, at 4 stages 219 -> 224.
 template <int FORM, int STEP, int TN, bool BOX>
+static int mdft_pairs(const MdftArgs& a, int gmax, int pairs)
+{
+    if constexpr (FORM == 0 && !BOX && TN == 128)
+    {
+        const int stages = MdftShape<FORM, STEP, TN, BOX, 2>::kPhases * a.nkb;
+        const bool worth = stages >= (STEP == 1 ? 16 : 8) && (long long)stages * a.n_units >= 3000;
+        if ((a.NBm & 1) == 0 && worth) return std::min(std::min(a.n_units, gmax) / 2, pairs);
+    }
+    return 0;
+}
+
+template <int FORM, int STEP, int TN, bool BOX>
 static cudaError_t mdft_step(const CUtensorMap& tA, const CUtensorMap& tB, const MdftArgs& a, int gmax, int pairs, cudaStream_t st)
 {
     if constexpr (FORM == 0 && !BOX && TN == 128)
     {
-        pairs = std::min(std::min(a.n_units, gmax) / 2, pairs);
-        const int stages = MdftShape<FORM, STEP, TN, BOX, 2>::kPhases * a.nkb;
-        const bool worth = stages >= (STEP == 1 ? 16 : 8) && (long long)stages * a.n_units >= 3000;
-        if ((a.NBm & 1) == 0 && pairs > 0 && worth)
+        const int two = mdft_pairs<FORM, STEP, TN, BOX>(a, gmax, pairs);
+        if (two > 0)
         {
-            const MdftLaunch L(2 * pairs, 2, MdftShape<FORM, STEP, TN, BOX, 2>::kSmem, st);
+            const MdftLaunch L(2 * two, 2, MdftShape<FORM, STEP, TN, BOX, 2>::kSmem, st);
             return cudaLaunchKernelEx(&L.cfg, mdft_kernel<FORM, STEP, TN, BOX, 2>, tA, tB, a);
         }
     }
@@ -1497,6 +1507,38 @@ extern "C" int gl_mdft_plan_set_center(gl_mdft_plan* plan, double center_x, doub
     return GL_OK;
 }
 
+// The sizes of both steps' reductions and units; a1 holds what they share.
+static void mdft_units(const MdftPlan* p, MdftArgs& a1, MdftArgs& a2)
+{
+    const int kbe = p->form == 0 ? 64 : 32, nl = (p->lam1 < 0 ? p->n_lambda : p->lam1) - p->lam0;
+    a1.KA = p->Kx;
+    a1.NB = a1.NBm = a1.NBt = p->Kx / 128;
+    a1.nh = p->nh; a1.nhr = p->nhr;
+    a1.nkb = (p->nh + kbe - 1) / kbe * (p->form == 0 && p->box ? 3 : 1);
+    a1.NI = p->nhr / 128;
+    a1.lam_base = p->lam0;
+    // step 1: (lambda, k block, pupil-row block, C / S); step 2: (lambda, output tile)
+    a1.n_units = nl * a1.NB * a1.NI * (is_folded(mdft_kernel_form(p->form, p->box)) ? 2 : 1);
+    a2 = a1;
+    a2.KA = p->Ky; a2.NBm = p->Ky / 128;
+    a2.NBt = p->Kx / p->tile_n;
+    a2.n_units = a2.NBm * a2.NBt * nl;
+}
+
+extern "C" int gl_mdft_plan_pairs(const gl_mdft_plan* plan, int* step1, int* step2)
+{
+    using namespace gl;
+    if (!plan || !step1 || !step2) return fail(GL_ERR_INVALID, "mdft_plan_pairs: null argument");
+    const MdftPlan* p = plan->p;
+    MdftArgs a1{}, a2;
+    mdft_units(p, a1, a2);
+    const int gmax = p->ctas > 0 ? p->ctas : p->sms;
+    const bool field = p->form == 0 && !p->box;
+    *step1 = field ? mdft_pairs<0, 1, 128, false>(a1, gmax, p->pairs) : 0;
+    *step2 = field && p->tile_n == 128 ? mdft_pairs<0, 2, 128, false>(a2, gmax, p->pairs) : 0;
+    return GL_OK;
+}
+
 extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, float* d_out_r, float* d_out_g,
                                      float* d_out_b, int accumulate, int out_w, int out_h, int x0, int y0, int win_w,
                                      int win_h, const float* tint_rgb, void* stream)
@@ -1508,7 +1550,6 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
         x0 + win_w > out_w || y0 + win_h > out_h)
         return fail(GL_ERR_INVALID, "mdft_plan_execute: the output window must lie inside the planes and the plan");
     cudaStream_t st = (cudaStream_t)stream;
-    const int NBx = p->Kx / 128, NBy = p->Ky / 128;
     const size_t npx = (size_t)out_w * out_h;
     int launches = 0;
     // zeroing blocks: one wave of the chip at most, one block at least (the error
@@ -1535,13 +1576,7 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     ++launches;
     if (shared && !accumulate)
         for (float* c : planes) GL_CUDA_TRY(cudaMemsetAsync(c, 0, sizeof(float) * npx, st));
-    MdftArgs a;
-    a.KA = p->Kx; a.NBm = NBx; a.NBt = NBx;
-    a.nh = p->nh; a.nhr = p->nhr;
-    const int kbe = p->form == 0 ? 64 : 32;
-    const bool folded = is_folded(mdft_kernel_form(p->form, p->box));
-    a.nkb = (p->nh + kbe - 1) / kbe * (p->form == 0 && p->box ? 3 : 1);
-    a.NB = NBx; a.NI = p->nhr / 128;
+    MdftArgs a{}, a2;
     a.tprime = p->tprime; a.out_r = d_out_r; a.out_g = d_out_g; a.out_b = d_out_b;
     a.weights = p->weights; a.err = p->err; a.parts = p->parts;
     a.out_w = out_w; a.x0 = x0; a.y0 = y0; a.win_w = win_w; a.win_h = win_h;
@@ -1549,14 +1584,8 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     a.vec = ((out_w | x0) & 3) == 0 && ((reinterpret_cast<uintptr_t>(d_out_r) | reinterpret_cast<uintptr_t>(d_out_g) |
                                          reinterpret_cast<uintptr_t>(d_out_b)) & 15) == 0;
     a.tint = tint_rgb ? make_float4(tint_rgb[0], tint_rgb[1], tint_rgb[2], 0.0f) : make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    const int l0 = p->lam0, l1 = p->lam1 < 0 ? p->n_lambda : p->lam1, nl = l1 - l0;
-    a.lam_base = l0;
-    a.n_units = nl * NBx * a.NI * (folded ? 2 : 1);   // step 1: (lambda, k block, pupil-row block, C / S)
-    const int gmax = p->ctas > 0 ? p->ctas : p->sms;
-    MdftArgs a2 = a;
-    a2.KA = p->Ky; a2.NBm = NBy;
-    a2.NBt = p->Kx / p->tile_n;
-    a2.n_units = NBy * a2.NBt * nl;                     // step 2: (lambda, output tile)
+    const int gmax = p->ctas > 0 ? p->ctas : p->sms, l1 = p->lam1 < 0 ? p->n_lambda : p->lam1;
+    mdft_units(p, a, a2);
     if (p->form == 2)
     {
         GL_CUDA_TRY(p->box ? mdft_simt<true>(p, a, a2, l1, &launches, st) : mdft_simt<false>(p, a, a2, l1, &launches, st));

@@ -119,6 +119,12 @@ class MdftPlan:
         _native.check(self._lib.gl_mdft_plan_set_tile(self._h, int(tile)), "mdft")
         self.launch = (int(ctas), int(tile))
 
+    def cta_pairs(self):
+        """Pairs of CTAs the two GEMMs of the next execute run in (0: single CTAs)."""
+        a, b = C.c_int(), C.c_int()
+        _native.check(self._lib.gl_mdft_plan_pairs(self._h, C.byref(a), C.byref(b)), "mdft")
+        return int(a.value), int(b.value)
+
     def execute_raw(self, pupil_ptr: int, r_ptr: int, g_ptr: int, b_ptr: int, stream=None, accumulate=False):
         """execute on raw device addresses (planes owned by another component,
         e.g. a serving request); the caller guarantees the sizes."""

@@ -385,10 +385,14 @@ int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int M, int N, 
  *   E_l = W_y A W_x^T  (K_out x K_out),  out_c += weights_rgb[3l+c] |E_l|^2.
  * form 0: three-term split-BF16 products on tcgen05 with FP32 accumulation;
  * form 1: TF32 tcgen05.  n and K_out multiples of 128.  The DFT matrices are
- * built once (phase reduced in FP64) and stay resident in the plan.  The
- * pupil amplitude is n x n float32 on the device; outputs are K_out x K_out
- * planar float32, overwritten.  Asynchronous; gl_mdft_plan_status reads the
- * device error word (non-zero = a bounded pipeline wait gave up). */
+ * built once (phase reduced in two-float arithmetic) and stay resident in the
+ * plan.  The pupil amplitude is n x n float32 on the device; outputs are K_out x
+ * K_out planar float32, overwritten (the pupil is read before that, so it may lie
+ * in their memory).  Any float address will do for either.  The tcgen05 forms add
+ * the wavelengths of a pixel in any order, so runs may differ in the last bits;
+ * form 2 (FP32 on the CUDA cores) repeats bit for bit.  Asynchronous;
+ * gl_mdft_plan_status reads the device error word (non-zero = a bounded pipeline
+ * wait gave up). */
 typedef struct gl_mdft_plan gl_mdft_plan;
 int gl_mdft_plan_create(int n, int K_out, int n_lambda, const double* scale_x,
                         const double* scale_y, double center_x, double center_y,
@@ -416,6 +420,9 @@ int gl_mdft_plan_set_launch(gl_mdft_plan* plan, int ctas);
  * counterpart in the reference (its starburst contracts with SIMT dot
  * products, mdft_render.cu:137-172).  Results agree to float rounding. */
 int gl_mdft_plan_set_tile(gl_mdft_plan* plan, int tile_n);
+/* Pairs of CTAs (one product of 256 rows each) that the next execute's two GEMMs
+ * run in; 0 = single CTAs. */
+int gl_mdft_plan_pairs(const gl_mdft_plan* plan, int* step1, int* step2);
 /* Restrict the next executes to wavelengths [lam_begin, lam_end) (0, -1:
  * all): a large pattern enqueued as several short wavelength ranges (each
  * accumulating) frees its CTAs' SMs between the ranges, so a serving loop's
