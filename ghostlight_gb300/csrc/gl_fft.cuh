@@ -37,8 +37,8 @@ __device__ __forceinline__ float2 cis(float2 a, float sign) { return make_float2
 // a times the constant c + sign i s.  FINE: the constant in two floats each; one
 // rounded to one float is off by up to 3e-8 in every product with it, the same way
 // every time.  Error of a transform of 1024^2 noise against 64 bits 2.0e-7, FINE
-// 1.65e-7.  The sprite's transforms take it at no cost in time, so do short ones
-// (latency); the convolution's long ones would be 4 % slower (161 -> 168 us).
+// 1.65e-7.  The sprite's transforms take it (1 to 2 us each, code to fetch) and the
+// convolution's short ones; its long ones would be 4 % slower (161 -> 168 us).
 template <bool FINE>
 __device__ __forceinline__ float2 cmul_const(float2 a, double c, double s, float sign)
 {

@@ -55,3 +55,48 @@ def test_convolution(W, H, kw, kh, bound):
         want = torch.fft.irfft2(torch.fft.rfft2(i.double(), s=s) * K, s=s)[kh // 2:kh // 2 + H, kw // 2:kw // 2 + W]
         assert _off(o, want) < bound
     plan.close()
+
+
+def test_sprite_kernels_follow_each_other():
+    """Bakes and autocorrelations without a wait between them (their launches are set
+    up early) and in a graph, against the same with waits: equal bit for bit but for
+    the energy's last bits (its FP64 sum has no fixed order)."""
+    from ghostlight_gb300.starburst import SpritePlan
+    spec = np.array([[450.0, 0.2, 0.3, 0.5], [550.0, 0.4, 0.5, 0.1], [650.0, 0.6, 0.1, 0.0]], np.float32)
+    for N, ds in [(512, 64), (1024, 2), (2048, 4)]:
+        plan = SpritePlan(N, spec)
+        grids = [_noise(N + i, N, N).abs() for i in range(2)]
+        lags = [torch.empty((65, 65), device="cuda") for _ in range(2)]
+        want = []
+        for g, l in zip(grids, lags):
+            plan.bake(g, ds)
+            torch.cuda.synchronize()
+            want.append(plan.read()[:2])
+            plan.autocorr(g, 32, l)
+            torch.cuda.synchronize()
+            want[-1] += (l.clone(),)
+
+        def chain():
+            got = []
+            for g, l in zip(grids, lags):
+                l.fill_(7.0)
+                plan.autocorr(g, 32, l)
+                plan.bake(g, ds)
+                got.append(plan.read()[:2] + (l.clone(),))
+            return got
+
+        for _ in range(5):
+            for a, b in zip(chain(), want):
+                assert torch.equal(a[0], b[0])
+                for x, y in zip(a[1:], b[1:]):
+                    assert float((x - y).abs().max()) <= 2.0 ** -22 * float(y.abs().max())
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.graph(graph, stream=side):
+            plan.bake(grids[0], ds)
+            plan.autocorr(grids[1], 32, lags[1])
+        lags[1].fill_(7.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float((lags[1] - want[1][2]).abs().max()) <= 2.0 ** -22 * float(want[1][2].abs().max())
+        plan.close()
