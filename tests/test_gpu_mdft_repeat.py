@@ -68,3 +68,36 @@ def test_peak_of_two_level_sums():
         off.append(float(out[0][50, 64]) / A.astype(np.float64).sum() ** 2 - 1.0)
     assert np.sqrt(np.mean(np.square(off))) < 3.2e-7
     plan.close()
+
+
+@pytest.mark.parametrize("form", ["fp32", "split_bf16"])
+def test_in_a_graph(form):
+    """Captured calls, after a copy and after another kernel, and with the pupil in a
+    plane (memsets between the launches): what the calls give outside the graph."""
+    import ghostlight_gb300 as gl
+    n, K, L = 128, 384, 1 if form == "split_bf16" else 6
+    r = np.random.default_rng(5)
+    A = torch.from_numpy(r.random((n, n)).astype(np.float32)).cuda()
+    plan = gl.MdftPlan(n, K, np.linspace(0.6, 0.9, L) / K, np.linspace(0.5, 0.8, L) / K, r.random((L, 3)).astype(np.float32), form)
+    want = torch.empty((3, K, K), device="cuda")
+    plan.execute(A, *want)
+    op, out, buf = torch.empty_like(A), torch.empty_like(want), torch.empty_like(want)
+    inside = buf.view(-1)[K * K - 100:K * K - 100 + n * n].view(n, n)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        op.copy_(A)
+        plan.execute(op, *out)
+        plan.execute(op, *out, accumulate=True)
+        inside.copy_(A)
+        plan.execute(inside, *buf)
+    for _ in range(3):
+        op.zero_()
+        out.fill_(3.0)
+        buf.fill_(5.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(buf, want)
+        assert torch.equal(out, want + want)
+    plan.close()
