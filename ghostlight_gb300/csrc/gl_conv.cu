@@ -23,9 +23,9 @@
 //     row FFTs, the cropped W x H planes written from registers.
 // The kernel spectrum (normalisation 1/(PQ) folded in) is built once per plan
 // and stays resident.
-// 2048^2 x 3 (*) 257^2: 0.325 -> 0.160 ms (two planes packed in one complex
+// 2048^2 x 3 (*) 257^2: 0.325 -> 0.157 ms (two planes packed in one complex
 // transform, the third alone, ping-pong buffers, 18 warps per SM before); the
-// passes take 47, 73 and 45 us cold, issue slots half busy: bound by instruction
+// passes take 46, 73 and 43 us cold, issue slots half busy: bound by instruction
 // issue and fetch (each CTA runs a long straight line of code once), not by HBM
 // (15%) or shared memory (40%).  Passes 2 and 3 are launched while the pass before
 // them drains (gl_launch.cuh): 100^2 (*) 7^2, calls back to back, 20.5 -> 16 us (18.5
@@ -59,10 +59,10 @@ constexpr int kPairs = 2;          // row pairs per CTA in the row passes
 constexpr int kColsPerCta = 2;     // one column pair per CTA in the column pass
 constexpr int kConvThreads = 384;  // 3072 points, two transforms of them, 16 elements per thread
 // Ping-pong stages (gl_fft.cuh) up to this length, in place above.  Three
-// planes, ping-pong against in place: 162 x 486 points 20.7 / 39.1 us (the
-// first is the call's own time), 512 x 729 30.9 / 37.0, 972 x 972 55.4 / 51.3,
-// 2304 x 2304 175 / 161.
-constexpr int kShort = 800;
+// planes, calls back to back, ping-pong against in place: 162 x 486 points 18.4 /
+// 34.9 us, 512 x 512 22.6 / 28.8, 512 x 729 27.0 / 31.1, 768 x 768 37.0 / 30.8, 972 x
+// 972 52 / 45.
+constexpr int kShort = 740;
 
 struct ConvPlanes {
     const float* in[3];
