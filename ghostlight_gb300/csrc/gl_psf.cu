@@ -238,7 +238,9 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
 // Bound by the FP32 pipes in step 2 (64 FMA per 4 shared 16-byte loads); the
 // trace before it is most of the time left.  8 x 8 tiles of 64^2, 16
 // wavelengths, radius 13 (the default settings): 3.96 -> 0.35 ms for both
-// kernels.  The trace stays a kernel of its own (landings through a scratch
+// kernels.  Taps below 1e-6 of their splat, which psf_kernel<false> drops, are
+// kept: at most 3.7e-6 of a splat with a radius of 2.5 sigma (sigma 0.86 px), none
+// above 1.7 px.  The trace stays a kernel of its own (landings through a scratch
 // that fits L2): inlined here it rounded some landings differently.
 constexpr int kDenseChunk = 32;       // landings per outer-product step
 constexpr size_t kDenseLandings = (size_t)4 << 20;   // 64 MB: stays in L2 between the two kernels

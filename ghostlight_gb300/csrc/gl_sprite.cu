@@ -47,7 +47,7 @@ struct StarSource { float px, py, r, g, b; };
 // N = 2048 with a pupil of 0.3 of it: rows then columns of the full complex
 // spectrum took 28 + 110 us (139 KB of shared memory and 8 warps per CTA, one
 // CTA per SM, 16-byte pieces of each row), the half spectrum's two passes
-// 17 + 18 us.
+// 19 + 20 us.
 constexpr int kShortGrid = 1024;    // ping-pong stages up to here, in place above (gl_fft.cuh)
 
 // Half spectrum of the first pass: column x, row ky <= N / 2 at

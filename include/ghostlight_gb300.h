@@ -494,9 +494,10 @@ int gl_survivor_envelope(const gl_surface* surfaces, int n, float lambda, const 
  * this path (its veil is an analytic glare-spread sprite splatted per source,
  * veil_render.cu:94-243); this is the flare path's image-space form.  FFT
  * route: zero-padded circular convolution of size P x Q = the smallest
- * 2^a 3^b sizes covering image + kernel - 1, two channels per complex
- * transform, three HBM passes; the kernel spectrum stays resident in the
- * plan.  Planes are W x H float32 on the device.  Asynchronous. */
+ * 2^a 3^b sizes covering image + kernel - 1, two rows of a plane per complex
+ * transform (half spectra), three passes; the kernel spectrum, made in FP64,
+ * stays resident in the plan.  Planes are W x H float32 on the device; outputs
+ * may be the inputs.  Asynchronous. */
 typedef struct gl_conv_plan gl_conv_plan;
 int gl_conv2d_plan_create(int width, int height, const float* h_kernel, int kw, int kh,
                           void* stream, gl_conv_plan** out);
