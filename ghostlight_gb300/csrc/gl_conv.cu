@@ -327,87 +327,11 @@ __global__ void __launch_bounds__(PP ? 512 : kConvThreads, PP ? 2 : 3) conv_rows
 // ---- kernel spectrum, once per plan ----------------------------------------------
 // In FP64 and rounded once: a third of the rounding of forward transform, product
 // and inverse was the kernel's own float transform, the same in every call (noise, 2048^2
-// (*) 257^2: 3.7e-7 off 64 bits with it, 2.8e-7 without).  Stockham stages
-// of radix 4, 3, 2 between two arrays in global memory, one thread a butterfly.
-
-// Rows of the kernel, its centre at column 0, wrapped.
-__global__ void spec_place(const float* __restrict__ k, int kw, int kh, int Q, double norm, double2* __restrict__ a)
-{
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (size_t)kh * Q) return;
-    const int u = (int)(t / Q), c = (int)(t - (size_t)u * Q), v = (c + kw / 2) % Q;
-    a[t] = make_double2(v < kw ? (double)k[(size_t)u * kw + v] * norm : 0.0, 0.0);
-}
-
-// The rows' spectra to P rows, the centre row at row 0, wrapped; columns past Q / 2 zero.
-__global__ void spec_turn(const double2* __restrict__ a, int kh, int Q, int P, int cols, double2* __restrict__ b)
-{
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (size_t)P * cols) return;
-    const int y = (int)(t / cols), q = (int)(t - (size_t)y * cols), u = (y + kh / 2) % P;
-    b[t] = (u < kh && q <= Q / 2) ? a[(size_t)u * Q + q] : make_double2(0.0, 0.0);
-}
-
-// To the column pairs of the intermediate (pair_index).
-__global__ void spec_store(const double2* __restrict__ b, int P, int cols, int k_rows, float2* __restrict__ khat)
-{
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (size_t)P * cols) return;
-    const int y = (int)(t / cols), q = (int)(t - (size_t)y * cols);
-    const double2 v = b[t];
-    khat[((size_t)(q >> 1) * k_rows + y) * 2 + (q & 1)] = make_float2((float)v.x, (float)v.y);
-}
-
-// One stage over nseq sequences; element i of sequence s at i es + s ss (one of
-// the strides is 1).  tw: exp(-2 pi i t / n), t < n.
-template <int R>
-__global__ void spec_stage(const double2* __restrict__ x, double2* __restrict__ y, int n, int Ls, int nseq, size_t es, size_t ss,
-                           const double2* __restrict__ tw)
-{
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int m = n / R;
-    if (t >= (size_t)m * nseq) return;
-    const int s = es == 1 ? (int)(t / m) : (int)(t % nseq), j = es == 1 ? (int)(t % m) : (int)(t / nseq);
-    const int g = j / Ls, k = j - g * Ls;
-    double2 v[R];
-    #pragma unroll
-    for (int q = 0; q < R; ++q)
-    {
-        const double2 a = x[(j + (size_t)q * m) * es + s * ss], w = tw[q * k * (m / Ls)];
-        v[q] = make_double2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
-    }
-    #pragma unroll
-    for (int p = 0; p < R; ++p)
-    {
-        double2 o = v[0];
-        #pragma unroll
-        for (int q = 1; q < R; ++q)
-        {
-            const double2 w = tw[p * q % R * m];
-            o.x += v[q].x * w.x - v[q].y * w.y;
-            o.y += v[q].x * w.y + v[q].y * w.x;
-        }
-        y[((size_t)g * Ls * R + k + (size_t)p * Ls) * es + s * ss] = o;
-    }
-}
-
-inline unsigned spec_blocks(size_t threads) { return (unsigned)((threads + 255) / 256); }
-
-// All stages of one axis; leaves the result's array in x.
-void spec_axis(double2*& x, double2*& y, int n, int nseq, size_t es, size_t ss, const double2* tw, cudaStream_t st)
-{
-    int Ls = 1;
-    while (Ls < n)
-    {
-        const int left = n / Ls, R = left % 4 == 0 ? 4 : (left % 2 == 0 ? 2 : 3);
-        const unsigned blocks = spec_blocks((size_t)(n / R) * nseq);
-        if (R == 4) spec_stage<4><<<blocks, 256, 0, st>>>(x, y, n, Ls, nseq, es, ss, tw);
-        else if (R == 3) spec_stage<3><<<blocks, 256, 0, st>>>(x, y, n, Ls, nseq, es, ss, tw);
-        else spec_stage<2><<<blocks, 256, 0, st>>>(x, y, n, Ls, nseq, es, ss, tw);
-        std::swap(x, y);
-        Ls *= R;
-    }
-}
+// (*) 257^2: 3.7e-7 off 64 bits with it, 2.8e-7 without).  One CTA a row of the
+// kernel, then one a column: Stockham stages of radix 4, 3, 2 between two arrays
+// in shared memory.  A plan for 2304^2 points takes the time it took with the float
+// transform (3.2 ms, most of it the tables).
+constexpr int kSpecThreads = 256;
 
 // exp(-2 pi i t / n), t < n
 __global__ void spec_circle(int n, double2* __restrict__ tw)
@@ -417,6 +341,89 @@ __global__ void spec_circle(int n, double2* __restrict__ tw)
     double s, c;
     sincospi(2.0 * (double)t / (double)n, &s, &c);
     tw[t] = make_double2(c, -s);
+}
+
+template <int R>
+__device__ __forceinline__ void spec_stage(const double2* x, double2* y, int n, int Ls, const double2* __restrict__ tw)
+{
+    const int m = n / R;
+    for (int j = threadIdx.x; j < m; j += kSpecThreads)
+    {
+        const int g = j / Ls, k = j - g * Ls;
+        double2 v[R];
+        #pragma unroll
+        for (int q = 0; q < R; ++q)
+        {
+            const double2 a = x[j + q * m], w = tw[q * k * (m / Ls)];
+            v[q] = make_double2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+        }
+        #pragma unroll
+        for (int p = 0; p < R; ++p)
+        {
+            double2 o = v[0];
+            #pragma unroll
+            for (int q = 1; q < R; ++q)
+            {
+                const double2 w = tw[p * q % R * m];
+                o.x += v[q].x * w.x - v[q].y * w.y;
+                o.y += v[q].x * w.y + v[q].y * w.x;
+            }
+            y[g * Ls * R + k + p * Ls] = o;
+        }
+    }
+    __syncthreads();
+}
+
+// The transform of x; returns the array that holds it (x or y).
+__device__ const double2* spec_fft(double2* x, double2* y, int n, const double2* __restrict__ tw)
+{
+    __syncthreads();
+    for (int Ls = 1; Ls < n;)
+    {
+        const int left = n / Ls, R = left % 4 == 0 ? 4 : (left % 2 == 0 ? 2 : 3);
+        if (R == 4) spec_stage<4>(x, y, n, Ls, tw);
+        else if (R == 3) spec_stage<3>(x, y, n, Ls, tw);
+        else spec_stage<2>(x, y, n, Ls, tw);
+        double2* t = x;
+        x = y;
+        y = t;
+        Ls *= R;
+    }
+    return x;
+}
+
+// Row blockIdx.x of the kernel, its centre at column 0, wrapped: its half spectrum
+// (cols of them, zero past Q / 2).
+__global__ void __launch_bounds__(kSpecThreads) spec_rows(const float* __restrict__ k, int kw, int Q, int cols, double norm,
+                                                          const double2* __restrict__ tw, double2* __restrict__ a)
+{
+    extern __shared__ double2 arrays[];
+    const float* row = k + (size_t)blockIdx.x * kw;
+    for (int c = threadIdx.x; c < Q; c += kSpecThreads)
+    {
+        const int v = (c + kw / 2) % Q;
+        arrays[c] = make_double2(v < kw ? (double)row[v] * norm : 0.0, 0.0);
+    }
+    const double2* r = spec_fft(arrays, arrays + Q, Q, tw);
+    for (int q = threadIdx.x; q < cols; q += kSpecThreads)
+        a[(size_t)blockIdx.x * cols + q] = q <= Q / 2 ? r[q] : make_double2(0.0, 0.0);
+}
+
+// Column blockIdx.x of the rows' spectra, the centre row at row 0, wrapped: its
+// transform to the column pairs of the intermediate (pair_index).
+__global__ void __launch_bounds__(kSpecThreads) spec_cols(const double2* __restrict__ a, int kh, int P, int cols, int k_rows,
+                                                          const double2* __restrict__ tw, float2* __restrict__ khat)
+{
+    extern __shared__ double2 arrays[];
+    const int q = blockIdx.x;
+    for (int y = threadIdx.x; y < P; y += kSpecThreads)
+    {
+        const int u = (y + kh / 2) % P;
+        arrays[y] = u < kh ? a[(size_t)u * cols + q] : make_double2(0.0, 0.0);
+    }
+    const double2* r = spec_fft(arrays, arrays + P, P, tw);
+    for (int y = threadIdx.x; y < P; y += kSpecThreads)
+        khat[((size_t)(q >> 1) * k_rows + y) * 2 + (q & 1)] = make_float2((float)r[y].x, (float)r[y].y);
 }
 
 int good_size(int need)
@@ -467,27 +474,24 @@ static void conv_free(ConvPlan* p)
 // 'same'-aligned; 1 / (P Q) folded in) into p->khat.
 static cudaError_t conv_spectrum(const ConvPlan* p, const float* h_kernel, cudaStream_t st)
 {
-    const size_t nk = (size_t)p->KH * p->KW, cols = 2 * (size_t)p->G;
-    const size_t cells = std::max((size_t)p->KH * p->Q, (size_t)p->P * cols);
-    const size_t k_at = sizeof(double2) * (2 * cells + (size_t)p->Q + p->P);
-    char* block = nullptr;         // two arrays, the circles of both axes, the kernel
+    const size_t nk = (size_t)p->KH * p->KW, cols = 2 * (size_t)p->G, cells = p->KH * cols;
+    const size_t k_at = sizeof(double2) * (cells + (size_t)p->Q + p->P);
+    const size_t smem_q = 2 * sizeof(double2) * p->Q, smem_p = 2 * sizeof(double2) * p->P;
+    char* block = nullptr;         // the rows' spectra, the circles of both axes, the kernel
     cudaError_t e = cudaMalloc(&block, k_at + sizeof(float) * nk);
     auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-    double2 *x = reinterpret_cast<double2*>(block), *y = x + cells, *twq = y + cells, *twp = twq + p->Q;
+    double2 *a = reinterpret_cast<double2*>(block), *twq = a + cells, *twp = twq + p->Q;
     float* k = reinterpret_cast<float*>(block + k_at);
+    if (e == cudaSuccess) chk((cudaError_t)raise_smem_limit((const void*)spec_rows, smem_q));
+    if (e == cudaSuccess) chk((cudaError_t)raise_smem_limit((const void*)spec_cols, smem_p));
     if (e == cudaSuccess) chk(cudaMemcpyAsync(k, h_kernel, sizeof(float) * nk, cudaMemcpyHostToDevice, st));
     if (e == cudaSuccess)
     {
-        double2 *a = x, *b = y;
         const double norm = 1.0 / ((double)p->P * (double)p->Q);
-        spec_circle<<<spec_blocks((size_t)p->Q), 256, 0, st>>>(p->Q, twq);
-        spec_circle<<<spec_blocks((size_t)p->P), 256, 0, st>>>(p->P, twp);
-        spec_place<<<spec_blocks((size_t)p->KH * p->Q), 256, 0, st>>>(k, p->KW, p->KH, p->Q, norm, a);
-        spec_axis(a, b, p->Q, p->KH, 1, (size_t)p->Q, twq, st);
-        spec_turn<<<spec_blocks((size_t)p->P * cols), 256, 0, st>>>(a, p->KH, p->Q, p->P, (int)cols, b);
-        std::swap(a, b);
-        spec_axis(a, b, p->P, (int)cols, cols, 1, twp, st);
-        spec_store<<<spec_blocks((size_t)p->P * cols), 256, 0, st>>>(a, p->P, (int)cols, p->k_rows, p->khat);
+        spec_circle<<<(p->Q + 255) / 256, 256, 0, st>>>(p->Q, twq);
+        spec_circle<<<(p->P + 255) / 256, 256, 0, st>>>(p->P, twp);
+        spec_rows<<<p->KH, kSpecThreads, smem_q, st>>>(k, p->KW, p->Q, (int)cols, norm, twq, a);
+        spec_cols<<<(unsigned)cols, kSpecThreads, smem_p, st>>>(a, p->KH, p->P, (int)cols, p->k_rows, twp, p->khat);
         chk(cudaGetLastError());
     }
     chk(cudaStreamSynchronize(st));
