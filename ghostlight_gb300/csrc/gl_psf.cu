@@ -23,6 +23,8 @@ namespace gl {
 namespace {
 
 constexpr int kPsfThreads = 256;
+constexpr float kTapMin = 1e-6f;        // taps of less of their splat are left out
+constexpr float kDepositMin = 1e-14f;   // colour times weight up to which a plane takes nothing of a ray
 
 struct PsfArgs {
     const SurfRec* recs;
@@ -57,25 +59,25 @@ __device__ __forceinline__ void deposit(const PsfArgs& A, float* tile, int tx, i
         const int t = ty * A.tile_w + tx, plane = A.tile_w * A.tile_h;
         if (A.mono)
         {
-            if (fabsf(lum) > 1e-14f) atomicAdd(tile + t, lum * wt);
+            if (fabsf(lum) > kDepositMin) atomicAdd(tile + t, lum * wt);
         }
         else
         {
-            if (fabsf(cr) > 1e-14f) atomicAdd(tile + t, cr * wt);
-            if (fabsf(cg) > 1e-14f) atomicAdd(tile + plane + t, cg * wt);
-            if (fabsf(cb) > 1e-14f) atomicAdd(tile + 2 * plane + t, cb * wt);
+            if (fabsf(cr) > kDepositMin) atomicAdd(tile + t, cr * wt);
+            if (fabsf(cg) > kDepositMin) atomicAdd(tile + plane + t, cg * wt);
+            if (fabsf(cb) > kDepositMin) atomicAdd(tile + 2 * plane + t, cb * wt);
         }
         return;
     }
     if (A.mono)
     {
-        if (fabsf(lum) > 1e-14f) atomicAdd(A.out_r + pix, lum * wt);
+        if (fabsf(lum) > kDepositMin) atomicAdd(A.out_r + pix, lum * wt);
     }
     else
     {
-        if (fabsf(cr) > 1e-14f) atomicAdd(A.out_r + pix, cr * wt);
-        if (fabsf(cg) > 1e-14f) atomicAdd(A.out_g + pix, cg * wt);
-        if (fabsf(cb) > 1e-14f) atomicAdd(A.out_b + pix, cb * wt);
+        if (fabsf(cr) > kDepositMin) atomicAdd(A.out_r + pix, cr * wt);
+        if (fabsf(cg) > kDepositMin) atomicAdd(A.out_g + pix, cg * wt);
+        if (fabsf(cb) > kDepositMin) atomicAdd(A.out_b + pix, cb * wt);
     }
 }
 
@@ -212,7 +214,7 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
                     if (xi < tx_min || xi >= tx_max || xi < 0 || xi >= A.comp_w) continue;
                     const float dxr = (float)dx - ox;
                     const float wt = expf(-(dxr * dxr + dyr * dyr) * inv2) * inv_wsum;
-                    if (wt < 1e-6f) continue;
+                    if (wt < kTapMin) continue;
                     deposit(A, tile, xi - S.tile_x0, yi - S.tile_y0, yi * A.comp_w + xi, lum, cr, cg, cb, wt);
                 }
             }
@@ -238,9 +240,8 @@ __device__ __forceinline__ void psf_trace_one(const PsfArgs& A, const SurfRec* l
 // Bound by the FP32 pipes in step 2 (64 FMA per 4 shared 16-byte loads); the
 // trace before it is most of the time left.  8 x 8 tiles of 64^2, 16
 // wavelengths, radius 13 (the default settings): 3.96 -> 0.35 ms for both
-// kernels.  Taps below 1e-6 of their splat, which psf_kernel<false> drops, are
-// kept: at most 3.7e-6 of a splat with a radius of 2.5 sigma (sigma 0.86 px), none
-// above 1.7 px.  The trace stays a kernel of its own (landings through a scratch
+// kernels.  Taps and rays that are too faint are left out as psf_kernel<false>
+// leaves them out.  The trace stays a kernel of its own (landings through a scratch
 // that fits L2): inlined here it rounded some landings differently.
 constexpr int kDenseChunk = 32;       // landings per outer-product step
 constexpr size_t kDenseLandings = (size_t)4 << 20;   // 64 MB: stays in L2 between the two kernels
@@ -268,6 +269,10 @@ inline size_t dense_smem_floats(const DenseGeom& g, int rounds)
     return 4 * (size_t)rounds * kPsfThreads + std::max(rows, plane);
 }
 
+// CUT: taps below kTapMin of their splat are left out one by one, as the tap kernel
+// leaves them out (a window much wider than 2.5 sigma has such taps): three
+// instructions per pixel and landing in place of one.
+template <bool CUT>
 __global__ void __launch_bounds__(kPsfThreads, 2) psf_dense_kernel(PsfArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -284,111 +289,150 @@ __global__ void __launch_bounds__(kPsfThreads, 2) psf_dense_kernel(PsfArgs A)
     const gl_psf_source S = A.src[si];
     const float4 sp = A.spec[l];
     const int R = A.radius_px;
+    const int planes = A.mono ? 1 : 3;
+    const float lum = (S.r + S.g + S.b) * (1.0f / 3.0f) * sp.z;
+    const float c[3] = {A.mono ? lum : S.r * sp.y, A.mono ? 0.0f : S.g * sp.z, A.mono ? 0.0f : S.b * sp.w};
     const float4* land = A.land + ((size_t)blockIdx.x * A.n_land + blockIdx.y) * A.n_grid;
+    // a plane takes nothing of a ray that is too faint in it; where that differs
+    // between planes (a dim source, the end of the spectrum) each has its own pass
+    int mixed = 0;
     for (int q = 0; q < A.rounds; ++q)
     {
         const int gi = (blockIdx.z * A.rounds + q) * kPsfThreads + tid;
         float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (gi < A.n_grid) e = land[gi];
-        const bool in = e.w != 0.0f;
+        int seen = 0, faint = 0;
+        #pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            const bool takes = fabsf(c[k] * e.z) > kDepositMin;
+            seen |= takes;
+            faint |= fabsf(c[k]) > 0.0f && !takes;
+        }
+        const bool in = e.w != 0.0f && seen;
+        mixed |= in && faint;
         const unsigned m = __ballot_sync(0xffffffffu, in);
         int base = 0;
         if (lane == 0 && m) base = atomicAdd(&n_list, __popc(m));
         base = __shfl_sync(0xffffffffu, base, 0);
         if (in) list[base + __popc(m & ((1u << lane) - 1u))] = e;
     }
-    __syncthreads();
+    mixed = __syncthreads_or(mixed);
     const int n = n_list;
     if (n == 0) return;
     const float inv2 = 1.0f / (2.0f * A.sigma_px * A.sigma_px);
     const int per = G.tx * G.ty, grp = tid / per, cell = tid - grp * per;
     const int mx = (cell % G.tx) * 8, my = (cell / G.tx) * 8;
-    float acc[8][8] = {};
-    for (int c0 = 0; c0 < n; c0 += kDenseChunk)
+    #pragma unroll 1
+    for (int p0 = 0; p0 < (mixed ? planes : 1); ++p0)
     {
-        const int cnt = min(kDenseChunk, n - c0);
-        for (int r = warp; r < cnt; r += kPsfThreads / 32)
+        const float cp = p0 == 0 ? c[0] : (p0 == 1 ? c[1] : c[2]);
+        float acc[8][8] = {};
+        for (int c0 = 0; c0 < n; c0 += kDenseChunk)
         {
-            const float4 e = list[c0 + r];
-            const int cx = (int)floorf(e.x), cy = (int)floorf(e.y);
-            const float ox = e.x - ((float)cx + 0.5f), oy = e.y - ((float)cy + 0.5f);
-            // window offset of this lane: R <= 16, at most 33 entries per axis
-            float wx = 0.0f, wy = 0.0f;
-            for (int d = lane - R; d <= R; d += 32)
+            const int cnt = min(kDenseChunk, n - c0);
+            for (int r = warp; r < cnt; r += kPsfThreads / 32)
             {
-                const float dx = (float)d - ox, dy = (float)d - oy;
-                wx += expf(-(dx * dx) * inv2);
-                wy += expf(-(dy * dy) * inv2);
+                const float4 e = list[c0 + r];
+                const int cx = (int)floorf(e.x), cy = (int)floorf(e.y);
+                const float ox = e.x - ((float)cx + 0.5f), oy = e.y - ((float)cy + 0.5f);
+                // window offset of this lane: R <= 16, at most 33 entries per axis
+                float wx = 0.0f, wy = 0.0f;
+                for (int d = lane - R; d <= R; d += 32)
+                {
+                    const float dx = (float)d - ox, dy = (float)d - oy;
+                    wx += expf(-(dx * dx) * inv2);
+                    wy += expf(-(dy * dy) * inv2);
+                }
+                #pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                {
+                    wx += __shfl_xor_sync(0xffffffffu, wx, o);
+                    wy += __shfl_xor_sync(0xffffffffu, wy, o);
+                }
+                const float ws = wx * wy;
+                const bool seen = ws > 1e-20f && (!mixed || fabsf(cp * e.z) > kDepositMin);
+                const float amp = !seen ? 0.0f : (CUT ? 1.0f / ws : e.z / ws);
+                const int lx = cx - S.tile_x0, ly = cy - S.tile_y0;
+                for (int i = lane; i < W8; i += 32)
+                {
+                    const float dx = (float)(i - lx) - ox;
+                    gx[r * W8 + i] = (i < A.tile_w && abs(i - lx) <= R) ? expf(-(dx * dx) * inv2) : 0.0f;
+                }
+                for (int i = lane; i < H8; i += 32)
+                {
+                    const float dy = (float)(i - ly) - oy;
+                    gy[r * H8 + i] = (i < A.tile_h && abs(i - ly) <= R) ? expf(-(dy * dy) * inv2) * amp : 0.0f;
+                }
             }
-            #pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
+            __syncthreads();
+            if (grp < G.groups)
             {
-                wx += __shfl_xor_sync(0xffffffffu, wx, o);
-                wy += __shfl_xor_sync(0xffffffffu, wy, o);
+                for (int r = grp; r < cnt; r += G.groups)
+                {
+                    const float4* px = reinterpret_cast<const float4*>(gx + r * W8 + mx);
+                    const float4* py = reinterpret_cast<const float4*>(gy + r * H8 + my);
+                    const float4 x0 = px[0], x1 = px[1], y0 = py[0], y1 = py[1];
+                    const float vx[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+                    const float vy[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+                    const float w = CUT ? list[c0 + r].z : 0.0f;
+                    #pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        #pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                        {
+                            if (!CUT) acc[j][i] = fmaf(vy[j], vx[i], acc[j][i]);
+                            else
+                            {
+                                const float t = vy[j] * vx[i];
+                                if (t >= kTapMin) acc[j][i] = fmaf(t, w, acc[j][i]);
+                            }
+                        }
+                }
             }
-            const float ws = wx * wy;
-            const float amp = ws > 1e-20f ? e.z / ws : 0.0f;
-            const int lx = cx - S.tile_x0, ly = cy - S.tile_y0;
-            for (int i = lane; i < W8; i += 32)
-            {
-                const float dx = (float)(i - lx) - ox;
-                gx[r * W8 + i] = (i < A.tile_w && abs(i - lx) <= R) ? expf(-(dx * dx) * inv2) : 0.0f;
-            }
-            for (int i = lane; i < H8; i += 32)
-            {
-                const float dy = (float)(i - ly) - oy;
-                gy[r * H8 + i] = (i < A.tile_h && abs(i - ly) <= R) ? expf(-(dy * dy) * inv2) * amp : 0.0f;
-            }
+            __syncthreads();
         }
-        __syncthreads();
-        if (grp < G.groups)
+        // sum of the groups, in order, in the rows' place (the loop ended on a barrier)
+        float* sum = gx;
+        for (int g = 0; g < G.groups; ++g)
         {
-            for (int r = grp; r < cnt; r += G.groups)
+            if (grp == g)
             {
-                const float4* px = reinterpret_cast<const float4*>(gx + r * W8 + mx);
-                const float4* py = reinterpret_cast<const float4*>(gy + r * H8 + my);
-                const float4 x0 = px[0], x1 = px[1], y0 = py[0], y1 = py[1];
-                const float vx[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-                const float vy[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
                 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[j][i] = fmaf(vy[j], vx[i], acc[j][i]);
+                    for (int i = 0; i < 8; ++i)
+                    {
+                        float* q = sum + (my + j) * W8 + mx + i;
+                        *q = g == 0 ? acc[j][i] : *q + acc[j][i];
+                    }
             }
+            __syncthreads();
         }
-        __syncthreads();
-    }
-    // sum of the groups, in order, in the rows' place (the loop ended on a barrier)
-    float* sum = gx;
-    for (int g = 0; g < G.groups; ++g)
-    {
-        if (grp == g)
+        float* const outs[3] = {A.out_r, A.out_g, A.out_b};
+        for (int t = tid; t < A.tile_w * A.tile_h; t += kPsfThreads)
         {
+            const int y = t / A.tile_w, x = t - y * A.tile_w;
+            const int xi = S.tile_x0 + x, yi = S.tile_y0 + y;
+            if (xi < 0 || xi >= A.comp_w || yi < 0 || yi >= A.comp_h) continue;
+            const float v = sum[y * W8 + x];
+            if (v == 0.0f) continue;
             #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                {
-                    float* q = sum + (my + j) * W8 + mx + i;
-                    *q = g == 0 ? acc[j][i] : *q + acc[j][i];
-                }
+            for (int pl = 0; pl < 3; ++pl)
+                if ((!mixed || pl == p0) && fabsf(c[pl]) > 0.0f) atomicAdd(outs[pl] + (size_t)yi * A.comp_w + xi, c[pl] * v);
         }
         __syncthreads();
     }
-    const float lum = (S.r + S.g + S.b) * (1.0f / 3.0f) * sp.z;
-    const float c[3] = {A.mono ? lum : S.r * sp.y, S.g * sp.z, S.b * sp.w};
-    float* outs[3] = {A.out_r, A.out_g, A.out_b};
-    const int planes = A.mono ? 1 : 3;
-    for (int t = tid; t < A.tile_w * A.tile_h; t += kPsfThreads)
-    {
-        const int y = t / A.tile_w, x = t - y * A.tile_w;
-        const int xi = S.tile_x0 + x, yi = S.tile_y0 + y;
-        if (xi < 0 || xi >= A.comp_w || yi < 0 || yi >= A.comp_h) continue;
-        const float v = sum[y * W8 + x];
-        if (v == 0.0f) continue;
-        for (int pl = 0; pl < planes; ++pl)
-            if (fabsf(c[pl]) > 0.0f) atomicAdd(outs[pl] + (size_t)yi * A.comp_w + xi, c[pl] * v);
-    }
+}
+
+// Whether a landing's window may hold taps below kTapMin: its corner, seen from
+// the far end of the centre pixel.
+inline bool faint_taps(float sigma_px, int radius_px)
+{
+    const double inv2 = 0.5 / ((double)sigma_px * sigma_px), far = radius_px + 0.5;
+    double wx = 0.0;
+    for (int d = -radius_px; d <= radius_px; ++d) wx += std::exp(-(d + 0.5) * (d + 0.5) * inv2);
+    return !(std::exp(-2.0 * far * far * inv2) >= 1.01 * (double)kTapMin * wx * wx);
 }
 
 // The dense kernel pays for the whole tile per landing, the sparse one for the
@@ -507,8 +551,9 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
     const size_t smem = recs.size() * sizeof(SurfRec) + at.size() * sizeof(float) + (tile_smem && !dense ? tile_bytes + 16 : 0);
     if (e == cudaSuccess && smem > 48 * 1024)
         e = (cudaError_t)raise_smem_limit(dense ? (const void*)psf_kernel<true> : (const void*)psf_kernel<false>, smem);
+    auto dense_kernel = faint_taps(splat_sigma_px, splat_radius_px) ? psf_dense_kernel<true> : psf_dense_kernel<false>;
     if (e == cudaSuccess && dense && dense_smem > 47 * 1024)   // the kernel has a static word besides
-        e = (cudaError_t)raise_smem_limit((const void*)psf_dense_kernel, dense_smem);
+        e = (cudaError_t)raise_smem_limit((const void*)dense_kernel, dense_smem);
     int launches = dense ? 0 : 1;
     if (e == cudaSuccess)
     {
@@ -542,7 +587,7 @@ static int psf_render_impl(const gl_surface* surfaces, int n_surfaces, const gl_
                 const int parts = (int)std::min<long long>(A.n_land, std::max(1LL, (want + ctas - 1) / ctas));
                 const int per = (A.n_land + parts - 1) / parts;
                 psf_kernel<true><<<dim3(ns, blocks, (unsigned)((A.n_land + per - 1) / per)), kPsfThreads, smem, st>>>(A);
-                psf_dense_kernel<<<dim3(ns, (unsigned)A.n_land, (unsigned)dense_z(rounds)), kPsfThreads, dense_smem, st>>>(A);
+                dense_kernel<<<dim3(ns, (unsigned)A.n_land, (unsigned)dense_z(rounds)), kPsfThreads, dense_smem, st>>>(A);
                 launches += 2;
             }
         e = cudaGetLastError();

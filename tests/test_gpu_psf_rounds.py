@@ -1,6 +1,6 @@
 """A wide splat's landings in several rounds over sources and wavelengths, and the
-atlas without them (each ray its own taps): the same terms in another order.
-Taps below 1e-6 of their splat are in the former only: at most 1e-5 of it at 2 px."""
+atlas without them (each ray its own taps): the same terms in another order, over
+windows wider than the splat needs, tiles off the composite and dim sources too."""
 import numpy as np
 import pytest
 
@@ -54,3 +54,63 @@ def test_more_landings_than_the_scratch():
             y, x = i // 8 * 32, i % 8 * 32
             a, b = out[k][y:y + 32, x:x + 32].double(), one[k].double()
             assert float(b.max()) > 0 and float((a - b).norm() / b.norm()) < 1e-6
+
+
+def _pair(inp):
+    """(with landings, taps) as float64 planes."""
+    from ghostlight_gb300.psf_grid import psf_launch
+    got = []
+    for landing_bytes in (None, 0):
+        out = torch.zeros((3, inp["comp_h"], inp["comp_w"]), device="cuda")
+        psf_launch(inp, out, torch.cuda.current_stream().cuda_stream, ordered=True, landing_bytes=landing_bytes)
+        torch.cuda.synchronize()
+        got.append((out.double(), __import__("ghostlight_gb300")._native.last_launch_count()))
+    assert got[0][1] == 2 and got[1][1] == 1          # landings and tiles; taps
+    return got[0][0], got[1][0]
+
+
+# radii of the splat (2.5 sigma: with and without taps below 1e-6) and beyond it;
+# float32 sums of some thousand terms in other orders, and taps within rounding of
+# the line on the other side of it, 1e-6 of a splat each
+@pytest.mark.parametrize("sigma,radius", [(0.85, 3), (1.1, 3), (1.25, 4), (1.62, 5), (5.12, 13), (0.3, 16), (0.9, 14), (1.5, 10),
+                                          (3.0, 16), (7.0, 4)])
+@pytest.mark.parametrize("mono", [False, True])
+def test_windows_equal_taps(sigma, radius, mono):
+    import ghostlight_gb300 as gl
+    from ghostlight_gb300 import prescriptions as P
+    from ghostlight_gb300.psf_grid import psf_inputs
+    lens = gl.OpticalSystem(P.double_gauss_12(seed=1))
+    src = np.array([[0.02 * i, 0.01 * i, 1.0, 0.8, -0.2 * i] for i in range(4)], np.float32)
+    cfg = gl.PSFConfig(grid_nx=2, grid_ny=2, tile_w=43, tile_h=30, tile_extent_mm=0.1, ray_grid=24, spectral_samples=5,
+                       monochromatic=mono)
+    inp = psf_inputs(src, lens, cfg)
+    inp["sigma"], inp["radius"] = sigma, radius
+    inp["sources"][1].tile_x0, inp["sources"][1].tile_y0 = 60, -7          # partly off the composite
+    a, b = _pair(inp)
+    assert float(b.abs().max()) > 0
+    assert float((a - b).norm() / b.norm()) < 2e-6
+
+
+def test_dim_sources_equal_taps():
+    """Colours around which a ray's share in a plane passes 1e-14, the least that a
+    plane takes: in all planes, in some, in none."""
+    import ghostlight_gb300 as gl
+    from ghostlight_gb300 import prescriptions as P
+    from ghostlight_gb300.psf_grid import psf_inputs
+    s = P.double_gauss_12(seed=1)
+    # weights over five decades: an attenuator's Gaussian
+    s[2].coating_model, s[2].gauss_sigma, s[2].gauss_background, s[2].gauss_peak = 4, 4.0, 1e-5, 1.0
+    lens = gl.OpticalSystem(s)
+    src = np.array([[0.0, 0.0, 1e-9, 1e-11, 1e-13], [0.02, 0.0, 1e-8, 1e-8, 1e-8], [0.0, 0.02, 1e-15, 1e-16, 0.0],
+                    [0.02, 0.02, 1e-10, 0.0, 1e-3]], np.float32)
+    cfg = gl.PSFConfig(grid_nx=2, grid_ny=2, tile_w=40, tile_h=40, tile_extent_mm=0.1, ray_grid=32, spectral_samples=9)
+    inp = psf_inputs(src, lens, cfg)
+    inp["sigma"], inp["radius"] = 2.0, 5
+    a, b = _pair(inp)
+    for k in range(3):
+        for y in (0, 40):
+            for x in (0, 40):
+                u, v = a[k, y:y + 40, x:x + 40], b[k, y:y + 40, x:x + 40]
+                assert bool((v != 0).any()) == bool((u != 0).any())
+                assert float((u - v).norm()) <= 2e-6 * float(v.norm())
+    assert float(b[0].abs().max()) > 0 and not b[:, 40:, :40].any()
