@@ -219,8 +219,11 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 // D2[Ti], Im E = D1[Ti] + D2[Tr]); the box form makes D1[Tr] and D2[Ti] only.
 // The pixel-integrated form in split BF16 is not folded either: its images are a
 // small window of dim pixels around a peak, where the order of the additions
-// shows.  It runs like TF32, with the reduction in three passes (hi hi, hi lo,
-// lo hi) over the same [hi | lo] rows.
+// shows.  Nor is the field form about another centre than the pupil's middle: the
+// halves do not match there, so less is saved and the error grows (256^2 disc,
+// centre at 0.4 of it: 2.1e-6 unfolded, 2.9e-6 folded; in the middle 2.1 and 1.3e-6).
+// Both run like TF32, with the reduction in three passes (hi hi, hi lo, lo hi) over
+// the same [hi | lo] rows.
 // FORM 2 (FP32 on the CUDA cores) is folded in the field form; its
 // pixel-integrated form makes the folded products over all signed distances, with
 // the operand in both parts (Te_r = C A, To_i = -S A).  Accumulation is FP32 in TMEM (or
@@ -233,15 +236,15 @@ extern "C" int gl_gemm_bf16_tc(const void* d_a, const void* d_b, float* d_c, int
 //   W'  [lam][C | S][k]                                  TF32: [Wr | Wi]
 //   A'  [ee | oe | eo | oo][row d]   FP32 box: A twice   (nhr rows each; TF32: A)
 //   T'  [lam][k / 128][Te_r | Te_i | To_i | -To_r][k % 128]   FP32 box: [Te_r | To_i]
-//                                                        TF32, split BF16 box: [Tr | Ti]
+//                                              TF32, unfolded split BF16: [Tr | Ti]
 // ===========================================================================
 namespace gl {
 namespace {
 
 constexpr int kMdftThreads = 192;     // warps 0-3 epilogue, warp 4 TMA, warp 5 MMA
 constexpr int kTf32 = 1;              // not folded
-constexpr int kSplitBox = 3;          // split BF16, pixel-integrated: not folded, three passes (a plan's form 0 with box)
-__host__ __device__ constexpr bool is_bf16(int form) { return form == 0 || form == kSplitBox; }
+constexpr int kSplitWhole = 3;        // split BF16, not folded, three passes (a plan's form 0 with box, or off the middle)
+__host__ __device__ constexpr bool is_bf16(int form) { return form == 0 || form == kSplitWhole; }
 __host__ __device__ constexpr bool is_folded(int form) { return form == 0 || form == 2; }
 constexpr int kOpTile = 128 * 128;    // bytes of one 128-row x 128-byte operand tile
 
@@ -424,9 +427,9 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                         uint8_t* st = smem + s * Sh::kStageBytes;
                         if (rank == 0) tc::mbar_expect_tx(&full[s], CL * Sh::kStageBytes);
                         // three passes: hi hi, hi lo, lo hi
-                        const int pass = FORM == kSplitBox ? kb / (args.nkb / 3) : 0;
-                        const int x = (FORM == kSplitBox ? kb % (args.nkb / 3) : kb) * kbe + (pass == 2 ? args.nh : 0);
-                        const int xB = FORM == kSplitBox ? (kb % (args.nkb / 3)) * kbe + (pass == 1 ? args.nh : 0) : x;
+                        const int pass = FORM == kSplitWhole ? kb / (args.nkb / 3) : 0;
+                        const int x = (FORM == kSplitWhole ? kb % (args.nkb / 3) : kb) * kbe + (pass == 2 ? args.nh : 0);
+                        const int xB = FORM == kSplitWhole ? (kb % (args.nkb / 3)) * kbe + (pass == 1 ? args.nh : 0) : x;
                         const uint32_t bar = CL == 2 ? tc::leader_u32(&full[s]) : 0u;
                         auto load = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1) {
                             if (CL == 2) tc::tma_load_2d_pair(dst, map, c0, c1, bar);
@@ -499,7 +502,7 @@ __global__ void __launch_bounds__(kMdftThreads, 1) mdft_kernel(const __grid_cons
                     // folded: the lo set; TF32 box: the Ti block
                     const uint64_t b1 = tc::sw128_desc(tc::smem_u32(st + 2 * kOpTile + (Sh::kFold ? Sh::kBBytes : Sh::kRows * 128)));
                     // the last step of a reduction may be partly past nh (whatever lies there is not multiplied)
-                    const int left = FORM == kSplitBox ? 4 : (args.nh - kb * kbe) / kStep;
+                    const int left = FORM == kSplitWhole ? 4 : (args.nh - kb * kbe) / kStep;
                     #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
                     {
@@ -1171,10 +1174,14 @@ __global__ void __launch_bounds__(256) mdft_simt_sum(const MdftArgs args, int nl
 constexpr double kMaxCentre = 12288.0;   // pattern centre range (pixels)
 
 // The kernels' form of a plan.
-static int mdft_kernel_form(int form, int box) { return form == 0 && box ? kSplitBox : form; }
+static int mdft_kernel_form(int form, int box, int n, float red_center)
+{
+    return form == 0 && (box || red_center != 0.5f * (float)(n - 1)) ? kSplitWhole : form;
+}
 
 struct MdftPlan {
     int n = 0, Kx = 0, Ky = 0, n_lambda = 0, form = 0, Kp = 0, elem = 2;
+    int kform = 0;          // the kernels' form
     // folded reduction: nf distances |j - cj|, padded to nh (16); nhr rows per
     // part of A' (128); h2 = 2 cj
     // (not folded: nf = nh = n); d0 = smallest distance (not folded: -cj)
@@ -1227,7 +1234,7 @@ static cudaError_t mdft_build_matrices(MdftPlan* p, cudaStream_t st)
     for (const DftRows& r : R)
     {
         const int grid = (p->n_lambda * r.K + (int)block.y - 1) / (int)block.y;
-        if (p->form == 0 && p->box) mdft_dft_kernel<kSplitBox><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
+        if (p->kform == kSplitWhole) mdft_dft_kernel<kSplitWhole><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
         else if (p->form == 0) mdft_dft_kernel<0><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
         else if (p->form == kTf32) mdft_dft_kernel<kTf32><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
         else mdft_dft_kernel<2><<<grid, block, 0, st>>>(r, p->n_lambda, p->nh, p->d0);
@@ -1402,7 +1409,8 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     p->cx = center_x; p->cy = center_y;
     p->box = box; p->cj = red_center;
     p->h2 = (int)(2.0f * red_center);
-    const bool folded = is_folded(mdft_kernel_form(form, box)), distances = folded && !box;
+    p->kform = mdft_kernel_form(form, box, n, red_center);
+    const bool folded = is_folded(p->kform), distances = folded && !box;
     p->nf = !distances ? n : (int)std::floor(std::max((double)red_center, (double)(n - 1) - (double)red_center)) + 1;
     p->d0 = !distances ? -red_center : ((p->h2 & 1) ? 0.5f : 0.0f);
     p->nh = (p->nf + 15) / 16 * 16;
@@ -1455,7 +1463,8 @@ extern "C" int gl_mdft_plan_create3(int n, int Kx, int Ky, int n_lambda, const d
     }
     chk(cudaStreamSynchronize(st));
     // shared-memory opt-in once here, so execute enqueues kernels only (graph capture)
-    if (form == 0) chk(box ? mdft_prepare_all<kSplitBox, true>(&p->pairs) : mdft_prepare_all<0, false>(&p->pairs));
+    if (p->kform == kSplitWhole) chk(box ? mdft_prepare_all<kSplitWhole, true>(&p->pairs) : mdft_prepare_all<kSplitWhole, false>(&p->pairs));
+    else if (form == 0) chk(mdft_prepare_all<0, false>(&p->pairs));
     else if (form == 1) chk(box ? mdft_prepare_all<1, true>(&p->pairs) : mdft_prepare_all<1, false>(&p->pairs));
     const CUtensorMapDataType dt = form == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const uint32_t bc = form == 0 ? 64 : 32;
@@ -1514,11 +1523,11 @@ static void mdft_units(const MdftPlan* p, MdftArgs& a1, MdftArgs& a2)
     a1.KA = p->Kx;
     a1.NB = a1.NBm = a1.NBt = p->Kx / 128;
     a1.nh = p->nh; a1.nhr = p->nhr;
-    a1.nkb = (p->nh + kbe - 1) / kbe * (p->form == 0 && p->box ? 3 : 1);
+    a1.nkb = (p->nh + kbe - 1) / kbe * (p->kform == kSplitWhole ? 3 : 1);
     a1.NI = p->nhr / 128;
     a1.lam_base = p->lam0;
     // step 1: (lambda, k block, pupil-row block, C / S); step 2: (lambda, output tile)
-    a1.n_units = nl * a1.NB * a1.NI * (is_folded(mdft_kernel_form(p->form, p->box)) ? 2 : 1);
+    a1.n_units = nl * a1.NB * a1.NI * (is_folded(p->kform) ? 2 : 1);
     a2 = a1;
     a2.KA = p->Ky; a2.NBm = p->Ky / 128;
     a2.NBt = p->Kx / p->tile_n;
@@ -1533,7 +1542,7 @@ extern "C" int gl_mdft_plan_pairs(const gl_mdft_plan* plan, int* step1, int* ste
     MdftArgs a1{}, a2;
     mdft_units(p, a1, a2);
     const int gmax = p->ctas > 0 ? p->ctas : p->sms;
-    const bool field = p->form == 0 && !p->box;
+    const bool field = p->kform == 0;
     *step1 = field ? mdft_pairs<0, 1, 128, false>(a1, gmax, p->pairs) : 0;
     *step2 = field && p->tile_n == 128 ? mdft_pairs<0, 2, 128, false>(a2, gmax, p->pairs) : 0;
     return GL_OK;
@@ -1569,7 +1578,7 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
         kernel<<<fold, 128, 0, st>>>(d_pupil, p->mask, p->n, p->nh, p->nhr, p->nf, p->h2, p->box, d_out_r, d_out_g,
                                      d_out_b, zero, p->err);
     };
-    if (p->form == 0 && p->box) run_fold(mdft_fold_kernel<kSplitBox>);
+    if (p->kform == kSplitWhole) run_fold(mdft_fold_kernel<kSplitWhole>);
     else if (p->form == 0) run_fold(mdft_fold_kernel<0>);
     else if (p->form == kTf32) run_fold(mdft_fold_kernel<kTf32>);
     else run_fold(mdft_fold_kernel<2>);
@@ -1592,7 +1601,8 @@ extern "C" int gl_mdft_plan_execute3(gl_mdft_plan* plan, const float* d_pupil, f
     }
     else if (p->form == 0)
     {
-        GL_CUDA_TRY(p->box ? (mdft_gemms<kSplitBox, true>(p, a, a2, gmax, st)) : (mdft_gemms<0, false>(p, a, a2, gmax, st)));
+        if (p->kform == 0) GL_CUDA_TRY((mdft_gemms<0, false>(p, a, a2, gmax, st)));
+        else GL_CUDA_TRY(p->box ? (mdft_gemms<kSplitWhole, true>(p, a, a2, gmax, st)) : (mdft_gemms<kSplitWhole, false>(p, a, a2, gmax, st)));
     }
     else
     {

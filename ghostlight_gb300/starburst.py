@@ -147,10 +147,11 @@ class MdftPlan:
         planes of single wavelengths (at most 64 MB or two)."""
         import torch
         tf32 = self.form == "tf32"
-        folded = not tf32 and not (self.form == "split_bf16" and self.box)
+        middle = self._red_center == 0.5 * (self.n - 1)
+        folded = not tf32 and not (self.form == "split_bf16" and (self.box or not middle))
         nh = self.n if self.box or not folded else (int(max(self._red_center, self.n - 1 - self._red_center)) + 16) // 16 * 16
         row = nh * 4                        # two bf16 terms or one float
-        parts, nl = (2 if self.box or tf32 else 4), self.n_lambda
+        parts, nl = (2 if self.box or not folded else 4), self.n_lambda
         px, sms = self.Kx * self.Ky, torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
         planes = 0
         if self.form == "fp32" and nl > 1 and px // 4096 < 4 * sms:
